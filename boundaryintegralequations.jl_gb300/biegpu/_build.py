@@ -23,6 +23,7 @@ SOURCES = [
     "bie_setup.cpp",
     "bie_assemble.cu",
     "bie_assemble_mixed.cu",
+    "bie_assemble_fix64.cu",
     "bie_matvec.cu",
     "bie_solver.cu",
     "bie_nearfield.cpp",

@@ -140,6 +140,45 @@ assemble_fp64_kernel(const double *__restrict__ rec, int stride, int nidx_off,
     if ((threadIdx.x & 31) == 0 && nqpe) atomicAdd(qpe_count, nqpe);
 }
 
+// C at points off the surface: the sums cancel there to the quadrature error, so
+// C keeps K1's FP64 operations and order while F and G come from the
+// fixed-point kernel.  A quarter of K1's FP64 instructions per point.
+template <int NP>
+__global__ void __launch_bounds__(kThreads)
+field_c_fp64_kernel(const double *__restrict__ rec, int stride, int64_t E, int S,
+                    const __grid_constant__ RuleInfo ri, const double *__restrict__ tgt, int64_t M,
+                    double *__restrict__ Cpart, int chunk) {
+    extern __shared__ __align__(16) double s_rec[];
+    __shared__ RuleInfo s_ri;
+    if (threadIdx.x == 0) s_ri = ri;
+    const int s = blockIdx.y;
+    const int64_t e0 = (int64_t)s * E / S, e1 = (int64_t)(s + 1) * E / S;
+    const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    const bool active = i < M;
+    double tx = 0, ty = 0, tz = 0;
+    if (active) {
+        tx = tgt[3 * i + 0];
+        ty = tgt[3 * i + 1];
+        tz = tgt[3 * i + 2];
+    }
+    double cacc = 0.0;
+    for (int64_t cb = e0; cb < e1; cb += chunk) {
+        const int n = (int)min((int64_t)chunk, e1 - cb);
+        __syncthreads();
+        const double2 *src = reinterpret_cast<const double2 *>(rec + cb * stride);
+        double2 *dst = reinterpret_cast<double2 *>(s_rec);
+        for (int t = threadIdx.x; t < n * stride / 2; t += kThreads) dst[t] = src[t];
+        __syncthreads();
+        if (!active) continue;
+        for (int el = 0; el < n; ++el) {
+            const double *r = s_rec + (size_t)el * stride;
+            const int c = dev::nearest_node<NP>(r, tx, ty, tz);
+            cacc += dev::element_c_fp64(r + s_ri.off[c], s_ri.Q[c], tx, ty, tz);
+        }
+    }
+    if (active) Cpart[(int64_t)s * M + i] = cacc;
+}
+
 template <int NP, bool CPLX>
 void launch_np(Ctx &c, const AssembleArgs &a, int S, int level, size_t smem, int chunk,
                double *Cpart) {
@@ -192,9 +231,6 @@ int wave_slice_level(const Ctx &c, int64_t M, int threads_per_row_tile) {
         ++level;
     return std::max(level, choose_slice_level(c, M, threads_per_row_tile));
 }
-
-void launch_reduce_c(Ctx &c, const double *Cpart, int S, const double *Cextra, int64_t M,
-                     double *C);
 
 LaunchShape resolve_shape(Ctx &c, int kernel, int64_t M, const LaunchShape &base, const ShapeAxes &ax,
                           const std::function<void(const LaunchShape &)> &run, const std::function<void()> &reset) {
@@ -253,6 +289,7 @@ LaunchShape resolve_shape(Ctx &c, int kernel, int64_t M, const LaunchShape &base
 }
 
 void launch_assemble_fp64(Ctx &c, const AssembleArgs &a) {
+    if (launch_assemble_fix64(c, a, false)) return;
     const RecordLayout &L = c.lay;
     const int64_t N = c.n_sources;
     if (a.flags & BIE_F) BIE_CUDA(cudaMemsetAsync(a.F, 0, (size_t)a.M * N * 16, c.stream));
@@ -282,6 +319,27 @@ void launch_assemble_fp64(Ctx &c, const AssembleArgs &a) {
         else launch_np<6, false>(c, a, S, level, smem, chunk, Cpart);
     }
     if (a.flags & BIE_C) launch_reduce_c(c, Cpart, S, nullptr, a.M, a.C);
+}
+
+void launch_field_c_fp64(Ctx &c, const double *targets, int64_t M, double *C) {
+    const RecordLayout &L = c.lay;
+    const int level = choose_slice_level(c, M, kThreads), S = 1 << level;
+    const size_t rec_bytes = (size_t)L.stride * sizeof(double);
+    const int chunk = (int)std::max<size_t>(1, std::min<size_t>(64, (40u << 10) / rec_bytes));
+    const size_t smem = (size_t)chunk * rec_bytes;
+    double *Cpart = static_cast<double *>(c.scratch(kScratchCpart, (size_t)S * M * sizeof(double)));
+    RuleInfo ri{};
+    for (int r = 0; r < L.R; ++r) {
+        ri.Q[r] = L.Q[r];
+        ri.off[r] = L.rule_off[r];
+    }
+    auto kern = L.NP == 1 ? field_c_fp64_kernel<1> : (L.NP == 3 ? field_c_fp64_kernel<3> : field_c_fp64_kernel<6>);
+    BIE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<dim3((unsigned)((M + kThreads - 1) / kThreads), (unsigned)S), kThreads, smem, c.stream>>>(
+        c.d_records, L.stride, c.n_elements, S, ri, targets, M, Cpart, chunk);
+    BIE_CUDA(cudaGetLastError());
+    ++c.kernel_launches;
+    launch_reduce_c(c, Cpart, S, nullptr, M, C);
 }
 
 // ---------------------------------------------------------------------------

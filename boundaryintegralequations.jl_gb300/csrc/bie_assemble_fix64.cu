@@ -1,0 +1,907 @@
+// K10: FP64-grade dense collocation assembly on the integer pipes
+// (BIE_PREC_FP64 and BIE_PREC_DF64, real and complex k).
+//
+// Same result as K1 (assemble_parallel!, src/3d/assembly_collocation.jl:
+// 270-479).  K1 is bound by the FP64 pipe, which GB300 runs at 1/64 of its
+// FP32 rate (86 % busy); here the regular pairs are evaluated in 64-bit fixed
+// point (bie_fix64.cuh), whose error is at or below FP64 rounding, and only the
+// near pairs and nearest-node near-ties stay in FP64 (a list and a correction
+// kernel, as in the mixed assembly).
+//
+// Measured (GB300, complete step): pulsating sphere, 10242 nodes, 3-node
+// physics 133.3 -> 20.8 ms; 362 nodes, 16-point rules 0.79 -> 0.23 ms;
+// BIE_PREC_DF64 (before: double-float kernel) 5762 nodes, 6-node physics
+// 4.98 -> 3.24 ms, 11562 nodes 17.3 -> 11.3 ms.  Errors against a 64-bit
+// evaluation are unchanged (pulsating sphere F 7.6e-14, dominated by near
+// pairs).
+// What bounds it now: instruction issue.  One point costs about 268
+// instructions (71 IMAD.WIDE) = 528 issue cycles per warp, a node's output
+// about 130 (48 IMAD.WIDE); measured per warp instruction IMAD.WIDE takes 2.45
+// cycles, shifts and logic 2.1, adds 1.2 and they do not overlap.  Not kept:
+// staging records in shared memory (same time as reading them through L1, plus
+// barriers), 3 or 5 resident blocks (+5 %), all four points of a group at once
+// (+15 %), integer-to-double conversion without the FP64 pipe (+3 %).
+//
+//   * one thread per target row, element slices in grid.y, records read through
+//     L1 (every lane of a warp reads the same words);
+//   * per pair the FP32 nearest-node choice with a near-tie margin, D = c - t as
+//     integers, and the scales of the pair;
+//   * per point the kernel values as integers, two points side by side; the
+//     values of four points go through shared memory to the sums with the
+//     physics basis (three IMAD.WIDE each: high x high and the two cross
+//     products), so that neither loop holds the other's registers (128 against
+//     214, 4 blocks per SM instead of 2: 4.4 -> 3.3 ms at 5762 nodes);
+//   * each (row, node) entry is a running 64-bit integer sum in units fixed by
+//     the row-node distance and the node's element weights, so sums are exact
+//     and independent of their order: the first contribution in the node's
+//     slice stores, later ones add, the last one converts to complex128; nodes
+//     shared between slices take 64-bit integer atomics and a widening pass.
+#include "bie_internal.h"
+#include "bie_device.cuh"
+#include "bie_df64.cuh"
+#include "bie_fix64.cuh"
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+namespace bie {
+
+namespace {
+
+using dev::RuleInfo;
+using fix64::i64;
+using fix64::Limb;
+using fix64::u64;
+constexpr int kThreads = 128;
+constexpr int kPointWords = 16;
+
+// header words of a record
+constexpr int kHdrNear2 = 0, kHdrRho = 1, kHdrEj = 2, kHdrEo = 3, kHdrCen = 4, kHdrNodes = 12;
+
+struct Fp64View {
+    const double *rec;
+    int stride;
+    int nidx_off;
+    const double *phi;   // global, R x qmax x NP
+    int qmax;
+    RuleInfo ri;
+};
+
+// Scales of a launch (host values)
+struct FxScale {
+    double x0[3];        // origin of the scaled coordinates
+    double inv;          // 2^-S
+    double len;          // 2^S
+    int S;
+    int pe;              // basis values are stored times 2^-pe
+    int extra;           // entry units times 2^extra (large node valences)
+    float rho_max;       // largest rho of the mesh
+};
+
+// k as mantissas and exponents (see fix64::pair_wavenumber, pair_damping)
+struct FxWave {
+    i64 km, ka;          // Re k / 2 pi, Re k
+    i64 kd, kai;         // Im k log2(e), Im k
+    int kx, kb, kdx;
+    float kl;            // Im k log2(e)
+    float rho_max;       // largest rho of the mesh
+};
+
+// integer nearest to (hi + lo) 2^n, |hi| 2^n below 2^62
+__device__ __forceinline__ i64 fx_round(double hi, double lo, int n) {
+    return __double2ll_rn(ldexp(hi, n)) + __double2ll_rn(ldexp(lo, n));
+}
+
+template <bool CPLX_K>
+__device__ __forceinline__ FxWave fx_wave(double kre, double kim, const FxScale &sc) {
+    // 1 / 2 pi and log2(e) as hi + lo
+    constexpr double kHi = 0x1.45f306dc9c883p-3, kLo = -0x1.6b01ec5417056p-57;
+    constexpr double lHi = 0x1.71547652b82fep+0, lLo = 0x1.777d0ffda0d24p-56;
+    const double k = kre * sc.len, ki = kim * sc.len;
+    FxWave w{0, 0, 0, 0, -1000, -1000, -1000, 0.f, sc.rho_max};
+    if (k != 0.0) {
+        const double hi = k * kHi, lo = fma(k, kHi, -hi) + k * kLo;
+        (void)frexp(hi, &w.kx);
+        (void)frexp(k, &w.kb);
+        w.km = fx_round(hi, lo, 62 - w.kx);
+    }
+    if (CPLX_K) {
+        int kb2 = -1000;
+        if (ki != 0.0) {
+            const double hi = ki * lHi, lo = fma(ki, lHi, -hi) + ki * lLo;
+            (void)frexp(hi, &w.kdx);
+            (void)frexp(ki, &kb2);
+            w.kd = fx_round(hi, lo, 62 - w.kdx);
+            w.kl = (float)hi;
+        }
+        w.kb = max(w.kb, kb2) + 1;   // |Re k|, |Im k| below 2^(kb - 1)
+        if (ki != 0.0) w.kai = fx_round(ki, 0.0, 62 - w.kb);
+    }
+    if (k != 0.0) w.ka = fx_round(k, 0.0, 62 - w.kb);
+    return w;
+}
+
+// Units of an entry (row, node): floor(log2 |t - x|) of the FP32 coordinates and,
+// for complex k, the base of its damping; evaluated the same way wherever they
+// are needed
+struct FxEntry {
+    int fl, base;
+};
+template <bool CPLX_K>
+__device__ __forceinline__ FxEntry fx_entry(float tx, float ty, float tz, float x, float y, float z, const FxWave &w) {
+    const float dx = __fsub_rn(x, tx), dy = __fsub_rn(y, ty), dz = __fsub_rn(z, tz);
+    const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+    return FxEntry{(fix64::float_exp(d2) - 1) >> 1, CPLX_K ? fix64::entry_base(w.kl, __fsqrt_rn(d2), w.rho_max) : 0};
+}
+
+// integer sum in units of 2^e as a double
+template <bool CPLX_K>
+__device__ __forceinline__ double fx_double(i64 v, int e) {
+    const double d = (double)v;
+    if (CPLX_K) return ldexp(d, e);   // strong damping may leave the normal range
+    // real k: exponents stay far inside it (coordinates within 2^+-300)
+    return v == 0 ? 0.0 : __hiloint2double(__double2hiint(d) + (e << 20), __double2loint(d));
+}
+template <bool CPLX_K>
+__device__ __forceinline__ longlong2 fx_complex(longlong2 v, int e) {
+    return make_longlong2(__double_as_longlong(fx_double<CPLX_K>(v.x, e)),
+                          __double_as_longlong(fx_double<CPLX_K>(v.y, e)));
+}
+
+struct FxTarget {
+    i64 x, y, z;         // fixed coordinates, 2^(59 - st) units
+    float fx, fy, fz;    // scaled FP32 coordinates
+    int st;
+    bool bad;            // not representable: every pair in FP64
+};
+
+__device__ __forceinline__ FxTarget fx_target(double tx, double ty, double tz, const FxScale &sc) {
+    FxTarget T;
+    const double x = (tx - sc.x0[0]) * sc.inv, y = (ty - sc.x0[1]) * sc.inv, z = (tz - sc.x0[2]) * sc.inv;
+    const double m = fmax(fmax(fabs(x), fabs(y)), fabs(z));
+    T.bad = !(m < 0x1p40) || isnan(x) || isnan(y) || isnan(z);
+    T.fx = (float)x;
+    T.fy = (float)y;
+    T.fz = (float)z;
+    int ex = 0;
+    if (!T.bad) (void)frexp(m, &ex);
+    T.st = ex > 0 ? ex : 0;
+    const double s = __hiloint2double((1023 + fix64::kCoordBits - T.st) << 20, 0);
+    T.x = T.bad ? 0 : __double2ll_rn(x * s);
+    T.y = T.bad ? 0 : __double2ll_rn(y * s);
+    T.z = T.bad ? 0 : __double2ll_rn(z * s);
+    return T;
+}
+
+struct FxPairInfo {
+    int c;               // rule: nearest physics node
+    int e;               // pair exponent
+    bool deferred;       // FP64
+    float r0, rho;       // |D|, largest offset in the element
+};
+
+// Set-up of one pair: nearest node in FP32 with near / near-tie detection (the
+// criteria of the mixed assembly), the pair's exponent, and D.
+template <int NP, bool CPLX_K>
+__device__ __forceinline__ FxPairInfo fx_pair(const float *r, const FxTarget &T, const FxWave &w, i64 &Dx, i64 &Dy,
+                                              i64 &Dz) {
+    FxPairInfo I;
+    const i64 *cen = reinterpret_cast<const i64 *>(r + kHdrCen);
+    Dx = (cen[0] >> T.st) - T.x;
+    Dy = (cen[1] >> T.st) - T.y;
+    Dz = (cen[2] >> T.st) - T.z;
+    // FP32 D from the bits above 2^(29 - 59): 22 significant bits at the smallest
+    // regular distance
+    const float u = __int_as_float((127 - fix64::kCoordBits + 29 + T.st) << 23);
+    const float fx = (float)(int)(Dx >> 29) * u, fy = (float)(int)(Dy >> 29) * u, fz = (float)(int)(Dz >> 29) * u;
+    float d2[NP];
+#pragma unroll
+    for (int a = 0; a < NP; ++a) {
+        const float ax = fx + r[kHdrNodes + 3 * a], ay = fy + r[kHdrNodes + 3 * a + 1],
+                    az = fz + r[kHdrNodes + 3 * a + 2];
+        d2[a] = ax * ax + ay * ay + az * az;
+    }
+    int c = 0;
+    float b = d2[0];
+#pragma unroll
+    for (int a = 1; a < NP; ++a)
+        if (d2[a] < b) {
+            b = d2[a];
+            c = a;
+        }
+    const float lim = b * (1.0f + 1e-5f);
+    bool tie = false;
+#pragma unroll
+    for (int a = 0; a < NP; ++a) tie |= (a != c) && (d2[a] <= lim);
+    const float r0f2 = fx * fx + fy * fy + fz * fz;
+    const float near2 = r[kHdrNear2], rho = r[kHdrRho];
+    const float r0 = sqrtf(r0f2);
+    const float rmin = r0 * (1.0f - 1e-6f) - rho;
+    I.c = c;
+    I.r0 = r0;
+    I.rho = rho;
+    I.e = fix64::float_exp(rmin);
+    I.deferred = T.bad || tie || r0f2 < near2 || 4.0f * b < near2 || !(r0 >= fix64::kRhoFactor * rho) ||
+                 I.e < T.st + fix64::kMinExp || w.kx + I.e > fix64::kMaxTurnExp;
+    if (CPLX_K)
+        I.deferred |= !(fabsf(w.kl) * rho <= fix64::kMaxDampSpread) || w.kdx + I.e > fix64::kMaxDampExp;
+    return I;
+}
+
+
+// Basis tables: per rule, group of four points and node the four values' limbs
+// (two int4), zero beyond the rule's points.
+constexpr int kGroup = 4;
+constexpr int kInterleave = 2;   // points evaluated side by side
+inline int phi_groups(int qmax) { return (qmax + kGroup - 1) / kGroup; }
+
+template <int NP, bool CPLX_K>
+__global__ void __launch_bounds__(kThreads, 4)
+assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int S,
+                      const int4 *__restrict__ phi, int nphi, int ngroups, const __grid_constant__ RuleInfo ri,
+                      const int4 *__restrict__ trig, const int2 *__restrict__ damp, const double *__restrict__ tgt, int64_t M,
+                      double kre, double kim, int flags, longlong2 *__restrict__ F, longlong2 *__restrict__ G,
+                      const uint32_t *__restrict__ kflags, double *__restrict__ Cpart,
+                      int2 *__restrict__ defer, unsigned int *__restrict__ defer_count, unsigned int defer_cap,
+                      int *__restrict__ over, const __grid_constant__ FxScale sc,
+                      unsigned long long *__restrict__ qpe_count, const double *__restrict__ kdev) {
+    if (kdev) {   // wavenumber read from device memory (recorded sweeps)
+        kre = kdev[0];
+        kim = kdev[1];
+    }
+    extern __shared__ __align__(16) float smemf[];
+    int4 *s_trig = reinterpret_cast<int4 *>(smemf);                              // 1024 entries
+    int4 *s_val = s_trig + fix64::kTrigEntries;                                  // 2 kGroup x kThreads
+    int4 *s_phi = s_val + 2 * kGroup * kThreads;                                      // nphi entries
+    int2 *s_damp = reinterpret_cast<int2 *>(s_phi + nphi);                       // 256 entries (complex k)
+    __shared__ RuleInfo s_ri;
+    __shared__ FxWave s_wave;
+
+    const int s = blockIdx.y;
+    const int64_t e0 = (int64_t)s * E / S;
+    const int64_t e1 = (int64_t)(s + 1) * E / S;
+    const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    const bool active = i < M;
+    const bool doF = flags & BIE_F, doG = flags & BIE_G, doC = flags & BIE_C;
+
+    double tx = 0, ty = 0, tz = 0;
+    if (active) {
+        tx = tgt[3 * i + 0];
+        ty = tgt[3 * i + 1];
+        tz = tgt[3 * i + 2];
+    }
+    const FxTarget T = fx_target(tx, ty, tz, sc);
+    for (int t = threadIdx.x; t < fix64::kTrigEntries; t += kThreads) s_trig[t] = trig[t];
+    for (int t = threadIdx.x; t < nphi; t += kThreads) s_phi[t] = phi[t];
+    if (threadIdx.x == 0) {
+        s_ri = ri;
+        s_wave = fx_wave<CPLX_K>(kre, kim, sc);
+    }
+    if (CPLX_K)
+        for (int t = threadIdx.x; t < fix64::kDampEntries; t += kThreads) s_damp[t] = damp[t];
+    auto table = [s_trig](int j, Limb &c, Limb &sn) {
+        const int4 v = s_trig[j];
+        c = Limb{v.x, v.y};
+        sn = Limb{v.z, v.w};
+    };
+    auto damp_table = [s_damp](int j) {
+        const int2 v = s_damp[j];
+        return Limb{v.x, v.y};
+    };
+
+    double cacc = 0.0;
+    int over_at = 0x7fffffff;
+    unsigned long long nqpe = 0;
+    __syncthreads();
+    const FxWave wv = s_wave;
+    const unsigned row_bytes = (unsigned)(M * 16);   // of a column
+    char *Fi = reinterpret_cast<char *>(F + i), *Gi = reinterpret_cast<char *>(G + i);
+    if (active) {
+        for (int64_t pe = e0; pe < e1; ++pe) {
+            const float *r = rec + pe * stride;
+            const int *ir = reinterpret_cast<const int *>(r);
+            fix64::Pair P;
+            const FxPairInfo I = fx_pair<NP, CPLX_K>(r, T, wv, P.Dx, P.Dy, P.Dz);
+            const uint32_t fw = __ldg(kflags + pe);
+            const int ej = ir[kHdrEj];
+            const float *abs_nodes = r + kHdrNodes + 3 * NP;
+            const int *node_ej = ir + kHdrNodes + 6 * NP;
+            const int *nid = node_ej + NP;
+            const int e = I.e;
+            int Q = 0;
+            if (I.deferred) {   // no points here, but the pair may open or close entries
+                const unsigned int slot = atomicAdd(defer_count, 1u);
+                if (slot < defer_cap) defer[slot] = make_int2((int)i, (int)pe);
+                else over_at = min(over_at, (int)pe);   // rescanned by the correction kernel
+            } else {
+                const int qs = T.st + 2 - e;   // 2^(59 - st) units -> Q61 of 2^e
+                P.Dx = (i64)((u64)P.Dx << qs);
+                P.Dy = (i64)((u64)P.Dy << qs);
+                P.Dz = (i64)((u64)P.Dz << qs);
+                P.osh = min(63, 1 + e - ir[kHdrEo]);
+                Q = s_ri.Q[I.c];
+                nqpe += Q;
+            }
+            fix64::pair_wavenumber(P, wv.km, wv.kx, wv.ka, wv.kb, e);
+            if (CPLX_K)
+                fix64::pair_damping(P, wv.kd, wv.kdx, wv.kai, wv.kb, e,
+                                    fix64::pair_base(wv.kl, I.r0, I.rho));
+            const int4 *g4 = reinterpret_cast<const int4 *>(r + s_ri.off[I.c]);
+            const int4 *phc = s_phi + (size_t)I.c * ngroups * NP * 2;
+            i64 ce = 0;
+            int q0 = 0;
+            do {
+                // kernel values of up to four points, through shared memory so that
+                // one copy of the point sequence serves all of them
+                for (int q = 0; q < kGroup; q += kInterleave) {
+                    int4 vf[kInterleave], vg[kInterleave];
+#pragma unroll
+                    for (int j = 0; j < kInterleave; ++j) vf[j] = vg[j] = make_int4(0, 0, 0, 0);
+                    if (q0 + q < Q) {
+#pragma unroll
+                        for (int j = 0; j < kInterleave; ++j) {
+                            const int qj = min(q0 + q + j, Q - 1);
+                            const int4 *w = g4 + 4 * qj;
+                            const int4 A = __ldg(w), B = __ldg(w + 1), C4 = __ldg(w + 2);
+                            const int2 D2 = __ldg(reinterpret_cast<const int2 *>(w + 3));
+                            const bool on = q0 + q + j < Q;   // beyond the rule: weight zero
+                            fix64::PointData g;
+                            g.ox = fix64::make64(A.y, (unsigned)A.x);
+                            g.oy = fix64::make64(A.w, (unsigned)A.z);
+                            g.oz = fix64::make64(B.y, (unsigned)B.x);
+                            g.nx = Limb{B.z, B.w};
+                            g.ny = Limb{C4.x, C4.y};
+                            g.nz = Limb{C4.z, C4.w};
+                            g.jw = Limb{on ? D2.x : 0, on ? D2.y : 0};
+                            const fix64::Point v = fix64::point<CPLX_K>(g, P, table, damp_table);
+                            ce += v.tq;
+                            const Limb a0 = fix64::split(v.Fr), a1 = fix64::split(v.Fi), a2 = fix64::split(v.Gr),
+                                       a3 = fix64::split(v.Gi);
+                            vf[j] = make_int4(a0.h, a0.l, a1.h, a1.l);
+                            vg[j] = make_int4(a2.h, a2.l, a3.h, a3.l);
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < kInterleave; ++j) {
+                        s_val[(2 * (q + j)) * kThreads + threadIdx.x] = vf[j];
+                        s_val[(2 * (q + j) + 1) * kThreads + threadIdx.x] = vg[j];
+                    }
+                }
+                if (doF || doG) {
+                    int4 vf[kGroup], vg[kGroup];
+#pragma unroll
+                    for (int q = 0; q < kGroup; ++q) {
+                        vf[q] = s_val[(2 * q) * kThreads + threadIdx.x];
+                        vg[q] = s_val[(2 * q + 1) * kThreads + threadIdx.x];
+                    }
+                    const bool open = q0 == 0, close = q0 + kGroup >= Q;
+#pragma unroll 1
+                    for (int a = 0; a < NP; ++a) {
+                        const u64 off = (u64)(unsigned)nid[a] * (u64)row_bytes;
+                        longlong2 *pF = reinterpret_cast<longlong2 *>(Fi + off);
+                        longlong2 *pG = reinterpret_cast<longlong2 *>(Gi + off);
+                        const bool shared = (fw >> (16 + a)) & 1u;
+                        const bool first = open && ((fw >> a) & 1u), last = close && ((fw >> (8 + a)) & 1u);
+                        // the entry's sums so far, read ahead of the products
+                        longlong2 vF = make_longlong2(0, 0), vG = vF;
+                        if (!shared && !first) {
+                            if (doF) vF = __ldcg(pF);
+                            if (doG) vG = __ldcg(pG);
+                        }
+                        int p[2 * kGroup];
+                        *reinterpret_cast<int4 *>(p) = phc[2 * a];
+                        *reinterpret_cast<int4 *>(p + 4) = phc[2 * a + 1];
+                        i64 fr = 0, fi = 0, gr = 0, gi = 0;       // high sums, Q55
+                        const i64 half = (i64)1 << 31;
+                        i64 frl = half, fil = half, grl = half, gil = half;   // cross sums
+#pragma unroll
+                        for (int q = 0; q < kGroup; ++q) {
+                            const Limb ph{p[2 * q], p[2 * q + 1]};
+                            const Limb a0{vf[q].x, vf[q].y}, a1{vf[q].z, vf[q].w}, a2{vg[q].x, vg[q].y},
+                                a3{vg[q].z, vg[q].w};
+                            fr = fix64::high(fr, a0, ph);
+                            fi = fix64::high(fi, a1, ph);
+                            gr = fix64::high(gr, a2, ph);
+                            gi = fix64::high(gi, a3, ph);
+                            frl = fix64::cross(frl, a0, ph);
+                            fil = fix64::cross(fil, a1, ph);
+                            grl = fix64::cross(grl, a2, ph);
+                            gil = fix64::cross(gil, a3, ph);
+                        }
+                        const FxEntry en = fx_entry<CPLX_K>(T.fx, T.fy, T.fz, abs_nodes[3 * a], abs_nodes[3 * a + 1],
+                                                            abs_nodes[3 * a + 2], wv);
+                        const int fl = en.fl, de = e - (fl - 1);
+                        const int dj = node_ej[a] - ej + sc.extra + (CPLX_K ? P.base - en.base : 0);
+                        const int sg = max(0, dj + de);
+                        const int sf = max(0, dj + 2 * de + fix64::amplitude_exp(wv.kb, fl - 1) - P.fe);
+                        vF.x += fix64::shift_right(fix64::fold(fr, frl), sf);
+                        vF.y += fix64::shift_right(fix64::fold(fi, fil), sf);
+                        vG.x += fix64::shift_right(fix64::fold(gr, grl), sg);
+                        vG.y += fix64::shift_right(fix64::fold(gi, gil), sg);
+                        if (shared) {
+                            unsigned long long *uF = reinterpret_cast<unsigned long long *>(pF);
+                            unsigned long long *uG = reinterpret_cast<unsigned long long *>(pG);
+                            if (doF) {
+                                atomicAdd(uF, (unsigned long long)vF.x);
+                                atomicAdd(uF + 1, (unsigned long long)vF.y);
+                            }
+                            if (doG) {
+                                atomicAdd(uG, (unsigned long long)vG.x);
+                                atomicAdd(uG + 1, (unsigned long long)vG.y);
+                            }
+                            continue;
+                        }
+                        if (last) {   // final complex128 entries
+                            const int adj = sc.pe + sc.extra - en.base;
+                            vF = fx_complex<CPLX_K>(vF, fix64::entry_exp_f(node_ej[a], fl, wv.kb) + adj);
+                            vG = fx_complex<CPLX_K>(vG, fix64::entry_exp_g(node_ej[a], fl) + adj + sc.S);
+                        }
+                        if (doF) *pF = vF;
+                        if (doG) *pG = vG;
+                    }
+                }
+                q0 += kGroup;
+                phc += NP * 2;
+            } while (q0 < Q);
+            if (doC && Q > 0) cacc -= fx_double<false>(ce, ej - 2 * e - 57);
+        }
+    }
+    if (active) {
+        if (doC) Cpart[(int64_t)s * M + i] = cacc;
+        over[(int64_t)s * M + i] = over_at;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) nqpe += __shfl_down_sync(0xffffffffu, nqpe, o);
+    if ((threadIdx.x & 31) == 0 && nqpe) atomicAdd(qpe_count, nqpe);
+}
+
+// Columns of the nodes shared between slices (and of untouched nodes): zeroed
+// before the assembly, converted after it.
+__global__ void fx_zero_kernel(const int32_t *__restrict__ fnode, int64_t nfix, int64_t M, longlong2 *__restrict__ F,
+                               longlong2 *__restrict__ G) {
+    const int64_t total = nfix * M;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t n = t / M;
+        const size_t off = (size_t)fnode[n] * (size_t)M + (size_t)(t - n * M);
+        if (F) F[off] = make_longlong2(0, 0);
+        if (G) G[off] = make_longlong2(0, 0);
+    }
+}
+
+template <bool CPLX_K>
+__global__ void fx_widen_kernel(const int32_t *__restrict__ fnode, int64_t nfix, const float4 *__restrict__ nodes,
+                                const double *__restrict__ tgt, int64_t M, double kre, double kim,
+                                const __grid_constant__ FxScale sc, longlong2 *__restrict__ F,
+                                longlong2 *__restrict__ G, const double *__restrict__ kdev) {
+    if (kdev) {
+        kre = kdev[0];
+        kim = kdev[1];
+    }
+    __shared__ FxWave s_wave;
+    if (threadIdx.x == 0) s_wave = fx_wave<CPLX_K>(kre, kim, sc);
+    __syncthreads();
+    const FxWave wv = s_wave;
+    const int64_t total = nfix * M;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t n = t / M, i = t - n * M;
+        const int32_t nd = fnode[n];
+        const size_t off = (size_t)nd * (size_t)M + (size_t)i;
+        const float4 x = nodes[nd];
+        const float fx = (float)((tgt[3 * i] - sc.x0[0]) * sc.inv), fy = (float)((tgt[3 * i + 1] - sc.x0[1]) * sc.inv),
+                    fz = (float)((tgt[3 * i + 2] - sc.x0[2]) * sc.inv);
+        const FxEntry en = fx_entry<CPLX_K>(fx, fy, fz, x.x, x.y, x.z, wv);
+        const int ej = __float_as_int(x.w), adj = sc.pe + sc.extra - en.base;
+        if (F) F[off] = fx_complex<CPLX_K>(F[off], fix64::entry_exp_f(ej, en.fl, wv.kb) + adj);
+        if (G) G[off] = fx_complex<CPLX_K>(G[off], fix64::entry_exp_g(ej, en.fl) + adj + sc.S);
+    }
+}
+
+template <int NP, bool CPLX_K, class Trig>
+__device__ __forceinline__ int fx_correct_pair(const Fp64View &v, int64_t i, int64_t p, const double *tgt, int64_t M,
+                                               double kre, double kim, bool doF, bool doG, bool doC, double2 *F,
+                                               double2 *G, double *Cnear) {
+    const double *r = v.rec + (size_t)p * v.stride;
+    const double tx = tgt[3 * i], ty = tgt[3 * i + 1], tz = tgt[3 * i + 2];
+    const int c = dev::nearest_node<NP>(r, tx, ty, tz);
+    double fr[NP], fi[NP], gr[NP], gi[NP];
+    const double ce = dev::element_fp64<NP, CPLX_K, Trig>(r + v.ri.off[c], v.ri.Q[c],
+                                                          v.phi + (size_t)c * v.qmax * NP, tx, ty, tz, kre, kim, fr,
+                                                          fi, gr, gi);
+    const int32_t *nid = reinterpret_cast<const int32_t *>(r + v.nidx_off);
+#pragma unroll
+    for (int a = 0; a < NP; ++a) {
+        const size_t off = (size_t)nid[a] * (size_t)M + (size_t)i;
+        if (doF) {
+            atomicAdd(&F[off].x, fr[a]);
+            atomicAdd(&F[off].y, fi[a]);
+        }
+        if (doG) {
+            atomicAdd(&G[off].x, gr[a]);
+            atomicAdd(&G[off].y, gi[a]);
+        }
+    }
+    if (doC) atomicAdd(&Cnear[i], ce);
+    return v.ri.Q[c];
+}
+
+// FP64 integration of the deferred pairs, added to the finished entries.  Where
+// the list was too short, every (row, slice) whose pairs did not all fit is
+// gone through again from its first pair that found no place.
+template <int NP, bool CPLX_K, class Trig>
+__global__ void __launch_bounds__(128)
+fx_correct_kernel(const int2 *__restrict__ defer, const unsigned int *__restrict__ defer_count,
+                  unsigned int defer_cap, const __grid_constant__ Fp64View v, const double *__restrict__ tgt,
+                  int64_t M, double kre, double kim, int flags, double2 *__restrict__ F, double2 *__restrict__ G,
+                  double *__restrict__ Cnear, const int *__restrict__ over, const float *__restrict__ rec, int stride,
+                  int64_t E, int S, const __grid_constant__ FxScale sc, unsigned long long *__restrict__ qpe_count,
+                  const double *__restrict__ kdev) {
+    if (kdev) {
+        kre = kdev[0];
+        kim = kdev[1];
+    }
+    const unsigned int total = *defer_count, n = min(total, defer_cap);
+    const bool doF = flags & BIE_F, doG = flags & BIE_G, doC = flags & BIE_C;
+    unsigned long long nqpe = 0;
+    for (unsigned int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
+        nqpe += fx_correct_pair<NP, CPLX_K, Trig>(v, defer[j].x, defer[j].y, tgt, M, kre, kim, doF, doG, doC, F, G,
+                                                  Cnear);
+    if (total > defer_cap) {
+        const FxWave wv = fx_wave<CPLX_K>(kre, kim, sc);
+        for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < M * S;
+             j += (int64_t)gridDim.x * blockDim.x) {
+            if (over[j] == 0x7fffffff) continue;
+            const int64_t s = j / M, i = j - s * M;
+            const FxTarget T = fx_target(tgt[3 * i], tgt[3 * i + 1], tgt[3 * i + 2], sc);
+            for (int64_t p = over[j]; p < (s + 1) * E / S; ++p) {
+                i64 dx, dy, dz;
+                if (!fx_pair<NP, CPLX_K>(rec + p * stride, T, wv, dx, dy, dz).deferred) continue;
+                nqpe += fx_correct_pair<NP, CPLX_K, Trig>(v, i, p, tgt, M, kre, kim, doF, doG, doC, F, G, Cnear);
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) nqpe += __shfl_down_sync(0xffffffffu, nqpe, o);
+    if ((threadIdx.x & 31) == 0 && nqpe) atomicAdd(qpe_count, nqpe);
+}
+
+inline unsigned stream_grid(const Ctx &c, int64_t total) {
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, 16LL * c.num_sms));
+}
+
+struct FxBuffers {
+    double *Cpart, *Cnear;
+    int2 *defer;
+    unsigned int *dcount, dcap;
+    int *over;
+};
+
+template <int NP, bool CPLX>
+void launch_np(Ctx &c, const AssembleArgs &a, bool df_trig, const LaunchShape &sh, size_t smem, const FxBuffers &b) {
+    const RecordLayout &L = c.lay;
+    const Fix64Layout &X = c.xlay;
+    RuleInfo ri{}, ri64{};
+    for (int r = 0; r < L.R; ++r) {
+        ri.Q[r] = ri64.Q[r] = L.Q[r];
+        ri.off[r] = X.rule_off[r];
+        ri64.off[r] = L.rule_off[r];
+    }
+    FxScale sc{};
+    for (int k = 0; k < 3; ++k) sc.x0[k] = c.fx_origin[k];
+    sc.S = c.fx_exp;
+    sc.inv = std::ldexp(1.0, -c.fx_exp);
+    sc.len = std::ldexp(1.0, c.fx_exp);
+    sc.pe = c.fx_phi_exp;
+    sc.extra = c.fx_extra;
+    sc.rho_max = c.fx_rho_max;
+    const Fp64View v{c.d_records, L.stride, L.nidx_off, c.d_phi, L.qmax, ri64};
+    const int level = sh.level, S = 1 << level;
+    const int64_t E = c.n_elements, nfix = c.k2_nfix[level];
+    longlong2 *F = (a.flags & BIE_F) ? reinterpret_cast<longlong2 *>(a.F) : nullptr;
+    longlong2 *G = (a.flags & BIE_G) ? reinterpret_cast<longlong2 *>(a.G) : nullptr;
+    const int32_t *fnode = c.d_k2_fix + c.k2_fix_off[level];
+    if (nfix > 0 && (F || G)) {
+        fx_zero_kernel<<<stream_grid(c, nfix * a.M), 256, 0, c.stream>>>(fnode, nfix, a.M, F, G);
+        BIE_CUDA(cudaGetLastError());
+        ++c.kernel_launches;
+    }
+    auto kern = assemble_fix64_kernel<NP, CPLX>;
+    BIE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const dim3 grid((unsigned)((a.M + kThreads - 1) / kThreads), (unsigned)S);
+    cudaEvent_t t0 = c.timer_begin();
+    kern<<<grid, kThreads, smem, c.stream>>>(
+        c.d_xrecords, X.stride, E, S, reinterpret_cast<const int4 *>(c.d_xphi), L.R * phi_groups(L.qmax) * NP * 2,
+        phi_groups(L.qmax), ri,
+        reinterpret_cast<const int4 *>(c.d_xtrig),
+        reinterpret_cast<const int2 *>(c.d_xtrig + 4 * fix64::kTrigEntries), a.targets, a.M, a.k_re, a.k_im, a.flags, F, G,
+        c.d_k2_flags + (size_t)level * E, b.Cpart, b.defer, b.dcount, b.dcap, b.over, sc, c.d_qpe, a.k_dev);
+    BIE_CUDA(cudaGetLastError());
+    c.timer_end(t0);
+    ++c.kernel_launches;
+    if (nfix > 0 && (F || G)) {
+        fx_widen_kernel<CPLX><<<stream_grid(c, nfix * a.M), 256, 0, c.stream>>>(
+            fnode, nfix, reinterpret_cast<const float4 *>(c.d_xnodes), a.targets, a.M, a.k_re, a.k_im, sc, F, G,
+            a.k_dev);
+        BIE_CUDA(cudaGetLastError());
+        ++c.kernel_launches;
+    }
+    auto corr = df_trig ? fx_correct_kernel<NP, CPLX, df64::TrigDf> : fx_correct_kernel<NP, CPLX, dev::TrigFp64>;
+    corr<<<(unsigned)(4 * c.num_sms), 128, 0, c.stream>>>(
+        b.defer, b.dcount, b.dcap, v, a.targets, a.M, a.k_re, a.k_im, a.flags, reinterpret_cast<double2 *>(F),
+        reinterpret_cast<double2 *>(G), b.Cnear, b.over, c.d_xrecords, X.stride, E, S, sc, c.d_qpe, a.k_dev);
+    BIE_CUDA(cudaGetLastError());
+    ++c.kernel_launches;
+}
+
+}  // namespace
+
+// Records of the fixed-point kernels from the FP64 ones (E x lay.stride).
+void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
+    const RecordLayout &L = c.lay;
+    Fix64Layout &X = c.xlay;
+    X = Fix64Layout{};
+    const int NP = L.NP;
+    const int64_t E = c.n_elements, N = c.n_sources;
+    c.fx_ok = false;
+    // scaled coordinates (x - x0) 2^-S with the largest in [1/2, 1).  x0 is zero
+    // unless the mesh lies far from the origin for its size, where the
+    // subtraction is exact for targets near the mesh.
+    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+    auto span = [&](const std::vector<double> &v) {
+        for (size_t j = 0; j < v.size(); j += 3)
+            for (int k = 0; k < 3; ++k) {
+                lo[k] = std::min(lo[k], v[j + k]);
+                hi[k] = std::max(hi[k], v[j + k]);
+            }
+    };
+    span(c.coords);
+    span(c.sources);
+    double ext = 0.0, top = 0.0;
+    for (int k = 0; k < 3; ++k) ext = std::max(ext, hi[k] - lo[k]);
+    for (int k = 0; k < 3; ++k) {
+        const double mid = 0.5 * (lo[k] + hi[k]);
+        c.fx_origin[k] = std::fabs(mid) > 4.0 * ext ? mid : 0.0;
+        top = std::max(top, std::max(std::fabs(lo[k] - c.fx_origin[k]), std::fabs(hi[k] - c.fx_origin[k])));
+    }
+    if (!(top > 0x1p-300 && top < 0x1p300)) return;   // such meshes stay with the FP64 kernel
+    (void)std::frexp(top, &c.fx_exp);
+    const double inv = std::ldexp(1.0, -c.fx_exp);
+    // integer nearest to (hi + lo) 2^n
+    auto fixed = [](double h, double l, double scale) { return (long long)std::llrint(h * scale) + (long long)std::llrint(l * scale); };
+    auto put_limbs = [](int32_t *w, long long v) {
+        const fix64::Limb s = fix64::split(v);
+        w[0] = s.h;
+        w[1] = s.l;
+    };
+
+    int off = kHdrNodes + 6 * NP + 2 * NP;
+    off = (off + 3) & ~3;
+    for (int r = 0; r < L.R; ++r) {
+        X.rule_off[r] = off;
+        off += kPointWords * L.Q[r];
+    }
+    X.stride = off;
+
+    // basis scale: |phi| 2^-pe <= 1
+    double pmax = 0.0;
+    for (double p : c.phi) pmax = std::max(pmax, std::fabs(p));
+    c.fx_phi_exp = 0;
+    while (std::ldexp(pmax, -c.fx_phi_exp) > 1.0) ++c.fx_phi_exp;
+    const int ng = phi_groups(L.qmax);
+    std::vector<int32_t> phi((size_t)L.R * ng * NP * 2 * kGroup, 0);
+    for (int r = 0; r < L.R; ++r)
+        for (int q = 0; q < L.Q[r]; ++q)
+            for (int a = 0; a < NP; ++a)
+                put_limbs(&phi[((((size_t)r * ng + q / kGroup) * NP + a) * kGroup + q % kGroup) * 2],
+                          (long long)std::llrint(std::ldexp(c.phi[((size_t)r * L.qmax + q) * NP + a], 61 - c.fx_phi_exp)));
+
+    std::vector<int32_t> rec((size_t)E * X.stride, 0);
+    std::vector<int> ej(E);
+    std::vector<int> node_ej(N, INT32_MIN);
+    std::vector<double> reach((size_t)E * NP);   // max over rules of sum |jw| |phi| in 2^(ej + pe)
+    for (int64_t p = 0; p < E; ++p) {
+        const int64_t e = c.order[p];
+        const double *R0 = &rec64[(size_t)p * L.stride];
+        int32_t *w = &rec[(size_t)p * X.stride];
+        float *wf = reinterpret_cast<float *>(w);
+        double cen[3] = {0, 0, 0}, hmax = 0;
+        for (int a = 0; a < 3; ++a)
+            for (int k = 0; k < 3; ++k) cen[k] += c.coords[3 * (int64_t)c.topo[c.NS * e + a] + k] / 3.0;
+        for (int a = 0; a < 3; ++a) {
+            const double *A = &c.coords[3 * (int64_t)c.topo[c.NS * e + a]];
+            const double *B = &c.coords[3 * (int64_t)c.topo[c.NS * e + (a + 1) % 3]];
+            const double d[3] = {(A[0] - B[0]) * inv, (A[1] - B[1]) * inv, (A[2] - B[2]) * inv};
+            hmax = std::max(hmax, std::sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]));
+        }
+        long long fc[3];
+        for (int k = 0; k < 3; ++k) {
+            const double s = cen[k] - c.fx_origin[k], bb = s - cen[k];
+            const double err = (cen[k] - (s - bb)) + (-c.fx_origin[k] - bb);   // two-sum
+            fc[k] = fixed(s * inv, err * inv, 0x1p59);
+            std::memcpy(w + kHdrCen + 2 * k, &fc[k], 8);
+        }
+        wf[kHdrNear2] = (float)(hmax * hmax);
+        double rho2 = 0.0, jmax = 0.0, omax = 0.0, jsum = 0.0;
+        for (int a = 0; a < NP; ++a) {
+            double d2 = 0.0;
+            for (int k = 0; k < 3; ++k) {
+                const double x = R0[3 * a + k], d = (x - cen[k]) * inv;
+                d2 += d * d;
+                wf[kHdrNodes + 3 * a + k] = (float)d;
+                wf[kHdrNodes + 3 * NP + 3 * a + k] = (float)((x - c.fx_origin[k]) * inv);
+            }
+            rho2 = std::max(rho2, d2);
+        }
+        for (int r = 0; r < L.R; ++r) {
+            const int Q = L.Q[r];
+            const double *g = R0 + L.rule_off[r];
+            double js = 0.0;
+            for (int q = 0; q < Q; ++q) {
+                double d2 = 0.0;
+                for (int k = 0; k < 3; ++k) {
+                    const double d = (g[k * Q + q] - cen[k]) * inv;
+                    d2 += d * d;
+                    omax = std::max(omax, std::fabs(d));
+                }
+                rho2 = std::max(rho2, d2);
+                const double j = std::fabs(g[6 * Q + q]) * (inv * inv) * dev::kInv4Pi;
+                jmax = std::max(jmax, j);
+                js += j;
+            }
+            jsum = std::max(jsum, js);
+        }
+        wf[kHdrRho] = (float)(std::sqrt(rho2) * (1.0 + 1e-6));
+        c.fx_rho_max = std::max(c.fx_rho_max, wf[kHdrRho]);
+        int eo = 0, je = 0;
+        (void)std::frexp(omax > 0 ? omax * (1.0 + 1e-9) : 0x1p-60, &eo);
+        (void)std::frexp(jmax > 0 ? jmax * 1.01 : 0x1p-200, &je);
+        while (std::ldexp(jsum, -je) > 8.0) ++je;   // sums over a rule: |sum t| < 8 * 4 2^57
+        if (je < -900) return;
+        ej[p] = je;
+        w[kHdrEj] = je;
+        w[kHdrEo] = eo;
+        const double so = std::ldexp(1.0, 62 - eo), sj = std::ldexp(inv * inv * dev::kInv4Pi, 63 - je);
+        for (int r = 0; r < L.R; ++r) {
+            const int Q = L.Q[r];
+            const double *g = R0 + L.rule_off[r];
+            for (int q = 0; q < Q; ++q) {
+                int32_t *P = w + X.rule_off[r] + kPointWords * q;
+                for (int k = 0; k < 3; ++k) {
+                    const double x = g[k * Q + q], s = x - cen[k], bb = s - x;
+                    const double err = (x - (s - bb)) + (-cen[k] - bb);
+                    const long long o = fixed(s * inv, err * inv, so);
+                    std::memcpy(P + 2 * k, &o, 8);
+                    put_limbs(P + 6 + 2 * k, (long long)std::llrint(g[(3 + k) * Q + q] * 0x1p61));
+                }
+                put_limbs(P + 12, (long long)std::llrint(g[6 * Q + q] * sj));
+            }
+        }
+        for (int a = 0; a < NP; ++a) {
+            const int32_t nd = c.ptopo[NP * e + a];
+            w[kHdrNodes + 7 * NP + a] = nd;
+            node_ej[nd] = std::max(node_ej[nd], je);
+            double best = 0.0;
+            for (int r = 0; r < L.R; ++r) {
+                double s = 0.0;
+                for (int q = 0; q < L.Q[r]; ++q)
+                    s += std::fabs(R0[L.rule_off[r] + 6 * L.Q[r] + q] * c.phi[((size_t)r * L.qmax + q) * NP + a]);
+                best = std::max(best, s);
+            }
+            reach[(size_t)p * NP + a] = std::ldexp(best * inv * inv * dev::kInv4Pi, -je - c.fx_phi_exp);
+        }
+    }
+    // entries hold |sum| <= 4 sqrt(2) 2^55 sum of the reaches: below 2^62
+    std::vector<double> node_reach(N, 0.0);
+    for (int64_t p = 0; p < E; ++p)
+        for (int a = 0; a < NP; ++a) {
+            const int32_t nd = c.ptopo[NP * c.order[p] + a];
+            rec[(size_t)p * X.stride + kHdrNodes + 6 * NP + a] = node_ej[nd];
+            node_reach[nd] += std::ldexp(reach[(size_t)p * NP + a], ej[p] - node_ej[nd]);
+        }
+    double worst = 0.0;
+    for (double v : node_reach) worst = std::max(worst, v);
+    c.fx_extra = 0;
+    while (std::ldexp(worst * 5.7, -c.fx_extra) > 127.0) ++c.fx_extra;
+
+    std::vector<float> nodes((size_t)4 * N);
+    for (int64_t j = 0; j < N; ++j) {
+        for (int k = 0; k < 3; ++k) nodes[4 * j + k] = (float)((c.sources[3 * j + k] - c.fx_origin[k]) * inv);
+        const int32_t v = node_ej[j] == INT32_MIN ? 0 : node_ej[j];
+        std::memcpy(&nodes[4 * j + 3], &v, 4);
+    }
+    // e^{2 pi i j / 1024} and 2^(-j / 256) as Q62 limbs
+    std::vector<int32_t> trig((size_t)4 * fix64::kTrigEntries + 2 * fix64::kDampEntries);
+    {
+        const int n = fix64::kTrigEntries;
+        const long double pi = 3.141592653589793238462643383279502884L;
+        auto q62 = [](long double x) { return (long long)std::llrint(std::ldexp(x, 62)); };
+        for (int j = 0; j < n; ++j) {
+            const long double th = 2.0L * pi * j / n;
+            put_limbs(&trig[4 * j], q62(std::cos(th)));
+            put_limbs(&trig[4 * j + 2], q62(std::sin(th)));
+        }
+        for (int j = 0; j < fix64::kDampEntries; ++j)   // 2^(-j / 256)
+            put_limbs(&trig[4 * n + 2 * j], q62(std::exp2(-(long double)j / fix64::kDampEntries)));
+    }
+    BIE_CUDA(cudaMalloc(&c.d_xrecords, rec.size() * 4));
+    BIE_CUDA(cudaMalloc(&c.d_xphi, phi.size() * 4));
+    BIE_CUDA(cudaMalloc(&c.d_xnodes, nodes.size() * 4));
+    BIE_CUDA(cudaMalloc(&c.d_xtrig, trig.size() * 4));
+    BIE_CUDA(cudaMemcpy(c.d_xrecords, rec.data(), rec.size() * 4, cudaMemcpyHostToDevice));
+    BIE_CUDA(cudaMemcpy(c.d_xphi, phi.data(), phi.size() * 4, cudaMemcpyHostToDevice));
+    BIE_CUDA(cudaMemcpy(c.d_xnodes, nodes.data(), nodes.size() * 4, cudaMemcpyHostToDevice));
+    BIE_CUDA(cudaMemcpy(c.d_xtrig, trig.data(), trig.size() * 4, cudaMemcpyHostToDevice));
+    c.fx_ok = true;
+}
+
+bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df_trig) {
+    AssembleArgs a = args;
+    if (!c.fx_ok || a.taylor_m >= 0 || a.g_weight) return false;
+    if (a.k_dev && !(a.k_abs_max > 0)) return false;   // no bound on |k|
+    const bool cplx = a.k_im != 0.0;
+    // wavenumbers whose phase or damping over the mesh or an element leaves the
+    // fixed-point ranges for many pairs stay with the FP64 kernel
+    const double bound = a.k_dev ? a.k_abs_max : 0.0, len = std::ldexp(1.0, c.fx_exp);
+    const double kr = std::max(std::fabs(a.k_re), bound) * len, ki = cplx ? std::max(std::fabs(a.k_im), bound) * len : 0.0;
+    if (!(kr < 500.0) || !(ki < 100.0) || !(ki * c.fx_rho_max * 1.45 < fix64::kMaxDampSpread)) return false;
+    // C at points off the surface cancels to the quadrature error, where any other
+    // rounding would show: it keeps the FP64 (double-float) operations
+    const bool nodes = a.targets >= c.d_sources && a.targets + 3 * a.M <= c.d_sources + 3 * c.n_sources;
+    if ((a.flags & BIE_C) && !nodes) {
+        AssembleArgs f = a;
+        f.flags = BIE_C;
+        f.F = f.G = nullptr;
+        if (!(df_trig && launch_assemble_k9(c, f))) launch_field_c_fp64(c, a.targets, a.M, a.C);
+        a.flags &= ~BIE_C;
+    }
+    if (!(a.flags & (BIE_F | BIE_G | BIE_C))) return true;
+    const RecordLayout &L = c.lay;
+    FxBuffers b{};
+    b.dcap = (unsigned int)std::min<int64_t>(a.M * 64 + 4096, (int64_t)1 << 30);
+    const size_t dbytes = (size_t)b.dcap * sizeof(int2);
+    char *dbuf = static_cast<char *>(c.scratch(kScratchDefer, dbytes + 256 + (size_t)a.M * 8));
+    b.defer = reinterpret_cast<int2 *>(dbuf);
+    b.dcount = reinterpret_cast<unsigned int *>(dbuf + dbytes);
+    b.Cnear = reinterpret_cast<double *>(dbuf + dbytes + 256);
+    auto reset = [&] { BIE_CUDA(cudaMemsetAsync(dbuf + dbytes, 0, 256 + (size_t)a.M * 8, c.stream)); };
+    reset();
+
+    auto run = [&](const LaunchShape &sh) {
+        const int S = 1 << sh.level;
+        // phase table, point values of the block's threads, basis tables
+        const size_t smem = ((size_t)fix64::kTrigEntries + 2 * kGroup * kThreads +
+                             (size_t)L.R * phi_groups(L.qmax) * L.NP * 2) * 16 +
+                            (cplx ? fix64::kDampEntries * 8 : 0);
+        // per (slice, row): the C partial sums, then the overflow marks
+        const size_t cp = (size_t)S * a.M * sizeof(double);
+        char *part = static_cast<char *>(c.scratch(kScratchCpart, cp + (size_t)S * a.M * sizeof(int)));
+        b.Cpart = reinterpret_cast<double *>(part);
+        b.over = reinterpret_cast<int *>(part + cp);
+        if (L.NP == 1) {
+            if (cplx) launch_np<1, true>(c, a, df_trig, sh, smem, b);
+            else launch_np<1, false>(c, a, df_trig, sh, smem, b);
+        } else if (L.NP == 3) {
+            if (cplx) launch_np<3, true>(c, a, df_trig, sh, smem, b);
+            else launch_np<3, false>(c, a, df_trig, sh, smem, b);
+        } else {
+            if (cplx) launch_np<6, true>(c, a, df_trig, sh, smem, b);
+            else launch_np<6, false>(c, a, df_trig, sh, smem, b);
+        }
+        if (a.flags & BIE_C) launch_reduce_c(c, b.Cpart, S, b.Cnear, a.M, a.C);
+    };
+    // The finest slicing with at least four elements per slice: blocks differ in
+    // cost (near pairs leave points out, midpoint rules add some), so many small
+    // ones even out.  Step at 128 / 64 / 32 slices: pulsating sphere 20.8 / 21.2 /
+    // 22.0 ms, rigid sphere P2 11.3 / 11.4 / 12.0, 5762 nodes P2 3.20 / 3.30 / 3.55,
+    // 362 nodes with 16-point rules 0.22 / 0.29 / 0.40.
+    int level = 0;
+    while (level + 1 < kMaxLevels && (c.n_elements >> (level + 1)) >= 4) ++level;
+    const LaunchShape base{level, 1, kThreads};   // (records are read through L1: no chunks)
+    ShapeAxes ax;
+    for (int l = level - 1; l <= level + 1; ++l)
+        if (l >= 0 && l < kMaxLevels && (int64_t(1) << l) <= c.n_elements) ax.levels.push_back(l);
+    run(df_trig ? resolve_shape(c, kShapeK9, a.M, base, ax, run, reset) : base);
+    return true;
+}
+
+}  // namespace bie

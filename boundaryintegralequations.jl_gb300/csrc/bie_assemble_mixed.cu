@@ -753,7 +753,9 @@ __device__ __noinline__ double k9_pair_inplace(const Fp64View &v64, int64_t p, d
     return ce;
 }
 
-template <int NP, bool CPLX_K>
+// FG = false: C alone (points off the surface, whose C keeps this arithmetic
+// while F and G come from the fixed-point kernel).
+template <int NP, bool CPLX_K, bool FG>
 __global__ void __launch_bounds__(kThreads, BIE_K9_MIN_BLOCKS)
 assemble_df64_kernel(const float *__restrict__ rec, int stride, int nidx_off, int64_t E, int S,
                      const uint32_t *__restrict__ smask, const float2 *__restrict__ phi, int nphi, int qmax,
@@ -778,7 +780,7 @@ assemble_df64_kernel(const float *__restrict__ rec, int stride, int nidx_off, in
     const int64_t e1 = (int64_t)(s + 1) * E / S;
     const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const bool active = i < M;
-    const bool doF = flags & BIE_F, doG = flags & BIE_G, doC = flags & BIE_C;
+    const bool doF = FG && (flags & BIE_F), doG = FG && (flags & BIE_G), doC = flags & BIE_C;
 
     double tx = 0, ty = 0, tz = 0;
     if (active) {
@@ -844,6 +846,7 @@ assemble_df64_kernel(const float *__restrict__ rec, int stride, int nidx_off, in
                 qpe_df64<CPLX_K>(g4[4 * q], g4[4 * q + 1], g4[4 * q + 2], g4[4 * q + 3], P, r0, E0r, E0i, K, Ki,
                                  deg, Fr, Fi, Gr, Gi, tq);
                 dd::acc_add(ce, tq);
+                if (!FG) continue;
                 const float2 *pq = phc + q * NP;
 #pragma unroll
                 for (int a = 0; a < NP; ++a) {
@@ -857,6 +860,7 @@ assemble_df64_kernel(const float *__restrict__ rec, int stride, int nidx_off, in
             }
             // C = -sum t
             dd::acc_add(cacc, dd::neg(dev::fast_two_sum(ce.hi, ce.lo)));
+            if (!FG) continue;
             if (gweight && doG) {   // element factor on the single layer, in double-float
                 const double2 w = gweight[cb + el];
                 const df wr = dd::to_df(w.x), wi = dd::to_df(w.y);
@@ -907,7 +911,7 @@ void launch_df64_np(Ctx &c, const AssembleArgs &a, int S, int level, size_t smem
         ri64.off[r] = L.rule_off[r];
     }
     Fp64View v{c.d_records, L.stride, L.nidx_off, c.d_phi, L.qmax, ri64};
-    auto kern = assemble_df64_kernel<NP, CPLX>;
+    auto kern = (a.flags & (BIE_F | BIE_G)) ? assemble_df64_kernel<NP, CPLX, true> : assemble_df64_kernel<NP, CPLX, false>;
     BIE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grid((unsigned)((a.M + kThreads - 1) / kThreads), (unsigned)S);
     cudaEvent_t t0 = c.timer_begin();
@@ -1006,6 +1010,10 @@ void build_df64_records(Ctx &c, const std::vector<double> &rec64, const std::vec
 }
 
 bool launch_assemble_df64(Ctx &c, const AssembleArgs &a) {
+    return launch_assemble_fix64(c, a, true) || launch_assemble_k9(c, a);
+}
+
+bool launch_assemble_k9(Ctx &c, const AssembleArgs &a) {
     const RecordLayout &L = c.lay;
     if (a.taylor_m >= 0 || (a.k_dev && !(a.k_abs_max > 0))) return false;
     df64::DfDegrees deg{};
@@ -1055,7 +1063,8 @@ bool launch_assemble_df64(Ctx &c, const AssembleArgs &a) {
     for (int l = base.level - 1; l <= base.level + 1; ++l)
         if (l >= 0 && l < kMaxLevels && (int64_t(1) << l) <= c.n_elements) ax.levels.push_back(l);
     ax.chunks = {std::max(1, chunk0 / 2), chunk0, std::min(64, 2 * chunk0)};
-    LaunchShape sh = resolve_shape(c, kShapeK9, a.M, base, ax, run, reset);
+    // C alone: the default shape (its slices are part of the sum's order)
+    LaunchShape sh = (a.flags & (BIE_F | BIE_G)) ? resolve_shape(c, kShapeK9, a.M, base, ax, run, reset) : base;
     sh.tpb = kThreads;   // the double-float kernel has one block size
     run(sh);
     return true;

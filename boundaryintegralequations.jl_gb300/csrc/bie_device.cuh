@@ -142,6 +142,24 @@ __device__ __forceinline__ double element_fp64(const double *g, int Q, const dou
     return ce;
 }
 
+// The C contribution of element_fp64 alone, with its operations in its order, so
+// that a C computed apart from F and G keeps every rounding.
+__device__ __forceinline__ double element_c_fp64(const double *g, int Q, double tx, double ty, double tz) {
+    double ce = 0.0;
+    for (int q = 0; q < Q; ++q) {
+        const double dx = g[q] - tx;
+        const double dy = g[Q + q] - ty;
+        const double dz = g[2 * Q + q] - tz;
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        const double rinv = rsqrt(r2);
+        const double jw = g[6 * Q + q];
+        const double dn = g[3 * Q + q] * dx + g[4 * Q + q] * dy + g[5 * Q + q] * dz;
+        const double tq = __dmul_rn(dn * (rinv * rinv * rinv) * kInv4Pi, jw);
+        ce = __dsub_rn(ce, tq);
+    }
+    return ce;
+}
+
 // ---------------------------------------------------------------------------
 // Double-float (unevaluated sum of two floats) arithmetic, ~48-bit significand.
 // Error-free transformations after Knuth (TwoSum) and Dekker (FastTwoSum,

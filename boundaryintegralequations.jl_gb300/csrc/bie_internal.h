@@ -135,6 +135,16 @@ struct Df64Layout {
     int stride = 0;
 };
 
+// Fixed-point element records (K10; 32-bit words): near radius^2, rho, ej, eo,
+// centroid (three 64-bit integers), two unused words, then per physics node
+// its FP32 offset from the centroid, its FP32 coordinates, the entry weight
+// exponent and the node index; per rule and point 16 words (see
+// fix64::PointData).  Lengths are scaled by 2^-fx_exp about fx_origin.
+struct Fix64Layout {
+    int rule_off[kMaxRules] = {};
+    int stride = 0;
+};
+
 // Near-field (sparse) structure for one (depth, offset, n_gauss): CSR pattern of
 // connected nodes per collocation node, the (row, element, CSR slots) pairs and
 // the rule tables (adaptive singular rules per element node + the coarse
@@ -229,6 +239,17 @@ struct Ctx {
     float *d_dphi = nullptr;             // R x qmax x NP (hi, lo) pairs
     double df_rho_max = 0.0;             // largest |x_q - c_e| over the mesh
     float *d_phase_tab = nullptr;        // e^{i j h} as (cos hi, lo, sin hi, lo), double-float kernels
+    Fix64Layout xlay;
+    bool fx_ok = false;                  // the fixed-point records exist (coordinates in range)
+    double fx_origin[3] = {};            // origin and scale 2^-fx_exp of their coordinates
+    int fx_exp = 0;
+    float fx_rho_max = 0.f;              // largest point or node offset from a centroid (scaled)
+    int fx_phi_exp = 0;                  // basis values are stored times 2^-fx_phi_exp
+    int fx_extra = 0;                    // entry units times 2^fx_extra (nodes with many elements)
+    float *d_xrecords = nullptr;         // E x xlay.stride words, element order
+    int32_t *d_xphi = nullptr;           // R x qmax x (4, 8, 12) limb words
+    float *d_xnodes = nullptr;           // N x (x, y, z, entry weight exponent)
+    int32_t *d_xtrig = nullptr;          // 1024 x (cos, sin) limbs, 256 x 2^(-j/256) limbs
     double *d_coords = nullptr;          // 3 x Nc geometry nodes (near-field kernels)
     int32_t *d_topo = nullptr;           // NS x E, 0-based
     std::vector<std::unique_ptr<NearField>> nearfields;
@@ -321,6 +342,9 @@ LaunchShape resolve_shape(Ctx &c, int kernel, int64_t M, const LaunchShape &base
                           const std::function<void(const LaunchShape &)> &run, const std::function<void()> &reset);
 void launch_reduce_c(Ctx &c, const double *Cpart, int S, const double *Cextra, int64_t M,
                      double *C);
+
+// C alone at targets off the surface, with K1's operations in K1's order
+void launch_field_c_fp64(Ctx &c, const double *targets, int64_t M, double *C);
 
 // Matrix-free products yF = F x, yG = G v (bie_matvec.cu); all pointers device
 struct MatvecArgs {
@@ -556,10 +580,20 @@ void launch_nearfield(Ctx &c, const NearField &nf, double k_re, double k_im, int
 // host: builds d_mrecords / d_mphi from the FP64 records (E x lay.stride) and uploads them
 void build_mixed_records(Ctx &c, const std::vector<double> &rec64);
 void launch_assemble_mixed(Ctx &c, const AssembleArgs &a);
-// Double-float assembly (K9); false when the arguments need the FP64 kernel
-// (element factors, k-derivatives, device-resident k, or phase rotations
-// beyond the Taylor tables)
+// FP64-grade assembly (BIE_PREC_DF64): the fixed-point kernel (K10) or, where its
+// ranges end, the double-float kernel (K9); false when the arguments need the
+// FP64 kernel (k-derivatives, device-resident k, or phase rotations beyond the
+// Taylor tables)
 bool launch_assemble_df64(Ctx &c, const AssembleArgs &a);
+bool launch_assemble_k9(Ctx &c, const AssembleArgs &a);   // the double-float kernel itself
+
+// Fixed-point assembly at FP64 accuracy (K10, bie_assemble_fix64.cu): records
+// from the FP64 ones; the launch returns false, enqueuing nothing, where the
+// arguments need another kernel (k-derivatives, element factors, phases or
+// damping beyond the fixed-point ranges, coordinates outside 2^+-300).  df_trig: double-float sine and cosine in the
+// FP64 integrals of the near pairs (BIE_PREC_DF64).
+void build_fix64_records(Ctx &c, const std::vector<double> &rec64);
+bool launch_assemble_fix64(Ctx &c, const AssembleArgs &a, bool df_trig);
 
 // FMA throughput probe (bie_peaks.cu)
 void measure_peaks(int device, bie_peaks &out);

@@ -846,6 +846,7 @@ void build_context(Ctx &c, const bie_mesh_desc &d, int device, int gauss_rule,
     if (!k2_fix.empty())
         BIE_CUDA(cudaMemcpy(c.d_k2_fix, k2_fix.data(), k2_fix.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     build_mixed_records(c, rec);
+    build_fix64_records(c, rec);
     prepare_noalloc(c);
 }
 
@@ -872,6 +873,14 @@ void destroy_context(Ctx &c) {
     cudaFree(c.d_dphi);
     cudaFree(c.d_phase_tab);
     c.d_phase_tab = nullptr;
+    cudaFree(c.d_xrecords);
+    cudaFree(c.d_xphi);
+    cudaFree(c.d_xnodes);
+    cudaFree(c.d_xtrig);
+    c.d_xrecords = nullptr;
+    c.d_xphi = nullptr;
+    c.d_xnodes = nullptr;
+    c.d_xtrig = nullptr;
     c.d_drecords = nullptr;
     c.d_dphi = nullptr;
     for (auto &nf : c.nearfields) free_nearfield(*nf);

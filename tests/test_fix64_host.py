@@ -1,0 +1,31 @@
+"""The fixed-point quadrature points of the FP64-grade assembly on the host: the
+functions the kernel calls (csrc/bie_fix64.cuh), compiled with g++ and compared
+with long double over random regular pairs (the complex-wavenumber damping is
+covered by tests/test_gpu_fix64.py)."""
+from __future__ import annotations
+
+import shutil
+import subprocess
+
+import pytest
+
+from conftest import PKG, ROOT
+
+GXX = shutil.which("g++")
+
+
+@pytest.fixture(scope="module")
+def driver(tmp_path_factory):
+    if GXX is None:
+        pytest.skip("g++ not available")
+    exe = tmp_path_factory.mktemp("fix64") / "fix64_points"
+    subprocess.run([GXX, "-O2", "-std=gnu++17", "-I", str(PKG / "csrc"), str(ROOT / "tests" / "fix64_points.cpp"),
+                    "-o", str(exe)], check=True)
+    return str(exe)
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_points_against_long_double(driver, seed):
+    out = subprocess.run([driver, str(seed)], check=True, capture_output=True, text=True).stdout.split()
+    assert out[0] == "1"            # every table index inside its table
+    assert float(out[1]) <= 1.0     # largest error as a multiple of its bound
