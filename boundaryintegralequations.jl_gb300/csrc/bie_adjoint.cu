@@ -26,6 +26,7 @@
 #include "bie_df64.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <complex>
 #include <vector>
@@ -293,6 +294,431 @@ adjoint_grad_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
     }
 }
 
+// ---------------------------------------------------------------------------
+// The reverse pass on the FP32 pipes.
+//
+// adjoint_grad_kernel is bound by the FP64 pipe (87 % busy, 79 ms for the
+// 4842-node ellipsoid, 46.9 M pairs).  Here the regular pairs run in double-float
+// (bie_df64.cuh) and only near pairs and nearest-node near-ties in FP64, in place:
+// 13.5 ms, bound by instruction issue (128 registers, 4 blocks per SM; two rows
+// per thread with one reduction for both took 19.7 ms at 255 registers).  Phases
+// are formed without cancellation, so gradients differ from the FP64 kernel's by
+// 3e-14 .. 8e-14, below the error of the solves (1e-13 .. 4e-13).  With
+// b = conj(w) p(x_q), z = b e^{ikr}, W = jw / 4 pi, n the unit normal, d = x_q - t,
+// g = z alpha_G Y_e, sc = Re conj(w) p_i (collocation rows):
+//   t3 = alpha_F (z_r + k r z_i) - sc,     gp = Re g (i k r - 1),
+//   A' = W/r^2 [ (d.n)/r (alpha_F k^2 z_r - 3 t3 / r^2) + gp / r ],  B = W t3 / r^3,
+//   dL/dx_q = A' d + B n,   dL/dnn = (B d + W g_r / r n) / J   (nn = u x v = J n).
+// Since x_q = sum_a N_a X_a, a pair needs only the scalars
+//   M_ab = sum_q A' N_a N_b,  SB_a = sum_q B N_a,  SG = sum_q W g_r / r,
+//   SZ = sum_q z W / r,
+// and over all rows an element needs the sums of M_ab, D M_a, SB_a, D SB, SG, SZ
+// (M_a = sum_b M_ab, D = centroid - t): 24 numbers, reduced over a warp's rows
+// and added to the element's accumulators; adjoint_finish_kernel forms the vertex
+// gradients from them once per element in FP64.
+// ---------------------------------------------------------------------------
+using dev::df;
+using df64::dd::Acc;
+namespace dd = df64::dd;
+constexpr int kAdjSums = 24;       // M 0..5, D M_a 6..14, SB_a 15..17, D SB 18..20, SG 21, SZ 22, 23
+constexpr int kAdjTab = 20;        // floats per rule point: N_a N_b (11 22 33 12 13 23), N_a as hi, lo
+
+struct AdjPair {                   // the scalars of one pair
+    double M[6], SB[3], SG, SZr, SZi;
+};
+
+struct AdjView {
+    const double *rec;             // FP64 records
+    int stride, nidx_off, qmax;
+    const double *phi;
+    dev::RuleInfo ri;
+};
+
+// One pair in FP64 (near pairs: the reference's rule choice and arithmetic).
+__device__ __noinline__ AdjPair adjoint_pair_fp64(const AdjView &v, int64_t pe, double tx, double ty, double tz,
+                                                  cd cw, double sc, double aF, double sgn, cd G0,
+                                                  const double2 *__restrict__ p, double kre) {
+    const double *r = v.rec + (size_t)pe * v.stride;
+    const int c = dev::nearest_node<3>(r, tx, ty, tz);
+    const int Q = v.ri.Q[c];
+    const double *g = r + v.ri.off[c], *ph = v.phi + (size_t)c * v.qmax * 3;
+    const int32_t *nid = reinterpret_cast<const int32_t *>(r + v.nidx_off);
+    const cd p0 = {p[nid[0]].x, p[nid[0]].y}, p1 = {p[nid[1]].x, p[nid[1]].y}, p2 = {p[nid[2]].x, p[nid[2]].y};
+    AdjPair o;
+    for (int j = 0; j < 6; ++j) o.M[j] = 0.0;
+    for (int j = 0; j < 3; ++j) o.SB[j] = 0.0;
+    o.SG = o.SZr = o.SZi = 0.0;
+    for (int q = 0; q < Q; ++q) {
+        const double N1 = ph[3 * q], N2 = ph[3 * q + 1], N3 = ph[3 * q + 2];
+        const double dx = g[q] - tx, dy = g[Q + q] - ty, dz = g[2 * Q + q] - tz;
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        const double ri = rsqrt(r2), rr = r2 * ri, ri2 = ri * ri;
+        double sn, cs;
+                df64::TrigDf::sincos_of(kre * rr, &sn, &cs);
+        const cd Ph = cadd(cadd(cscale(p0, N1), cscale(p1, N2)), cscale(p2, N3));
+        const cd z = cmul(cmul(cw, Ph), cd{cs, sn});
+        const double kr = kre * rr;
+        const double t3 = aF * (z.re + kr * z.im) - sc;
+        const cd gg = cmul(z, G0);
+        const double gp = -sgn * (gg.re + kr * gg.im);
+        const double wr = g[6 * Q + q] * dev::kInv4Pi * ri;
+        // (d.n)/r with the outward normal: the record holds its negative
+        const double dh = -(g[3 * Q + q] * dx + g[4 * Q + q] * dy + g[5 * Q + q] * dz) * ri;
+        const double A = wr * ri * (dh * (aF * kre * kre * z.re - 3.0 * t3 * ri2) + gp * ri);
+        const double B = wr * ri2 * t3;
+        o.M[0] += A * N1 * N1;
+        o.M[1] += A * N2 * N2;
+        o.M[2] += A * N3 * N3;
+        o.M[3] += A * N1 * N2;
+        o.M[4] += A * N1 * N3;
+        o.M[5] += A * N2 * N3;
+        o.SB[0] += B * N1;
+        o.SB[1] += B * N2;
+        o.SB[2] += B * N3;
+        o.SG += wr * sgn * gg.re;
+        o.SZr += wr * sgn * z.re;
+        o.SZi += wr * sgn * z.im;
+    }
+    return o;
+}
+
+// (K + k3) a with k3 the third float of the wavenumber: a wavenumber rounded to
+// 48 bits is a systematic relative error, which the sums over rows and elements do
+// not average (gradient error 2.4e-13 without it, 1e-13 from the solves alone)
+__device__ __forceinline__ df mul_k(df K, float k3, df a) {
+    const float p = __fmul_rn(K.hi, a.hi);
+    float e = __fmaf_rn(K.hi, a.hi, -p);
+    e = __fmaf_rn(K.hi, a.lo, e);
+    e = __fmaf_rn(K.lo, a.hi, e);
+    return dev::fast_two_sum(p, __fmaf_rn(k3, a.hi, e));
+}
+__device__ __forceinline__ float third(double x, df a) {
+    return (float)((x - (double)a.hi) - (double)a.lo);
+}
+__device__ __forceinline__ void acc_prod(Acc &s, df a, df b) { dd::acc_add(s, dd::mul_raw(a, b)); }
+__device__ __forceinline__ df acc_df(const Acc &s) { return dev::fast_two_sum(s.hi, s.lo); }
+__device__ __forceinline__ df scale2(df a, float s) { return {a.hi * s, a.lo * s}; }   // s a power of two, or +-1
+
+// Sum over the warp of 32 values per lane: lane l returns the sum of value l
+// (31 additions instead of 5 per value).
+__device__ __forceinline__ Acc warp_transpose_sum(Acc (&v)[32], int lane) {
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) {
+        const bool up = lane & s;
+#pragma unroll
+        for (int i = 0; i < s; ++i) {
+            const Acc keep = up ? v[i + s] : v[i], send = up ? v[i] : v[i + s];
+            const float h = __shfl_xor_sync(0xffffffffu, send.hi, s), l = __shfl_xor_sync(0xffffffffu, send.lo, s);
+            const df t = dev::two_sum(keep.hi, h);
+            v[i] = Acc{t.hi, __fadd_rn(__fadd_rn(keep.lo, l), t.lo)};
+        }
+    }
+    return v[0];
+}
+
+__global__ void __launch_bounds__(kT, 4)
+adjoint_df64_kernel(int64_t N, int64_t M, const double *__restrict__ src, const double *__restrict__ fpts,
+                    const double2 *__restrict__ w, const double2 *__restrict__ p, const float *__restrict__ rec,
+                    int stride, int nidx_off, const __grid_constant__ dev::RuleInfo ri,
+                    const double *__restrict__ coords, const double2 *__restrict__ Y, int64_t E, int S,
+                    const float *__restrict__ tab, int qmax, const __grid_constant__ AdjView v64, double kre,
+                    double rhock, df64::DfDegrees deg, int chunk, double *__restrict__ sums,
+                    double *__restrict__ dX) {
+    extern __shared__ __align__(16) float smemf[];
+    float *s_tab = smemf;                                        // 3 qmax kAdjTab
+    float *s_rec = s_tab + 3 * qmax * kAdjTab;                   // chunk * stride
+    float4 *s_ph = reinterpret_cast<float4 *>(s_rec + (size_t)chunk * stride);   // chunk * 3 qmax: p(x_q)
+    float *s_el = reinterpret_cast<float *>(s_ph + (size_t)chunk * 3 * qmax);    // chunk * 32: e_b, G0, centroid
+    __shared__ dev::RuleInfo s_ri;
+    if (threadIdx.x == 0) s_ri = ri;
+    for (int t = threadIdx.x; t < 3 * qmax * kAdjTab; t += kT) s_tab[t] = tab[t];
+    const int lane = threadIdx.x & 31;
+    const int s = blockIdx.y;
+    const int64_t e0 = (int64_t)s * E / S, e1 = (int64_t)(s + 1) * E / S;
+    const df K = dd::to_df(kre), K2 = dd::to_df(kre * kre);
+    const float kf = K.hi, k3 = third(kre, K), k23 = third(kre * kre, K2);
+
+    const int64_t row = (int64_t)blockIdx.x * kT + threadIdx.x;
+    const bool active = row < N + M, node = row < N;   // collocation row, else field row
+    const float aF = node ? 1.0f : -1.0f;              // alpha_F, and the sign of alpha_G's factor
+    double tx = 0, ty = 0, tz = 0;
+    double2 wv = make_double2(0, 0), pv = wv;
+    if (active) {
+        const double *t = node ? src + 3 * row : fpts + 3 * (row - N);
+        tx = t[0];
+        ty = t[1];
+        tz = t[2];
+        wv = w[row];
+        if (node) pv = p[row];
+    }
+    const mixed::Target T{dd::to_df(tx), dd::to_df(ty), dd::to_df(tz)};
+    const df cwr = dd::to_df(wv.x), cwi = dd::to_df(-wv.y);
+    const df sc = dd::to_df(node ? wv.x * pv.x + wv.y * pv.y : 0.0);   // Re conj(w) p_i
+    Acc gt[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+    for (int64_t cb = e0; cb < e1; cb += chunk) {
+        const int n = (int)min((int64_t)chunk, e1 - cb);
+        __syncthreads();
+        {
+            const float4 *a = reinterpret_cast<const float4 *>(rec + cb * stride);
+            float4 *b = reinterpret_cast<float4 *>(s_rec);
+            for (int t = threadIdx.x; t < n * stride / 4; t += kT) b[t] = a[t];
+        }
+        __syncthreads();
+        for (int t = threadIdx.x; t < n * 3 * qmax; t += kT) {   // p at the points, in FP64
+            const int el = t / (3 * qmax), c = (t - el * 3 * qmax) / qmax, q = t - el * 3 * qmax - c * qmax;
+            const int32_t *nid = reinterpret_cast<const int32_t *>(s_rec + (size_t)el * stride + nidx_off);
+            if (q >= s_ri.Q[c]) continue;
+            double re = 0, im = 0;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const double Na = v64.phi[((size_t)c * v64.qmax + q) * 3 + a];
+                const double2 pa = p[nid[a]];
+                re += Na * pa.x;
+                im += Na * pa.y;
+            }
+            const df x = dd::to_df(re), y = dd::to_df(im);
+            s_ph[t] = make_float4(x.hi, x.lo, y.hi, y.lo);
+        }
+        for (int t = threadIdx.x; t < n * 11; t += kT) {         // X_b - centroid, rhock (Im Y, -Re Y)
+            const int el = t / 11, j = t - el * 11;
+            const float *r = s_rec + (size_t)el * stride;
+            double x;
+            if (j < 9) {
+                const int b = j / 3, k = j - 3 * b;
+                const double cen = (double)r[k] + (double)r[3 + k];
+                x = coords[3 * (int64_t)reinterpret_cast<const int32_t *>(r + nidx_off)[b] + k] - cen;
+            } else {
+                const double2 y = Y[cb + el];
+                x = j == 9 ? rhock * y.y : -rhock * y.x;
+            }
+            const df h = dd::to_df(x);
+            s_el[32 * el + 2 * j] = h.hi;
+            s_el[32 * el + 2 * j + 1] = h.lo;
+            if (j < 3)
+                reinterpret_cast<double *>(s_el + 32 * el + 24)[j] = (double)r[j] + (double)r[3 + j];   // centroid
+        }
+        __syncthreads();
+
+        for (int el = 0; el < n; ++el) {
+            const float *r = s_rec + (size_t)el * stride;
+            const float2 *se = reinterpret_cast<const float2 *>(s_el + 32 * el);
+            const df G0r{se[9].x, se[9].y}, G0i{se[10].x, se[10].y};
+            Acc v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = Acc{0.f, 0.f};
+            if (active) {
+                const mixed::PairSetup P = mixed::pair_setup<3>(r, T);
+                df r0, ri0;
+                dd::sqrt_rcp_df(dev::df_add(dev::df_add(dev::df_sqr(P.Dxd), dev::df_sqr(P.Dyd)), dev::df_sqr(P.Dzd)),
+                                r0, ri0);
+                Acc m[6], sb[3], sg{0.f, 0.f}, szr{0.f, 0.f}, szi{0.f, 0.f};
+#pragma unroll
+                for (int a = 0; a < 6; ++a) m[a] = Acc{0.f, 0.f};
+#pragma unroll
+                for (int a = 0; a < 3; ++a) sb[a] = Acc{0.f, 0.f};
+                                if (P.deferred || !(fabsf(kf * r0.hi) < df64::kDfMaxPhase)) {
+                    const cd g0 = {(double)G0r.hi + (double)G0r.lo, (double)G0i.hi + (double)G0i.lo};
+                    const AdjPair o = adjoint_pair_fp64(
+                        v64, cb + el, tx, ty, tz,
+                        cd{(double)cwr.hi + (double)cwr.lo, (double)cwi.hi + (double)cwi.lo},
+                        (double)sc.hi + (double)sc.lo, (double)aF, (double)aF, g0, p, kre);
+                    auto acc_of = [](double x) {
+                        const df t = dd::to_df(x);
+                        return Acc{t.hi, t.lo};
+                    };
+#pragma unroll
+                    for (int a = 0; a < 6; ++a) m[a] = acc_of(o.M[a]);
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) sb[a] = acc_of(o.SB[a]);
+                    sg = acc_of(o.SG);
+                    szr = acc_of(o.SZr);
+                    szi = acc_of(o.SZi);
+                } else {
+                    // e^{i k r0}: phase and quadrant in FP64 (fifteen operations of an
+                    // otherwise idle pipe), series in double-float
+                    df E0r, E0i;
+                    {
+                        const double *cen = reinterpret_cast<const double *>(s_el + 32 * el + 24);
+                        const double ax = cen[0] - tx, ay = cen[1] - ty, az = cen[2] - tz;
+                        const double q2 = ax * ax + ay * ay + az * az;
+                        const double x = kre * (q2 * rsqrt(q2));
+                        const double nq = rint(x * 0.63661977236758134308);   // 2 / pi
+                        const double y = fma(-nq, 6.123233995736766036e-17, fma(-nq, 1.57079632679489655800, x));
+                        dd::sincos_df(dd::to_df(y), E0i, E0r);
+                        const int quad = ((int)nq) & 3;
+                        if (quad & 1) {
+                            const df t = E0r;
+                            E0r = dd::neg(E0i);
+                            E0i = t;
+                        }
+                        if (quad & 2) {
+                            E0r = dd::neg(E0r);
+                            E0i = dd::neg(E0i);
+                        }
+                    }
+                    // conj(w) e^{i k r0}
+                    const df hr = dev::df_sub(dev::df_mul(cwr, E0r), dev::df_mul(cwi, E0i));
+                    const df hi = dev::df_add(dev::df_mul(cwr, E0i), dev::df_mul(cwi, E0r));
+                    const int c = P.c, Q = s_ri.Q[c];
+                    const float4 *g4 = reinterpret_cast<const float4 *>(r + s_ri.off[c]);
+                    const float4 *ph = s_ph + ((size_t)el * 3 + c) * qmax;
+                    const float4 *tb = reinterpret_cast<const float4 *>(s_tab + (size_t)c * qmax * kAdjTab);
+                    for (int q = 0; q < Q; ++q) {
+                        const float4 A = g4[4 * q], B4 = g4[4 * q + 1], Cn = g4[4 * q + 2], Dn = g4[4 * q + 3];
+                        const df ox{A.x, B4.x}, oy{A.y, B4.y}, oz{A.z, B4.z};
+                        const df dx = dev::df_add(P.Dxd, ox), dy = dev::df_add(P.Dyd, oy), dz = dev::df_add(P.Dzd, oz);
+                        df rr, ri1;
+                        dd::sqrt_rcp_df(dev::df_add(dev::df_add(dev::df_sqr(dx), dev::df_sqr(dy)), dev::df_sqr(dz)),
+                                        rr, ri1);
+                        // r - r0 = (2 D.o + |o|^2) / (r + r0), free of cancellation: at a
+                        // distance of 10 the difference of two rounded lengths would cost
+                        // the phase 1e-13
+                        const df Do = dev::df_add(dev::df_add(dev::df_mul(P.Dxd, ox), dev::df_mul(P.Dyd, oy)),
+                                                  dev::df_mul(P.Dzd, oz));
+                        const df dr = dev::df_mul(dev::df_add(scale2(Do, 2.0f), df{Cn.w, Dn.w}),
+                                                  dd::rcp(dev::df_add(rr, r0)));
+                        df ct, st;
+                        df64::rotation_df64(mul_k(K, k3, dr), deg, ct, st);
+                        const float4 pq = ph[q];
+                        const df pr{pq.x, pq.y}, pi{pq.z, pq.w};
+                        // z = conj(w) e^{i k r0} (p(x_q) e^{i k (r - r0)})
+                        const df ar = dev::df_sub(dev::df_mul(pr, ct), dev::df_mul(pi, st));
+                        const df ai = dev::df_add(dev::df_mul(pr, st), dev::df_mul(pi, ct));
+                        const df zr = dev::df_sub(dev::df_mul(hr, ar), dev::df_mul(hi, ai));
+                        const df zi = dev::df_add(dev::df_mul(hr, ai), dev::df_mul(hi, ar));
+                        const df kr = mul_k(K, k3, rr);
+                        const df ri2 = dev::df_sqr(ri1);
+                        const df t3 = dev::df_sub(scale2(dev::df_add(zr, dev::df_mul(kr, zi)), aF), sc);
+                        const df gr = dev::df_sub(dev::df_mul(zr, G0r), dev::df_mul(zi, G0i));
+                        const df gi = dev::df_add(dev::df_mul(zr, G0i), dev::df_mul(zi, G0r));
+                        const df gp = scale2(dev::df_add(gr, dev::df_mul(kr, gi)), -aF);
+                        const df wr = dev::df_mul(df{A.w, B4.w}, ri1);
+                        const df dh = dev::df_mul(
+                            dev::df_add(dev::df_add(dev::df_mul(dx, df{Cn.x, Dn.x}), dev::df_mul(dy, df{Cn.y, Dn.y})),
+                                        dev::df_mul(dz, df{Cn.z, Dn.z})), ri1);   // -(d.n)/r
+                        const df tr = dev::df_mul(t3, ri2);
+                        // aF k^2 z_r - 3 t3 / r^2 (3 x = 2 x + x)
+                        const df q1 = dev::df_sub(scale2(mul_k(K2, k23, zr), aF), dev::df_add(scale2(tr, 2.0f), tr));
+                        const df A1 = dev::df_mul(dev::df_mul(wr, ri1),
+                                                  dev::df_sub(dev::df_mul(gp, ri1), dev::df_mul(dh, q1)));
+                        const df B1 = dev::df_mul(wr, tr);
+                        const float4 t0 = tb[5 * q], t1 = tb[5 * q + 1], t2 = tb[5 * q + 2], t4 = tb[5 * q + 3],
+                                     t5 = tb[5 * q + 4];
+                        acc_prod(m[0], A1, df{t0.x, t0.y});
+                        acc_prod(m[1], A1, df{t0.z, t0.w});
+                        acc_prod(m[2], A1, df{t1.x, t1.y});
+                        acc_prod(m[3], A1, df{t1.z, t1.w});
+                        acc_prod(m[4], A1, df{t2.x, t2.y});
+                        acc_prod(m[5], A1, df{t2.z, t2.w});
+                        acc_prod(sb[0], B1, df{t4.x, t4.y});
+                        acc_prod(sb[1], B1, df{t4.z, t4.w});
+                        acc_prod(sb[2], B1, df{t5.x, t5.y});
+                        const df ws = scale2(wr, aF);
+                        acc_prod(sg, ws, gr);
+                        acc_prod(szr, ws, zr);
+                        acc_prod(szi, ws, zi);
+                    }
+                }
+                // over the element: M, D M_a, SB, D SB, SG, SZ; and the row's gradient
+                // -(sum_q A' d + B n)
+                df mm[6], mb[3], sbd[3];
+#pragma unroll
+                for (int a = 0; a < 6; ++a) mm[a] = acc_df(m[a]);
+                mb[0] = dev::df_add(dev::df_add(mm[0], mm[3]), mm[4]);
+                mb[1] = dev::df_add(dev::df_add(mm[1], mm[3]), mm[5]);
+                mb[2] = dev::df_add(dev::df_add(mm[2], mm[4]), mm[5]);
+#pragma unroll
+                for (int a = 0; a < 3; ++a) sbd[a] = acc_df(sb[a]);
+                const df sbt = dev::df_add(dev::df_add(sbd[0], sbd[1]), sbd[2]);
+                const df mt = dev::df_add(dev::df_add(mb[0], mb[1]), mb[2]);
+                const df D[3] = {P.Dxd, P.Dyd, P.Dzd};
+#pragma unroll
+                for (int a = 0; a < 6; ++a) dd::acc_add(v[a], mm[a]);
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) acc_prod(v[6 + 3 * a + k], D[k], mb[a]);
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    dd::acc_add(v[15 + a], sbd[a]);
+                    acc_prod(v[18 + a], D[a], sbt);
+                }
+                dd::acc_add(v[21], acc_df(sg));
+                dd::acc_add(v[22], acc_df(szr));
+                dd::acc_add(v[23], acc_df(szi));
+                if (node) {
+                    const float4 Cn = *reinterpret_cast<const float4 *>(r + s_ri.off[0] + 8);
+                    const float4 Dn = *reinterpret_cast<const float4 *>(r + s_ri.off[0] + 12);
+                    const df nr[3] = {{Cn.x, Dn.x}, {Cn.y, Dn.y}, {Cn.z, Dn.z}};   // -n
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        acc_prod(gt[k], dd::neg(D[k]), mt);
+                        acc_prod(gt[k], nr[k], sbt);
+#pragma unroll
+                        for (int b = 0; b < 3; ++b) {
+                            const float2 eb = se[3 * b + k];
+                            acc_prod(gt[k], df{-eb.x, -eb.y}, mb[b]);
+                        }
+                    }
+                }
+            }
+            const Acc t = warp_transpose_sum(v, lane);
+            if (lane < kAdjSums) atomicAdd(sums + (size_t)(cb + el) * kAdjSums + lane, dd::acc_value(t));
+        }
+    }
+    if (node)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) atomicAdd(&dX[3 * row + k], dd::acc_value(gt[k]));
+}
+
+// Vertex gradients and admittance sensitivities of every element from its sums.
+__global__ void adjoint_finish_kernel(const double *__restrict__ sums, const double *__restrict__ coords,
+                                      const int32_t *__restrict__ topo, const int32_t *__restrict__ order, int64_t E,
+                                      double rhock, double *__restrict__ dX, double2 *__restrict__ sY) {
+    const int64_t pe = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (pe >= E) return;
+    const int64_t e = order[pe];
+    const double *s = sums + pe * kAdjSums;
+    double X[3][3], cen[3], n[3], eb[3][3], u[3], v[3];
+    for (int b = 0; b < 3; ++b)
+        for (int k = 0; k < 3; ++k) X[b][k] = coords[3 * (int64_t)topo[3 * e + b] + k];
+    for (int k = 0; k < 3; ++k) {
+        cen[k] = X[0][k] / 3.0;
+        cen[k] += X[1][k] / 3.0;
+        cen[k] += X[2][k] / 3.0;   // as the records form it
+        u[k] = X[1][k] - X[0][k];
+        v[k] = X[2][k] - X[0][k];
+        for (int b = 0; b < 3; ++b) eb[b][k] = X[b][k] - cen[k];
+    }
+    n[0] = u[1] * v[2] - u[2] * v[1];
+    n[1] = u[2] * v[0] - u[0] * v[2];
+    n[2] = u[0] * v[1] - u[1] * v[0];
+    const double J = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+    for (int k = 0; k < 3; ++k) n[k] /= J;
+    const int ix[3][3] = {{0, 3, 4}, {3, 1, 5}, {4, 5, 2}};
+    double g[3][3], Gn[3];
+    for (int k = 0; k < 3; ++k) {
+        Gn[k] = s[18 + k] + n[k] * s[21];
+        for (int a = 0; a < 3; ++a) {
+            double t = s[6 + 3 * a + k] + n[k] * s[15 + a];
+            for (int b = 0; b < 3; ++b) t += eb[b][k] * s[ix[a][b]];
+            g[a][k] = t;
+            Gn[k] += eb[a][k] * s[15 + a];
+        }
+    }
+    for (int k = 0; k < 3; ++k) Gn[k] /= J;
+    // nn = u x v: dL/du = v x Gn, dL/dv = Gn x u
+    const double au[3] = {v[1] * Gn[2] - v[2] * Gn[1], v[2] * Gn[0] - v[0] * Gn[2], v[0] * Gn[1] - v[1] * Gn[0]};
+    const double av[3] = {Gn[1] * u[2] - Gn[2] * u[1], Gn[2] * u[0] - Gn[0] * u[2], Gn[0] * u[1] - Gn[1] * u[0]};
+    for (int k = 0; k < 3; ++k) {
+        atomicAdd(&dX[3 * (int64_t)topo[3 * e] + k], g[0][k] - au[k] - av[k]);
+        atomicAdd(&dX[3 * (int64_t)topo[3 * e + 1] + k], g[1][k] + au[k]);
+        atomicAdd(&dX[3 * (int64_t)topo[3 * e + 2] + k], g[2][k] + av[k]);
+    }
+    // sum of sgn z W / r times -i rhock
+    sY[e] = make_double2(rhock * s[23], -rhock * s[22]);
+}
+
 inline unsigned nblocks(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
@@ -334,14 +760,26 @@ void run_adjoint(Ctx &c, const AdjointArgs &a, AdjointOut &out) {
     const double2 aBc = make_double2(0.0, a.rho_c * a.k_re);
     // ---- forward: A, B ----------------------------------------------------------
     {
+        // |Re Y|, |Im Y| < 2^exp for the fixed-point assembly
+        double ymax = 0.0;
+        const std::complex<double> *Zh = reinterpret_cast<const std::complex<double> *>(a.Z);
+        for (int64_t e = 0; e < E; ++e) {
+            const double n = std::norm(Zh[e]);
+            const double y = std::max(std::fabs(Zh[e].real()), std::fabs(Zh[e].imag())) / n;
+            if (!(y <= ymax)) ymax = y;   // a NaN or infinity stays
+        }
+        int yexp = INT_MIN;
+        if (ymax > 0x1p-200 && ymax < 0x1p200) (void)std::frexp(ymax * 1.0001, &yexp);
         AssembleArgs s{a.k_re, a.k_im, c.d_sources, N, BIE_F | BIE_G | BIE_C, A.d(), G.d(), Cv.d()};
         s.g_weight = Y.d();
+        s.g_weight_exp = yexp;
         if (!(a.precision == BIE_PREC_DF64 && launch_assemble_df64(c, s))) launch_assemble_fp64(c, s);
         combine_system_kernel<<<std::min<unsigned>(nblocks(N * N), 65535u), 256, 0, st>>>(
             A.d2(), G.d2(), aAc, Cv.d2(), N, N);
         BIE_CUDA(cudaGetLastError());
         AssembleArgs f{a.k_re, a.k_im, fp.d(), M, BIE_F | BIE_G, B.d(), Gx.d(), nullptr};
         f.g_weight = Y.d();
+        f.g_weight_exp = yexp;
         if (!(a.precision == BIE_PREC_DF64 && launch_assemble_df64(c, f))) launch_assemble_fp64(c, f);
         // stored: F_x - i rho c k G_x  (= -B)
         combine_system_kernel<<<std::min<unsigned>(nblocks(M * N), 65535u), 256, 0, st>>>(
@@ -433,16 +871,64 @@ void run_adjoint(Ctx &c, const AdjointArgs &a, AdjointOut &out) {
         BIE_CUDA(cudaMemcpyAsync(tab.p, ht.data(), ht.size() * 8, cudaMemcpyHostToDevice, st));
         BIE_CUDA(cudaMemsetAsync(dX.p, 0, 3 * N * 8, st));
         BIE_CUDA(cudaMemsetAsync(sY.p, 0, E * 16, st));
-        int S = 1;
-        const int64_t tiles = (N + M + kT - 1) / kT;
-        while (tiles * S < 8LL * c.num_sms && S < 256 && S * 2 <= E) S *= 2;
         const double rhock_re = a.rho_c * a.k_re;
-        dim3 grid((unsigned)tiles, (unsigned)S);
-        adjoint_grad_kernel<false><<<grid, kT, 0, st>>>(N, M, c.d_sources, fp.d(), w.d2(), p.d2(),
-                                                        c.d_coords, c.d_topo, ord.i32(), Y.d2(), E, S,
-                                                        tab.d(), rt, a.k_re, a.k_im, rhock_re, dX.d(),
-                                                        sY.d2());
-        BIE_CUDA(cudaGetLastError());
+        df64::DfDegrees deg{};
+        if (df64::df_degrees(std::fabs(a.k_re) * c.df_rho_max, 0.0, deg)) {
+            deg.tab = reinterpret_cast<const float4 *>(c.d_phase_tab);
+            const RecordLayout &L = c.lay;
+            const Df64Layout &X = c.dlay;
+            AdjView v{c.d_records, L.stride, L.nidx_off, L.qmax, c.d_phi, {}};
+            dev::RuleInfo ri{};
+            for (int r = 0; r < 3; ++r) {
+                ri.Q[r] = v.ri.Q[r] = L.Q[r];
+                ri.off[r] = X.rule_off[r];
+                v.ri.off[r] = L.rule_off[r];
+            }
+            // N_a N_b and N_a per rule point as hi, lo
+            std::vector<float> tb((size_t)3 * L.qmax * kAdjTab, 0.f);
+            for (int r = 0; r < 3; ++r)
+                for (int q = 0; q < L.Q[r]; ++q) {
+                    const double *Nv = &c.phi[((size_t)r * L.qmax + q) * 3];
+                    const double x[10] = {Nv[0] * Nv[0], Nv[1] * Nv[1], Nv[2] * Nv[2], Nv[0] * Nv[1],
+                                          Nv[0] * Nv[2], Nv[1] * Nv[2], Nv[0], Nv[1], Nv[2], 0.0};
+                    float *t = &tb[((size_t)r * L.qmax + q) * kAdjTab];
+                    for (int j = 0; j < 10; ++j) {
+                        t[2 * j] = (float)x[j];
+                        t[2 * j + 1] = (float)(x[j] - (double)t[2 * j]);
+                    }
+                }
+            Buf dtab(tb.size() * 4), sums((size_t)E * kAdjSums * 8);
+            BIE_CUDA(cudaMemcpyAsync(dtab.p, tb.data(), tb.size() * 4, cudaMemcpyHostToDevice, st));
+            BIE_CUDA(cudaMemsetAsync(sums.p, 0, (size_t)E * kAdjSums * 8, st));
+            // chunks of ~24 KB: four blocks per SM with room for L1
+            const size_t el_bytes = (size_t)X.stride * 4 + (size_t)3 * L.qmax * 16 + 32 * 4;
+            const int chunk = (int)std::max<size_t>(1, std::min<size_t>(32, (24u << 10) / el_bytes));
+            const size_t smem = tb.size() * 4 + chunk * el_bytes;
+            const int64_t tiles = (N + M + kT - 1) / kT;
+            int S = 1;
+            // many small blocks: their cost differs with the near pairs in them (13.5 ms
+            // at 64 blocks per SM, 14.0 at 32, 14.9 at 16, 16.4 at 8)
+            while (tiles * S < 64LL * c.num_sms && S * 2 * 8 <= E) S *= 2;
+            BIE_CUDA(cudaFuncSetAttribute(adjoint_df64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            adjoint_df64_kernel<<<dim3((unsigned)tiles, (unsigned)S), kT, smem, st>>>(
+                N, M, c.d_sources, fp.d(), w.d2(), p.d2(), c.d_drecords, X.stride, X.nidx_off, ri, c.d_coords, Y.d2(),
+                E, S, static_cast<const float *>(dtab.p), L.qmax, v, a.k_re, rhock_re, deg, chunk, sums.d(), dX.d());
+            BIE_CUDA(cudaGetLastError());
+            adjoint_finish_kernel<<<nblocks(E), 256, 0, st>>>(sums.d(), c.d_coords, c.d_topo, ord.i32(), E, rhock_re,
+                                                              dX.d(), sY.d2());
+            BIE_CUDA(cudaGetLastError());
+            BIE_CUDA(cudaStreamSynchronize(st));   // the call's buffers go out of scope
+        } else {   // phase rotations beyond the double-float tables
+            int S = 1;
+            const int64_t tiles = (N + M + kT - 1) / kT;
+            while (tiles * S < 8LL * c.num_sms && S < 256 && S * 2 <= E) S *= 2;
+            dim3 grid((unsigned)tiles, (unsigned)S);
+            adjoint_grad_kernel<false><<<grid, kT, 0, st>>>(N, M, c.d_sources, fp.d(), w.d2(), p.d2(),
+                                                            c.d_coords, c.d_topo, ord.i32(), Y.d2(), E, S,
+                                                            tab.d(), rt, a.k_re, a.k_im, rhock_re, dX.d(),
+                                                            sY.d2());
+            BIE_CUDA(cudaGetLastError());
+        }
         std::vector<double> hdX(3 * N);
         std::vector<std::complex<double>> hs(E), hpI(N);
         BIE_CUDA(cudaMemcpyAsync(hdX.data(), dX.p, 3 * N * 8, cudaMemcpyDeviceToHost, st));

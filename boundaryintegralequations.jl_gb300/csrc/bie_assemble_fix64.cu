@@ -77,6 +77,7 @@ struct FxScale {
     int pe;              // basis values are stored times 2^-pe
     int extra;           // entry units times 2^extra (large node valences)
     float rho_max;       // largest rho of the mesh
+    int wexp;            // element factors on G are held times 2^-wexp
 };
 
 // k as mantissas and exponents (see fix64::pair_wavenumber, pair_damping)
@@ -236,7 +237,8 @@ constexpr int kGroup = 4;
 constexpr int kInterleave = 2;   // points evaluated side by side
 inline int phi_groups(int qmax) { return (qmax + kGroup - 1) / kGroup; }
 
-template <int NP, bool CPLX_K>
+// GW: per-element complex factors on G (the adjoint's element admittances)
+template <int NP, bool CPLX_K, bool GW>
 __global__ void __launch_bounds__(kThreads, 4)
 assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int S,
                       const int4 *__restrict__ phi, int nphi, int ngroups, const __grid_constant__ RuleInfo ri,
@@ -244,7 +246,7 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
                       double kre, double kim, int flags, longlong2 *__restrict__ F, longlong2 *__restrict__ G,
                       const uint32_t *__restrict__ kflags, double *__restrict__ Cpart,
                       int2 *__restrict__ defer, unsigned int *__restrict__ defer_count, unsigned int defer_cap,
-                      int *__restrict__ over, const __grid_constant__ FxScale sc,
+                      int *__restrict__ over, const int4 *__restrict__ gweight, const __grid_constant__ FxScale sc,
                       unsigned long long *__restrict__ qpe_count, const double *__restrict__ kdev) {
     if (kdev) {   // wavenumber read from device memory (recorded sweeps)
         kre = kdev[0];
@@ -356,8 +358,14 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
                             g.jw = Limb{on ? D2.x : 0, on ? D2.y : 0};
                             const fix64::Point v = fix64::point<CPLX_K>(g, P, table, damp_table);
                             ce += v.tq;
-                            const Limb a0 = fix64::split(v.Fr), a1 = fix64::split(v.Fi), a2 = fix64::split(v.Gr),
-                                       a3 = fix64::split(v.Gi);
+                            const Limb a0 = fix64::split(v.Fr), a1 = fix64::split(v.Fi);
+                            Limb a2 = fix64::split(v.Gr), a3 = fix64::split(v.Gi);
+                            if (GW) {
+                                const int4 f = __ldg(gweight + pe);
+                                const fix64::Values2 u = fix64::complex_mul(a2, a3, Limb{f.x, f.y}, Limb{f.z, f.w});
+                                a2 = fix64::split(u.re);
+                                a3 = fix64::split(u.im);
+                            }
                             vf[j] = make_int4(a0.h, a0.l, a1.h, a1.l);
                             vg[j] = make_int4(a2.h, a2.l, a3.h, a3.l);
                         }
@@ -435,7 +443,7 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
                         if (last) {   // final complex128 entries
                             const int adj = sc.pe + sc.extra - en.base;
                             vF = fx_complex<CPLX_K>(vF, fix64::entry_exp_f(node_ej[a], fl, wv.kb) + adj);
-                            vG = fx_complex<CPLX_K>(vG, fix64::entry_exp_g(node_ej[a], fl) + adj + sc.S);
+                            vG = fx_complex<CPLX_K>(vG, fix64::entry_exp_g(node_ej[a], fl) + adj + sc.S + sc.wexp);
                         }
                         if (doF) *pF = vF;
                         if (doG) *pG = vG;
@@ -493,14 +501,22 @@ __global__ void fx_widen_kernel(const int32_t *__restrict__ fnode, int64_t nfix,
         const FxEntry en = fx_entry<CPLX_K>(fx, fy, fz, x.x, x.y, x.z, wv);
         const int ej = __float_as_int(x.w), adj = sc.pe + sc.extra - en.base;
         if (F) F[off] = fx_complex<CPLX_K>(F[off], fix64::entry_exp_f(ej, en.fl, wv.kb) + adj);
-        if (G) G[off] = fx_complex<CPLX_K>(G[off], fix64::entry_exp_g(ej, en.fl) + adj + sc.S);
+        if (G) G[off] = fx_complex<CPLX_K>(G[off], fix64::entry_exp_g(ej, en.fl) + adj + sc.S + sc.wexp);
     }
+}
+
+// element factors as Q62 limbs times 2^-wexp
+__global__ void fx_weight_kernel(const double2 *__restrict__ w, int64_t E, int wexp, int4 *__restrict__ out) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= E) return;
+    const Limb a = fix64::split(fx_round(w[p].x, 0.0, 62 - wexp)), b = fix64::split(fx_round(w[p].y, 0.0, 62 - wexp));
+    out[p] = make_int4(a.h, a.l, b.h, b.l);
 }
 
 template <int NP, bool CPLX_K, class Trig>
 __device__ __forceinline__ int fx_correct_pair(const Fp64View &v, int64_t i, int64_t p, const double *tgt, int64_t M,
                                                double kre, double kim, bool doF, bool doG, bool doC, double2 *F,
-                                               double2 *G, double *Cnear) {
+                                               double2 *G, double *Cnear, const double2 *gweight) {
     const double *r = v.rec + (size_t)p * v.stride;
     const double tx = tgt[3 * i], ty = tgt[3 * i + 1], tz = tgt[3 * i + 2];
     const int c = dev::nearest_node<NP>(r, tx, ty, tz);
@@ -508,6 +524,15 @@ __device__ __forceinline__ int fx_correct_pair(const Fp64View &v, int64_t i, int
     const double ce = dev::element_fp64<NP, CPLX_K, Trig>(r + v.ri.off[c], v.ri.Q[c],
                                                           v.phi + (size_t)c * v.qmax * NP, tx, ty, tz, kre, kim, fr,
                                                           fi, gr, gi);
+    if (gweight && doG) {
+        const double2 w = gweight[p];
+#pragma unroll
+        for (int a = 0; a < NP; ++a) {
+            const double t = gr[a] * w.x - gi[a] * w.y;
+            gi[a] = gr[a] * w.y + gi[a] * w.x;
+            gr[a] = t;
+        }
+    }
     const int32_t *nid = reinterpret_cast<const int32_t *>(r + v.nidx_off);
 #pragma unroll
     for (int a = 0; a < NP; ++a) {
@@ -535,7 +560,7 @@ fx_correct_kernel(const int2 *__restrict__ defer, const unsigned int *__restrict
                   int64_t M, double kre, double kim, int flags, double2 *__restrict__ F, double2 *__restrict__ G,
                   double *__restrict__ Cnear, const int *__restrict__ over, const float *__restrict__ rec, int stride,
                   int64_t E, int S, const __grid_constant__ FxScale sc, unsigned long long *__restrict__ qpe_count,
-                  const double *__restrict__ kdev) {
+                  const double *__restrict__ kdev, const double2 *__restrict__ gweight) {
     if (kdev) {
         kre = kdev[0];
         kim = kdev[1];
@@ -545,7 +570,7 @@ fx_correct_kernel(const int2 *__restrict__ defer, const unsigned int *__restrict
     unsigned long long nqpe = 0;
     for (unsigned int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
         nqpe += fx_correct_pair<NP, CPLX_K, Trig>(v, defer[j].x, defer[j].y, tgt, M, kre, kim, doF, doG, doC, F, G,
-                                                  Cnear);
+                                                  Cnear, gweight);
     if (total > defer_cap) {
         const FxWave wv = fx_wave<CPLX_K>(kre, kim, sc);
         for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < M * S;
@@ -556,7 +581,7 @@ fx_correct_kernel(const int2 *__restrict__ defer, const unsigned int *__restrict
             for (int64_t p = over[j]; p < (s + 1) * E / S; ++p) {
                 i64 dx, dy, dz;
                 if (!fx_pair<NP, CPLX_K>(rec + p * stride, T, wv, dx, dy, dz).deferred) continue;
-                nqpe += fx_correct_pair<NP, CPLX_K, Trig>(v, i, p, tgt, M, kre, kim, doF, doG, doC, F, G, Cnear);
+                nqpe += fx_correct_pair<NP, CPLX_K, Trig>(v, i, p, tgt, M, kre, kim, doF, doG, doC, F, G, Cnear, gweight);
             }
         }
     }
@@ -594,6 +619,15 @@ void launch_np(Ctx &c, const AssembleArgs &a, bool df_trig, const LaunchShape &s
     sc.pe = c.fx_phi_exp;
     sc.extra = c.fx_extra;
     sc.rho_max = c.fx_rho_max;
+    int4 *gw = nullptr;
+    if (a.g_weight && (a.flags & BIE_G)) {
+        sc.wexp = a.g_weight_exp;
+        gw = static_cast<int4 *>(c.scratch(kScratchFxWeight, (size_t)c.n_elements * sizeof(int4)));
+        fx_weight_kernel<<<(unsigned)((c.n_elements + 255) / 256), 256, 0, c.stream>>>(
+            reinterpret_cast<const double2 *>(a.g_weight), c.n_elements, sc.wexp, gw);
+        BIE_CUDA(cudaGetLastError());
+        ++c.kernel_launches;
+    }
     const Fp64View v{c.d_records, L.stride, L.nidx_off, c.d_phi, L.qmax, ri64};
     const int level = sh.level, S = 1 << level;
     const int64_t E = c.n_elements, nfix = c.k2_nfix[level];
@@ -605,7 +639,9 @@ void launch_np(Ctx &c, const AssembleArgs &a, bool df_trig, const LaunchShape &s
         BIE_CUDA(cudaGetLastError());
         ++c.kernel_launches;
     }
-    auto kern = assemble_fix64_kernel<NP, CPLX>;
+    auto kern = assemble_fix64_kernel<NP, CPLX, false>;
+    if constexpr (NP == 3 && !CPLX)
+        if (gw) kern = assemble_fix64_kernel<NP, CPLX, true>;
     BIE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const dim3 grid((unsigned)((a.M + kThreads - 1) / kThreads), (unsigned)S);
     cudaEvent_t t0 = c.timer_begin();
@@ -614,7 +650,7 @@ void launch_np(Ctx &c, const AssembleArgs &a, bool df_trig, const LaunchShape &s
         phi_groups(L.qmax), ri,
         reinterpret_cast<const int4 *>(c.d_xtrig),
         reinterpret_cast<const int2 *>(c.d_xtrig + 4 * fix64::kTrigEntries), a.targets, a.M, a.k_re, a.k_im, a.flags, F, G,
-        c.d_k2_flags + (size_t)level * E, b.Cpart, b.defer, b.dcount, b.dcap, b.over, sc, c.d_qpe, a.k_dev);
+        c.d_k2_flags + (size_t)level * E, b.Cpart, b.defer, b.dcount, b.dcap, b.over, gw, sc, c.d_qpe, a.k_dev);
     BIE_CUDA(cudaGetLastError());
     c.timer_end(t0);
     ++c.kernel_launches;
@@ -628,12 +664,36 @@ void launch_np(Ctx &c, const AssembleArgs &a, bool df_trig, const LaunchShape &s
     auto corr = df_trig ? fx_correct_kernel<NP, CPLX, df64::TrigDf> : fx_correct_kernel<NP, CPLX, dev::TrigFp64>;
     corr<<<(unsigned)(4 * c.num_sms), 128, 0, c.stream>>>(
         b.defer, b.dcount, b.dcap, v, a.targets, a.M, a.k_re, a.k_im, a.flags, reinterpret_cast<double2 *>(F),
-        reinterpret_cast<double2 *>(G), b.Cnear, b.over, c.d_xrecords, X.stride, E, S, sc, c.d_qpe, a.k_dev);
+        reinterpret_cast<double2 *>(G), b.Cnear, b.over, c.d_xrecords, X.stride, E, S, sc, c.d_qpe, a.k_dev,
+        reinterpret_cast<const double2 *>(a.g_weight));
     BIE_CUDA(cudaGetLastError());
     ++c.kernel_launches;
 }
 
 }  // namespace
+
+// e^{2 pi i j / 1024} and 2^(-j / 256) as Q62 limbs (constants: built once; the
+// extended arithmetic is software on some hosts)
+static const std::vector<int32_t> &unit_tables() {
+    static const std::vector<int32_t> table = [] {
+        const int n = fix64::kTrigEntries;
+        std::vector<int32_t> t((size_t)4 * n + 2 * fix64::kDampEntries);
+        const long double pi = 3.141592653589793238462643383279502884L;
+        auto put = [](int32_t *w, long double x) {
+            const fix64::Limb s = fix64::split((long long)std::llrint(std::ldexp(x, 62)));
+            w[0] = s.h;
+            w[1] = s.l;
+        };
+        for (int j = 0; j < n; ++j) {
+            put(&t[4 * j], std::cos(2.0L * pi * j / n));
+            put(&t[4 * j + 2], std::sin(2.0L * pi * j / n));
+        }
+        for (int j = 0; j < fix64::kDampEntries; ++j)
+            put(&t[4 * n + 2 * j], std::exp2(-(long double)j / fix64::kDampEntries));
+        return t;
+    }();
+    return table;
+}
 
 // Records of the fixed-point kernels from the FP64 ones (E x lay.stride).
 void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
@@ -809,20 +869,7 @@ void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
         const int32_t v = node_ej[j] == INT32_MIN ? 0 : node_ej[j];
         std::memcpy(&nodes[4 * j + 3], &v, 4);
     }
-    // e^{2 pi i j / 1024} and 2^(-j / 256) as Q62 limbs
-    std::vector<int32_t> trig((size_t)4 * fix64::kTrigEntries + 2 * fix64::kDampEntries);
-    {
-        const int n = fix64::kTrigEntries;
-        const long double pi = 3.141592653589793238462643383279502884L;
-        auto q62 = [](long double x) { return (long long)std::llrint(std::ldexp(x, 62)); };
-        for (int j = 0; j < n; ++j) {
-            const long double th = 2.0L * pi * j / n;
-            put_limbs(&trig[4 * j], q62(std::cos(th)));
-            put_limbs(&trig[4 * j + 2], q62(std::sin(th)));
-        }
-        for (int j = 0; j < fix64::kDampEntries; ++j)   // 2^(-j / 256)
-            put_limbs(&trig[4 * n + 2 * j], q62(std::exp2(-(long double)j / fix64::kDampEntries)));
-    }
+    const std::vector<int32_t> &trig = unit_tables();
     BIE_CUDA(cudaMalloc(&c.d_xrecords, rec.size() * 4));
     BIE_CUDA(cudaMalloc(&c.d_xphi, phi.size() * 4));
     BIE_CUDA(cudaMalloc(&c.d_xnodes, nodes.size() * 4));
@@ -836,9 +883,10 @@ void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
 
 bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df_trig) {
     AssembleArgs a = args;
-    if (!c.fx_ok || a.taylor_m >= 0 || a.g_weight) return false;
+    if (!c.fx_ok || a.taylor_m >= 0 || (a.g_weight && a.g_weight_exp == INT32_MIN)) return false;
     if (a.k_dev && !(a.k_abs_max > 0)) return false;   // no bound on |k|
     const bool cplx = a.k_im != 0.0;
+    if (a.g_weight && (c.lay.NP != 3 || cplx)) return false;   // (the adjoint: 3-node physics, real k)
     // wavenumbers whose phase or damping over the mesh or an element leaves the
     // fixed-point ranges for many pairs stay with the FP64 kernel
     const double bound = a.k_dev ? a.k_abs_max : 0.0, len = std::ldexp(1.0, c.fx_exp);

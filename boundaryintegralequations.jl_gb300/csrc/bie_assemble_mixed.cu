@@ -978,7 +978,7 @@ void build_df64_records(Ctx &c, const std::vector<double> &rec64, const std::vec
                 float *P = w + 16 * q;
                 const double o[3] = {g[q] - cen[0], g[Q + q] - cen[1], g[2 * Q + q] - cen[2]};
                 rho = std::max(rho, std::sqrt(o[0] * o[0] + o[1] * o[1] + o[2] * o[2]));
-                // (ox oy oz jw/4pi)_hi, (...)_lo, (nx ny nz 0)_hi, (...)_lo
+                // (ox oy oz jw/4pi)_hi, (...)_lo, (nx ny nz |o|^2)_hi, (...)_lo
                 split(o[0], P[0], P[4]);
                 split(o[1], P[1], P[5]);
                 split(o[2], P[2], P[6]);
@@ -986,6 +986,7 @@ void build_df64_records(Ctx &c, const std::vector<double> &rec64, const std::vec
                 split(g[3 * Q + q], P[8], P[12]);
                 split(g[4 * Q + q], P[9], P[13]);
                 split(g[5 * Q + q], P[10], P[14]);
+                split(o[0] * o[0] + o[1] * o[1] + o[2] * o[2], P[11], P[15]);   // |o|^2
             }
         }
         std::copy(M0 + c.mlay.nidx_off, M0 + c.mlay.nidx_off + NP, W + X.nidx_off);

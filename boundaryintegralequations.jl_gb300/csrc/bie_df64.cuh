@@ -84,6 +84,18 @@ __device__ __forceinline__ df sqrt_df(df a) {
     const float e = __fadd_rn(__fmaf_rn(-y, y, a.hi), a.lo);
     return dev::fast_two_sum(y, __fmul_rn(e, 0.5f * rsqrtf(a.hi)));
 }
+// sqrt(a) and 1 / sqrt(a), a > 0, without the bias of sqrt_df and rcp (whose
+// correction terms inherit the float reciprocal square root's error and drop the
+// square): both corrections use one correctly rounded reciprocal
+__device__ __forceinline__ void sqrt_rcp_df(df a, df &s, df &i) {
+    const float y = __fsqrt_rn(a.hi);
+    const float q = __frcp_rn(y);
+    const float e = __fadd_rn(__fmaf_rn(-y, y, a.hi), a.lo);
+    s = dev::fast_two_sum(y, __fmul_rn(e, 0.5f * q));
+    float r = __fmaf_rn(-s.hi, q, 1.0f);
+    r = __fmaf_rn(-s.lo, q, r);
+    i = dev::fast_two_sum(q, __fmul_rn(q, __fmaf_rn(r, r, r)));
+}
 // a * b with the product left unnormalised (hi, lo): for sums that
 // renormalise later
 __device__ __forceinline__ df mul_raw(df a, df b) {
@@ -193,6 +205,24 @@ inline bool df_degrees(double theta, double kappa, DfDegrees &d) {
 }
 
 
+// e^{i theta}, |theta| < kPhaseTabHalf kPhaseTabStep: the table entry at the nearest
+// j h times the Taylor series of the remainder
+__device__ __forceinline__ void rotation_df64(dev::df th, const DfDegrees &deg, dev::df &ct, dev::df &st) {
+    using dev::df;
+    const float jf = rintf(__fmul_rn(th.hi, 1.0f / kPhaseTabStep));
+    const df dl = dd::add_f(th, -__fmul_rn(jf, kPhaseTabStep));    // exact product
+    const df z = dev::df_sqr(dl);
+    const df cd = dd::poly(kDfCos, 2, z);                            // to dl^4: dl^6/6! < 5e-18
+    const df sd = dev::df_mul(dl, dd::poly(kDfSin, 2, z));
+    // (|jf| <= 0.9 kPhaseTabHalf by the host's bound on |k| x element radius;
+    // clamped so that no value can index outside the table)
+    const int jt = min(kPhaseTabHalf, max(-kPhaseTabHalf, __float2int_rn(jf)));
+    const float4 T = __ldg(deg.tab + kPhaseTabHalf + jt);
+    const df Tc{T.x, T.y}, Ts{T.z, T.w};
+    ct = dev::df_sub(dev::df_mul(Tc, cd), dev::df_mul(Ts, sd));
+    st = dev::df_add(dev::df_mul(Ts, cd), dev::df_mul(Tc, sd));
+}
+
 // Kernel values at one quadrature point of a regular pair in double-float
 // (greens3d!, freens3d!, freens3dk0! of src/3d/kernels.jl:13-55 times the
 // jacobian-weight product): D = c_e - t, record point (A, B: o and jw/4pi as
@@ -209,20 +239,8 @@ __device__ __forceinline__ void qpe_df64(const float4 A, const float4 B, const f
     const df dz = dev::df_add(P.Dzd, df{A.z, B.z});
     const df rr = dd::sqrt_df(dev::df_add(dev::df_add(dev::df_sqr(dx), dev::df_sqr(dy)), dev::df_sqr(dz)));
     const df ri_ = dd::rcp(rr);
-    // e^{i k (r - r0)} = e^{i j h} e^{i (theta - j h)}, |theta| < kPhaseTabHalf h
-    const df th = dev::df_mul(K, dev::df_sub(rr, r0));
-    const float jf = rintf(__fmul_rn(th.hi, 1.0f / kPhaseTabStep));
-    const df dl = dd::add_f(th, -__fmul_rn(jf, kPhaseTabStep));    // exact product
-    const df z = dev::df_sqr(dl);
-    const df cd = dd::poly(kDfCos, 2, z);                            // to dl^4: dl^6/6! < 5e-18
-    const df sd = dev::df_mul(dl, dd::poly(kDfSin, 2, z));
-    // (|jf| <= 0.9 kPhaseTabHalf by the host's bound on |k| x element radius;
-    // clamped so that no value can index outside the table)
-    const int jt = min(kPhaseTabHalf, max(-kPhaseTabHalf, __float2int_rn(jf)));
-    const float4 T = __ldg(deg.tab + kPhaseTabHalf + jt);
-    const df Tc{T.x, T.y}, Ts{T.z, T.w};
-    df ct = dev::df_sub(dev::df_mul(Tc, cd), dev::df_mul(Ts, sd));
-    df st = dev::df_add(dev::df_mul(Ts, cd), dev::df_mul(Tc, sd));
+    df ct, st;   // e^{i k (r - r0)}
+    rotation_df64(dev::df_mul(K, dev::df_sub(rr, r0)), deg, ct, st);
     if (CPLX_K) {
         const df damp = dd::poly(kDfExp, deg.Je, dd::neg(dev::df_mul(Ki, dev::df_sub(rr, r0))));
         ct = dev::df_mul(ct, damp);

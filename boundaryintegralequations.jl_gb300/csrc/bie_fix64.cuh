@@ -98,6 +98,16 @@ FX_FN i64 fold_up(i64 H, i64 L) { return (i64)((u64)H << S) + (L >> (32 - S)); }
 template <int S>
 FX_FN i64 mulhi_up(Limb a, Limb b) { return fold_up<S>(wide(a.h, b.h), cross<S>(a, b)); }
 
+// (ar + i ai) (br + i bi) 2^-62, b in Q62
+struct Values2 {
+    i64 re, im;
+};
+FX_FN Values2 complex_mul(Limb ar, Limb ai, Limb br, Limb bi) {
+    const Limb mbi = split(-((i64)((u64)(i64)bi.h << 32) + (i64)bi.l));
+    return Values2{fold_up<2>(high(wide(ar.h, br.h), ai, mbi), cross(cross<2>(ar, br), ai, mbi)),
+                   fold_up<2>(high(wide(ar.h, bi.h), ai, br), cross(cross<2>(ar, bi), ai, br))};
+}
+
 constexpr int kTrigBits = 10;                      // e^{2 pi i j / 1024}
 constexpr int kTrigEntries = 1 << kTrigBits;
 constexpr int kCoordBits = 59;                     // fixed coordinates: largest |x| -> 2^59

@@ -107,6 +107,7 @@ enum ScratchSlot {
     kScratchLowp = 12,     // multi-RHS products: strips, 16-bit tiles, partial sums
     kScratchSolverNested = 13,  // GMRES workspace + partials of nested solves, two slots
                                 // per level 1, 2 (solves inside another solve's product)
+    kScratchFxWeight = 16, // fixed-point assembly: element factors as limbs
     kScratchK2Side = 17,   // mixed assembly: per-slice partial sums of nodes shared between slices
     kScratchCount = 18
 };
@@ -127,8 +128,8 @@ struct MixedLayout {
 
 // Double-float element records (K9, BIE_PREC_DF64): the mixed header (centroid
 // hi/lo, near radius^2, FP32 node offsets), then per rule and point 16 floats
-// (o = x_q - c_e and jw / 4 pi as hi, lo; the unit normal as hi, lo), then the
-// physics node indices.
+// (o = x_q - c_e and jw / 4 pi as hi, lo; the unit normal and |o|^2 as hi, lo),
+// then the physics node indices.
 struct Df64Layout {
     int rule_off[kMaxRules] = {};
     int nidx_off = 0;
@@ -316,8 +317,10 @@ struct AssembleArgs {
     int flags;
     double *F, *G, *C;       // device outputs (interleaved complex), may be null
     bool c64_out = false;    // mixed only: F, G are complex64 (float2) buffers, not widened
-    const double *g_weight = nullptr;   // FP64 only: per-element complex factor on G
+    const double *g_weight = nullptr;   // not mixed: per-element complex factor on G
                                         // (record order), e.g. an element admittance
+    int g_weight_exp = INT32_MIN;       // |Re|, |Im| of the factors < 2^g_weight_exp; INT32_MIN:
+                                        // not known (no fixed-point assembly)
     int taylor_m = -1;                  // FP64 only: >= 0 assembles the taylor_m-th
                                         // k-derivative (corner rules only)
     const double *k_dev = nullptr;      // device (re, im): the kernels read k here instead
