@@ -881,8 +881,7 @@ void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
     c.fx_ok = true;
 }
 
-bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df_trig) {
-    AssembleArgs a = args;
+bool fix64_covers(const Ctx &c, const AssembleArgs &a) {
     if (!c.fx_ok || a.taylor_m >= 0 || (a.g_weight && a.g_weight_exp == INT32_MIN)) return false;
     if (a.k_dev && !(a.k_abs_max > 0)) return false;   // no bound on |k|
     const bool cplx = a.k_im != 0.0;
@@ -891,7 +890,13 @@ bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df_trig) {
     // fixed-point ranges for many pairs stay with the FP64 kernel
     const double bound = a.k_dev ? a.k_abs_max : 0.0, len = std::ldexp(1.0, c.fx_exp);
     const double kr = std::max(std::fabs(a.k_re), bound) * len, ki = cplx ? std::max(std::fabs(a.k_im), bound) * len : 0.0;
-    if (!(kr < 500.0) || !(ki < 100.0) || !(ki * c.fx_rho_max * 1.45 < fix64::kMaxDampSpread)) return false;
+    return kr < 500.0 && ki < 100.0 && ki * c.fx_rho_max * 1.45 < fix64::kMaxDampSpread;
+}
+
+bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df_trig) {
+    if (!fix64_covers(c, args)) return false;
+    AssembleArgs a = args;
+    const bool cplx = a.k_im != 0.0;
     // C at points off the surface cancels to the quadrature error, where any other
     // rounding would show: it keeps the FP64 (double-float) operations
     const bool nodes = a.targets >= c.d_sources && a.targets + 3 * a.M <= c.d_sources + 3 * c.n_sources;
@@ -944,7 +949,10 @@ bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df_trig) {
     // 362 nodes with 16-point rules 0.22 / 0.29 / 0.40.
     int level = 0;
     while (level + 1 < kMaxLevels && (c.n_elements >> (level + 1)) >= 4) ++level;
-    const LaunchShape base{level, 1, kThreads};   // (records are read through L1: no chunks)
+    // (records are read through L1: the chunk is the double-float kernel's, which
+    // shares the tuned shape)
+    const int chunk0 = (int)std::max<size_t>(1, std::min<size_t>(32, (32u << 10) / ((size_t)c.dlay.stride * sizeof(float))));
+    const LaunchShape base{level, chunk0, kThreads};
     ShapeAxes ax;
     for (int l = level - 1; l <= level + 1; ++l)
         if (l >= 0 && l < kMaxLevels && (int64_t(1) << l) <= c.n_elements) ax.levels.push_back(l);

@@ -597,6 +597,7 @@ bool launch_assemble_k9(Ctx &c, const AssembleArgs &a);   // the double-float ke
 // FP64 integrals of the near pairs (BIE_PREC_DF64).
 void build_fix64_records(Ctx &c, const std::vector<double> &rec64);
 bool launch_assemble_fix64(Ctx &c, const AssembleArgs &a, bool df_trig);
+bool fix64_covers(const Ctx &c, const AssembleArgs &a);   // whether it launches
 
 // FMA throughput probe (bie_peaks.cu)
 void measure_peaks(int device, bie_peaks &out);

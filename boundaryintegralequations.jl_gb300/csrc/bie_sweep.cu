@@ -245,12 +245,16 @@ struct MeshRun {
 
     // assembly of one wavenumber (k_re, k_im; or from device memory kd, with k_im
     // only selecting the complex-k code path)
-    void assemble(double kr, double ki, const double *kd) {
+    AssembleArgs assemble_args(double kr, double ki, const double *kd) const {
         AssembleArgs a{kr, ki, c.d_sources, N, BIE_F | BIE_G | BIE_C, F.as<double>(), G.as<double>(),
                        reinterpret_cast<double *>(Cv)};
         a.c64_out = mixed;
         a.k_dev = kd;
         a.k_abs_max = kmax;
+        return a;
+    }
+    void assemble(double kr, double ki, const double *kd) {
+        const AssembleArgs a = assemble_args(kr, ki, kd);
         if (mixed) launch_assemble_mixed(c, a);
         else if (!(df64 && launch_assemble_df64(c, a))) launch_assemble_fp64(c, a);
     }
@@ -281,6 +285,14 @@ struct MeshRun {
         BIE_CUDA(cudaEventElapsedTime(&tsv, e[1], e[2]));
         asm_ms += ta;
         sol_ms += tsv;
+    }
+    // The recorded assembly bounds Re k and Im k by the sweep's largest |k|, so it can
+    // take another kernel than the first wavenumber did: that kernel runs once
+    // before the recording, which sizes its scratch.
+    void size_recorded(const double *ks, bool cplx) {
+        const double ki = cplx ? 1.0 : 0.0;
+        if (!mixed && fix64_covers(c, assemble_args(ks[0], ks[1], nullptr)) != fix64_covers(c, assemble_args(0.0, ki, ks_d)))
+            assemble(0.0, ki, ks_d);
     }
     // amp[j] from y and A z
     void finish_probe(const int *jdev, int jhost) {
@@ -486,6 +498,7 @@ void run_sweep(Ctx *const *ctxs, int nmesh, const double *ks, int nk, const doub
         runs.push_back(std::make_unique<MeshRun>(c, nk, ks, w[m], o));
         for (int j = 0; j < nk; ++j) runs.back()->kmax = std::max(runs.back()->kmax, std::hypot(ks[2 * j], ks[2 * j + 1]));
         runs.back()->eager(0, ks, ev.e);   // sizes the scratch, tunes the slicing
+        runs.back()->size_recorded(ks, cplx);
     }
     GraphScope gs(uniq);
     const auto t0 = std::chrono::steady_clock::now();
