@@ -184,3 +184,37 @@ def test_gmres_host_entry_matrix_free_and_not_converged():
     # maxiter reached: x is still returned with the info filled, as gmres does
     x3, r3 = gmres(Diagonal(1.0 - C) - Ff, b, maxiter=2, log=True)
     assert not r3.converged and r3.iterations == 2 and np.all(np.isfinite(x3))
+
+
+@pytest.mark.parametrize("f", [1, 2, 5, 6, 9])
+@pytest.mark.parametrize("kind", ["plain", "wide rows", "rising", "tiny"])
+def test_dense_product_error(f, kind):
+    """Residual |b - A x0| of an exact right-hand side: the rounding error of the
+    dense complex128 product.  Rows of 12 to 812 columns; "wide rows" scale rows
+    and columns over 1e+-150, "rising" lets each row grow by 2^40 from its first
+    column to its last, "tiny" reaches subnormals and holds zero rows.
+
+    Bound: at most 64 slice sums, n / 64 block sums and 8 further roundings of
+    2^-53 each on the absolute row sums."""
+    mesh = bm.icosphere(f)
+    n = mesh.n_sources
+    r = np.random.default_rng(n)
+    A = r.normal(size=(n, n)) + 1j * r.normal(size=(n, n))
+    x = rand_c(n, 5)
+    if kind == "wide rows":
+        s = 10.0 ** r.uniform(-150, 150, n)
+        A = A * s[None, :]
+        x = x / s
+        A *= 10.0 ** r.uniform(-100, 0, n)[:, None]
+    elif kind == "rising":
+        A *= 2.0 ** np.linspace(-40, 0, n)[None, :]
+    elif kind == "tiny":
+        A *= 10.0 ** r.uniform(-320, 0, n)[:, None]
+        A[::5] = 0
+    ctx = biegpu.get_context(mesh, n=2, m=2)
+    L = np.clongdouble
+    b = (A.astype(L) @ x.astype(L)).astype(np.complex128)
+    bound = (64 + n / 64 + 8) * 2.0 ** -53 * np.linalg.norm(np.abs(A) @ np.abs(x))
+    x1, res = gmres(A, b, ctx=ctx, x0=x, abstol=np.inf, maxiter=1, log=True)
+    assert np.array_equal(x1, x)
+    assert res.residual_norm <= bound
