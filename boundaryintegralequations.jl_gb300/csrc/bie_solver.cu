@@ -10,8 +10,8 @@
 //
 // Arnoldi uses classical Gram-Schmidt with one reorthogonalisation pass
 // (CGS2, the same numerical role as IterativeSolvers' default DGKS
-// orthogonalisation); the small Hessenberg least-squares problem is solved on
-// the host with Givens rotations (FP64).  Mixed-precision iterative refinement
+// orthogonalisation); the small Hessenberg least-squares problem is solved with
+// Givens rotations on the device (FP64).  Mixed-precision iterative refinement
 // (opts->refine) runs the inner GMRES on the cheaper operator (complex64 dense
 // copy or mixed matrix-free product) and forms the outer residual b - A x with
 // the FP64 operator.
@@ -21,14 +21,12 @@
 
 #include <algorithm>
 #include <cmath>
-#include <complex>
 #include <vector>
 
 namespace bie {
 
 namespace {
 
-using cplx = std::complex<double>;
 constexpr int kT = 256;
 
 // part[s n + i] = sum_j A[i + j n] x[j] (complex128) over the columns of slice
@@ -410,119 +408,228 @@ dense_gemv_c64_rows_kernel(const float2 *__restrict__ A, int64_t n, const double
                                                 dev::f2d(yi.hi) + dev::f2d(yi.lo));
 }
 
-// y = s * sum_slices(part) + d .* x   (d may be null)
-__global__ void combine_kernel(const double2 *__restrict__ part, int S, int64_t n, double2 sc,
-                               const double2 *__restrict__ d, const double2 *__restrict__ x,
-                               double2 *__restrict__ y, const int *__restrict__ stop) {
-    if (stop && *stop) return;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double re = 0, im = 0;
-    for (int s = 0; s < S; ++s) {
-        const double2 p = part[(int64_t)s * n + i];
-        re += p.x;
-        im += p.y;
-    }
-    double yr = sc.x * re - sc.y * im, yi = sc.x * im + sc.y * re;
-    if (d) {
-        const double2 dv = d[i], xv = x[i];
-        yr += dv.x * xv.x - dv.y * xv.y;
-        yi += dv.x * xv.y + dv.y * xv.x;
-    }
-    y[i] = make_double2(yr, yi);
+// ---- vector work of an Arnoldi step -------------------------------------------
+// Between two products a step sums the product's slices, runs two Gram-Schmidt
+// passes over the basis and normalises.  The vectors are short (77 KB at 4842
+// nodes) and live in L2, so launches and the FP64 pipe bound them: a warp waits
+// 62 cycles for each FP64 operation whatever its parallelism (measured; 16 cycles
+// per warp operation and SM), and a launch costs about 2 us.  The step is four
+// launches: each block owns a range of rows, keeps them through a launch, and
+// takes for itself the sums of the partial sums that the launch before left per
+// block (152 blocks at most), instead of a launch for each.  Threads work
+// on real components, not complex numbers: half the operations in a row for each
+// warp, and a warp per scheduler is enough to keep the pipe busy.
+// 2562 nodes, 8 to 13 columns, 64 slices: 26 us a step in 4 launches; with one
+// launch per sum, update and rotation 75 us in 7.  Solves of 8 wavenumbers (refined,
+// with a sensitivity probe) 13.8 -> 7.6 ms.
+constexpr int kRedBlocks = 152;   // most blocks of a vector kernel: one per SM
+constexpr int kHs = 32;           // columns whose sums a block takes itself
+constexpr int kVT = 128;          // threads where a block has few rows,
+constexpr int kVTLong = 512;      // ... and many
+constexpr int kLongRows = 128;
+struct RowSplit {
+    int64_t rows;   // per block, a multiple of 32
+    int nb;
+};
+inline RowSplit row_split(int64_t n) {
+    const int64_t rows = 32 * std::max<int64_t>(1, (n + 32 * kRedBlocks - 1) / (32 * kRedBlocks));
+    return RowSplit{rows, (int)((n + rows - 1) / rows)};
 }
+// (a complex vector as components)
+__device__ __forceinline__ const double *comps(const double2 *p) { return reinterpret_cast<const double *>(p); }
+__device__ __forceinline__ double *comps(double2 *p) { return reinterpret_cast<double *>(p); }
 
-// partial[col * nb + block] = sum over the block's rows of conj(V[:, col]) . w
-__global__ void __launch_bounds__(kT)
-multidot_kernel(const double2 *__restrict__ V, int64_t ldv, const double2 *__restrict__ w,
-                int64_t n, double2 *__restrict__ partial, const int *__restrict__ stop) {
-    if (stop && *stop) return;
-    const int col = blockIdx.y;
-    const double2 *v = V + (int64_t)col * ldv;
-    double re = 0, im = 0;
-    for (int64_t i = (int64_t)blockIdx.x * kT + threadIdx.x; i < n; i += (int64_t)gridDim.x * kT) {
-        const double2 a = v[i], b = w[i];
-        re += a.x * b.x + a.y * b.y;
-        im += a.x * b.y - a.y * b.x;
-    }
-    __shared__ double sr[kT], si[kT];
-    sr[threadIdx.x] = re;
-    si[threadIdx.x] = im;
-    __syncthreads();
-    for (int o = kT / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) {
-            sr[threadIdx.x] += sr[threadIdx.x + o];
-            si[threadIdx.x] += si[threadIdx.x + o];
+// done(i, sum over the groups g of term(i, g), the same of the row's other
+// component) for the components i of rows r0 .. r1; two groups share the terms
+// where the rows are few
+template <int T>
+constexpr int kGroups = T == kVT ? 2 : 1;
+template <int T, typename Term, typename Done>
+__device__ __forceinline__ void over_rows(int64_t r0, int64_t r1, double *red, Term term, Done done) {
+    constexpr int G = kGroups<T>, RC = T / G;
+    const int lane = threadIdx.x % RC, g = threadIdx.x / RC;
+    for (int64_t base = 2 * r0; base < 2 * r1; base += RC) {
+        const int64_t i = base + lane;
+        double acc = i < 2 * r1 ? term(i, g) : 0.0;
+        if (G > 1) {
+            __syncthreads();
+            if (g > 0) red[lane] = acc;
+            __syncthreads();
+            if (g == 0) acc += red[lane];
         }
+        const double other = __shfl_xor_sync(0xffffffffu, acc, 1);
+        if (g == 0 && i < 2 * r1) done(i, acc, other);
+    }
+}
+
+// sum over groups of L neighbouring lanes (L a power of two up to 32)
+__device__ __forceinline__ double lane_sum(double v, int L) {
+    for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// lanes per component for ncol columns: the block's threads spread over them
+template <int T>
+__device__ __forceinline__ int lanes_per(int ncol) {
+    int L = 32;
+    while (L > 1 && L * 2 * ncol > T) L >>= 1;
+    return L;
+}
+
+// partial[c nb + block] = sum over rows r0 .. r1 of conj(V[:, c]) w
+template <int T>
+__device__ __forceinline__ void block_dots(const double2 *__restrict__ V, int64_t ldv, int ncol, const double2 *w,
+                                           int64_t r0, int64_t r1, double2 *__restrict__ partial, int nb) {
+    const int L = lanes_per<T>(ncol), lane = threadIdx.x % L;
+    for (int q0 = 0; q0 < 2 * ncol; q0 += T / L) {
+        const int q = q0 + threadIdx.x / L, c = q >> 1;
+        const bool im = q & 1;
+        double s = 0;
+        if (q < 2 * ncol) {
+            const double2 *v = V + (int64_t)c * ldv;
+#pragma unroll 8
+            for (int64_t i = r0 + lane; i < r1; i += L) {
+                const double2 a = v[i], b = w[i];
+                s = fma(a.x, im ? b.y : b.x, s);
+                s = fma(im ? -a.y : a.y, im ? b.x : b.y, s);
+            }
+        }
+        s = lane_sum(s, L);
+        if (lane == 0 && q < 2 * ncol) comps(partial)[2 * ((int64_t)c * nb + blockIdx.x) + (q & 1)] = s;
+    }
+}
+// h[c] = sum of column c's nb partial sums, by the whole block
+template <int T>
+__device__ __forceinline__ void block_sums(const double2 *__restrict__ partial, int nb, int ncol, double2 *h) {
+    const int L = lanes_per<T>(ncol), lane = threadIdx.x % L;
+    for (int q0 = 0; q0 < 2 * ncol; q0 += T / L) {
+        const int q = q0 + threadIdx.x / L;
+        double s = 0;
+        if (q < 2 * ncol) {
+            const double *p = comps(partial) + 2 * (int64_t)(q >> 1) * nb + (q & 1);
+#pragma unroll 16
+            for (int b = lane; b < nb; b += L) s += p[2 * b];
+        }
+        s = lane_sum(s, L);
+        if (lane == 0 && q < 2 * ncol) comps(h)[q] = s;
+    }
+}
+// sum of the squares of one value per thread -> partial[block]
+template <int T>
+__device__ __forceinline__ void block_norm(double s, double *red, double *__restrict__ partial) {
+    s = lane_sum(s, 32);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = red[0];
+        for (int k = 1; k < T / 32; ++k) t += red[k];
+        partial[blockIdx.x] = t;
+    }
+}
+// the squared norm from block_norm's partial sums, in every thread
+__device__ __forceinline__ double block_norm_value(const double *__restrict__ partial, int nb, double *red) {
+    if (threadIdx.x < 32) {
+        double s = 0;
+#pragma unroll
+        for (int k = 0; k <= kRedBlocks / 32; ++k) {
+            const int b = threadIdx.x + k * 32;
+            if (k * 32 < nb) s += b < nb ? partial[b] : 0.0;
+        }
+        s = lane_sum(s, 32);
+        if (threadIdx.x == 0) red[0] = s;
+    }
+    __syncthreads();
+    return fmax(red[0], 0.0);
+}
+
+// A product that is still in slices: y = sc sum_s part[s n + i] + d .* x (d may
+// be null; part may be y if S == 1); S == 0: y already holds it.
+struct Sliced {
+    const double2 *part = nullptr;
+    int S = 0;
+    double2 sc = {1.0, 0.0};
+    const double2 *d = nullptr, *x = nullptr;
+};
+
+// y = the product (or rhs - product, or rhs where *zero), then what the next
+// launch needs: ncol > 0 the partial dot products with V, ncol < 0 the partial
+// squared norms.
+template <int T>
+__global__ void __launch_bounds__(T)
+gm_product_kernel(Sliced p, int64_t n, int64_t rows, double2 *y, const double2 *__restrict__ rhs,
+                  const int *__restrict__ zero, const double2 *__restrict__ V, int ncol, double2 *__restrict__ dots,
+                  double *__restrict__ norms, const int *__restrict__ stop) {
+    if (stop && *stop) return;
+    __shared__ double red[T];
+    const int64_t r0 = (int64_t)blockIdx.x * rows, r1 = min(n, r0 + rows);
+    double nrm = 0;
+    const bool skip = zero && *zero;
+    if (p.S > 0 || rhs || ncol < 0) {
+        over_rows<T>(r0, r1, red,
+            [&](int64_t i, int g) {
+                double s = 0;
+                if (skip) return s;
+#pragma unroll 16
+                for (int k = g; k < p.S; k += kGroups<T>) s += comps(p.part)[2 * (int64_t)k * n + i];
+                return s;
+            },
+            [&](int64_t i, double s, double o) {
+                const bool im = i & 1;
+                double v;
+                if (skip) {
+                    v = 0;
+                } else if (p.S == 0) {
+                    v = comps(y)[i];
+                } else {
+                    v = fma(im ? p.sc.y : -p.sc.y, o, p.sc.x * s);
+                    if (p.d) {
+                        const double2 dv = p.d[i >> 1], xv = p.x[i >> 1];
+                        v = fma(dv.x, im ? xv.y : xv.x, v);
+                        v = fma(im ? dv.y : -dv.y, im ? xv.x : xv.y, v);
+                    }
+                }
+                if (rhs) v = comps(rhs)[i] - v;
+                if (p.S > 0 || rhs) comps(y)[i] = v;
+                nrm = fma(v, v, nrm);
+            });
+    }
+    if (ncol < 0) block_norm<T>(nrm, red, norms);
+    if (ncol > 0) {
         __syncthreads();
+        block_dots<T>(V, n, ncol, y, r0, r1, dots, gridDim.x);
     }
-    if (threadIdx.x == 0) partial[(int64_t)col * gridDim.x + blockIdx.x] = make_double2(sr[0], si[0]);
 }
 
-__global__ void sum_partials_kernel(const double2 *__restrict__ partial, int nb, int ncol,
-                                    double2 *__restrict__ out, const int *__restrict__ stop) {
+// out[c] = sum of column c's partial sums, one warp per column (bases of more
+// than kHs columns, where each block's own sums would cost more than a launch)
+__global__ void __launch_bounds__(kT)
+sum_partials_kernel(const double2 *__restrict__ partial, int nb, int ncol, double2 *__restrict__ out,
+                    const int *__restrict__ stop) {
     if (stop && *stop) return;
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= ncol) return;
+    const int c = blockIdx.x * (kT / 32) + threadIdx.x / 32;
     double re = 0, im = 0;
-    for (int b = 0; b < nb; ++b) {
-        re += partial[(int64_t)col * nb + b].x;
-        im += partial[(int64_t)col * nb + b].y;
-    }
-    out[col] = make_double2(re, im);
-}
-
-// w -= V[:, 0..ncol) h
-__global__ void gs_update_kernel(const double2 *__restrict__ V, int64_t ldv, int ncol,
-                                 const double2 *__restrict__ h, double2 *__restrict__ w, int64_t n,
-                                 const int *__restrict__ stop) {
-    if (stop && *stop) return;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double re = w[i].x, im = w[i].y;
-    for (int c = 0; c < ncol; ++c) {
-        const double2 v = V[(int64_t)c * ldv + i], hc = h[c];
-        re -= v.x * hc.x - v.y * hc.y;
-        im -= v.x * hc.y + v.y * hc.x;
-    }
-    w[i] = make_double2(re, im);
-}
-
-// y = a - b
-__global__ void sub_kernel(const double2 *__restrict__ a, const double2 *__restrict__ b,
-                           double2 *__restrict__ y, int64_t n) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) y[i] = make_double2(a[i].x - b[i].x, a[i].y - b[i].y);
-}
-
-// x += sum_c V[:, c] yc  (yc in constant-size device array)
-__global__ void combo_add_kernel(const double2 *__restrict__ V, int64_t ldv, int ncol,
-                                 const double2 *__restrict__ yc, double2 *__restrict__ x, int64_t n) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double re = x[i].x, im = x[i].y;
-    for (int c = 0; c < ncol; ++c) {
-        const double2 v = V[(int64_t)c * ldv + i], y = yc[c];
-        re += v.x * y.x - v.y * y.y;
-        im += v.x * y.y + v.y * y.x;
-    }
-    x[i] = make_double2(re, im);
+    if (c < ncol)
+        for (int b = threadIdx.x & 31; b < nb; b += 32) {
+            re += partial[(int64_t)c * nb + b].x;
+            im += partial[(int64_t)c * nb + b].y;
+        }
+    re = lane_sum(re, 32);
+    im = lane_sum(im, 32);
+    if ((threadIdx.x & 31) == 0 && c < ncol) out[c] = make_double2(re, im);
 }
 
 // ---- device-resident Arnoldi state (one GMRES cycle without host round trips)
 // Layout in one device block: H (m+1) x m, g (m+1), sn (m), h1 (m+1), h2 (m+1),
 // y (m) complex; cs (m) real; scalars.
 struct GmScalars {
-    double2 nrm2;      // output of the last norm reduction (|w|^2 in .x)
     double beta;       // residual norm at the start of the cycle
-    double inv_beta;
-    double inv_hn;     // 1 / h_{j+1,j} of the last step
     double res;        // |g_{j+1}| after the last step
     double tol;
-    int done;          // 1: converged (or breakdown); later kernels of the cycle skip
+    int done;          // 1: converged, breakdown or jmax steps; later kernels of the cycle skip
     int start_ok;      // 1: the starting residual already met the tolerance
     int jdone;         // Arnoldi steps completed in this cycle
-    int pad;
+    int jlast;         // ... in the cycle before
+    int jmax;          // ... at most
 };
 struct GmState {
     double2 *H, *g, *sn, *h1, *h2, *y;
@@ -535,103 +642,244 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
-__device__ __forceinline__ double cabs2(double2 a) { return hypot(a.x, a.y); }
 
-// start of a cycle: beta = |w|, g = (beta, 0, ...), done = beta <= tol
-__global__ void gm_init_kernel(GmState st, double tol) {
-    GmScalars &s = *st.s;
-    s.tol = tol;
-    const double beta = sqrt(fmax(s.nrm2.x, 0.0));
-    s.beta = beta;
-    s.res = beta;
-    s.jdone = 0;
-    s.start_ok = beta <= s.tol ? 1 : 0;
-    s.done = s.start_ok;
-    s.inv_beta = beta > 0.0 ? 1.0 / beta : 0.0;
-    for (int k = 0; k <= st.m; ++k) st.g[k] = make_double2(0.0, 0.0);
-    st.g[0] = make_double2(beta, 0.0);
+// out = a w over the block's rows
+__device__ __forceinline__ void scale_rows(const double2 *__restrict__ w, double a, int64_t n, int64_t rows,
+                                           double2 *__restrict__ out) {
+    const int64_t r0 = (int64_t)blockIdx.x * rows, r1 = min(n, r0 + rows);
+#pragma unroll 4
+    for (int64_t i = 2 * r0 + threadIdx.x; i < 2 * r1; i += kVT) comps(out)[i] = a * comps(w)[i];
 }
 
-// Arnoldi step j: column j of H from the two Gram-Schmidt passes and |w|,
-// previous rotations applied, new rotation, residual estimate, stop test.
-// The rotation follows the host form used before (cs real, sn complex).
-__global__ void gm_givens_kernel(GmState st, int j) {
+// state at the start of a cycle: g = (beta, 0, ...), done = beta <= tol
+__device__ __forceinline__ void gm_begin(const GmState &st, double beta, double tol, int jmax) {
     GmScalars &s = *st.s;
-    if (s.done) return;
-    const int ld = st.m + 1;
-    double2 *col = st.H + (int64_t)j * ld;
-    for (int k = 0; k <= j; ++k) col[k] = make_double2(st.h1[k].x + st.h2[k].x, st.h1[k].y + st.h2[k].y);
-    const double hn = sqrt(fmax(s.nrm2.x, 0.0));
-    col[j + 1] = make_double2(hn, 0.0);
-    s.inv_hn = hn > 0.0 ? 1.0 / hn : 0.0;
-    for (int k = 0; k < j; ++k) {
-        const double c = st.cs[k];
-        const double2 sn = st.sn[k];
-        const double2 a = col[k], b = col[k + 1];
-        const double2 t = make_double2(c * a.x + cmul(sn, b).x, c * a.y + cmul(sn, b).y);
-        const double2 u = cmul(cconj(sn), a);
-        col[k + 1] = make_double2(-u.x + c * b.x, -u.y + c * b.y);
-        col[k] = t;
+    for (int k = threadIdx.x; k <= st.m; k += kVT) st.g[k] = make_double2(k ? 0.0 : beta, 0.0);
+    if (threadIdx.x > 0) return;
+    s.tol = tol;
+    s.beta = beta;
+    s.res = beta;
+    s.jlast = s.jdone;
+    s.jdone = 0;
+    s.jmax = jmax;
+    s.start_ok = beta <= tol ? 1 : 0;
+    s.done = s.start_ok;
+}
+
+// start of a cycle: beta from the partial squared norms, V_0 = w / beta; the
+// last block keeps the state
+__global__ void __launch_bounds__(kVT)
+gm_start_kernel(GmState st, double tol, const double *__restrict__ norms, int nb, const double2 *__restrict__ w,
+                int64_t n, int64_t rows, double2 *__restrict__ v0) {
+    __shared__ double red[1];
+    const double beta = sqrt(block_norm_value(norms, nb, red));
+    if (blockIdx.x == nb) {
+        gm_begin(st, beta, tol, st.m);   // (the host ends the cycle)
+        return;
     }
-    // rotation zeroing col[j + 1]
-    const double2 a = col[j], b = col[j + 1];
-    const double na = cabs2(a), nb = cabs2(b);
-    double c;
+    scale_rows(w, beta > 0.0 ? 1.0 / beta : 0.0, n, rows, v0);
+}
+
+// Column j of H before its last rotation: the two passes' coefficients with the
+// rotations of the columns before applied.  Each rotation is one pass of four
+// lanes of a warp (the two components of both results): three FP64 operations
+// in a row instead of twelve.
+template <int T>
+__device__ __forceinline__ void gm_rotate_column(const GmState &st, int j, const double2 *h2) {
+    __shared__ double2 s_col[kHs + 1], s_sn[kHs + 1];
+    __shared__ double s_cs[kHs + 1];
+    double2 *out = st.H + (int64_t)j * (st.m + 1);
+    const bool small = j < kHs;
+    double2 *col = small ? s_col : out;
+    const double2 *sn = small ? s_sn : st.sn;
+    const double *cs = small ? s_cs : st.cs;
+    for (int k = threadIdx.x; k <= j; k += T) {
+        col[k] = make_double2(st.h1[k].x + h2[k].x, st.h1[k].y + h2[k].y);
+        if (small && k < j) {
+            s_sn[k] = st.sn[k];
+            s_cs[k] = st.cs[k];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        // lanes 0, 1: the components of -conj(sn) a + c b, which the next rotation
+        // takes; lanes 2, 3: those of c a + sn b, the finished entry
+        const bool im = threadIdx.x & 1, fin = threadIdx.x & 2;
+        double2 a = col[0];
+        for (int k = 0; k < j; ++k) {
+            const double2 b = col[k + 1], s = sn[k];
+            const double c = cs[k];
+            const double2 p = fin ? a : b, q = fin ? b : a;
+            double v = c * (im ? p.y : p.x);
+            v = fma(fin ? s.x : -s.x, im ? q.y : q.x, v);
+            v = fma(im ? s.y : -s.y, im ? q.x : q.y, v);
+            if (fin) comps(col)[2 * k + im] = v;
+            a = make_double2(__shfl_sync(0xfu, v, 0), __shfl_sync(0xfu, v, 1));
+        }
+        if (threadIdx.x == 0) col[j] = a;
+    }
+    __syncthreads();
+    if (small)
+        for (int k = threadIdx.x; k <= j; k += T) out[k] = col[k];
+}
+
+// w -= V h (ncol columns, h the sums of dots_in, or hsum already summed), then
+// the partial dot products with V (first pass) or, LAST, the partial squared
+// norms.  The first pass stores h in h1; in the last one a further block applies
+// the earlier rotations to the new column of H.
+template <int T, bool LAST>
+__global__ void __launch_bounds__(T)
+gm_update_kernel(GmState st, const double2 *__restrict__ V, int ncol, const double2 *__restrict__ dots_in,
+                 const double2 *__restrict__ hsum, int nb, double2 *w, int64_t n, int64_t rows,
+                 double2 *__restrict__ dots_out, double *__restrict__ norms, const int *__restrict__ stop) {
+    if (stop && *stop) return;
+    __shared__ double red[T];
+    __shared__ double2 hs[kHs];
+    const double2 *h = hsum;
+    if (!hsum) {
+        block_sums<T>(dots_in, nb, ncol, hs);
+        __syncthreads();
+        h = hs;
+        if (!LAST && blockIdx.x == 0 && threadIdx.x < ncol) st.h1[threadIdx.x] = hs[threadIdx.x];
+    }
+    if (LAST && blockIdx.x == nb) {
+        gm_rotate_column<T>(st, ncol - 1, h);
+        return;
+    }
+    const int64_t r0 = (int64_t)blockIdx.x * rows, r1 = min(n, r0 + rows);
+    double nrm = 0;
+    over_rows<T>(r0, r1, red,
+        [&](int64_t i, int g) {
+            const bool im = i & 1;
+            double s = 0;
+#pragma unroll 8
+            for (int c = g; c < ncol; c += kGroups<T>) {
+                const double2 v = V[(int64_t)c * n + (i >> 1)], hc = h[c];
+                s = fma(v.x, im ? hc.y : hc.x, s);
+                s = fma(im ? v.y : -v.y, im ? hc.x : hc.y, s);
+            }
+            return s;
+        },
+        [&](int64_t i, double s, double) {
+            const double v = comps(w)[i] - s;
+            comps(w)[i] = v;
+            if (LAST) nrm = fma(v, v, nrm);
+        });
+    if (LAST) {
+        block_norm<T>(nrm, red, norms);
+    } else {
+        __syncthreads();
+        block_dots<T>(V, n, ncol, w, r0, r1, dots_out, nb);
+    }
+}
+
+// The last rotation of Arnoldi step j, residual estimate and stop test (cs
+// real, sn complex), by one block: a = col[j] of H, hn2 = |w|^2.  Warps share the
+// square roots, whose FP64 operations no warp can overlap.  The squares are
+// those of norms taken as roots of a sum of squares, so a scaled hypot would not
+// widen the range; |g_j| is the residual before the step.
+__device__ __forceinline__ void gm_givens(const GmState &st, int j, const double *__restrict__ norms, int nb) {
+    __shared__ double red[1], s_na2, s_ia, s_rh;
+    GmScalars &s = *st.s;
+    double2 *col = st.H + (int64_t)j * (st.m + 1);
+    const double2 a = col[j], gj = st.g[j];   // (and g_{j+1} = 0)
+    if (threadIdx.x == 32) {
+        s_na2 = fma(a.x, a.x, a.y * a.y);
+        s_ia = rsqrt(s_na2);
+    }
+    const double hn2 = block_norm_value(norms, nb, red), na2 = s_na2, ia = s_ia;
+    if (threadIdx.x == 32) s_rh = rsqrt(hn2);
+    double in = 0;
+    if (threadIdx.x == 0) in = rsqrt(na2 + hn2);
+    __syncthreads();
+    if (threadIdx.x > 0) return;
+    double c, q;
     double2 sn, r;
-    if (nb == 0.0) {
+    if (hn2 == 0.0) {
         c = 1.0;
+        q = 0.0;
         sn = make_double2(0.0, 0.0);
         r = a;
-    } else if (na == 0.0) {
+    } else if (na2 == 0.0) {
         c = 0.0;
-        sn = make_double2(b.x / nb, -b.y / nb);
-        r = make_double2(nb, 0.0);
+        q = 1.0;
+        sn = make_double2(1.0, 0.0);
+        r = make_double2(hn2 * s_rh, 0.0);
     } else {
-        const double nrm = hypot(na, nb);
-        const double2 alpha = make_double2(a.x / na, a.y / na);
-        c = na / nrm;
-        const double2 t = cmul(alpha, cconj(b));
-        sn = make_double2(t.x / nrm, t.y / nrm);
-        r = make_double2(alpha.x * nrm, alpha.y * nrm);
+        c = na2 * ia * in;
+        q = hn2 * s_rh * in;
+        const double t = q * ia, u = (na2 + hn2) * in * ia;
+        sn = make_double2(a.x * t, a.y * t);
+        r = make_double2(a.x * u, a.y * u);
     }
+    const double res = s.res * q;
+    s.res = res;
+    s.jdone = j + 1;
+    if (res <= s.tol || hn2 == 0.0 || j + 1 >= s.jmax) s.done = 1;
     st.cs[j] = c;
     st.sn[j] = sn;
     col[j] = r;
     col[j + 1] = make_double2(0.0, 0.0);
-    const double2 gj = st.g[j], gj1 = st.g[j + 1];
-    const double2 sg = cmul(sn, gj1);
     const double2 ug = cmul(cconj(sn), gj);
-    st.g[j] = make_double2(c * gj.x + sg.x, c * gj.y + sg.y);
-    st.g[j + 1] = make_double2(-ug.x + c * gj1.x, -ug.y + c * gj1.y);
-    s.res = cabs2(st.g[j + 1]);
-    s.jdone = j + 1;
-    if (s.res <= s.tol || hn == 0.0) s.done = 1;
+    st.g[j] = make_double2(c * gj.x, c * gj.y);
+    st.g[j + 1] = make_double2(-ug.x, -ug.y);
 }
 
-// y = R^{-1} g over the jdone columns (back substitution)
-__global__ void gm_trisolve_kernel(GmState st) {
-    const int j = st.s->jdone;
-    const int ld = st.m + 1;
-    for (int k = j - 1; k >= 0; --k) {
-        double2 acc = st.g[k];
-        for (int l = k + 1; l < j; ++l) {
-            const double2 t = cmul(st.H[(int64_t)l * ld + k], st.y[l]);
-            acc.x -= t.x;
-            acc.y -= t.y;
-        }
-        const double2 d = st.H[(int64_t)k * ld + k];
-        const double den = d.x * d.x + d.y * d.y;
-        st.y[k] = make_double2((acc.x * d.x + acc.y * d.y) / den, (acc.y * d.x - acc.x * d.y) / den);
+// V_{j+1} = w / |w|, and in a further block the state of step j.  (A block that
+// already sees the flag which that block raises skips a vector nothing reads.)
+__global__ void __launch_bounds__(kVT)
+gm_finish_kernel(GmState st, int j, const double *__restrict__ norms, int nb, const double2 *__restrict__ w, int64_t n,
+                 int64_t rows, double2 *__restrict__ vn) {
+    __shared__ double red[1];
+    if (__syncthreads_or(threadIdx.x == 0 && *static_cast<volatile int *>(&st.s->done))) return;
+    if (blockIdx.x == nb) {
+        gm_givens(st, j, norms, nb);
+        return;
     }
+    const double hn2 = block_norm_value(norms, nb, red);
+    scale_rows(w, hn2 > 0.0 ? rsqrt(hn2) : 0.0, n, rows, vn);
 }
 
-// y = x * (*alpha) (alpha real, on the device)
-__global__ void scale_dev_kernel(const double2 *__restrict__ x, const double *__restrict__ alpha,
-                                 double2 *__restrict__ y, int64_t n, const int *__restrict__ stop) {
-    if (stop && *stop) return;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const double a = *alpha;
-    if (i < n) y[i] = make_double2(a * x[i].x, a * x[i].y);
+// y = R^{-1} g over the jdone columns (back substitution by columns, one warp)
+__global__ void __launch_bounds__(32) gm_trisolve_kernel(GmState st) {
+    constexpr int kS = 32;
+    __shared__ double2 s_y[kS], s_R[kS * kS];
+    const int j = st.s->jdone, ld = st.m + 1, lane = threadIdx.x;
+    const bool small = j <= kS;
+    double2 *y = small ? s_y : st.y;
+    const double2 *R = small ? s_R : st.H;
+    const int ldr = small ? kS : ld;
+    for (int k = lane; k < j; k += 32) y[k] = st.g[k];
+    if (small && lane < j)
+#pragma unroll 8
+        for (int k = 0; k < j; ++k) s_R[k * kS + lane] = st.H[(int64_t)k * ld + lane];
+    __syncwarp();
+    double2 inv = make_double2(0.0, 0.0);   // 1 / R(lane, lane)
+    if (small && lane < j) {
+        const double2 d = R[(int64_t)lane * ldr + lane];
+        const double i = 1.0 / fma(d.x, d.x, d.y * d.y);
+        inv = make_double2(d.x * i, -d.y * i);
+    }
+    for (int k = j - 1; k >= 0; --k) {
+        double2 ik;
+        if (small) {
+            ik = make_double2(__shfl_sync(0xffffffffu, inv.x, k), __shfl_sync(0xffffffffu, inv.y, k));
+        } else {
+            const double2 d = R[(int64_t)k * ldr + k];
+            const double den = fma(d.x, d.x, d.y * d.y);
+            ik = make_double2(d.x / den, -d.y / den);
+        }
+        const double2 yk = cmul(y[k], ik);
+        __syncwarp();
+        if (lane == 0) y[k] = yk;
+        for (int l = lane; l < k; l += 32) {
+            const double2 t = cmul(R[(int64_t)k * ldr + l], yk);
+            y[l] = make_double2(y[l].x - t.x, y[l].y - t.y);
+        }
+        __syncwarp();
+    }
+    if (small)
+        for (int k = lane; k < j; k += 32) st.y[k] = y[k];
 }
 
 // x += V[:, 0..*ncol) yc  (column count on the device)
@@ -641,6 +889,7 @@ __global__ void combo_add_dev_kernel(const double2 *__restrict__ V, int64_t ldv,
     if (i >= n) return;
     const int nc = *ncol;
     double re = x[i].x, im = x[i].y;
+#pragma unroll 4
     for (int c = 0; c < nc; ++c) {
         const double2 v = V[(int64_t)c * ldv + i], y = yc[c];
         re += v.x * y.x - v.y * y.y;
@@ -662,24 +911,9 @@ struct RfState {
     int iters, restarts, refinements;
     int outer_zero;        // x == 0: the outer residual is b (its product skipped)
     int inner_zero;        // dx == 0: the cycle residual is the right-hand side
-    int jmax;              // Arnoldi steps allowed in the current cycle
     int steps, cycles;     // loop counters (bounds of the WHILE nodes)
     int pad;
 };
-
-// out = *zero ? r : r - w   (out may be w)
-__global__ void resid_flag_kernel(const double2 *__restrict__ r, const double2 *w, double2 *out, int64_t n,
-                                  const int *__restrict__ zero) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double2 a = r[i];
-    if (*zero) {
-        out[i] = a;
-    } else {
-        const double2 b = w[i];
-        out[i] = make_double2(a.x - b.x, a.y - b.y);
-    }
-}
 
 // x += d
 __global__ void axpy1_kernel(const double2 *__restrict__ d, double2 *__restrict__ x, int64_t n) {
@@ -688,10 +922,13 @@ __global__ void axpy1_kernel(const double2 *__restrict__ d, double2 *__restrict_
 }
 
 // |b| from the norm reduction, tolerance, counters; enter the outer loop
-__global__ void rf_start_kernel(GmState st, RfState *rf, double reltol, double abstol,
-                                cudaGraphConditionalHandle h_outer) {
+__global__ void __launch_bounds__(32)
+rf_start_kernel(RfState *rf, const double *__restrict__ norms, int nb, double reltol, double abstol,
+                cudaGraphConditionalHandle h_outer) {
+    __shared__ double red[1];
+    const double bn = sqrt(block_norm_value(norms, nb, red));
+    if (threadIdx.x > 0) return;
     RfState &r = *rf;
-    const double bn = sqrt(fmax(st.s->nrm2.x, 0.0));
     r = RfState{};
     r.bnorm = bn;
     r.tol = fmax(reltol * bn, abstol);
@@ -704,14 +941,16 @@ __global__ void rf_start_kernel(GmState st, RfState *rf, double reltol, double a
 // Top of an outer pass.  Refinement: the outer residual |b - A x| decides
 // whether another inner solve runs (the host loop of run_gmres); plain GMRES:
 // one pass whose inner solve is the whole solve.
-__global__ void rf_check_kernel(GmState st, RfState *rf, int refine, int maxiter, int max_outer,
-                                double inner_rel, cudaGraphConditionalHandle h_outer,
-                                cudaGraphConditionalHandle h_cycle) {
+__global__ void __launch_bounds__(32)
+rf_check_kernel(RfState *rf, const double *__restrict__ norms, int nb, int refine, int maxiter, int max_outer,
+                double inner_rel, cudaGraphConditionalHandle h_outer, cudaGraphConditionalHandle h_cycle) {
+    __shared__ double red[1];
+    const double res = refine ? sqrt(block_norm_value(norms, nb, red)) : 0.0;
+    if (threadIdx.x > 0) return;
     RfState &r = *rf;
     if (refine) {
         if (!r.outer_zero) r.matvecs += 1;
         r.outer_zero = 0;
-        const double res = sqrt(fmax(st.s->nrm2.x, 0.0));
         r.res = res;
         if (res <= r.tol || r.iters >= maxiter || r.refinements >= max_outer) {
             cudaGraphSetConditional(h_outer, 0u);
@@ -729,41 +968,39 @@ __global__ void rf_check_kernel(GmState st, RfState *rf, int refine, int maxiter
     cudaGraphSetConditional(h_cycle, 1u);
 }
 
-// Start of a restart cycle (gm_init_kernel with the inner tolerance read from
+// Start of a restart cycle (gm_start_kernel with the inner tolerance read from
 // the device); opens the Arnoldi loop unless the true residual already meets it.
-__global__ void gm_cycle_init_kernel(GmState st, RfState *rf, int maxiter, int restart,
-                                     cudaGraphConditionalHandle h_step, cudaGraphConditionalHandle h_sel) {
-    GmScalars &s = *st.s;
-    RfState &r = *rf;
-    s.tol = r.inner_tol;
-    const double beta = sqrt(fmax(s.nrm2.x, 0.0));
-    s.beta = beta;
-    s.res = beta;
-    s.jdone = 0;
-    s.start_ok = beta <= s.tol ? 1 : 0;
-    s.done = s.start_ok;
-    s.inv_beta = beta > 0.0 ? 1.0 / beta : 0.0;
-    for (int k = 0; k <= st.m; ++k) st.g[k] = make_double2(0.0, 0.0);
-    st.g[0] = make_double2(beta, 0.0);
-    if (!r.inner_zero) r.matvecs += 1;
-    r.inner_zero = 0;
-    r.last_beta = beta;
-    r.jmax = min(restart, max(0, maxiter - r.iters));
-    r.steps = 0;
-    cudaGraphSetConditional(h_step, (!s.start_ok && r.jmax > 0) ? 1u : 0u);
-    cudaGraphSetConditional(h_sel, 0u);
+__global__ void __launch_bounds__(kVT)
+gm_cycle_start_kernel(GmState st, RfState *rf, int maxiter, int restart, const double *__restrict__ norms, int nb,
+                      const double2 *__restrict__ w, int64_t n, int64_t rows, double2 *__restrict__ v0,
+                      cudaGraphConditionalHandle h_step, cudaGraphConditionalHandle h_sel) {
+    __shared__ double red[1];
+    const double beta = sqrt(block_norm_value(norms, nb, red));
+    if (blockIdx.x == nb) {
+        RfState &r = *rf;
+        const int jmax = min(restart, max(0, maxiter - r.iters));
+        gm_begin(st, beta, r.inner_tol, jmax);
+        if (threadIdx.x > 0) return;
+        if (!r.inner_zero) r.matvecs += 1;
+        r.inner_zero = 0;
+        r.last_beta = beta;
+        r.steps = 0;
+        cudaGraphSetConditional(h_step, (!st.s->start_ok && jmax > 0) ? 1u : 0u);
+        cudaGraphSetConditional(h_sel, 0u);
+        return;
+    }
+    scale_rows(w, beta > 0.0 ? 1.0 / beta : 0.0, n, rows, v0);
 }
 
-// After each Arnoldi step: the next step index, and whether it runs (not
-// converged, steps left in the cycle; at most `restart` passes)
-__global__ void gm_step_guard_kernel(GmState st, RfState *rf, int restart, cudaGraphConditionalHandle h_step,
+// After each group of Arnoldi steps: the next group, and whether it runs (not
+// converged, steps left in the cycle; at most `groups` passes)
+__global__ void gm_step_guard_kernel(GmState st, RfState *rf, int groups, cudaGraphConditionalHandle h_step,
                                      cudaGraphConditionalHandle h_sel) {
     const GmScalars &s = *st.s;
     RfState &r = *rf;
     r.steps += 1;
-    const int jd = s.jdone;
-    cudaGraphSetConditional(h_step, (!s.done && jd < r.jmax && r.steps < restart) ? 1u : 0u);
-    cudaGraphSetConditional(h_sel, (unsigned)jd);
+    cudaGraphSetConditional(h_step, (!s.done && r.steps < groups) ? 1u : 0u);
+    cudaGraphSetConditional(h_sel, (unsigned)r.steps);
 }
 
 // End of a cycle: tallies; another cycle (whose first action re-checks the true
@@ -821,12 +1058,14 @@ struct Solver {
     Ctx &c;
     int64_t n;
     int m;                        // restart length
-    double2 *part = nullptr;      // gemv slices / multidot partials
-    int nbdot = 1;
-    double2 *hdev = nullptr;      // device scratch for dot results (>= restart + 2)
-    std::vector<double2> hhost;
+    RowSplit rs;                  // rows of the vector kernels' blocks
+    double2 *part = nullptr;      // gemv slices
+    double2 *dot1 = nullptr, *dot2 = nullptr;
+    double *norms = nullptr;      // partial sums of the vector kernels
     GmState st{};                 // device-resident Arnoldi state
     RfState *rf = nullptr;        // device-resident refinement state (graph form)
+    const void *slices_of = nullptr;   // kernel whose slices were asked for last
+    int n_slices = 1;
     const int *stop = nullptr;    // device stop flag honoured by the launches below
     cudaStream_t stream;          // launch stream (a capture stream while recording a graph)
     DevOp *devop = nullptr;       // operator applied through DevOp::apply (else bie_operator)
@@ -835,17 +1074,19 @@ struct Solver {
     Solver(Ctx &ctx, int64_t n_, int restart, int level = 0)
         : c(ctx), n(n_), m(restart), stream(ctx.stream) {
         const int part_slot = level == 0 ? kScratchSolverPart : kScratchSolverNested + 2 * (level - 1) + 1;
-        // dot-product blocks per column; vectors up to 4096 entries take one
-        // block per column, which writes its result directly (no second launch)
-        nbdot = n <= 4096 ? 1 : (int)std::min<int64_t>(std::max<int64_t>(1, (n + kT * 8 - 1) / (kT * 8)), 256);
-        const size_t part_bytes = (size_t)std::max<int64_t>(kMaxSlices * n, (int64_t)(restart + 2) * nbdot) * 16;
-        const size_t hbytes = (size_t)(restart + 2) * 16;
+        rs = row_split(n);
+        const size_t part_bytes = (size_t)kMaxSlices * n * 16;
+        const size_t dot_bytes = (size_t)(restart + 1) * rs.nb * 16;
         const size_t nc = (size_t)(restart + 1) * restart + 4 * (size_t)(restart + 1) + restart;
         const size_t st_bytes = nc * 16 + (size_t)restart * 8 + sizeof(GmScalars) + sizeof(RfState) + 96;
-        char *base = static_cast<char *>(c.scratch(part_slot, part_bytes + hbytes + st_bytes));
+        char *base = static_cast<char *>(
+            c.scratch(part_slot, part_bytes + 2 * dot_bytes + (size_t)rs.nb * 16 + st_bytes));
         part = reinterpret_cast<double2 *>(base);
-        hdev = reinterpret_cast<double2 *>(base + part_bytes);
-        double2 *z = reinterpret_cast<double2 *>(base + part_bytes + hbytes);
+        dot1 = reinterpret_cast<double2 *>(base + part_bytes);
+        dot2 = dot1 + (size_t)(restart + 1) * rs.nb;
+        double2 *z = dot2 + (size_t)(restart + 1) * rs.nb;
+        norms = reinterpret_cast<double *>(z);
+        z += rs.nb;
         st.m = restart;
         st.H = z;
         z += (size_t)(restart + 1) * restart;
@@ -862,16 +1103,24 @@ struct Solver {
         st.cs = reinterpret_cast<double *>(z);
         st.s = reinterpret_cast<GmScalars *>(reinterpret_cast<char *>(st.cs) + (((size_t)restart * 8 + 15) & ~size_t(15)));
         rf = reinterpret_cast<RfState *>(reinterpret_cast<char *>(st.s) + ((sizeof(GmScalars) + 15) & ~size_t(15)));
-        hhost.resize(restart + 2);
     }
 
     void launched() { ++c.kernel_launches; }
 
-    // y = s (K x) + d .* x   (dense kernels skip when *stop is set)
-    void apply(const bie_operator &op, int precision, const double2 *x, double2 *y) {
+    // y = s (K x) + d .* x up to the sum of its slices, which gm_product_kernel
+    // takes (dense kernels skip when *stop is set)
+    // slices of a product kernel over `rows` row threads (asked once per solver)
+    int slices(const void *kern, int64_t rows) {
+        if (kern != slices_of) {
+            slices_of = kern;
+            n_slices = gemv_slices(kern, rows, c.num_sms);
+        }
+        return n_slices;
+    }
+    Sliced product(const bie_operator &op, int precision, const double2 *x, double2 *y) {
         if (devop) {
             devop->apply(x, y, stop);
-            return;
+            return Sliced{};
         }
         const double2 sc = make_double2(op.scale_re, op.scale_im);
         const double2 *d = reinterpret_cast<const double2 *>(op.diag);
@@ -885,36 +1134,34 @@ struct Solver {
                 const bool exact = precision != BIE_PREC_MIXED;
                 if (n % 2 == 0) {
                     if (exact) {
-                        S = gemv_slices((const void *)dense_gemv_c64_exact_kernel, n / 2, c.num_sms);
+                        S = slices((const void *)dense_gemv_c64_exact_kernel, n / 2);
                         dense_gemv_c64_exact_kernel<<<dim3(blocks(n / 2, kT), (unsigned)S), kT, 0, stream>>>(
                             reinterpret_cast<const float4 *>(op.A32), n, x, part, S, stop);
                     } else {
-                        S = gemv_slices((const void *)dense_gemv_c64_kernel, n / 2, c.num_sms);
+                        S = slices((const void *)dense_gemv_c64_kernel, n / 2);
                         dense_gemv_c64_kernel<<<dim3(blocks(n / 2, kT), (unsigned)S), kT, 0, stream>>>(
                             reinterpret_cast<const float4 *>(op.A32), n, x, part, S, stop);
                     }
                 } else {
                     if (exact) {
-                        S = gemv_slices((const void *)dense_gemv_c64_rows_exact_kernel, n, c.num_sms);
+                        S = slices((const void *)dense_gemv_c64_rows_exact_kernel, n);
                         dense_gemv_c64_rows_exact_kernel<<<dim3(blocks(n, kT), (unsigned)S), kT, 0, stream>>>(
                             reinterpret_cast<const float2 *>(op.A32), n, x, part, S, stop);
                     } else {
-                        S = gemv_slices((const void *)dense_gemv_c64_rows_kernel, n, c.num_sms);
+                        S = slices((const void *)dense_gemv_c64_rows_kernel, n);
                         dense_gemv_c64_rows_kernel<<<dim3(blocks(n, kT), (unsigned)S), kT, 0, stream>>>(
                             reinterpret_cast<const float2 *>(op.A32), n, x, part, S, stop);
                     }
                 }
             } else {
-                S = gemv_slices((const void *)dense_gemv_kernel, n, c.num_sms);
+                S = slices((const void *)dense_gemv_kernel, n);
                 dense_gemv_kernel<<<dim3(blocks(n, kT), (unsigned)S), kT, 0, stream>>>(
                     reinterpret_cast<const double2 *>(op.A), n, x, part, S, stop);
             }
             BIE_CUDA(cudaGetLastError());
             c.timer_end(t0);
             launched();
-            combine_kernel<<<blocks(n, 32), 32, 0, stream>>>(part, S, n, sc, d, x, y, stop);
-            BIE_CUDA(cudaGetLastError());
-            launched();
+            return Sliced{part, S, sc, d, x};
         } else {
             // matrix-free F x (or the fast operator) into y, then y = s y + d .* x
             // (these products do not look at the stop flag: the caller checks it
@@ -928,69 +1175,81 @@ struct Solver {
                               nullptr, reinterpret_cast<double *>(y), nullptr, precision};
                 launch_matvec(c, mv);
             }
-            combine_kernel<<<blocks(n), 256, 0, c.stream>>>(y, 1, n, sc, d, x, y, stop);
-            BIE_CUDA(cudaGetLastError());
-            launched();
+            return Sliced{y, 1, sc, d, x};
         }
     }
 
-    // out[0..ncol) = V[:, 0..ncol)^H w on the device (no host copy)
-    void multidot_dev(const double2 *V, int64_t ldv, int ncol, const double2 *w, double2 *out) {
-        dim3 grid((unsigned)nbdot, (unsigned)ncol);
-        multidot_kernel<<<grid, kT, 0, stream>>>(V, ldv, w, n, nbdot == 1 ? out : part, stop);
-        BIE_CUDA(cudaGetLastError());
-        launched();
-        if (nbdot == 1) return;   // partial[col] is the sum already
-        sum_partials_kernel<<<blocks(ncol, 64), 64, 0, stream>>>(part, nbdot, ncol, out, stop);
+    // blocks of few rows or of many (over_rows)
+    bool few() const { return rs.rows < kLongRows; }
+    void finish_product(const Sliced &p, double2 *y, const double2 *rhs, const int *zero, const double2 *V, int ncol) {
+        auto kern = few() ? gm_product_kernel<kVT> : gm_product_kernel<kVTLong>;
+        kern<<<rs.nb, few() ? kVT : kVTLong, 0, stream>>>(p, n, rs.rows, y, rhs, zero, V, ncol, dot1, norms, stop);
         BIE_CUDA(cudaGetLastError());
         launched();
     }
-
-    // out[0..ncol) = V[:, 0..ncol)^H w  (copied to host)
-    void multidot(const double2 *V, int64_t ldv, int ncol, const double2 *w, std::vector<cplx> &out) {
-        multidot_dev(V, ldv, ncol, w, hdev);
-        BIE_CUDA(cudaMemcpyAsync(hhost.data(), hdev, ncol * sizeof(double2), cudaMemcpyDeviceToHost, c.stream));
-        BIE_CUDA(cudaStreamSynchronize(c.stream));
-        out.resize(ncol);
-        for (int k = 0; k < ncol; ++k) out[k] = cplx(hhost[k].x, hhost[k].y);
+    // y = s (K x) + d .* x
+    void apply(const bie_operator &op, int precision, const double2 *x, double2 *y) {
+        const Sliced p = product(op, precision, x, y);
+        if (p.S > 0) finish_product(p, y, nullptr, nullptr, nullptr, 0);
+    }
+    // w = rhs - A x (rhs where *zero, whose product is skipped), partial norms
+    void residual(const bie_operator &op, int precision, const double2 *rhs, const double2 *x, double2 *w,
+                  const int *zero) {
+        stop = zero;
+        const Sliced p = product(op, precision, x, w);
+        stop = nullptr;
+        finish_product(p, w, rhs, zero, nullptr, -1);
     }
 
-    double norm(const double2 *w) {
-        std::vector<cplx> o;
-        multidot(w, n, 1, w, o);
-        return std::sqrt(std::max(o[0].real(), 0.0));
-    }
-
-    void upload_coeffs(const std::vector<cplx> &h) {
-        for (size_t k = 0; k < h.size(); ++k) hhost[k] = make_double2(h[k].real(), h[k].imag());
-        BIE_CUDA(cudaMemcpyAsync(hdev, hhost.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice,
-                                 c.stream));
-    }
-
-    // w -= V[:, 0..ncol) h  with h on the device
-    void gs_update_dev(const double2 *V, int64_t ldv, int ncol, double2 *w, const double2 *h) {
-        gs_update_kernel<<<blocks(n), 256, 0, stream>>>(V, ldv, ncol, h, w, n, stop);
-        BIE_CUDA(cudaGetLastError());
-        launched();
-    }
-
-    void combo_add(const double2 *V, int64_t ldv, int ncol, const std::vector<cplx> &y, double2 *x) {
-        upload_coeffs(y);
-        combo_add_kernel<<<blocks(n), 256, 0, c.stream>>>(V, ldv, ncol, hdev, x, n);
-        BIE_CUDA(cudaGetLastError());
-        launched();
-    }
-
-    void scale_dev(const double2 *x, const double *a, double2 *y) {
-        scale_dev_kernel<<<blocks(n), 256, 0, stream>>>(x, a, y, n, stop);
+    // Arnoldi step j: w = A V_j, orthogonalised against V_0 .. V_j (CGS2), V_{j+1}
+    void arnoldi_step(const bie_operator &op, int precision, double2 *V, double2 *w, int j) {
+        const int nc = j + 1;
+        const Sliced p = product(op, precision, V + (int64_t)j * n, w);
+        finish_product(p, w, nullptr, nullptr, V, nc);
+        for (int pass = 0; pass < 2; ++pass) {
+            const double2 *in = pass ? dot2 : dot1;
+            const double2 *hsum = nullptr;
+            if (nc > kHs) {
+                double2 *h = pass ? st.h2 : st.h1;
+                sum_partials_kernel<<<blocks(nc, kT / 32), kT, 0, stream>>>(in, rs.nb, nc, h, stop);
+                BIE_CUDA(cudaGetLastError());
+                launched();
+                hsum = h;
+            }
+            auto kern = pass ? (few() ? gm_update_kernel<kVT, true> : gm_update_kernel<kVTLong, true>)
+                             : (few() ? gm_update_kernel<kVT, false> : gm_update_kernel<kVTLong, false>);
+            kern<<<rs.nb + pass, few() ? kVT : kVTLong, 0, stream>>>(st, V, nc, in, hsum, rs.nb, w, n, rs.rows, dot2,
+                                                                    norms, stop);
+            BIE_CUDA(cudaGetLastError());
+            launched();
+        }
+        gm_finish_kernel<<<rs.nb + 1, kVT, 0, stream>>>(st, j, norms, rs.nb, w, n, rs.rows, V + (int64_t)nc * n);
         BIE_CUDA(cudaGetLastError());
         launched();
     }
 
-    void sub(const double2 *a, const double2 *b, double2 *y) {
-        sub_kernel<<<blocks(n), 256, 0, stream>>>(a, b, y, n);
+    // x += V y, R y = g
+    void add_solution(const double2 *V, double2 *x) {
+        gm_trisolve_kernel<<<1, 32, 0, stream>>>(st);
         BIE_CUDA(cudaGetLastError());
         launched();
+        combo_add_dev_kernel<<<blocks(n, 64), 64, 0, stream>>>(V, n, &st.s->jdone, st.y, x, n);
+        BIE_CUDA(cudaGetLastError());
+        launched();
+    }
+
+    // partial squared norms of w
+    void norm_partials(const double2 *w) {
+        finish_product(Sliced{}, const_cast<double2 *>(w), nullptr, nullptr, nullptr, -1);
+    }
+    // the norm from these
+    double norm_value() {
+        std::vector<double> h(rs.nb);
+        BIE_CUDA(cudaMemcpyAsync(h.data(), norms, h.size() * sizeof(double), cudaMemcpyDeviceToHost, stream));
+        BIE_CUDA(cudaStreamSynchronize(stream));
+        double s = 0;
+        for (double v : h) s += v;
+        return std::sqrt(std::max(s, 0.0));
     }
 };
 
@@ -1000,8 +1259,8 @@ struct Solver {
 //
 // Each restart cycle runs on the device without host round trips: the
 // Gram-Schmidt coefficients, the Hessenberg column, the Givens rotations and
-// the residual estimate stay in device memory (GmState), a single-thread
-// kernel decides convergence and raises a stop flag, and every later kernel of
+// the residual estimate stay in device memory (GmState), one block of a step
+// decides convergence and raises a stop flag, and every later kernel of
 // the cycle returns at once when it sees the flag.  The host reads the state
 // once per cycle (dense operators) or once per step (matrix-free and fast
 // operators, whose products do not look at the flag).
@@ -1015,46 +1274,35 @@ int gmres_core(Solver &S, const bie_operator &op, int prec, const double2 *b, do
     cudaStream_t stream = S.stream;
     int it = 0, restarts = 0;
     double beta = 0.0;
-    bool first = true;
     GmScalars hs{};
-    while (true) {
+    for (bool first = true;; first = false) {
         // r = b - A x  (r = b for a zero start), beta = |r|
-        S.stop = nullptr;
         if (first && x_zero) {
             BIE_CUDA(cudaMemcpyAsync(w, b, (size_t)n * 16, cudaMemcpyDeviceToDevice, stream));
+            S.stop = nullptr;
+            S.norm_partials(w);
         } else {
-            S.apply(op, prec, x, w);
+            S.residual(op, prec, b, x, w, nullptr);
             ++*matvecs;
-            S.sub(b, w, w);
         }
-        first = false;
-        S.multidot_dev(w, n, 1, w, &st.s->nrm2);
-        gm_init_kernel<<<1, 1, 0, stream>>>(st, tol);
+        gm_start_kernel<<<S.rs.nb + 1, kVT, 0, stream>>>(st, tol, S.norms, S.rs.nb, w, n, S.rs.rows, V);
         BIE_CUDA(cudaGetLastError());
         S.launched();
-        const int jmax = std::min(restart, std::max(0, maxiter - it));
         BIE_CUDA(cudaMemcpyAsync(&hs, st.s, sizeof(GmScalars), cudaMemcpyDeviceToHost, stream));
         BIE_CUDA(cudaStreamSynchronize(stream));
+        if (!first) {
+            it += hs.jlast;
+            *matvecs += hs.jlast;
+            ++restarts;
+        }
+        const int jmax = std::min(restart, std::max(0, maxiter - it));
         if (hs.start_ok || jmax == 0) {
             beta = hs.beta;
             break;
         }
         S.stop = stop_flag;
-        S.scale_dev(w, &st.s->inv_beta, V);
         for (int j = 0; j < jmax; ++j) {
-            const double2 *vj = V + (int64_t)j * n;
-            double2 *vn = V + (int64_t)(j + 1) * n;
-            S.apply(op, prec, vj, w);
-            // CGS2
-            S.multidot_dev(V, n, j + 1, w, st.h1);
-            S.gs_update_dev(V, n, j + 1, w, st.h1);
-            S.multidot_dev(V, n, j + 1, w, st.h2);
-            S.gs_update_dev(V, n, j + 1, w, st.h2);
-            S.multidot_dev(w, n, 1, w, &st.s->nrm2);
-            gm_givens_kernel<<<1, 1, 0, stream>>>(st, j);
-            BIE_CUDA(cudaGetLastError());
-            S.launched();
-            S.scale_dev(w, &st.s->inv_hn, vn);
+            S.arnoldi_step(op, prec, V, w, j);
             // the host looks at the stop flag after every step for operators whose
             // products ignore it, every kCheck steps for dense ones (at most
             // kCheck - 1 skipped steps are queued after convergence)
@@ -1066,19 +1314,8 @@ int gmres_core(Solver &S, const bie_operator &op, int prec, const double2 *b, do
                 if (done) break;
             }
         }
-        // x += V y,  R y = g
         S.stop = nullptr;
-        gm_trisolve_kernel<<<1, 1, 0, stream>>>(st);
-        BIE_CUDA(cudaGetLastError());
-        combo_add_dev_kernel<<<blocks(n), 256, 0, stream>>>(V, n, &st.s->jdone, st.y, x, n);
-        BIE_CUDA(cudaGetLastError());
-        S.launched();
-        S.launched();
-        BIE_CUDA(cudaMemcpyAsync(&hs, st.s, sizeof(GmScalars), cudaMemcpyDeviceToHost, stream));
-        BIE_CUDA(cudaStreamSynchronize(stream));
-        it += hs.jdone;
-        *matvecs += hs.jdone;
-        ++restarts;
+        S.add_solution(V, x);
     }
     *res_out = beta;
     *restarts_out = restarts;
@@ -1119,6 +1356,8 @@ void graph_add_conditional(cudaStream_t s, cudaGraphConditionalHandle h, cudaGra
     for (unsigned i = 0; i < size; ++i) bodies[i] = p.conditional.phGraph_out[i];
 }
 
+constexpr int kStepGroup = 4;   // Arnoldi steps per pass of the graph form's loop
+
 void capture_gmres(Ctx &c, const bie_operator &op, const double *b_, double *x_, const bie_gmres_opts &o,
                    bie_gmres_info *d_info, const cudaStream_t *body) {
     if (op.kind != BIE_OP_DENSE) fail(BIE_ERR_UNSUPPORTED, "graph GMRES needs a dense operator");
@@ -1147,9 +1386,9 @@ void capture_gmres(Ctx &c, const bie_operator &op, const double *b_, double *x_,
     cudaStream_t s0 = c.stream;
 
     BIE_CUDA(cudaMemsetAsync(x, 0, (size_t)n * 16, s0));
-    S.multidot_dev(b, n, 1, b, &st.s->nrm2);
+    S.norm_partials(b);
     const cudaGraphConditionalHandle h_outer = graph_new_handle(s0);
-    rf_start_kernel<<<1, 1, 0, s0>>>(st, rf, reltol, abstol, h_outer);
+    rf_start_kernel<<<1, 32, 0, s0>>>(rf, S.norms, S.rs.nb, reltol, abstol, h_outer);
     BIE_CUDA(cudaGetLastError());
     S.launched();
     cudaGraph_t g_outer;
@@ -1160,20 +1399,14 @@ void capture_gmres(Ctx &c, const bie_operator &op, const double *b_, double *x_,
         BodyCapture bc1(body[0], g_outer);
         S.stream = body[0];
         if (refine) {
-            S.stop = &rf->outer_zero;
-            S.apply(op, o.precision == BIE_PREC_DF64 ? BIE_PREC_DF64 : BIE_PREC_FP64, x, w);
-            S.stop = nullptr;
-            resid_flag_kernel<<<blocks(n), 256, 0, S.stream>>>(b, w, rr, n, &rf->outer_zero);
-            BIE_CUDA(cudaGetLastError());
-            S.launched();
-            S.multidot_dev(rr, n, 1, rr, &st.s->nrm2);
+            S.residual(op, o.precision == BIE_PREC_DF64 ? BIE_PREC_DF64 : BIE_PREC_FP64, b, x, rr, &rf->outer_zero);
             BIE_CUDA(cudaMemsetAsync(dx, 0, (size_t)n * 16, S.stream));
         }
         const double2 *rhs = refine ? rr : b;
         double2 *sol = refine ? dx : x;
         const cudaGraphConditionalHandle h_cycle = graph_new_handle(S.stream);
-        rf_check_kernel<<<1, 1, 0, S.stream>>>(st, rf, refine ? 1 : 0, maxiter, max_outer, inner_rel, h_outer,
-                                                h_cycle);
+        rf_check_kernel<<<1, 32, 0, S.stream>>>(rf, S.norms, S.rs.nb, refine ? 1 : 0, maxiter, max_outer, inner_rel,
+                                                h_outer, h_cycle);
         BIE_CUDA(cudaGetLastError());
         S.launched();
         cudaGraph_t g_cycle;
@@ -1183,59 +1416,43 @@ void capture_gmres(Ctx &c, const bie_operator &op, const double *b_, double *x_,
             // then up to `restart` Arnoldi steps
             BodyCapture bc2(body[1], g_cycle);
             S.stream = body[1];
-            S.stop = &rf->inner_zero;
-            S.apply(op, prec, sol, w);
-            S.stop = nullptr;
-            resid_flag_kernel<<<blocks(n), 256, 0, S.stream>>>(rhs, w, w, n, &rf->inner_zero);
-            BIE_CUDA(cudaGetLastError());
-            S.launched();
-            S.multidot_dev(w, n, 1, w, &st.s->nrm2);
+            S.residual(op, prec, rhs, sol, w, &rf->inner_zero);
             const cudaGraphConditionalHandle h_step = graph_new_handle(S.stream);
             const cudaGraphConditionalHandle h_sel = graph_new_handle(S.stream);
-            gm_cycle_init_kernel<<<1, 1, 0, S.stream>>>(st, rf, maxiter, restart, h_step, h_sel);
+            gm_cycle_start_kernel<<<S.rs.nb + 1, kVT, 0, S.stream>>>(st, rf, maxiter, restart, S.norms, S.rs.nb, w, n,
+                                                                   S.rs.rows, V, h_step, h_sel);
             BIE_CUDA(cudaGetLastError());
             S.launched();
-            S.scale_dev(w, &st.s->inv_beta, V);
             cudaGraph_t g_step;
             graph_add_conditional(S.stream, h_step, cudaGraphCondTypeWhile, 1, &g_step);
             {
-                // one Arnoldi step per pass: a switch over the step index j runs
-                // the body recorded for that j (CGS2 over j + 1 basis vectors)
+                // kStepGroup Arnoldi steps per pass: a switch over the group runs the
+                // body recorded for its steps (CGS2 over j + 1 basis vectors for step
+                // j); steps after the last one skip.  Solves of 8 wavenumbers at 2562
+                // nodes: 7.9 ms with 1 step per pass, 7.8 with 2, 7.6 with 4, 7.7 with 8.
                 BodyCapture bc3(body[2], g_step);
                 S.stream = body[2];
-                std::vector<cudaGraph_t> branch(restart);
-                graph_add_conditional(S.stream, h_sel, cudaGraphCondTypeSwitch, (unsigned)restart, branch.data());
-                gm_step_guard_kernel<<<1, 1, 0, S.stream>>>(st, rf, restart, h_step, h_sel);
+                const int groups = (restart + kStepGroup - 1) / kStepGroup;
+                std::vector<cudaGraph_t> branch(groups);
+                graph_add_conditional(S.stream, h_sel, cudaGraphCondTypeSwitch, (unsigned)groups, branch.data());
+                gm_step_guard_kernel<<<1, 1, 0, S.stream>>>(st, rf, groups, h_step, h_sel);
                 BIE_CUDA(cudaGetLastError());
                 S.launched();
-                for (int j = 0; j < restart; ++j) {
-                    BodyCapture bc4(body[3], branch[j]);
+                S.stop = &st.s->done;
+                for (int g = 0; g < groups; ++g) {
+                    BodyCapture bc4(body[3], branch[g]);
                     S.stream = body[3];
-                    const double2 *vj = V + (int64_t)j * n;
-                    double2 *vn = V + (int64_t)(j + 1) * n;
-                    S.apply(op, prec, vj, w);
-                    S.multidot_dev(V, n, j + 1, w, st.h1);
-                    S.gs_update_dev(V, n, j + 1, w, st.h1);
-                    S.multidot_dev(V, n, j + 1, w, st.h2);
-                    S.gs_update_dev(V, n, j + 1, w, st.h2);
-                    S.multidot_dev(w, n, 1, w, &st.s->nrm2);
-                    gm_givens_kernel<<<1, 1, 0, S.stream>>>(st, j);
-                    BIE_CUDA(cudaGetLastError());
-                    S.launched();
-                    S.scale_dev(w, &st.s->inv_hn, vn);
+                    for (int j = g * kStepGroup; j < std::min(restart, (g + 1) * kStepGroup); ++j)
+                        S.arnoldi_step(op, prec, V, w, j);
                     bc4.end();
                 }
+                S.stop = nullptr;
                 bc3.end();
             }
             S.stream = body[1];
-            gm_trisolve_kernel<<<1, 1, 0, S.stream>>>(st);
-            BIE_CUDA(cudaGetLastError());
-            combo_add_dev_kernel<<<blocks(n), 256, 0, S.stream>>>(V, n, &st.s->jdone, st.y, sol, n);
-            BIE_CUDA(cudaGetLastError());
+            S.add_solution(V, sol);
             gm_cycle_end_kernel<<<1, 1, 0, S.stream>>>(st, rf, maxiter, h_cycle);
             BIE_CUDA(cudaGetLastError());
-            S.launched();
-            S.launched();
             S.launched();
             bc2.end();
         }
@@ -1275,7 +1492,8 @@ void gmres_solve(Ctx &c, const bie_operator &op, DevOp *devop, int64_t n, int le
     double2 *dx = rr + n;
     Solver S(c, n, restart, level);
     S.devop = devop;
-    const double bnorm = S.norm(b);
+    S.norm_partials(b);
+    const double bnorm = S.norm_value();
     const double tol = std::max(reltol * bnorm, abstol);
     if (!o.initially_nonzero) BIE_CUDA(cudaMemsetAsync(x, 0, (size_t)n * 16, c.stream));
     int64_t matvecs = 0;
@@ -1292,10 +1510,9 @@ void gmres_solve(Ctx &c, const bie_operator &op, DevOp *devop, int64_t n, int le
         const int max_outer = o.max_refine > 0 ? o.max_refine : 10;
         bie_operator low = op;
         for (outer = 0; outer < max_outer; ++outer) {
-            S.apply(op, o.precision == BIE_PREC_DF64 ? BIE_PREC_DF64 : BIE_PREC_FP64, x, w);
+            S.residual(op, o.precision == BIE_PREC_DF64 ? BIE_PREC_DF64 : BIE_PREC_FP64, b, x, rr, nullptr);
             ++matvecs;
-            S.sub(b, w, rr);
-            res = S.norm(rr);
+            res = S.norm_value();
             if (res <= tol || iters >= maxiter) break;
             BIE_CUDA(cudaMemsetAsync(dx, 0, (size_t)n * 16, c.stream));
             double ires = 0;
@@ -1303,9 +1520,9 @@ void gmres_solve(Ctx &c, const bie_operator &op, DevOp *devop, int64_t n, int le
             iters += gmres_core(S, low, BIE_PREC_MIXED, rr, dx, true, V, w, restart, maxiter - iters,
                                 std::max(inner_rel * res, tol * 0.5), &ires, &irs, &matvecs);
             restarts += irs;
-            // x += dx
-            std::vector<cplx> one{cplx(1.0, 0.0)};
-            S.combo_add(dx, n, 1, one, x);
+            axpy1_kernel<<<blocks(n), 256, 0, c.stream>>>(dx, x, n);
+            BIE_CUDA(cudaGetLastError());
+            S.launched();
         }
     }
     BIE_CUDA(cudaStreamSynchronize(c.stream));

@@ -218,3 +218,26 @@ def test_dense_product_error(f, kind):
     x1, res = gmres(A, b, ctx=ctx, x0=x, abstol=np.inf, maxiter=1, log=True)
     assert np.array_equal(x1, x)
     assert res.residual_norm <= bound
+
+
+@pytest.mark.parametrize("f,restart", [(1, 12), (2, 5), (5, 33), (9, 40), (9, 64)])
+def test_gmres_restart_lengths(f, restart):
+    """Arnoldi cycles shorter and longer than the 32 columns whose sums each block
+    takes itself, on vectors of 12 to 812 rows (no multiples of 32), against a
+    direct solve: the residual test at 1e-12 bounds the error of a matrix with
+    singular values in 0.5 .. 2 by 2e-12 relative (4x for rounding)."""
+    mesh = bm.icosphere(f)
+    n = mesh.n_sources
+    r = np.random.default_rng(n + restart)
+    q = [np.linalg.qr(r.normal(size=(n, n)) + 1j * r.normal(size=(n, n)))[0] for _ in range(2)]
+    A = (q[0] * r.uniform(0.5, 2.0, n)) @ q[1]
+    A = A + 2.5 * np.eye(n)
+    b = rand_c(n, 8)
+    ctx = biegpu.get_context(mesh, n=2, m=2)
+    x, res = gmres(A, b, ctx=ctx, reltol=1e-12, restart=restart, maxiter=400, log=True)
+    xd = np.linalg.solve(A, b)
+    assert res.converged
+    assert rel(x, xd) <= 4 * 1e-12 * np.linalg.cond(A)
+    # a step count that ends a cycle early
+    x7, r7 = gmres(A, b, ctx=ctx, reltol=1e-12, restart=restart, maxiter=min(7, n - 1), log=True)
+    assert r7.iterations == min(7, n - 1) and not r7.converged
