@@ -24,6 +24,7 @@
 #include "bie_internal.h"
 #include "bie_device.cuh"
 #include "bie_df64.cuh"
+#include "bie_fixmath.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -167,8 +168,9 @@ adjoint_grad_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
                     const double2 *__restrict__ w, const double2 *__restrict__ p,
                     const double *__restrict__ coords, const int32_t *__restrict__ topo,
                     const int32_t *__restrict__ order, const double2 *__restrict__ Y, int64_t E, int S,
-                    const double *__restrict__ tab, RuleTab rt, double kre, double kim, double rhock,
-                    double *__restrict__ dX, double2 *__restrict__ sY) {
+                    const double *__restrict__ tab, RuleTab rt, const int32_t *__restrict__ trig_tab, double kre,
+                    double kim, double rhock, double *__restrict__ dX, double2 *__restrict__ sY) {
+    const dev::TrigFix trig{trig_tab};
     const int64_t row = (int64_t)blockIdx.x * kT + threadIdx.x;
     const bool active = row < N + M;
     const bool arow = row < N;
@@ -221,14 +223,11 @@ adjoint_grad_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
                 const double yz = N1 * X[2] + N2 * X[5] + N3 * X[8];
                 const double dx = yx - tx, dy = yy - ty, dz = yz - tz;
                 const double r2 = dx * dx + dy * dy + dz * dz;
-                const double rinv = rsqrt(r2);
-                const double r = r2 * rinv;
-                double sn, cs;
-                // on the FP32 pipes in double-float (~2^-46 relative): the FP64
-                // sine and cosine would be a quarter of this loop's FP64 work
-                df64::TrigDf::sincos_of(kre * r, &sn, &cs);
+                double rinv, r, sn, cs;
+                trig.root_of(r2, rinv, r);
+                trig.sincos_of(kre * r, &sn, &cs);
                 if (CPLX_K) {
-                    const double dmp = exp(-kim * r);
+                    const double dmp = trig.exp_minus(kim * r);
                     sn *= dmp;
                     cs *= dmp;
                 }
@@ -331,6 +330,7 @@ struct AdjView {
     const double *rec;             // FP64 records
     int stride, nidx_off, qmax;
     const double *phi;
+    const int32_t *tab;            // tables of dev::TrigFix
     dev::RuleInfo ri;
 };
 
@@ -341,6 +341,7 @@ __device__ __noinline__ AdjPair adjoint_pair_fp64(const AdjView &v, int64_t pe, 
     const double *r = v.rec + (size_t)pe * v.stride;
     const int c = dev::nearest_node<3>(r, tx, ty, tz);
     const int Q = v.ri.Q[c];
+    const dev::TrigFix trig{v.tab};
     const double *g = r + v.ri.off[c], *ph = v.phi + (size_t)c * v.qmax * 3;
     const int32_t *nid = reinterpret_cast<const int32_t *>(r + v.nidx_off);
     const cd p0 = {p[nid[0]].x, p[nid[0]].y}, p1 = {p[nid[1]].x, p[nid[1]].y}, p2 = {p[nid[2]].x, p[nid[2]].y};
@@ -352,9 +353,10 @@ __device__ __noinline__ AdjPair adjoint_pair_fp64(const AdjView &v, int64_t pe, 
         const double N1 = ph[3 * q], N2 = ph[3 * q + 1], N3 = ph[3 * q + 2];
         const double dx = g[q] - tx, dy = g[Q + q] - ty, dz = g[2 * Q + q] - tz;
         const double r2 = dx * dx + dy * dy + dz * dz;
-        const double ri = rsqrt(r2), rr = r2 * ri, ri2 = ri * ri;
-        double sn, cs;
-                df64::TrigDf::sincos_of(kre * rr, &sn, &cs);
+        double ri, rr, sn, cs;
+        trig.root_of(r2, ri, rr);
+        const double ri2 = ri * ri;
+        trig.sincos_of(kre * rr, &sn, &cs);
         const cd Ph = cadd(cadd(cscale(p0, N1), cscale(p1, N2)), cscale(p2, N3));
         const cd z = cmul(cmul(cw, Ph), cd{cs, sn});
         const double kr = kre * rr;
@@ -877,7 +879,7 @@ void run_adjoint(Ctx &c, const AdjointArgs &a, AdjointOut &out) {
             deg.tab = reinterpret_cast<const float4 *>(c.d_phase_tab);
             const RecordLayout &L = c.lay;
             const Df64Layout &X = c.dlay;
-            AdjView v{c.d_records, L.stride, L.nidx_off, L.qmax, c.d_phi, {}};
+            AdjView v{c.d_records, L.stride, L.nidx_off, L.qmax, c.d_phi, c.d_xtrig, {}};
             dev::RuleInfo ri{};
             for (int r = 0; r < 3; ++r) {
                 ri.Q[r] = v.ri.Q[r] = L.Q[r];
@@ -925,8 +927,8 @@ void run_adjoint(Ctx &c, const AdjointArgs &a, AdjointOut &out) {
             dim3 grid((unsigned)tiles, (unsigned)S);
             adjoint_grad_kernel<false><<<grid, kT, 0, st>>>(N, M, c.d_sources, fp.d(), w.d2(), p.d2(),
                                                             c.d_coords, c.d_topo, ord.i32(), Y.d2(), E, S,
-                                                            tab.d(), rt, a.k_re, a.k_im, rhock_re, dX.d(),
-                                                            sY.d2());
+                                                            tab.d(), rt, c.d_xtrig, a.k_re, a.k_im, rhock_re,
+                                                            dX.d(), sY.d2());
             BIE_CUDA(cudaGetLastError());
         }
         std::vector<double> hdX(3 * N);

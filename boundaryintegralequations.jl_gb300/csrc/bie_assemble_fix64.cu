@@ -38,8 +38,7 @@
 //     shared between slices take 64-bit integer atomics and a widening pass.
 #include "bie_internal.h"
 #include "bie_device.cuh"
-#include "bie_df64.cuh"
-#include "bie_fix64.cuh"
+#include "bie_fixmath.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -66,6 +65,7 @@ struct Fp64View {
     const double *phi;   // global, R x qmax x NP
     int qmax;
     RuleInfo ri;
+    const int32_t *tab;   // tables of dev::TrigFix
 };
 
 // Scales of a launch (host values)
@@ -513,7 +513,7 @@ __global__ void fx_weight_kernel(const double2 *__restrict__ w, int64_t E, int w
     out[p] = make_int4(a.h, a.l, b.h, b.l);
 }
 
-template <int NP, bool CPLX_K, class Trig>
+template <int NP, bool CPLX_K>
 __device__ __forceinline__ int fx_correct_pair(const Fp64View &v, int64_t i, int64_t p, const double *tgt, int64_t M,
                                                double kre, double kim, bool doF, bool doG, bool doC, double2 *F,
                                                double2 *G, double *Cnear, const double2 *gweight) {
@@ -521,9 +521,9 @@ __device__ __forceinline__ int fx_correct_pair(const Fp64View &v, int64_t i, int
     const double tx = tgt[3 * i], ty = tgt[3 * i + 1], tz = tgt[3 * i + 2];
     const int c = dev::nearest_node<NP>(r, tx, ty, tz);
     double fr[NP], fi[NP], gr[NP], gi[NP];
-    const double ce = dev::element_fp64<NP, CPLX_K, Trig>(r + v.ri.off[c], v.ri.Q[c],
-                                                          v.phi + (size_t)c * v.qmax * NP, tx, ty, tz, kre, kim, fr,
-                                                          fi, gr, gi);
+    const double ce = dev::element_fp64<NP, CPLX_K, dev::TrigFix>(r + v.ri.off[c], v.ri.Q[c],
+                                                                  v.phi + (size_t)c * v.qmax * NP, tx, ty, tz, kre,
+                                                                  kim, fr, fi, gr, gi, -1, dev::TrigFix{v.tab});
     if (gweight && doG) {
         const double2 w = gweight[p];
 #pragma unroll
@@ -553,7 +553,7 @@ __device__ __forceinline__ int fx_correct_pair(const Fp64View &v, int64_t i, int
 // FP64 integration of the deferred pairs, added to the finished entries.  Where
 // the list was too short, every (row, slice) whose pairs did not all fit is
 // gone through again from its first pair that found no place.
-template <int NP, bool CPLX_K, class Trig>
+template <int NP, bool CPLX_K>
 __global__ void __launch_bounds__(128)
 fx_correct_kernel(const int2 *__restrict__ defer, const unsigned int *__restrict__ defer_count,
                   unsigned int defer_cap, const __grid_constant__ Fp64View v, const double *__restrict__ tgt,
@@ -569,7 +569,7 @@ fx_correct_kernel(const int2 *__restrict__ defer, const unsigned int *__restrict
     const bool doF = flags & BIE_F, doG = flags & BIE_G, doC = flags & BIE_C;
     unsigned long long nqpe = 0;
     for (unsigned int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-        nqpe += fx_correct_pair<NP, CPLX_K, Trig>(v, defer[j].x, defer[j].y, tgt, M, kre, kim, doF, doG, doC, F, G,
+        nqpe += fx_correct_pair<NP, CPLX_K>(v, defer[j].x, defer[j].y, tgt, M, kre, kim, doF, doG, doC, F, G,
                                                   Cnear, gweight);
     if (total > defer_cap) {
         const FxWave wv = fx_wave<CPLX_K>(kre, kim, sc);
@@ -581,7 +581,7 @@ fx_correct_kernel(const int2 *__restrict__ defer, const unsigned int *__restrict
             for (int64_t p = over[j]; p < (s + 1) * E / S; ++p) {
                 i64 dx, dy, dz;
                 if (!fx_pair<NP, CPLX_K>(rec + p * stride, T, wv, dx, dy, dz).deferred) continue;
-                nqpe += fx_correct_pair<NP, CPLX_K, Trig>(v, i, p, tgt, M, kre, kim, doF, doG, doC, F, G, Cnear, gweight);
+                nqpe += fx_correct_pair<NP, CPLX_K>(v, i, p, tgt, M, kre, kim, doF, doG, doC, F, G, Cnear, gweight);
             }
         }
     }
@@ -602,7 +602,7 @@ struct FxBuffers {
 };
 
 template <int NP, bool CPLX>
-void launch_np(Ctx &c, const AssembleArgs &a, bool df_trig, const LaunchShape &sh, size_t smem, const FxBuffers &b) {
+void launch_np(Ctx &c, const AssembleArgs &a, const LaunchShape &sh, size_t smem, const FxBuffers &b) {
     const RecordLayout &L = c.lay;
     const Fix64Layout &X = c.xlay;
     RuleInfo ri{}, ri64{};
@@ -628,7 +628,7 @@ void launch_np(Ctx &c, const AssembleArgs &a, bool df_trig, const LaunchShape &s
         BIE_CUDA(cudaGetLastError());
         ++c.kernel_launches;
     }
-    const Fp64View v{c.d_records, L.stride, L.nidx_off, c.d_phi, L.qmax, ri64};
+    const Fp64View v{c.d_records, L.stride, L.nidx_off, c.d_phi, L.qmax, ri64, c.d_xtrig};
     const int level = sh.level, S = 1 << level;
     const int64_t E = c.n_elements, nfix = c.k2_nfix[level];
     longlong2 *F = (a.flags & BIE_F) ? reinterpret_cast<longlong2 *>(a.F) : nullptr;
@@ -661,7 +661,7 @@ void launch_np(Ctx &c, const AssembleArgs &a, bool df_trig, const LaunchShape &s
         BIE_CUDA(cudaGetLastError());
         ++c.kernel_launches;
     }
-    auto corr = df_trig ? fx_correct_kernel<NP, CPLX, df64::TrigDf> : fx_correct_kernel<NP, CPLX, dev::TrigFp64>;
+    auto corr = fx_correct_kernel<NP, CPLX>;
     corr<<<(unsigned)(4 * c.num_sms), 128, 0, c.stream>>>(
         b.defer, b.dcount, b.dcap, v, a.targets, a.M, a.k_re, a.k_im, a.flags, reinterpret_cast<double2 *>(F),
         reinterpret_cast<double2 *>(G), b.Cnear, b.over, c.d_xrecords, X.stride, E, S, sc, c.d_qpe, a.k_dev,
@@ -703,6 +703,9 @@ void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
     const int NP = L.NP;
     const int64_t E = c.n_elements, N = c.n_sources;
     c.fx_ok = false;
+    const std::vector<int32_t> &trig = unit_tables();   // (the near pairs of every precision use them)
+    BIE_CUDA(cudaMalloc(&c.d_xtrig, trig.size() * 4));
+    BIE_CUDA(cudaMemcpy(c.d_xtrig, trig.data(), trig.size() * 4, cudaMemcpyHostToDevice));
     // scaled coordinates (x - x0) 2^-S with the largest in [1/2, 1).  x0 is zero
     // unless the mesh lies far from the origin for its size, where the
     // subtraction is exact for targets near the mesh.
@@ -869,15 +872,12 @@ void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
         const int32_t v = node_ej[j] == INT32_MIN ? 0 : node_ej[j];
         std::memcpy(&nodes[4 * j + 3], &v, 4);
     }
-    const std::vector<int32_t> &trig = unit_tables();
     BIE_CUDA(cudaMalloc(&c.d_xrecords, rec.size() * 4));
     BIE_CUDA(cudaMalloc(&c.d_xphi, phi.size() * 4));
     BIE_CUDA(cudaMalloc(&c.d_xnodes, nodes.size() * 4));
-    BIE_CUDA(cudaMalloc(&c.d_xtrig, trig.size() * 4));
     BIE_CUDA(cudaMemcpy(c.d_xrecords, rec.data(), rec.size() * 4, cudaMemcpyHostToDevice));
     BIE_CUDA(cudaMemcpy(c.d_xphi, phi.data(), phi.size() * 4, cudaMemcpyHostToDevice));
     BIE_CUDA(cudaMemcpy(c.d_xnodes, nodes.data(), nodes.size() * 4, cudaMemcpyHostToDevice));
-    BIE_CUDA(cudaMemcpy(c.d_xtrig, trig.data(), trig.size() * 4, cudaMemcpyHostToDevice));
     c.fx_ok = true;
 }
 
@@ -893,7 +893,7 @@ bool fix64_covers(const Ctx &c, const AssembleArgs &a) {
     return kr < 500.0 && ki < 100.0 && ki * c.fx_rho_max * 1.45 < fix64::kMaxDampSpread;
 }
 
-bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df_trig) {
+bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df64) {
     if (!fix64_covers(c, args)) return false;
     AssembleArgs a = args;
     const bool cplx = a.k_im != 0.0;
@@ -904,7 +904,7 @@ bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df_trig) {
         AssembleArgs f = a;
         f.flags = BIE_C;
         f.F = f.G = nullptr;
-        if (!(df_trig && launch_assemble_k9(c, f))) launch_field_c_fp64(c, a.targets, a.M, a.C);
+        if (!(df64 && launch_assemble_k9(c, f))) launch_field_c_fp64(c, a.targets, a.M, a.C);
         a.flags &= ~BIE_C;
     }
     if (!(a.flags & (BIE_F | BIE_G | BIE_C))) return true;
@@ -931,14 +931,14 @@ bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df_trig) {
         b.Cpart = reinterpret_cast<double *>(part);
         b.over = reinterpret_cast<int *>(part + cp);
         if (L.NP == 1) {
-            if (cplx) launch_np<1, true>(c, a, df_trig, sh, smem, b);
-            else launch_np<1, false>(c, a, df_trig, sh, smem, b);
+            if (cplx) launch_np<1, true>(c, a, sh, smem, b);
+            else launch_np<1, false>(c, a, sh, smem, b);
         } else if (L.NP == 3) {
-            if (cplx) launch_np<3, true>(c, a, df_trig, sh, smem, b);
-            else launch_np<3, false>(c, a, df_trig, sh, smem, b);
+            if (cplx) launch_np<3, true>(c, a, sh, smem, b);
+            else launch_np<3, false>(c, a, sh, smem, b);
         } else {
-            if (cplx) launch_np<6, true>(c, a, df_trig, sh, smem, b);
-            else launch_np<6, false>(c, a, df_trig, sh, smem, b);
+            if (cplx) launch_np<6, true>(c, a, sh, smem, b);
+            else launch_np<6, false>(c, a, sh, smem, b);
         }
         if (a.flags & BIE_C) launch_reduce_c(c, b.Cpart, S, b.Cnear, a.M, a.C);
     };
@@ -956,7 +956,7 @@ bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df_trig) {
     ShapeAxes ax;
     for (int l = level - 1; l <= level + 1; ++l)
         if (l >= 0 && l < kMaxLevels && (int64_t(1) << l) <= c.n_elements) ax.levels.push_back(l);
-    run(df_trig ? resolve_shape(c, kShapeK9, a.M, base, ax, run, reset) : base);
+    run(df64 ? resolve_shape(c, kShapeK9, a.M, base, ax, run, reset) : base);
     return true;
 }
 

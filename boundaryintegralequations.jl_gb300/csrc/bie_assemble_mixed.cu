@@ -35,6 +35,7 @@
 #include "bie_device.cuh"
 #include "bie_mixed.cuh"
 #include "bie_df64.cuh"
+#include "bie_fixmath.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -406,7 +407,7 @@ correct_fp64_kernel(const int2 *__restrict__ defer, const unsigned int *__restri
                     double kre, double kim, int flags, T2 *__restrict__ F,
                     T2 *__restrict__ G, double *__restrict__ Cnear,
                     unsigned long long *__restrict__ qpe_count, const double *__restrict__ kdev,
-                    const double2 *__restrict__ gweight = nullptr) {
+                    const int32_t *__restrict__ tab, const double2 *__restrict__ gweight = nullptr) {
     if (kdev) {
         kre = kdev[0];
         kim = kdev[1];
@@ -422,9 +423,9 @@ correct_fp64_kernel(const int2 *__restrict__ defer, const unsigned int *__restri
         const int c = dev::nearest_node<NP>(r, tx, ty, tz);
         nqpe += v.ri.Q[c];
         double fr[NP], fi[NP], gr[NP], gi[NP];
-        const double ce = dev::element_fp64<NP, CPLX_K, df64::TrigDf>(r + v.ri.off[c], v.ri.Q[c],
+        const double ce = dev::element_fp64<NP, CPLX_K, dev::TrigFix>(r + v.ri.off[c], v.ri.Q[c],
                                                         v.phi + (size_t)c * v.qmax * NP, tx, ty, tz,
-                                                        kre, kim, fr, fi, gr, gi);
+                                                        kre, kim, fr, fi, gr, gi, -1, dev::TrigFix{tab});
         if (gweight && doG) {   // element factor on the single layer
             const double2 w = gweight[pr.y];
 #pragma unroll
@@ -499,7 +500,7 @@ void launch_np(Ctx &c, const AssembleArgs &a, int level, size_t smem, int chunk,
     using T2 = typename std::conditional<C64, float2, double2>::type;
     correct_fp64_kernel<NP, CPLX, T2><<<(unsigned)(4 * c.num_sms), 128, 0, c.stream>>>(
         defer, dcount, dcap, v, a.targets, a.M, a.k_re, a.k_im, a.flags, reinterpret_cast<T2 *>(a.F),
-        reinterpret_cast<T2 *>(a.G), Cnear, c.d_qpe, a.k_dev);
+        reinterpret_cast<T2 *>(a.G), Cnear, c.d_qpe, a.k_dev, c.d_xtrig);
     BIE_CUDA(cudaGetLastError());
     ++c.kernel_launches;
 }
@@ -934,7 +935,7 @@ void launch_df64_np(Ctx &c, const AssembleArgs &a, int S, int level, size_t smem
     }
     correct_fp64_kernel<NP, CPLX, double2><<<(unsigned)(4 * c.num_sms), 128, 0, c.stream>>>(
         defer, dcount, dcap, v, a.targets, a.M, a.k_re, a.k_im, a.flags,
-        reinterpret_cast<double2 *>(a.F), reinterpret_cast<double2 *>(a.G), Cnear, c.d_qpe, a.k_dev,
+        reinterpret_cast<double2 *>(a.F), reinterpret_cast<double2 *>(a.G), Cnear, c.d_qpe, a.k_dev, c.d_xtrig,
         reinterpret_cast<const double2 *>(a.g_weight));
     BIE_CUDA(cudaGetLastError());
     ++c.kernel_launches;

@@ -66,22 +66,28 @@ __device__ __forceinline__ int nearest_node(const double *P, double tx, double t
     return c;
 }
 
-// sin and cos of the phase k r in FP64: the plain FP64 kernels keep the
-// reference's arithmetic (Julia's sincos of a Float64)
+// sine and cosine of the phase k r, r and 1 / r and the damping e^{-Im k r} in FP64:
+// the plain FP64 kernel keeps the reference's arithmetic (Julia's sincos of a
+// Float64)
 struct TrigFp64 {
-    static __device__ __forceinline__ void sincos_of(double x, double *s, double *c) { sincos(x, s, c); }
+    __device__ __forceinline__ void sincos_of(double x, double *s, double *c) const { sincos(x, s, c); }
+    __device__ __forceinline__ void root_of(double r2, double &rinv, double &r) const {
+        rinv = rsqrt(r2);
+        r = r2 * rinv;
+    }
+    __device__ __forceinline__ double exp_minus(double x) const { return exp(-x); }
 };
 
 // FP64 integration of one element for one target with the rule clustered at
 // node c: computing_integrals! (src/3d/assembly_collocation.jl:213-252).
 // g: rule data x[Q] y[Q] z[Q] nx[Q] ny[Q] nz[Q] jw[Q]; ph: Phi[q][a].
 // Accumulates F, G per node and returns the C contribution.  Trig: how the
-// sine and cosine of k r are formed (TrigFp64, or df64::TrigDf).
+// functions of r are formed (TrigFp64, or TrigFix on the integer pipes).
 template <int NP, bool CPLX_K, class Trig = TrigFp64>
 __device__ __forceinline__ double element_fp64(const double *g, int Q, const double *ph, double tx,
                                                double ty, double tz, double kre, double kim,
                                                double *fr, double *fi, double *gr, double *gi,
-                                               int tm = -1) {
+                                               int tm = -1, const Trig &trig = Trig()) {
     // tm >= 0: tm-th derivative with respect to k (taylor_greens3d!,
     // taylor_freens3d!, src/3d/kernels.jl:94-118): both kernels times (i r)^tm,
     // and F's factor (i k r - 1) becomes (i k r - 1 + tm).
@@ -93,14 +99,14 @@ __device__ __forceinline__ double element_fp64(const double *g, int Q, const dou
         const double dy = g[Q + q] - ty;
         const double dz = g[2 * Q + q] - tz;
         const double r2 = dx * dx + dy * dy + dz * dz;
-        const double rinv = rsqrt(r2);
-        const double rr = r2 * rinv;
+        double rinv, rr;
+        trig.root_of(r2, rinv, rr);
         const double jw = g[6 * Q + q];
         const double dn = g[3 * Q + q] * dx + g[4 * Q + q] * dy + g[5 * Q + q] * dz;
         double sn, cs;
-        Trig::sincos_of(kre * rr, &sn, &cs);
+        trig.sincos_of(kre * rr, &sn, &cs);
         if (CPLX_K) {
-            const double damp = exp(-kim * rr);
+            const double damp = trig.exp_minus(kim * rr);
             sn *= damp;
             cs *= damp;
         }

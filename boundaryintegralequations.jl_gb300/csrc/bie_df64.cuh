@@ -137,12 +137,12 @@ __device__ __forceinline__ void sincos_df(df x, df &s, df &c) {
 
 // sin and cos of an FP64 phase through sincos_df on the FP32 pipes (relative
 // error ~2^-46, well inside the FP64-grade and mixed-precision budgets), FP64
-// sincos beyond its range.  For the FP64 element integrals of the deferred
-// (near) pairs of the mixed and double-float paths: the FP64 sine and cosine
-// are most of their FP64-pipe work, and this GPU's FP64 pipe runs at 1/64 of
-// the FP32 rate.
+// sincos beyond its range.  For the pairs that the mixed and double-float
+// kernels integrate in place when their deferred list is full: dev::TrigFix, as
+// in the correction kernels, would cost the kernels around it 1 to 2 % (its
+// registers count against theirs across the call).
 struct TrigDf {
-    static __device__ __forceinline__ void sincos_of(double x, double *s, double *c) {
+    __device__ __forceinline__ void sincos_of(double x, double *s, double *c) const {
         if (!(fabs(x) < (double)kDfMaxPhase)) {
             sincos(x, s, c);
             return;
@@ -152,6 +152,11 @@ struct TrigDf {
         *s = dev::f2d(sd.hi) + dev::f2d(sd.lo);
         *c = dev::f2d(cd.hi) + dev::f2d(cd.lo);
     }
+    __device__ __forceinline__ void root_of(double r2, double &rinv, double &r) const {
+        rinv = rsqrt(r2);
+        r = r2 * rinv;
+    }
+    __device__ __forceinline__ double exp_minus(double x) const { return exp(-x); }
 };
 
 namespace dd {

@@ -185,8 +185,9 @@ FX_FN i64 rcp_sqrt(i64 r2, Limb r2l) {
 }
 
 // E = e^{i theta} (Q62) from theta as a 64-bit fraction of a turn: the table
-// entry T nearest below or above plus T (cos d - 1 + i sin d), |d| <= pi / 1024
-template <class Table>
+// entry T nearest below or above plus T (cos d - 1 + i sin d), |d| <= pi / 1024.
+// Largest error 2^-55 (the series in 32-bit steps), FINE 2^-60.
+template <bool FINE = false, class Table>
 FX_FN void unit_circle(u64 frac, const Table &table, i64 &Er, i64 &Ei) {
     const unsigned top = (unsigned)(frac >> 32) + 0x00200000u;
     Limb Tc, Ts;
@@ -201,23 +202,30 @@ FX_FN void unit_circle(u64 frac, const Table &table, i64 &Er, i64 &Ei) {
     const int zA = (int)(z >> 17);                                     // Q47
     const i64 z3 = wide(zA, 1431655765);                               // d^2 / 3, Q79
     const int q = hi32(wide(zA, hi32(z3)));                            // d^4 / 3, Q62
-    const int w = hi32(wide_add(z3, q, -6554));                        // d^2/6 - d^4/120, Q48
-    const int dA = (int)(d >> 25);                                     // Q39
-    const int dw = (int)(wide(dA, w) >> 29);                           // Q58
-    const i64 sn = wide_add(d, dw, -64);                               // sin, Q64
+    i64 sn, c1 = ((i64)q - z) >> 1;                                    // sin and cos - 1, Q64
+    if (FINE) {
+        // d^2/6 - d^4/120 in Q77, and the next term of cos
+        const i64 w = mulhi(split((i64)((u64)z << 13)), split(3074457345618258603LL)) - (wide(q, 26214) >> 5);
+        sn = d - ((mulhi(dl, split(w)) + 4096) >> 13);
+        c1 -= (i64)hi32(wide(hi32(wide(q, zA)), 2185));
+    } else {
+        const int w = hi32(wide_add(z3, q, -6554));                    // d^2/6 - d^4/120, Q48
+        const int dA = (int)(d >> 25);                                 // Q39
+        const int dw = (int)(wide(dA, w) >> 29);                       // Q58
+        sn = wide_add(d, dw, -64);
+    }
     const Limb s = split(sn), ms = split(-sn);
-    const Limb c = split(((i64)q - z) >> 1);                           // cos - 1, Q64
+    const Limb c = split(c1);
     Er = fold(make64(Tc.h, 0) + (i64)Tc.l + high(wide(Tc.h, c.h), Ts, ms), cross(cross(Tc, c), Ts, ms));
     Ei = fold(make64(Ts.h, 0) + (i64)Ts.l + high(wide(Ts.h, c.h), Tc, s), cross(cross(Ts, c), Tc, s));
 }
 
-// 2^-(x - base) (Q62) from x = T 2^(6 + ds) 2^-64 (T: Q58 of 2^ds, tl: the next 32
-// bits) and the table of 2^(-j / 256) limbs
+// 2^-(f - carry) (Q62), f = frac 2^-64: the next table entry below or above
+// (carry) times a series
 template <class Table>
-FX_FN i64 damping(i64 T, unsigned tl, int dsh, int base, const Table &table) {
-    const u64 frac = ((u64)T << dsh) | (u64)(tl >> (32 - dsh));
+FX_FN i64 exp2_fraction(u64 frac, int &carry, const Table &table) {
     const u64 up = frac + ((u64)1 << 55);
-    const int xi = (int)(T >> (64 - dsh)) + (up < frac ? 1 : 0);
+    carry = up < frac ? 1 : 0;
     const Limb Td = table((int)(up >> 56));
     const i64 f = (i64)((frac - (up & 0xff00000000000000ull)) << 7);  // Q63 of a table step
     const Limb C = split(99893036290645747LL);                        // ln 2 / 256, Q65
@@ -227,12 +235,22 @@ FX_FN i64 damping(i64 T, unsigned tl, int dsh, int base, const Table &table) {
     const int uA = (int)(u >> 24), u2A = (int)(u2 >> 15);              // Q40, Q49
     const int u3 = hi32(wide(uA, u2A));                                // Q57
     const int u4 = hi32(wide(u2A, u2A));                               // Q66
-    // e^-u - 1 = -u + u^2/2 - u^3/6 + u^4/24
+    const int u5 = hi32(wide(uA, u4));                                 // Q74
+    // e^-u - 1 = -u + u^2/2 - u^3/6 + u^4/24 - u^5/120
     i64 p = (u2 >> 1) - u;
     p = wide_add(p, hi32(wide(u3, 715827883)), -128);
-    p += (i64)hi32(wide(u4, 44739243));
-    const i64 v = make64(Td.h, 0) + (i64)Td.l + mulhi(Td, split(p));
-    return shift_right(v, xi - base);
+    p += (i64)hi32(wide(u4, 44739243)) - (i64)hi32(wide(u5, 34953));
+    return make64(Td.h, 0) + (i64)Td.l + mulhi(Td, split(p));
+}
+
+// 2^-(x - base) (Q62) from x = T 2^(6 + ds) 2^-64 (T: Q58 of 2^ds, tl: the next 32
+// bits) and the table of 2^(-j / 256) limbs
+template <class Table>
+FX_FN i64 damping(i64 T, unsigned tl, int dsh, int base, const Table &table) {
+    const u64 frac = ((u64)T << dsh) | (u64)(tl >> (32 - dsh));
+    int carry;
+    const i64 v = exp2_fraction(frac, carry, table);
+    return shift_right(v, (int)(T >> (64 - dsh)) + carry - base);
 }
 
 // One quadrature point of a regular pair: greens3d!, freens3d!, freens3dk0!

@@ -1,0 +1,177 @@
+// FP64 functions of near-pair integrals on the integer and FP32 pipes: sine and
+// cosine, decaying exponential, square root and its reciprocal of a double,
+// with the fixed-point primitives of the assembly.
+//
+// GB300 issues an FP64 instruction for a warp every 62 cycles per scheduler
+// (measured), an IMAD.WIDE every 2.5: the library's sincos (some 35 FP64
+// operations) and rsqrt (8) are most of a quadrature point's time.  Here the
+// argument's bits are taken apart, the function is evaluated on 64-bit integers
+// (about 150 and 80 instructions) and the double is put together from bits.
+// Errors against extended precision: roots 0.51 ulp, exponential 0.7 ulp, sine
+// and cosine 2^-60 of 1 besides the final rounding (an error of the modulus of
+// e^{ikr}).  Arguments beyond the ranges below take the library's
+// functions.  Measured: corrections of the near pairs of the mixed assembly at 11562
+// nodes 232 -> 202 us and of the mixed product at 40962 nodes 1.56 -> 1.36 ms
+// (which had sine and cosine in double-float), FP64 matrix-free product at 5762
+// nodes 16.7 -> 11.7 ms.
+//
+// The host compiles this header too (the tests drive it on the CPU).
+#pragma once
+
+#include "bie_fix64.cuh"
+
+#include <cstring>
+#ifndef __CUDACC__
+#include <cmath>
+#endif
+
+namespace bie {
+namespace fix64 {
+
+FX_FN u64 double_bits(double x) {
+#ifdef __CUDA_ARCH__
+    return (u64)__double_as_longlong(x);
+#else
+    u64 u;
+    std::memcpy(&u, &x, 8);
+    return u;
+#endif
+}
+FX_FN double bits_double(u64 u) {
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)u);
+#else
+    double x;
+    std::memcpy(&x, &u, 8);
+    return x;
+#endif
+}
+FX_FN int leading_zeros(u64 v) {
+#ifdef __CUDA_ARCH__
+    return __clzll((long long)v);
+#else
+    return v ? __builtin_clzll(v) : 64;
+#endif
+}
+FX_FN u64 mul_high(u64 a, u64 b) {
+#ifdef __CUDA_ARCH__
+    return __umul64hi(a, b);
+#else
+    return (u64)(((unsigned __int128)a * b) >> 64);
+#endif
+}
+
+// v 2^e as a double (round half up in magnitude); the result must be normal
+FX_FN double fixed_double(i64 v, int e) {
+    const u64 s = (u64)(v >> 63), a = ((u64)v ^ s) - s;
+    const int z = leading_zeros(a);
+    const u64 n = a << (z & 63);
+    const u64 m = (n >> 11) + ((n >> 10) & 1);   // 53 bits and a carry
+    const u64 bits = ((u64)(unsigned)(e + 1085 - z) << 52) + m;
+    return a ? bits_double(bits | (s & ((u64)1 << 63))) : 0.0;
+}
+
+// rinv = 1 / sqrt(r2), r = sqrt(r2); false (nothing set) outside [2^-1000, 2^1000]
+FX_FN bool root(double r2, double &rinv, double &r) {
+    const u64 u = double_bits(r2);
+    const int ex = (int)(u >> 52);
+    if ((unsigned)(ex - 23) > 2000u) return false;
+    const int h = (ex - 1023) >> 1, odd = (ex - 1023) & 1;
+    const i64 m = (i64)(((u & 0xfffffffffffffull) | 0x10000000000000ull) << (6 + odd));   // r2 4^-h, Q58 in [1, 4)
+    const Limb ml = split(m);
+    const i64 ri = rcp_sqrt(m, ml);                        // Q61
+    const Limb rl = split(ri);
+    rinv = fixed_double(ri, -61 - h);
+    r = fixed_double(fold_up<5>(wide(ml.h, rl.h), cross<5>(ml, rl) + hi32(wide(ml.l, rl.l))), -60 + h);
+    return true;
+}
+
+// (m j) >> sh of a 53-bit and a 64-bit number, 0 < sh: the low 64 bits, the rest in top
+FX_FN u64 scaled_product(u64 m, u64 j, int sh, u64 &top) {
+    const u64 hi = mul_high(m, j), lo = m * j;
+    const int a = sh < 64 ? sh : 63, b = sh < 64 ? 0 : (sh < 127 ? sh - 64 : 63);
+    top = sh < 64 ? hi >> a : 0;
+    return sh < 64 ? (hi << (64 - a)) | (lo >> a) : hi >> b;
+}
+
+// sine and cosine of x; false (nothing set) for |x| >= 2^20 and NaN
+template <class Table>
+FX_FN bool sine_cosine(double x, const Table &table, double &s, double &c) {
+    const u64 u = double_bits(x);
+    const int ex = (int)(u >> 52) & 0x7ff;
+    if (ex >= 1043) return false;
+    // x / 2 pi as a 64-bit fraction of a turn (2^66 / 2 pi; a subnormal is below 2^-64)
+    u64 top;
+    const u64 frac = scaled_product((u & 0xfffffffffffffull) | 0x10000000000000ull, 0xa2f9836e4e44152aull, 1077 - ex, top);
+    i64 Er, Ei;
+    unit_circle<true>(frac, table, Er, Ei);
+    c = fixed_double(Er, -62);
+    s = fixed_double((i64)u < 0 ? -Ei : Ei, -62);
+    return true;
+}
+
+// e^-x; false (nothing set) for |x| >= 700 and NaN
+template <class Table>
+FX_FN bool exp_minus(double x, const Table &table, double &v) {
+    const u64 u = double_bits(x);
+    const int ex = (int)(u >> 52) & 0x7ff;
+    if ((u & 0x7fffffffffffffffull) >= 0x4085e00000000000ull) return false;
+    // x log2(e) = top + frac 2^-64 (log2(e) 2^63)
+    u64 top;
+    u64 frac = scaled_product((u & 0xfffffffffffffull) | 0x10000000000000ull, 0xb8aa3b295c17f0bcull, 1074 - ex, top);
+    if ((i64)u < 0) {
+        frac = (u64)0 - frac;
+        top = ~top + (frac == 0 ? 1 : 0);
+    }
+    int carry;
+    const i64 w = exp2_fraction(frac, carry, table);
+    v = fixed_double(w, -62 - (int)(i64)top - carry);
+    return true;
+}
+
+}  // namespace fix64
+
+#ifdef __CUDACC__
+namespace dev {
+
+// out of line: the ranges of no quadrature point of a sound mesh
+static __device__ __noinline__ double2 sincos_library(double x) {
+    double s, c;
+    sincos(x, &s, &c);
+    return make_double2(s, c);
+}
+static __device__ __noinline__ double exp_library(double x) { return exp(x); }
+
+// The functions above as element_fp64 takes them; tab: the context's tables of
+// e^{2 pi i j / 1024} and 2^(-j / 256) as limbs.
+struct TrigFix {
+    const int32_t *tab;
+    __device__ __forceinline__ void sincos_of(double x, double *s, double *c) const {
+        auto table = [&](int j, fix64::Limb &tc, fix64::Limb &ts) {
+            const int4 t = __ldg(reinterpret_cast<const int4 *>(tab) + j);
+            tc = fix64::Limb{t.x, t.y};
+            ts = fix64::Limb{t.z, t.w};
+        };
+        if (fix64::sine_cosine(x, table, *s, *c)) return;
+        const double2 v = sincos_library(x);
+        *s = v.x;
+        *c = v.y;
+    }
+    __device__ __forceinline__ void root_of(double r2, double &rinv, double &r) const {
+        if (fix64::root(r2, rinv, r)) return;
+        rinv = rsqrt(r2);
+        r = r2 * rinv;
+    }
+    __device__ __forceinline__ double exp_minus(double x) const {
+        auto table = [&](int j) {
+            const int2 t = __ldg(reinterpret_cast<const int2 *>(tab + 4 * fix64::kTrigEntries) + j);
+            return fix64::Limb{t.x, t.y};
+        };
+        double v;
+        return fix64::exp_minus(x, table, v) ? v : exp_library(-x);
+    }
+};
+
+}  // namespace dev
+#endif
+}  // namespace bie

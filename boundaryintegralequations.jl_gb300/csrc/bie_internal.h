@@ -593,10 +593,10 @@ bool launch_assemble_k9(Ctx &c, const AssembleArgs &a);   // the double-float ke
 // Fixed-point assembly at FP64 accuracy (K10, bie_assemble_fix64.cu): records
 // from the FP64 ones; the launch returns false, enqueuing nothing, where the
 // arguments need another kernel (k-derivatives, element factors, phases or
-// damping beyond the fixed-point ranges, coordinates outside 2^+-300).  df_trig: double-float sine and cosine in the
-// FP64 integrals of the near pairs (BIE_PREC_DF64).
+// damping beyond the fixed-point ranges, coordinates outside
+// 2^+-300).  df64: BIE_PREC_DF64, which keeps its own slicing and off-surface C.
 void build_fix64_records(Ctx &c, const std::vector<double> &rec64);
-bool launch_assemble_fix64(Ctx &c, const AssembleArgs &a, bool df_trig);
+bool launch_assemble_fix64(Ctx &c, const AssembleArgs &a, bool df64);
 bool fix64_covers(const Ctx &c, const AssembleArgs &a);   // whether it launches
 
 // FMA throughput probe (bie_peaks.cu)

@@ -22,6 +22,7 @@
 #include "bie_device.cuh"
 #include "bie_mixed.cuh"
 #include "bie_df64.cuh"
+#include "bie_fixmath.cuh"
 
 #include <algorithm>
 
@@ -249,7 +250,7 @@ matvec_fp64_kernel(const double *__restrict__ rec, int stride, int nidx_off, int
                    const double2 *__restrict__ x, const double2 *__restrict__ v,
                    const double *__restrict__ tgt, int64_t M, double kre, double kim,
                    double2 *__restrict__ yFpart, double2 *__restrict__ yGpart, int chunk,
-                   unsigned long long *__restrict__ qpe_count) {
+                   const int32_t *__restrict__ tab, unsigned long long *__restrict__ qpe_count) {
     extern __shared__ __align__(16) double smem[];
     double *s_phi = smem;
     double *s_rec = smem + ((nphi + 1) & ~1);
@@ -285,8 +286,8 @@ matvec_fp64_kernel(const double *__restrict__ rec, int stride, int nidx_off, int
             const int c = dev::nearest_node<NP>(r, tx, ty, tz);
             nqpe += s_ri.Q[c];
             double fr[NP], fi[NP], gr[NP], gi[NP];
-            dev::element_fp64<NP, CPLX_K>(r + s_ri.off[c], s_ri.Q[c], s_phi + (size_t)c * qmax * NP, tx,
-                                          ty, tz, kre, kim, fr, fi, gr, gi);
+            dev::element_fp64<NP, CPLX_K, dev::TrigFix>(r + s_ri.off[c], s_ri.Q[c], s_phi + (size_t)c * qmax * NP,
+                                                        tx, ty, tz, kre, kim, fr, fi, gr, gi, -1, dev::TrigFix{tab});
             const int32_t *nid = reinterpret_cast<const int32_t *>(r + nidx_off);
 #pragma unroll
             for (int a = 0; a < NP; ++a) {
@@ -321,7 +322,7 @@ matvec_correct_kernel(const int2 *__restrict__ defer, const unsigned int *__rest
                       const double2 *__restrict__ x, const double2 *__restrict__ v,
                       const double *__restrict__ tgt, double kre, double kim,
                       double2 *__restrict__ yFn, double2 *__restrict__ yGn,
-                      unsigned long long *__restrict__ qpe_count) {
+                      const int32_t *__restrict__ tab, unsigned long long *__restrict__ qpe_count) {
     const unsigned int n = min(*defer_count, defer_cap);
     unsigned long long nqpe = 0;
     for (unsigned int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
@@ -332,8 +333,8 @@ matvec_correct_kernel(const int2 *__restrict__ defer, const unsigned int *__rest
         const int c = dev::nearest_node<NP>(r, tx, ty, tz);
         nqpe += ri.Q[c];
         double fr[NP], fi[NP], gr[NP], gi[NP];
-        dev::element_fp64<NP, CPLX_K, df64::TrigDf>(r + ri.off[c], ri.Q[c], phi + (size_t)c * qmax * NP, tx, ty,
-                                      tz, kre, kim, fr, fi, gr, gi);
+        dev::element_fp64<NP, CPLX_K, dev::TrigFix>(r + ri.off[c], ri.Q[c], phi + (size_t)c * qmax * NP, tx, ty,
+                                      tz, kre, kim, fr, fi, gr, gi, -1, dev::TrigFix{tab});
         const int32_t *nid = reinterpret_cast<const int32_t *>(r + nidx_off);
         double yfr = 0, yfi = 0, ygr = 0, ygi = 0;
 #pragma unroll
@@ -447,7 +448,7 @@ void run_mixed(Ctx &c, const MatvecArgs &a) {
         matvec_correct_kernel<NP, CPLX><<<(unsigned)(4 * c.num_sms), 128, 0, c.stream>>>(
             defer, dcount, dcap, c.d_records, L.stride, L.nidx_off, c.d_phi, L.qmax, ri64,
             reinterpret_cast<const double2 *>(a.x), reinterpret_cast<const double2 *>(a.v), a.targets,
-            a.k_re, a.k_im, yFn, yGn, c.d_qpe);
+            a.k_re, a.k_im, yFn, yGn, c.d_xtrig, c.d_qpe);
         BIE_CUDA(cudaGetLastError());
         ++c.kernel_launches;
         if (doF) {
@@ -499,7 +500,7 @@ void run_fp64(Ctx &c, const MatvecArgs &a) {
     kern<<<grid, kThreads, smem, c.stream>>>(
         c.d_records, L.stride, L.nidx_off, c.n_elements, S, c.d_phi, nphi, L.qmax, ri,
         reinterpret_cast<const double2 *>(a.x), reinterpret_cast<const double2 *>(a.v), a.targets, M,
-        a.k_re, a.k_im, yFpart, yGpart, chunk, c.d_qpe);
+        a.k_re, a.k_im, yFpart, yGpart, chunk, c.d_xtrig, c.d_qpe);
     BIE_CUDA(cudaGetLastError());
     c.timer_end(t0);
     ++c.kernel_launches;
@@ -560,7 +561,7 @@ void prime_noalloc_kernels(Ctx &c, unsigned int *zero_word) {
     BIE_CUDA(cudaGetLastError());
     matvec_correct_kernel<NP, CPLX><<<1, 128, 0, c.stream>>>(
         nullptr, zero_word, 0, c.d_records, c.lay.stride, c.lay.nidx_off, c.d_phi, c.lay.qmax, ri,
-        nullptr, nullptr, c.d_sources, 0.0, 0.0, nullptr, nullptr, c.d_qpe);
+        nullptr, nullptr, c.d_sources, 0.0, 0.0, nullptr, nullptr, c.d_xtrig, c.d_qpe);
     BIE_CUDA(cudaGetLastError());
 }
 
@@ -676,7 +677,7 @@ void run_mixed_noalloc(Ctx &c, const MatvecArgs &a) {
     matvec_correct_kernel<NP, CPLX><<<(unsigned)(4 * c.num_sms), 128, 0, c.stream>>>(
         defer, dcount, dcap, c.d_records, L.stride, L.nidx_off, c.d_phi, L.qmax, ri64,
         reinterpret_cast<const double2 *>(a.x), reinterpret_cast<const double2 *>(a.v), a.targets,
-        a.k_re, a.k_im, yFn, yGn, c.d_qpe);
+        a.k_re, a.k_im, yFn, yGn, c.d_xtrig, c.d_qpe);
     BIE_CUDA(cudaGetLastError());
     if (doF) {
         reduce_y_kernel<<<(unsigned)((M + 255) / 256), 256, 0, c.stream>>>(
@@ -920,7 +921,7 @@ void run_df64(Ctx &c, const MatvecArgs &a, DfDegrees deg) {
     matvec_correct_kernel<NP, CPLX><<<(unsigned)(4 * c.num_sms), 128, 0, c.stream>>>(
         defer, dcount, dcap, c.d_records, L.stride, L.nidx_off, c.d_phi, L.qmax, ri64,
         reinterpret_cast<const double2 *>(a.x), reinterpret_cast<const double2 *>(a.v), a.targets,
-        a.k_re, a.k_im, yFn, yGn, c.d_qpe);
+        a.k_re, a.k_im, yFn, yGn, c.d_xtrig, c.d_qpe);
     BIE_CUDA(cudaGetLastError());
     ++c.kernel_launches;
     if (doF) {

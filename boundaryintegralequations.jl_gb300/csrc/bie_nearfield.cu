@@ -12,10 +12,12 @@
 // derivatives), the jacobian and negated unit normal formed as in jacobian!
 // (src/3d/jacobian.jl:78-87), and the F and G integrands of kernels.jl:13-37
 // accumulated per physics node.  A warp-shuffle reduction gives the element's
-// contributions, which lane 0 adds (FP64 atomics) to the pair's CSR slots.
-// FP64 throughout: these are the singular and near-singular integrals.
+// contributions, which the lanes add (FP64 atomics) to the pair's CSR slots.
+// FP64 throughout (roots, sine, cosine and exponential at FP64 accuracy on the
+// integer pipes): these are the singular and near-singular integrals.
 #include "bie_internal.h"
 #include "bie_device.cuh"
+#include "bie_fixmath.cuh"
 
 namespace bie {
 
@@ -30,23 +32,52 @@ struct RuleSet {
     int coarse_q;
 };
 
-__device__ __forceinline__ double warp_sum(double v) {
+// Sums of V = 16 or 32 values over the warp's lanes, halving the values with
+// each exchange (V adds instead of 5 V): lane l gets value l (32) or l / 2 (16).
+template <int V>
+__device__ __forceinline__ double warp_sums(double (&v)[V], int lane) {
+    int n = V / 2, o = 16;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    for (; n >= 1; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < V / 2; ++i)
+            if (i < n) {
+                const double keep = up ? v[i + n] : v[i], send = up ? v[i] : v[i + n];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+    }
+    if (V == 16) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    return v[0];
 }
 
-template <int NS, int NP, bool CPLX_K>
+// r and 1 / r where r^2 leaves the range of fix64::root
+__device__ __noinline__ double2 distance_library(double dx, double dy, double dz) {
+    const double r = dev::julia_hypot3(dx, dy, dz);
+    return make_double2(r, __ddiv_rn(1.0, r));
+}
+
+// FLAT: three-node elements with linear shape functions, whose derivatives and
+// so normal and jacobian are the same at every point.
+//
+// Bound by the FP64 pipe (62 cycles per operation and scheduler): 230
+// operations per point when roots, divisions, sine, cosine and exponential came
+// from the library and flat elements formed their normal at every point, some
+// 50 now, with about 280 integer instructions beside them.  Flat elements, 1962
+// nodes: 19.9 -> 4.3 ms (with a complex wavenumber 21.6 -> 4.8); 6-node elements,
+// whose geometry stays in FP64 at every point, 36.0 -> 27.4 ms at 2562 nodes.
+template <int NS, int NP, bool CPLX_K, bool FLAT>
 __global__ void __launch_bounds__(256)
 nearfield_kernel(const int32_t *__restrict__ pairs, int pstride, int64_t npairs,
-                 const double *__restrict__ table, int tstride, RuleSet rs, bool coarse,
+                 const double *__restrict__ table, int tstride, const __grid_constant__ RuleSet rs, bool coarse,
                  const double *__restrict__ coords, const int32_t *__restrict__ topo,
                  const double *__restrict__ tgt, double kre, double kim, int flags, double sign,
-                 double2 *__restrict__ Fv, double2 *__restrict__ Gv) {
+                 const int32_t *__restrict__ trig_tab, double2 *__restrict__ Fv, double2 *__restrict__ Gv) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const bool doF = flags & BIE_F, doG = flags & BIE_G;
+    const dev::TrigFix trig{trig_tab};
     for (int64_t p = warp; p < npairs; p += nwarps) {
         const int32_t *pr = pairs + p * pstride;
         const int64_t i = pr[0];
@@ -70,24 +101,15 @@ nearfield_kernel(const int32_t *__restrict__ pairs, int pstride, int64_t npairs,
             base = rs.off[c];
             Q = rs.q[c];
         }
-        double fr[NP], fi[NP], gr[NP], gi[NP];
-#pragma unroll
-        for (int a = 0; a < NP; ++a) fr[a] = fi[a] = gr[a] = gi[a] = 0.0;
-        for (int q = lane; q < Q; q += 32) {
-            // The subdivided rules put points within 1e-6 element sizes of the
-            // singular node, where x_q - t and n.(x_q - t) cancel: the geometry
-            // is therefore evaluated with separately rounded products and sums
-            // in the reference's order (interpolation, cross product, Julia
-            // hypot for the jacobian and the distance, IEEE division for the
-            // normal), so the result does not depend on FMA contraction.
-            const double *P = table + (base + q) * tstride;
-            double x[3] = {0, 0, 0}, tu[3] = {0, 0, 0}, tv[3] = {0, 0, 0};
+        // negated unit normal, jacobian / 4 pi
+        double nx = 0, ny = 0, nz = 0, jac4 = 0;
+        auto normal = [&](const double *P) {
+            double tu[3] = {0, 0, 0}, tv[3] = {0, 0, 0};
 #pragma unroll
             for (int a = 0; a < NS; ++a) {
-                const double Na = P[a], Ua = P[NS + a], Va = P[2 * NS + a];
+                const double Ua = P[NS + a], Va = P[2 * NS + a];
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
-                    x[k] = __dadd_rn(x[k], __dmul_rn(X[3 * a + k], Na));
                     tu[k] = __dadd_rn(tu[k], __dmul_rn(X[3 * a + k], Ua));
                     tv[k] = __dadd_rn(tv[k], __dmul_rn(X[3 * a + k], Va));
                 }
@@ -96,59 +118,86 @@ nearfield_kernel(const int32_t *__restrict__ pairs, int pstride, int64_t npairs,
             const double n1 = __dsub_rn(__dmul_rn(tu[2], tv[0]), __dmul_rn(tu[0], tv[2]));
             const double n2 = __dsub_rn(__dmul_rn(tu[0], tv[1]), __dmul_rn(tu[1], tv[0]));
             const double jac = dev::julia_hypot3(n0, n1, n2);
-            const double jw = __dmul_rn(jac, P[3 * NS + NP]);
-            const double nx = __ddiv_rn(-n0, jac), ny = __ddiv_rn(-n1, jac), nz = __ddiv_rn(-n2, jac);
+            nx = __ddiv_rn(-n0, jac);
+            ny = __ddiv_rn(-n1, jac);
+            nz = __ddiv_rn(-n2, jac);
+            jac4 = jac * kInv4Pi;
+        };
+        if (FLAT) normal(table + base * tstride);
+        constexpr int V = NP <= 4 ? 16 : 32;
+        double acc[V];   // fr, fi, gr, gi per node
+#pragma unroll
+        for (int a = 0; a < V; ++a) acc[a] = 0.0;
+        for (int q = lane; q < Q; q += 32) {
+            // The subdivided rules put points within 1e-6 element sizes of the
+            // singular node, where x_q - t and n.(x_q - t) cancel (on flat elements
+            // F is that rounding): the geometry is therefore evaluated with
+            // separately rounded products and sums in the reference's order
+            // (interpolation, cross product, Julia hypot for the jacobian, IEEE
+            // division for the normal), so the result does not depend on FMA
+            // contraction.  The functions of r only scale it.
+            const double *P = table + (base + q) * tstride;
+            double x[3] = {0, 0, 0};
+#pragma unroll
+            for (int a = 0; a < NS; ++a) {
+                const double Na = P[a];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const double m = __dmul_rn(X[3 * a + k], Na);
+                    x[k] = a == 0 ? m : __dadd_rn(x[k], m);
+                }
+            }
+            if (!FLAT) normal(P);
+            const double jw = jac4 * P[3 * NS + NP];
             const double dx = __dsub_rn(x[0], tx), dy = __dsub_rn(x[1], ty), dz = __dsub_rn(x[2], tz);
-            const double rr = dev::julia_hypot3(dx, dy, dz);
-            const double rinv = __ddiv_rn(1.0, rr);
+            double rinv, rr;
+            if (!fix64::root(dx * dx + dy * dy + dz * dz, rinv, rr)) {
+                const double2 d = distance_library(dx, dy, dz);
+                rr = d.x;
+                rinv = d.y;
+            }
+            const double ai = kre * rr;
             double sn, cs;
-            sincos(kre * rr, &sn, &cs);
+            trig.sincos_of(ai, &sn, &cs);
             if (CPLX_K) {
-                const double damp = exp(-kim * rr);
+                const double damp = trig.exp_minus(kim * rr);
                 sn *= damp;
                 cs *= damp;
             }
-            const double wg = rinv * kInv4Pi * jw;
-            const double Gr = cs * wg, Gi = sn * wg;
-            const double dn = __dadd_rn(__dadd_rn(__dmul_rn(nx, dx), __dmul_rn(ny, dy)), __dmul_rn(nz, dz));
-            const double tq = dn * (rinv * rinv * rinv) * kInv4Pi * jw;
-            const double ar = CPLX_K ? (-1.0 - kim * rr) : -1.0;
-            const double ai = kre * rr;
-            const double Fr = (cs * ar - sn * ai) * tq;
-            const double Fi = (cs * ai + sn * ar) * tq;
+            const double wg = rinv * jw;
             const double *ph = P + 3 * NS;
-#pragma unroll
-            for (int a = 0; a < NP; ++a) {
-                fr[a] += Fr * ph[a];
-                fi[a] += Fi * ph[a];
-                gr[a] += Gr * ph[a];
-                gi[a] += Gi * ph[a];
-            }
-        }
-#pragma unroll
-        for (int a = 0; a < NP; ++a) {
             if (doF) {
-                fr[a] = warp_sum(fr[a]);
-                fi[a] = warp_sum(fi[a]);
+                const double dn = __dadd_rn(__dadd_rn(__dmul_rn(nx, dx), __dmul_rn(ny, dy)), __dmul_rn(nz, dz));
+                const double tq = dn * (wg * rinv) * rinv;
+                double Fr, Fi;   // e^{ikr} (i k r - 1) tq
+                if (CPLX_K) {
+                    const double ar = -1.0 - kim * rr;
+                    Fr = (cs * ar - sn * ai) * tq;
+                    Fi = (cs * ai + sn * ar) * tq;
+                } else {
+                    Fr = -(sn * ai + cs) * tq;
+                    Fi = (cs * ai - sn) * tq;
+                }
+#pragma unroll
+                for (int a = 0; a < NP; ++a) {
+                    acc[4 * a] += Fr * ph[a];
+                    acc[4 * a + 1] += Fi * ph[a];
+                }
             }
             if (doG) {
-                gr[a] = warp_sum(gr[a]);
-                gi[a] = warp_sum(gi[a]);
+                const double Gr = cs * wg, Gi = sn * wg;
+#pragma unroll
+                for (int a = 0; a < NP; ++a) {
+                    acc[4 * a + 2] += Gr * ph[a];
+                    acc[4 * a + 3] += Gi * ph[a];
+                }
             }
         }
-        if (lane == 0) {
-#pragma unroll
-            for (int a = 0; a < NP; ++a) {
-                const int64_t slot = pr[2 + a];
-                if (doF) {
-                    atomicAdd(&Fv[slot].x, sign * fr[a]);
-                    atomicAdd(&Fv[slot].y, sign * fi[a]);
-                }
-                if (doG) {
-                    atomicAdd(&Gv[slot].x, sign * gr[a]);
-                    atomicAdd(&Gv[slot].y, sign * gi[a]);
-                }
-            }
+        const double sum = warp_sums<V>(acc, lane);
+        const int v = V == 32 ? lane : lane >> 1, a = v >> 2;
+        if (v < 4 * NP && (V == 32 || !(lane & 1)) && ((v & 2) ? doG : doF)) {
+            double2 *dst = ((v & 2) ? Gv : Fv) + pr[2 + a];
+            atomicAdd((v & 1) ? &dst->y : &dst->x, sign * sum);
         }
     }
 }
@@ -167,16 +216,11 @@ void launch_ns_np(Ctx &c, const NearField &nf, double kre, double kim, int flags
     const unsigned blocks = (unsigned)std::max<int64_t>(1, (warps * 32 + 255) / 256);
     const bool cplx = kim != 0.0;
     cudaEvent_t t0 = c.timer_begin();
-    if (cplx)
-        nearfield_kernel<NS, NP, true><<<blocks, 256, 0, c.stream>>>(
-            nf.d_pairs, nf.pair_stride, nf.npairs, nf.d_table, nf.point_stride, rs, coarse,
-            c.d_coords, c.d_topo, c.d_sources, kre, kim, flags, sign,
-            reinterpret_cast<double2 *>(Fv), reinterpret_cast<double2 *>(Gv));
-    else
-        nearfield_kernel<NS, NP, false><<<blocks, 256, 0, c.stream>>>(
-            nf.d_pairs, nf.pair_stride, nf.npairs, nf.d_table, nf.point_stride, rs, coarse,
-            c.d_coords, c.d_topo, c.d_sources, kre, kim, flags, sign,
-            reinterpret_cast<double2 *>(Fv), reinterpret_cast<double2 *>(Gv));
+    constexpr bool kFlat = NS == 3;   // (three-node shape functions are linear)
+    auto kern = cplx ? nearfield_kernel<NS, NP, true, kFlat> : nearfield_kernel<NS, NP, false, kFlat>;
+    kern<<<blocks, 256, 0, c.stream>>>(nf.d_pairs, nf.pair_stride, nf.npairs, nf.d_table, nf.point_stride, rs, coarse,
+                                       c.d_coords, c.d_topo, c.d_sources, kre, kim, flags, sign, c.d_xtrig,
+                                       reinterpret_cast<double2 *>(Fv), reinterpret_cast<double2 *>(Gv));
     BIE_CUDA(cudaGetLastError());
     c.timer_end(t0);
     ++c.kernel_launches;
