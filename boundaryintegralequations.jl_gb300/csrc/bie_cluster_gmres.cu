@@ -18,7 +18,13 @@
 //     fixed order, so every CTA holds bit-identical coefficients and takes the
 //     same branches;
 //   * the Hessenberg column, Givens rotations, residual estimate and back
-//     substitution run on one thread of each CTA on its own copy of the state.
+//     substitution run on one warp of each CTA on its own copy of the state, the
+//     rotations while the other warps update w;
+//   * a warp waits 62 cycles for each FP64 operation whatever its parallelism, so
+//     the work is laid out for few operations in a row: real components, eight
+//     lanes per matrix row, lanes shared between the columns of a dot product.
+//     Solves of 2562 and 7686 rows, 3 steps, with a polling loop that reads the
+//     error word seldom: 108 -> 74 us on average.
 // Two synchronisation forms:
 //   * grid (large systems): one CTA per SM, partials in global memory, a
 //     grid barrier of this file (one monotonic arrival counter: barrier b
@@ -37,6 +43,7 @@
 // residual, stop when |r| <= max(reltol |b|, abstol) or after maxiter steps.
 // Every loop has a bound.
 #include "bie_internal.h"
+#include "bie_krylov.cuh"
 
 #include <cooperative_groups.h>
 
@@ -55,7 +62,7 @@ constexpr int kMaxRestart = 48;        // longest restart cycle of the one-launc
 constexpr size_t kMaxSmem = 224 * 1024;
 constexpr int kClusterThreads = 512;
 constexpr int kGridThreads = 256;
-constexpr long long kSpinLimit = 1LL << 23;   // grid-barrier polls (about a second)
+constexpr unsigned kSpinLimit = 1u << 22;     // grid-barrier polls (a few seconds)
 
 struct CgArgs {
     const int64_t *rp;
@@ -79,20 +86,16 @@ struct CgArgs {
 
 struct CgScalars {
     double res;     // |g_{j+1}| after the last step
-    double hn;      // h_{j+1,j} of the last step
+    double na2, ia; // |a|^2 and 1 / |a| of the new column's last entry a
+    double rh, in;  // 1 / h_{j+1,j}, 1 / sqrt(na2 + h_{j+1,j}^2)
     int done;       // converged or breakdown in this cycle
     int jdone;      // steps completed in this cycle
 };
 
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
-
-__device__ __forceinline__ double warp_sum(double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
+using namespace krylov;
+// Threads of a CTA that share the partial sums: one warp per scheduler, since
+// further warps only queue for its FP64 unit.
+constexpr int kSumThreads = 128;
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
     unsigned v;
@@ -124,13 +127,13 @@ struct ClusterSync {
     __device__ int stride() const { return 1; }
     // out[c] = sum over CTAs of their slot-s partial of column c (after sync)
     __device__ void gather(int s, int nc, double2 *out) {
-        const unsigned C = cl.num_blocks();
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        for (int c = warp; c < nc; c += NT / 32) {
-            double2 v = make_double2(0.0, 0.0);
-            if ((unsigned)lane < C) v = cl.map_shared_rank(spart + s * ps, (unsigned)lane)[c];
-            const double re = warp_sum(v.x), im = warp_sum(v.y);
-            if (lane == 0) out[c] = make_double2(re, im);
+        const int C = (int)cl.num_blocks(), L = 16;
+        for (int q0 = threadIdx.x / 32 * (32 / L); q0 < 2 * nc; q0 += NT / L) {
+            const int q = q0 + threadIdx.x % 32 / L, k = threadIdx.x % L;
+            double v = 0.0;
+            if (q < 2 * nc && k < C) v = comps(cl.map_shared_rank(spart + s * ps, (unsigned)k))[q];
+            v = lane_sum(v, L);
+            if (k == 0 && q < 2 * nc) comps(out)[q] = v;
         }
     }
     __device__ void finish() { cl.sync(); }   // no CTA leaves while another reads its shared memory
@@ -148,123 +151,92 @@ struct GridSync {
     int *err;
     int ps;
     unsigned nb, r, target;
+    bool dead = false;   // thread 0: a wait ran out, here or elsewhere
     __device__ GridSync(const CgArgs &a, double2 *, int ps_)
         : gpart(a.gpart), count(a.bar), err(a.err), ps(ps_), nb(gridDim.x), r(blockIdx.x), target(0) {}
     __device__ unsigned rank() const { return r; }
     __device__ void sync() {
         target += nb;
         __syncthreads();
-        if (threadIdx.x == 0 && ld_relaxed(err) == 0) {
+        if (threadIdx.x == 0 && !dead) {
             red_add_release(count, 1u);
-            long long spins = 0;
-            while ((int)(ld_acquire(count) - target) < 0) {
-                if (++spins > kSpinLimit || ld_relaxed(err) != 0) {
+            // (the error word only every 64 polls: reading it with each one doubles
+            // the time between two looks at the counter)
+            for (unsigned spins = 1; (int)(ld_acquire(count) - target) < 0; ++spins) {
+                if (spins % 64 == 0 && (spins > kSpinLimit || ld_relaxed(err) != 0)) {
                     atomicExch(err, 1);
+                    dead = true;
                     break;
                 }
             }
-            asm volatile("fence.acq_rel.gpu;" ::: "memory");
         }
         __syncthreads();
     }
     __device__ double2 *mine(int s) const { return gpart + (size_t)s * ps * nb + r; }
     __device__ int stride() const { return (int)nb; }
     __device__ void gather(int s, int nc, double2 *out) {
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const double2 *base = gpart + (size_t)s * ps * nb;
-        for (int c = warp; c < nc; c += NT / 32) {
-            double re = 0.0, im = 0.0;
-            for (unsigned q0 = 0; q0 < nb; q0 += 128) {   // four independent loads per lane in flight
-                double2 v[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const unsigned q = q0 + 32 * u + lane;
-                    v[u] = q < nb ? __ldcg(base + (size_t)c * nb + q) : make_double2(0.0, 0.0);
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    re += v[u].x;
-                    im += v[u].y;
-                }
+        if (threadIdx.x >= kSumThreads) return;
+        const double *base = comps(gpart + (size_t)s * ps * nb);
+        const int L = lanes_per<kSumThreads>(nc), k = threadIdx.x % L;
+        for (int q0 = 0; q0 < 2 * nc; q0 += kSumThreads / L) {
+            const int q = q0 + threadIdx.x / L;
+            double v = 0.0;
+            if (q < 2 * nc) {
+                const double *p = base + 2 * (size_t)(q >> 1) * nb + (q & 1);
+#pragma unroll 8
+                for (unsigned b = k; b < nb; b += L) v += __ldcg(p + 2 * b);
             }
-            re = warp_sum(re);
-            im = warp_sum(im);
-            if (lane == 0) out[c] = make_double2(re, im);
+            v = lane_sum(v, L);
+            if (k == 0 && q < 2 * nc) comps(out)[q] = v;
         }
     }
     __device__ void finish() {}
 };
 
-// (A s)[i] for global row i; s was written by other CTAs before the last
-// barrier, so it is read through L2 (ld.global.cg).
-__device__ __forceinline__ double2 csr_row(const CgArgs &a, const double2 *s, int64_t i) {
-    const int64_t blk = i / a.N;
-    const int64_t r = i - blk * a.N;
-    const double2 *sb = s + blk * a.N;
-    const int64_t p0 = __ldg(a.rp + r), p1 = __ldg(a.rp + r + 1);
-    double re = 0.0, im = 0.0;
-    int64_t p = p0;
-    for (; p + 4 <= p1; p += 4) {
-        const int c0 = __ldg(a.cols + p), c1 = __ldg(a.cols + p + 1), c2 = __ldg(a.cols + p + 2),
-                  c3 = __ldg(a.cols + p + 3);
-        const double2 v0 = __ldg(a.val + p), v1 = __ldg(a.val + p + 1), v2 = __ldg(a.val + p + 2),
-                      v3 = __ldg(a.val + p + 3);
-        const double2 x0 = __ldcg(sb + c0), x1 = __ldcg(sb + c1), x2 = __ldcg(sb + c2), x3 = __ldcg(sb + c3);
-        re += v0.x * x0.x - v0.y * x0.y;
-        im += v0.x * x0.y + v0.y * x0.x;
-        re += v1.x * x1.x - v1.y * x1.y;
-        im += v1.x * x1.y + v1.y * x1.x;
-        re += v2.x * x2.x - v2.y * x2.y;
-        im += v2.x * x2.y + v2.y * x2.x;
-        re += v3.x * x3.x - v3.y * x3.y;
-        im += v3.x * x3.y + v3.y * x3.x;
+// out(i, im, component im of (A s)[lo + i]) for the CTA's rows; s was written by
+// other CTAs before the last barrier, so it is read through L2
+template <int NT, class Out>
+__device__ __forceinline__ void csr_rows(const CgArgs &a, const double2 *s, int64_t lo, int cnt, Out out) {
+    const int lane = threadIdx.x & 31;
+    const bool im = lane & 1;
+    for (int r0 = threadIdx.x / 32 * 4; r0 < cnt; r0 += NT / 8) {
+        const int i = r0 + (lane >> 3);
+        const bool in = i < cnt;
+        const int64_t blk = in ? (lo + i) / a.N : 0, r = lo + i - blk * a.N;
+        double v = row_product<true>(a.rp, a.cols, a.val, s + blk * a.N, r, in, lane);
+        if (in && (lane & 6) == 0) {
+            if (a.diag) v = mul_step(v, __ldg(a.diag + r), __ldcg(s + lo + i), im);
+            out(i, im, v);
+        }
     }
-    for (; p < p1; ++p) {
-        const double2 v = __ldg(a.val + p), xv = __ldcg(sb + __ldg(a.cols + p));
-        re += v.x * xv.x - v.y * xv.y;
-        im += v.x * xv.y + v.y * xv.x;
-    }
-    if (a.diag) {
-        const double2 d = __ldg(a.diag + r), xv = __ldcg(s + i);
-        re += d.x * xv.x - d.y * xv.y;
-        im += d.x * xv.y + d.y * xv.x;
-    }
-    return make_double2(re, im);
 }
 
-// part[c * ps] = V[:, c]^H w over this CTA's rows, c < nc (one warp per
-// column); column c of the CTA's rows starts at Vl + c * ld
-template <int NT>
+// part[c * pst] = V[:, c]^H w over this CTA's rows, c < nc; column c of the CTA's
+// rows starts at Vl + c * ld
 __device__ __forceinline__ void local_multidot(const double2 *Vl, int64_t ld, int cnt, int nc, const double2 *w_s,
                                                double2 *part, int pst) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int c = warp; c < nc; c += NT / 32) {
-        const double2 *vc = Vl + (int64_t)c * ld;
-        double re = 0.0, im = 0.0;
-        for (int i = lane; i < cnt; i += 32) {
-            const double2 a = vc[i], w = w_s[i];
-            re += a.x * w.x + a.y * w.y;
-            im += a.x * w.y - a.y * w.x;
+    if (threadIdx.x >= kSumThreads) return;
+    const int L = lanes_per<kSumThreads>(nc), lane = threadIdx.x % L;
+    for (int q0 = 0; q0 < 2 * nc; q0 += kSumThreads / L) {
+        const int q = q0 + threadIdx.x / L;
+        double v = 0.0;
+        if (q < 2 * nc) {
+            const double2 *vc = Vl + (int64_t)(q >> 1) * ld;
+#pragma unroll 4
+            for (int i = lane; i < cnt; i += L) v = dot_step(v, vc[i], w_s[i], q & 1);
         }
-        re = warp_sum(re);
-        im = warp_sum(im);
-        if (lane == 0) part[(int64_t)c * pst] = make_double2(re, im);
+        v = lane_sum(v, L);
+        if (lane == 0 && q < 2 * nc) comps(part + (int64_t)(q >> 1) * pst)[q & 1] = v;
     }
 }
 
-// part[0] = |w|^2 over this CTA's rows
-template <int NT>
-__device__ __forceinline__ void local_norm2(int cnt, const double2 *w_s, double2 *part, double *wred) {
+// part[0] = |w|^2 over this CTA's rows, by the first warp
+__device__ __forceinline__ void local_norm2(int cnt, const double2 *w_s, double2 *part) {
+    if (threadIdx.x >= 32) return;
     double s = 0.0;
-    for (int i = threadIdx.x; i < cnt; i += NT) s += w_s[i].x * w_s[i].x + w_s[i].y * w_s[i].y;
-    s = warp_sum(s);
-    if ((threadIdx.x & 31) == 0) wred[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int k = 0; k < NT / 32; ++k) t += wred[k];
-        part[0] = make_double2(t, 0.0);
-    }
+    for (int i = threadIdx.x; i < 2 * cnt; i += 32) s = fma(comps(w_s)[i], comps(w_s)[i], s);
+    s = lane_sum(s, 32);
+    if (threadIdx.x == 0) part[0] = make_double2(s, 0.0);
 }
 
 template <class Sync, bool VS>
@@ -276,7 +248,7 @@ __global__ void __launch_bounds__(Sync::kThreads, 1) csr_gmres_one_kernel(CgArgs
 
     // shared memory: [VS: basis (m + 1) x rows_per], w (rows_per), three
     // partial slots (m + 2 each; cluster form), h1, h2, y (m + 2 each),
-    // H ((m + 1) x m), g (m + 1), sn (m), cs (m), warp partials, scalars
+    // H ((m + 1) x m), g (m + 1), sn (m), cs (m), scalars
     extern __shared__ double2 smem[];
     double2 *V_s = smem;
     double2 *w_s = VS ? smem + (int64_t)(m + 1) * a.rows_per : smem;
@@ -288,11 +260,12 @@ __global__ void __launch_bounds__(Sync::kThreads, 1) csr_gmres_one_kernel(CgArgs
     double2 *g = H + (int64_t)(m + 1) * m;
     double2 *sn = g + (m + 1);
     double *cs = reinterpret_cast<double *>(sn + m);
-    double *wred = cs + m;
-    CgScalars *sc = reinterpret_cast<CgScalars *>(wred + NT / 32);
+    CgScalars *sc = reinterpret_cast<CgScalars *>(cs + m);
 
     Sync S(a, spart, ps);
     const int rank = (int)S.rank();
+    const int lane = threadIdx.x & 31;
+    const bool last = threadIdx.x >= NT - 32;   // the warp that keeps the Hessenberg system
     const int64_t lo0 = (int64_t)rank * a.rows_per;
     const int64_t lo = lo0 < n ? lo0 : n;
     const int64_t hi = lo + a.rows_per < n ? lo + a.rows_per : n;
@@ -322,7 +295,7 @@ __global__ void __launch_bounds__(Sync::kThreads, 1) csr_gmres_one_kernel(CgArgs
     __syncthreads();
     {
         const int s = next_slot();
-        local_norm2<NT>(cnt, w_s, S.mine(s), wred);
+        local_norm2(cnt, w_s, S.mine(s));
         reduce(s, 1, h1);
     }
     const double bnorm = sqrt(fmax(h1[0].x, 0.0));
@@ -335,14 +308,13 @@ __global__ void __launch_bounds__(Sync::kThreads, 1) csr_gmres_one_kernel(CgArgs
         if (cycle > 0) {
             // w = b - A x with the x of every CTA
             S.sync();
-            for (int i = threadIdx.x; i < cnt; i += NT) {
-                const double2 ax = csr_row(a, a.x, lo + i), bv = a.b[lo + i];
-                w_s[i] = make_double2(bv.x - ax.x, bv.y - ax.y);
-            }
+            csr_rows<NT>(a, a.x, lo, cnt, [&](int i, int im, double v) {
+                comps(w_s)[2 * i + im] = comps(a.b)[2 * (lo + i) + im] - v;
+            });
             ++matvecs;
             __syncthreads();
             const int s = next_slot();
-            local_norm2<NT>(cnt, w_s, S.mine(s), wred);
+            local_norm2(cnt, w_s, S.mine(s));
             reduce(s, 1, h1);
             beta = sqrt(fmax(h1[0].x, 0.0));
         }
@@ -359,123 +331,97 @@ __global__ void __launch_bounds__(Sync::kThreads, 1) csr_gmres_one_kernel(CgArgs
         if (threadIdx.x == 0) {
             for (int k = 0; k <= m; ++k) g[k] = make_double2(0.0, 0.0);
             g[0] = make_double2(beta, 0.0);
+            sc->res = beta;
             sc->done = 0;
             sc->jdone = 0;
         }
         for (int j = 0; j < jmax; ++j) {
             S.sync();   // v_j of every CTA is in global memory
             const double2 *vj = VS ? a.V : a.V + (int64_t)j * n;
-            for (int i = threadIdx.x; i < cnt; i += NT) w_s[i] = csr_row(a, vj, lo + i);
+            csr_rows<NT>(a, vj, lo, cnt, [&](int i, int im, double v) { comps(w_s)[2 * i + im] = v; });
             __syncthreads();
             // classical Gram-Schmidt, two passes
             for (int pass = 0; pass < 2; ++pass) {
                 double2 *h = pass == 0 ? h1 : h2;
                 const int s = next_slot();
-                local_multidot<NT>(Vl, ldv, cnt, j + 1, w_s, S.mine(s), S.stride());
+                local_multidot(Vl, ldv, cnt, j + 1, w_s, S.mine(s), S.stride());
                 reduce(s, j + 1, h);
-                for (int i = threadIdx.x; i < cnt; i += NT) {
-                    double re = w_s[i].x, im = w_s[i].y;
-                    for (int c = 0; c <= j; ++c) {
-                        const double2 v = Vl[(int64_t)c * ldv + i], hc = h[c];
-                        re -= v.x * hc.x - v.y * hc.y;
-                        im -= v.x * hc.y + v.y * hc.x;
+                if (!last) {
+                    for (int i = threadIdx.x; i < 2 * cnt; i += NT - 32) {
+                        double v = 0.0;
+#pragma unroll 4
+                        for (int c = 0; c <= j; ++c) v = mul_step(v, Vl[(int64_t)c * ldv + (i >> 1)], h[c], i & 1);
+                        comps(w_s)[i] -= v;
                     }
-                    w_s[i] = make_double2(re, im);
+                } else if (pass == 1 && lane < 4) {
+                    // meanwhile the earlier rotations of Hessenberg column j
+                    double2 *col = H + (int64_t)j * (m + 1);
+                    for (int k = lane; k <= j; k += 4) col[k] = make_double2(h1[k].x + h2[k].x, h1[k].y + h2[k].y);
+                    __syncwarp(0xfu);
+                    rotate_column(col, sn, cs, j, lane);
+                    if (lane == 0) {
+                        const double2 u = col[j];
+                        sc->na2 = fma(u.x, u.x, u.y * u.y);
+                        sc->ia = rsqrt(sc->na2);
+                    }
                 }
                 __syncthreads();
             }
             {
                 const int s = next_slot();
-                local_norm2<NT>(cnt, w_s, S.mine(s), wred);
+                local_norm2(cnt, w_s, S.mine(s));
                 reduce(s, 1, y);
             }
-            if (threadIdx.x == 0) {
-                // Hessenberg column j, earlier rotations, the new rotation
-                const int ld = m + 1;
-                double2 *col = H + (int64_t)j * ld;
-                for (int k = 0; k <= j; ++k) col[k] = make_double2(h1[k].x + h2[k].x, h1[k].y + h2[k].y);
-                const double hn = sqrt(fmax(y[0].x, 0.0));
-                col[j + 1] = make_double2(hn, 0.0);
-                for (int k = 0; k < j; ++k) {
-                    const double c = cs[k];
-                    const double2 s = sn[k];
-                    const double2 u = col[k], v = col[k + 1];
-                    const double2 sv = cmul(s, v), su = cmul(cconj(s), u);
-                    col[k] = make_double2(c * u.x + sv.x, c * u.y + sv.y);
-                    col[k + 1] = make_double2(-su.x + c * v.x, -su.y + c * v.y);
+            const double hn2 = fmax(y[0].x, 0.0);
+            if (threadIdx.x == 0) sc->in = rsqrt(sc->na2 + hn2);
+            if (threadIdx.x == 32) sc->rh = rsqrt(hn2);
+            __syncthreads();
+            Rotation rot{};
+            if (!last) {
+                // v_{j+1} = w / h_{j+1,j}
+                const double inv_hn = hn2 > 0.0 ? sc->rh : 0.0;
+                double *vn = comps(Vl + (int64_t)(j + 1) * ldv);
+                for (int i = threadIdx.x; i < 2 * cnt; i += NT - 32) {
+                    const double v = comps(w_s)[i] * inv_hn;
+                    vn[i] = v;
+                    // the global copy of v_j was last read by the products before
+                    // this step's first reduction barrier
+                    if (VS) comps(a.V + lo)[i] = v;
                 }
-                const double2 u = col[j], v = col[j + 1];
-                const double nu = hypot(u.x, u.y), nv = hypot(v.x, v.y);
-                double c;
-                double2 s, r;
-                if (nv == 0.0) {
-                    c = 1.0;
-                    s = make_double2(0.0, 0.0);
-                    r = u;
-                } else if (nu == 0.0) {
-                    c = 0.0;
-                    s = make_double2(v.x / nv, -v.y / nv);
-                    r = make_double2(nv, 0.0);
-                } else {
-                    const double nrm = hypot(nu, nv);
-                    const double2 al = make_double2(u.x / nu, u.y / nu);
-                    c = nu / nrm;
-                    const double2 t = cmul(al, cconj(v));
-                    s = make_double2(t.x / nrm, t.y / nrm);
-                    r = make_double2(al.x * nrm, al.y * nrm);
-                }
-                cs[j] = c;
-                sn[j] = s;
-                col[j] = r;
-                col[j + 1] = make_double2(0.0, 0.0);
-                const double2 gj = g[j], gj1 = g[j + 1];
-                const double2 sg = cmul(s, gj1), ug = cmul(cconj(s), gj);
-                g[j] = make_double2(c * gj.x + sg.x, c * gj.y + sg.y);
-                g[j + 1] = make_double2(-ug.x + c * gj1.x, -ug.y + c * gj1.y);
-                sc->res = hypot(g[j + 1].x, g[j + 1].y);
-                sc->hn = hn;
+            } else if (lane == 0) {
+                rot = last_rotation(H[(int64_t)j * (m + 1) + j], sc->na2, sc->ia, hn2, sc->rh, sc->in);
+                sc->res *= rot.q;   // (|g_{j+1}|: g_{j+1} was 0)
                 sc->jdone = j + 1;
-                sc->done = (sc->res <= tol || hn == 0.0) ? 1 : 0;
+                sc->done = (sc->res <= tol || hn2 == 0.0) ? 1 : 0;
             }
             __syncthreads();
-            // v_{j+1} = w / h_{j+1,j}
-            const double hn = sc->hn;
-            const double inv_hn = hn > 0.0 ? 1.0 / hn : 0.0;
-            double2 *vn = Vl + (int64_t)(j + 1) * ldv;
-            for (int i = threadIdx.x; i < cnt; i += NT) {
-                const double2 v = make_double2(w_s[i].x * inv_hn, w_s[i].y * inv_hn);
-                vn[i] = v;
-                // the global copy of v_j was last read by the products before
-                // this step's first reduction barrier
-                if (VS) a.V[lo + i] = v;
+            const bool done = sc->done;
+            if (last && lane == 0) {   // (read by this warp, or after a barrier)
+                double2 *col = H + (int64_t)j * (m + 1);
+                cs[j] = rot.c;
+                sn[j] = rot.sn;
+                col[j] = rot.r;
+                col[j + 1] = make_double2(0.0, 0.0);
+                const double2 gj = g[j], ug = cmul(cconj(rot.sn), gj);
+                g[j] = make_double2(rot.c * gj.x, rot.c * gj.y);
+                g[j + 1] = make_double2(-ug.x, -ug.y);
             }
-            if (sc->done) break;
+            if (done) break;
         }
         // y = R^{-1} g; x += V y (this CTA's rows)
+        __syncthreads();
         const int jd = sc->jdone;
-        if (threadIdx.x == 0) {
-            const int ld = m + 1;
-            for (int k = jd - 1; k >= 0; --k) {
-                double2 acc = g[k];
-                for (int l = k + 1; l < jd; ++l) {
-                    const double2 t = cmul(H[(int64_t)l * ld + k], y[l]);
-                    acc.x -= t.x;
-                    acc.y -= t.y;
-                }
-                const double2 d = H[(int64_t)k * ld + k];
-                const double den = d.x * d.x + d.y * d.y;
-                y[k] = make_double2((acc.x * d.x + acc.y * d.y) / den, (acc.y * d.x - acc.x * d.y) / den);
-            }
+        if (threadIdx.x < 32) {
+            for (int k = lane; k < jd; k += 32) y[k] = g[k];
+            __syncwarp();
+            back_substitute(H, m + 1, jd, y, lane);
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < cnt; i += NT) {
-            double2 xv = a.x[lo + i];
-            for (int c = 0; c < jd; ++c) {
-                const double2 v = Vl[(int64_t)c * ldv + i], yc = y[c];
-                xv.x += v.x * yc.x - v.y * yc.y;
-                xv.y += v.x * yc.y + v.y * yc.x;
-            }
-            a.x[lo + i] = xv;
+        for (int i = threadIdx.x; i < 2 * cnt; i += NT) {
+            double v = comps(a.x + lo)[i];
+#pragma unroll 4
+            for (int c = 0; c < jd; ++c) v = mul_step(v, Vl[(int64_t)c * ldv + (i >> 1)], y[c], i & 1);
+            comps(a.x + lo)[i] = v;
         }
         it += jd;
         matvecs += jd;
@@ -501,10 +447,10 @@ __global__ void __launch_bounds__(Sync::kThreads, 1) csr_gmres_one_kernel(CgArgs
     S.finish();
 }
 
-size_t smem_bytes(int64_t rows_per, int m, bool vs, int threads) {
+size_t smem_bytes(int64_t rows_per, int m, bool vs) {
     const size_t c2 = (size_t)rows_per * (vs ? m + 2 : 1) + 3 * (m + 2) + 3 * (m + 2) + (size_t)(m + 1) * m +
                       (m + 1) + m;
-    return c2 * 16 + (size_t)m * 8 + (size_t)(threads / 32) * 8 + sizeof(CgScalars) + 16;
+    return c2 * 16 + (size_t)m * 8 + sizeof(CgScalars) + 16;
 }
 
 // Whether kernel `kern` launches with `blocks` CTAs of `threads` threads and
@@ -597,7 +543,7 @@ bool csr_gmres_one_launch(Ctx &c, const CsrSystem &A, const double2 *b, double2 
     size_t smem = 0;
     for (const auto &cd : cands) {
         const int64_t rp = (n + cd.second - 1) / cd.second;
-        const size_t sm = smem_bytes(rp, m, cd.first.vs, cd.first.threads);
+        const size_t sm = smem_bytes(rp, m, cd.first.vs);
         if (sm > kMaxSmem || !launch_fits(cd.first.kern, cd.first.cluster, c.device, c.num_sms, sm, cd.second,
                                           cd.first.threads))
             continue;

@@ -18,6 +18,7 @@
 #include "bie_internal.h"
 #include "bie_device.cuh"
 #include "bie_fix64.cuh"
+#include "bie_krylov.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -435,9 +436,7 @@ inline RowSplit row_split(int64_t n) {
     const int64_t rows = 32 * std::max<int64_t>(1, (n + 32 * kRedBlocks - 1) / (32 * kRedBlocks));
     return RowSplit{rows, (int)((n + rows - 1) / rows)};
 }
-// (a complex vector as components)
-__device__ __forceinline__ const double *comps(const double2 *p) { return reinterpret_cast<const double *>(p); }
-__device__ __forceinline__ double *comps(double2 *p) { return reinterpret_cast<double *>(p); }
+using namespace krylov;
 
 // done(i, sum over the groups g of term(i, g), the same of the row's other
 // component) for the components i of rows r0 .. r1; two groups share the terms
@@ -462,19 +461,6 @@ __device__ __forceinline__ void over_rows(int64_t r0, int64_t r1, double *red, T
     }
 }
 
-// sum over groups of L neighbouring lanes (L a power of two up to 32)
-__device__ __forceinline__ double lane_sum(double v, int L) {
-    for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-// lanes per component for ncol columns: the block's threads spread over them
-template <int T>
-__device__ __forceinline__ int lanes_per(int ncol) {
-    int L = 32;
-    while (L > 1 && L * 2 * ncol > T) L >>= 1;
-    return L;
-}
-
 // partial[c nb + block] = sum over rows r0 .. r1 of conj(V[:, c]) w
 template <int T>
 __device__ __forceinline__ void block_dots(const double2 *__restrict__ V, int64_t ldv, int ncol, const double2 *w,
@@ -488,9 +474,7 @@ __device__ __forceinline__ void block_dots(const double2 *__restrict__ V, int64_
             const double2 *v = V + (int64_t)c * ldv;
 #pragma unroll 8
             for (int64_t i = r0 + lane; i < r1; i += L) {
-                const double2 a = v[i], b = w[i];
-                s = fma(a.x, im ? b.y : b.x, s);
-                s = fma(im ? -a.y : a.y, im ? b.x : b.y, s);
+                s = dot_step(s, v[i], w[i], im);
             }
         }
         s = lane_sum(s, L);
@@ -582,11 +566,7 @@ gm_product_kernel(Sliced p, int64_t n, int64_t rows, double2 *y, const double2 *
                     v = comps(y)[i];
                 } else {
                     v = fma(im ? p.sc.y : -p.sc.y, o, p.sc.x * s);
-                    if (p.d) {
-                        const double2 dv = p.d[i >> 1], xv = p.x[i >> 1];
-                        v = fma(dv.x, im ? xv.y : xv.x, v);
-                        v = fma(im ? dv.y : -dv.y, im ? xv.x : xv.y, v);
-                    }
+                    if (p.d) v = mul_step(v, p.d[i >> 1], p.x[i >> 1], im);
                 }
                 if (rhs) v = comps(rhs)[i] - v;
                 if (p.S > 0 || rhs) comps(y)[i] = v;
@@ -638,11 +618,6 @@ struct GmState {
     int m;
 };
 
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
-
 // out = a w over the block's rows
 __device__ __forceinline__ void scale_rows(const double2 *__restrict__ w, double a, int64_t n, int64_t rows,
                                            double2 *__restrict__ out) {
@@ -681,9 +656,7 @@ gm_start_kernel(GmState st, double tol, const double *__restrict__ norms, int nb
 }
 
 // Column j of H before its last rotation: the two passes' coefficients with the
-// rotations of the columns before applied.  Each rotation is one pass of four
-// lanes of a warp (the two components of both results): three FP64 operations
-// in a row instead of twelve.
+// rotations of the columns before applied.
 template <int T>
 __device__ __forceinline__ void gm_rotate_column(const GmState &st, int j, const double2 *h2) {
     __shared__ double2 s_col[kHs + 1], s_sn[kHs + 1];
@@ -701,23 +674,7 @@ __device__ __forceinline__ void gm_rotate_column(const GmState &st, int j, const
         }
     }
     __syncthreads();
-    if (threadIdx.x < 4) {
-        // lanes 0, 1: the components of -conj(sn) a + c b, which the next rotation
-        // takes; lanes 2, 3: those of c a + sn b, the finished entry
-        const bool im = threadIdx.x & 1, fin = threadIdx.x & 2;
-        double2 a = col[0];
-        for (int k = 0; k < j; ++k) {
-            const double2 b = col[k + 1], s = sn[k];
-            const double c = cs[k];
-            const double2 p = fin ? a : b, q = fin ? b : a;
-            double v = c * (im ? p.y : p.x);
-            v = fma(fin ? s.x : -s.x, im ? q.y : q.x, v);
-            v = fma(im ? s.y : -s.y, im ? q.x : q.y, v);
-            if (fin) comps(col)[2 * k + im] = v;
-            a = make_double2(__shfl_sync(0xfu, v, 0), __shfl_sync(0xfu, v, 1));
-        }
-        if (threadIdx.x == 0) col[j] = a;
-    }
+    if (threadIdx.x < 4) rotate_column(col, sn, cs, j, threadIdx.x);
     __syncthreads();
     if (small)
         for (int k = threadIdx.x; k <= j; k += T) out[k] = col[k];
@@ -754,9 +711,7 @@ gm_update_kernel(GmState st, const double2 *__restrict__ V, int ncol, const doub
             double s = 0;
 #pragma unroll 8
             for (int c = g; c < ncol; c += kGroups<T>) {
-                const double2 v = V[(int64_t)c * n + (i >> 1)], hc = h[c];
-                s = fma(v.x, im ? hc.y : hc.x, s);
-                s = fma(im ? v.y : -v.y, im ? hc.x : hc.y, s);
+                s = mul_step(s, V[(int64_t)c * n + (i >> 1)], h[c], im);
             }
             return s;
         },
@@ -775,9 +730,8 @@ gm_update_kernel(GmState st, const double2 *__restrict__ V, int ncol, const doub
 
 // The last rotation of Arnoldi step j, residual estimate and stop test (cs
 // real, sn complex), by one block: a = col[j] of H, hn2 = |w|^2.  Warps share the
-// square roots, whose FP64 operations no warp can overlap.  The squares are
-// those of norms taken as roots of a sum of squares, so a scaled hypot would not
-// widen the range; |g_j| is the residual before the step.
+// square roots, whose FP64 operations no warp can overlap.  |g_j| is the
+// residual before the step.
 __device__ __forceinline__ void gm_givens(const GmState &st, int j, const double *__restrict__ norms, int nb) {
     __shared__ double red[1], s_na2, s_ia, s_rh;
     GmScalars &s = *st.s;
@@ -793,35 +747,17 @@ __device__ __forceinline__ void gm_givens(const GmState &st, int j, const double
     if (threadIdx.x == 0) in = rsqrt(na2 + hn2);
     __syncthreads();
     if (threadIdx.x > 0) return;
-    double c, q;
-    double2 sn, r;
-    if (hn2 == 0.0) {
-        c = 1.0;
-        q = 0.0;
-        sn = make_double2(0.0, 0.0);
-        r = a;
-    } else if (na2 == 0.0) {
-        c = 0.0;
-        q = 1.0;
-        sn = make_double2(1.0, 0.0);
-        r = make_double2(hn2 * s_rh, 0.0);
-    } else {
-        c = na2 * ia * in;
-        q = hn2 * s_rh * in;
-        const double t = q * ia, u = (na2 + hn2) * in * ia;
-        sn = make_double2(a.x * t, a.y * t);
-        r = make_double2(a.x * u, a.y * u);
-    }
-    const double res = s.res * q;
+    const Rotation rot = last_rotation(a, na2, ia, hn2, s_rh, in);
+    const double res = s.res * rot.q;
     s.res = res;
     s.jdone = j + 1;
     if (res <= s.tol || hn2 == 0.0 || j + 1 >= s.jmax) s.done = 1;
-    st.cs[j] = c;
-    st.sn[j] = sn;
-    col[j] = r;
+    st.cs[j] = rot.c;
+    st.sn[j] = rot.sn;
+    col[j] = rot.r;
     col[j + 1] = make_double2(0.0, 0.0);
-    const double2 ug = cmul(cconj(sn), gj);
-    st.g[j] = make_double2(c * gj.x, c * gj.y);
+    const double2 ug = cmul(cconj(rot.sn), gj);
+    st.g[j] = make_double2(rot.c * gj.x, rot.c * gj.y);
     st.g[j + 1] = make_double2(-ug.x, -ug.y);
 }
 
@@ -854,30 +790,7 @@ __global__ void __launch_bounds__(32) gm_trisolve_kernel(GmState st) {
 #pragma unroll 8
         for (int k = 0; k < j; ++k) s_R[k * kS + lane] = st.H[(int64_t)k * ld + lane];
     __syncwarp();
-    double2 inv = make_double2(0.0, 0.0);   // 1 / R(lane, lane)
-    if (small && lane < j) {
-        const double2 d = R[(int64_t)lane * ldr + lane];
-        const double i = 1.0 / fma(d.x, d.x, d.y * d.y);
-        inv = make_double2(d.x * i, -d.y * i);
-    }
-    for (int k = j - 1; k >= 0; --k) {
-        double2 ik;
-        if (small) {
-            ik = make_double2(__shfl_sync(0xffffffffu, inv.x, k), __shfl_sync(0xffffffffu, inv.y, k));
-        } else {
-            const double2 d = R[(int64_t)k * ldr + k];
-            const double den = fma(d.x, d.x, d.y * d.y);
-            ik = make_double2(d.x / den, -d.y / den);
-        }
-        const double2 yk = cmul(y[k], ik);
-        __syncwarp();
-        if (lane == 0) y[k] = yk;
-        for (int l = lane; l < k; l += 32) {
-            const double2 t = cmul(R[(int64_t)k * ldr + l], yk);
-            y[l] = make_double2(y[l].x - t.x, y[l].y - t.y);
-        }
-        __syncwarp();
-    }
+    back_substitute(R, ldr, j, y, lane);
     if (small)
         for (int k = lane; k < j; k += 32) st.y[k] = y[k];
 }
