@@ -142,41 +142,34 @@ assemble_fp64_kernel(const double *__restrict__ rec, int stride, int nidx_off,
 
 // C at points off the surface: the sums cancel there to the quadrature error, so
 // C keeps K1's FP64 operations and order while F and G come from the
-// fixed-point kernel.  A quarter of K1's FP64 instructions per point.
+// fixed-point kernel.  A quarter of K1's FP64 instructions per point, bound by the
+// FP64 pipe (1.3 ms for 1333 points and 1280 elements with 9-point rules).  A few
+// warps per SM keep that pipe busy, so it runs beside the fixed-point kernel (1.9
+// ms, which hardly uses FP64) on two blocks of 64 registers per SM, each going
+// through its share of the (row tile, slice) pairs: F, G and C 3.27 -> 2.41 ms
+// (one block per SM 2.49, three 2.67).
 template <int NP>
-__global__ void __launch_bounds__(kThreads)
-field_c_fp64_kernel(const double *__restrict__ rec, int stride, int64_t E, int S,
+__global__ void __launch_bounds__(kThreads, 8)
+field_c_fp64_kernel(const double *__restrict__ rec, int stride, int64_t E, int S, int tiles,
                     const __grid_constant__ RuleInfo ri, const double *__restrict__ tgt, int64_t M,
-                    double *__restrict__ Cpart, int chunk) {
-    extern __shared__ __align__(16) double s_rec[];
+                    double *__restrict__ Cpart) {
     __shared__ RuleInfo s_ri;
     if (threadIdx.x == 0) s_ri = ri;
-    const int s = blockIdx.y;
-    const int64_t e0 = (int64_t)s * E / S, e1 = (int64_t)(s + 1) * E / S;
-    const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    const bool active = i < M;
-    double tx = 0, ty = 0, tz = 0;
-    if (active) {
-        tx = tgt[3 * i + 0];
-        ty = tgt[3 * i + 1];
-        tz = tgt[3 * i + 2];
-    }
-    double cacc = 0.0;
-    for (int64_t cb = e0; cb < e1; cb += chunk) {
-        const int n = (int)min((int64_t)chunk, e1 - cb);
-        __syncthreads();
-        const double2 *src = reinterpret_cast<const double2 *>(rec + cb * stride);
-        double2 *dst = reinterpret_cast<double2 *>(s_rec);
-        for (int t = threadIdx.x; t < n * stride / 2; t += kThreads) dst[t] = src[t];
-        __syncthreads();
-        if (!active) continue;
-        for (int el = 0; el < n; ++el) {
-            const double *r = s_rec + (size_t)el * stride;
+    __syncthreads();
+    for (int64_t job = blockIdx.x; job < (int64_t)tiles * S; job += gridDim.x) {
+        const int s = (int)(job / tiles);
+        const int64_t e0 = (int64_t)s * E / S, e1 = (int64_t)(s + 1) * E / S;
+        const int64_t i = (job - (int64_t)s * tiles) * kThreads + threadIdx.x;
+        if (i >= M) continue;
+        const double tx = tgt[3 * i], ty = tgt[3 * i + 1], tz = tgt[3 * i + 2];
+        double cacc = 0.0;
+        for (int64_t el = e0; el < e1; ++el) {
+            const double *r = rec + el * stride;
             const int c = dev::nearest_node<NP>(r, tx, ty, tz);
             cacc += dev::element_c_fp64(r + s_ri.off[c], s_ri.Q[c], tx, ty, tz);
         }
+        Cpart[(int64_t)s * M + i] = cacc;
     }
-    if (active) Cpart[(int64_t)s * M + i] = cacc;
 }
 
 template <int NP, bool CPLX>
@@ -321,25 +314,39 @@ void launch_assemble_fp64(Ctx &c, const AssembleArgs &a) {
     if (a.flags & BIE_C) launch_reduce_c(c, Cpart, S, nullptr, a.M, a.C);
 }
 
-void launch_field_c_fp64(Ctx &c, const double *targets, int64_t M, double *C) {
+void launch_field_c_fp64(Ctx &c, const double *targets, int64_t M, double *C, bool beside) {
     const RecordLayout &L = c.lay;
     const int level = choose_slice_level(c, M, kThreads), S = 1 << level;
-    const size_t rec_bytes = (size_t)L.stride * sizeof(double);
-    const int chunk = (int)std::max<size_t>(1, std::min<size_t>(64, (40u << 10) / rec_bytes));
-    const size_t smem = (size_t)chunk * rec_bytes;
-    double *Cpart = static_cast<double *>(c.scratch(kScratchCpart, (size_t)S * M * sizeof(double)));
+    // (beside another assembly of the call: its own partial sums)
+    double *Cpart = static_cast<double *>(
+        c.scratch(beside ? kScratchFieldC : kScratchCpart, (size_t)S * M * sizeof(double)));
     RuleInfo ri{};
     for (int r = 0; r < L.R; ++r) {
         ri.Q[r] = L.Q[r];
         ri.off[r] = L.rule_off[r];
     }
+    const int tiles = (int)((M + kThreads - 1) / kThreads);
+    const int64_t jobs = (int64_t)tiles * S;
+    if (beside && !c.side_stream) {
+        for (auto &e : c.side_ev) BIE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        BIE_CUDA(cudaStreamCreateWithFlags(&c.side_stream, cudaStreamNonBlocking));
+    }
+    const cudaStream_t st = beside ? c.side_stream : c.stream;
+    if (beside) {
+        BIE_CUDA(cudaEventRecord(c.side_ev[0], c.stream));
+        BIE_CUDA(cudaStreamWaitEvent(st, c.side_ev[0], 0));
+    }
     auto kern = L.NP == 1 ? field_c_fp64_kernel<1> : (L.NP == 3 ? field_c_fp64_kernel<3> : field_c_fp64_kernel<6>);
-    BIE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<dim3((unsigned)((M + kThreads - 1) / kThreads), (unsigned)S), kThreads, smem, c.stream>>>(
-        c.d_records, L.stride, c.n_elements, S, ri, targets, M, Cpart, chunk);
+    // (an SM changes its shared-memory split only when idle: without this the two
+    // kernels never share one)
+    BIE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  cudaSharedmemCarveoutMaxShared));
+    kern<<<(unsigned)(beside ? std::min<int64_t>(jobs, 2LL * c.num_sms) : jobs), kThreads, 0, st>>>(
+        c.d_records, L.stride, c.n_elements, S, tiles, ri, targets, M, Cpart);
     BIE_CUDA(cudaGetLastError());
     ++c.kernel_launches;
-    launch_reduce_c(c, Cpart, S, nullptr, M, C);
+    launch_reduce_c(c, Cpart, S, nullptr, M, C, st);
+    if (beside) BIE_CUDA(cudaEventRecord(c.side_ev[1], st));
 }
 
 // ---------------------------------------------------------------------------
@@ -352,15 +359,45 @@ __global__ void reduce_c_kernel(const double *__restrict__ Cpart, int S,
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M) return;
     double acc = 0.0;
+#pragma unroll 16
     for (int s = 0; s < S; ++s) acc += Cpart[(int64_t)s * M + i];
+    if (Cextra) acc += Cextra[i];
+    C[i] = make_double2(acc, 0.0);
+}
+
+// ... with the slices of a row shared by eight warps (up to 2432 slices)
+__global__ void __launch_bounds__(256)
+reduce_c_groups_kernel(const double *__restrict__ Cpart, int S, const double *__restrict__ Cextra, int64_t M,
+                       double2 *__restrict__ C) {
+    __shared__ double part[8][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int64_t i = (int64_t)blockIdx.x * 32 + lane;
+    double acc = 0.0;
+    if (i < M)
+#pragma unroll 16
+        for (int s = g; s < S; s += 8) acc += Cpart[(int64_t)s * M + i];
+    part[g][lane] = acc;
+    __syncthreads();
+    if (g > 0 || i >= M) return;
+#pragma unroll
+    for (int k = 1; k < 8; ++k) acc += part[k][lane];
     if (Cextra) acc += Cextra[i];
     C[i] = make_double2(acc, 0.0);
 }
 }  // namespace
 
 void launch_reduce_c(Ctx &c, const double *Cpart, int S, const double *Cextra, int64_t M,
-                     double *C) {
-    reduce_c_kernel<<<(unsigned)((M + 255) / 256), 256, 0, c.stream>>>(
+                     double *C, cudaStream_t st, bool any_order) {
+    if (any_order) {
+        reduce_c_groups_kernel<<<(unsigned)((M + 31) / 32), 256, 0, st ? st : c.stream>>>(
+            Cpart, S, Cextra, M, reinterpret_cast<double2 *>(C));
+        BIE_CUDA(cudaGetLastError());
+        ++c.kernel_launches;
+        return;
+    }
+    // (small blocks over all SMs, 16 loads in flight: the sums of 128 slices are FP64
+    // additions in a row)
+    reduce_c_kernel<<<(unsigned)((M + 31) / 32), 32, 0, st ? st : c.stream>>>(
         Cpart, S, Cextra, M, reinterpret_cast<double2 *>(C));
     BIE_CUDA(cudaGetLastError());
     ++c.kernel_launches;

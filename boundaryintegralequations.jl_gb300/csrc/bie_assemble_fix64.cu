@@ -305,7 +305,8 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
             const int *ir = reinterpret_cast<const int *>(r);
             fix64::Pair P;
             const FxPairInfo I = fx_pair<NP, CPLX_K>(r, T, wv, P.Dx, P.Dy, P.Dz);
-            const uint32_t fw = __ldg(kflags + pe);
+            // (no flags: every node shared)
+            const uint32_t fw = kflags ? __ldg(kflags + pe) : 0x00ff0000u;
             const int ej = ir[kHdrEj];
             const float *abs_nodes = r + kHdrNodes + 3 * NP;
             const int *node_ej = ir + kHdrNodes + 6 * NP;
@@ -464,14 +465,14 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
     if ((threadIdx.x & 31) == 0 && nqpe) atomicAdd(qpe_count, nqpe);
 }
 
-// Columns of the nodes shared between slices (and of untouched nodes): zeroed
-// before the assembly, converted after it.
+// Columns of the nodes shared between slices (and of untouched nodes; without a
+// list, of all nodes): zeroed before the assembly, converted after it.
 __global__ void fx_zero_kernel(const int32_t *__restrict__ fnode, int64_t nfix, int64_t M, longlong2 *__restrict__ F,
                                longlong2 *__restrict__ G) {
     const int64_t total = nfix * M;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t n = t / M;
-        const size_t off = (size_t)fnode[n] * (size_t)M + (size_t)(t - n * M);
+        const size_t off = (size_t)(fnode ? fnode[n] : n) * (size_t)M + (size_t)(t - n * M);
         if (F) F[off] = make_longlong2(0, 0);
         if (G) G[off] = make_longlong2(0, 0);
     }
@@ -493,7 +494,7 @@ __global__ void fx_widen_kernel(const int32_t *__restrict__ fnode, int64_t nfix,
     const int64_t total = nfix * M;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t n = t / M, i = t - n * M;
-        const int32_t nd = fnode[n];
+        const int64_t nd = fnode ? fnode[n] : n;
         const size_t off = (size_t)nd * (size_t)M + (size_t)i;
         const float4 x = nodes[nd];
         const float fx = (float)((tgt[3 * i] - sc.x0[0]) * sc.inv), fy = (float)((tgt[3 * i + 1] - sc.x0[1]) * sc.inv),
@@ -602,7 +603,7 @@ struct FxBuffers {
 };
 
 template <int NP, bool CPLX>
-void launch_np(Ctx &c, const AssembleArgs &a, const LaunchShape &sh, size_t smem, const FxBuffers &b) {
+void launch_np(Ctx &c, const AssembleArgs &a, const LaunchShape &sh, int spread, size_t smem, const FxBuffers &b) {
     const RecordLayout &L = c.lay;
     const Fix64Layout &X = c.xlay;
     RuleInfo ri{}, ri64{};
@@ -629,11 +630,11 @@ void launch_np(Ctx &c, const AssembleArgs &a, const LaunchShape &sh, size_t smem
         ++c.kernel_launches;
     }
     const Fp64View v{c.d_records, L.stride, L.nidx_off, c.d_phi, L.qmax, ri64, c.d_xtrig};
-    const int level = sh.level, S = 1 << level;
-    const int64_t E = c.n_elements, nfix = c.k2_nfix[level];
+    const int level = sh.level, S = spread ? spread : 1 << level;
+    const int64_t E = c.n_elements, nfix = spread ? c.n_sources : c.k2_nfix[level];
     longlong2 *F = (a.flags & BIE_F) ? reinterpret_cast<longlong2 *>(a.F) : nullptr;
     longlong2 *G = (a.flags & BIE_G) ? reinterpret_cast<longlong2 *>(a.G) : nullptr;
-    const int32_t *fnode = c.d_k2_fix + c.k2_fix_off[level];
+    const int32_t *fnode = spread ? nullptr : c.d_k2_fix + c.k2_fix_off[level];
     if (nfix > 0 && (F || G)) {
         fx_zero_kernel<<<stream_grid(c, nfix * a.M), 256, 0, c.stream>>>(fnode, nfix, a.M, F, G);
         BIE_CUDA(cudaGetLastError());
@@ -650,7 +651,7 @@ void launch_np(Ctx &c, const AssembleArgs &a, const LaunchShape &sh, size_t smem
         phi_groups(L.qmax), ri,
         reinterpret_cast<const int4 *>(c.d_xtrig),
         reinterpret_cast<const int2 *>(c.d_xtrig + 4 * fix64::kTrigEntries), a.targets, a.M, a.k_re, a.k_im, a.flags, F, G,
-        c.d_k2_flags + (size_t)level * E, b.Cpart, b.defer, b.dcount, b.dcap, b.over, gw, sc, c.d_qpe, a.k_dev);
+        spread ? nullptr : c.d_k2_flags + (size_t)level * E, b.Cpart, b.defer, b.dcount, b.dcap, b.over, gw, sc, c.d_qpe, a.k_dev);
     BIE_CUDA(cudaGetLastError());
     c.timer_end(t0);
     ++c.kernel_launches;
@@ -881,7 +882,7 @@ void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
     c.fx_ok = true;
 }
 
-bool fix64_covers(const Ctx &c, const AssembleArgs &a) {
+static bool fix64_covers(const Ctx &c, const AssembleArgs &a) {
     if (!c.fx_ok || a.taylor_m >= 0 || (a.g_weight && a.g_weight_exp == INT32_MIN)) return false;
     if (a.k_dev && !(a.k_abs_max > 0)) return false;   // no bound on |k|
     const bool cplx = a.k_im != 0.0;
@@ -893,18 +894,39 @@ bool fix64_covers(const Ctx &c, const AssembleArgs &a) {
     return kr < 500.0 && ki < 100.0 && ki * c.fx_rho_max * 1.45 < fix64::kMaxDampSpread;
 }
 
+static bool on_nodes(const Ctx &c, const AssembleArgs &a) {
+    return a.targets >= c.d_sources && a.targets + 3 * a.M <= c.d_sources + 3 * c.n_sources;
+}
+
+// Where the double-float kernel is available (BIE_PREC_DF64), the fixed-point one
+// takes the node rows of 4-point rules: its entries cost less, its points more.
+// Against the double-float kernel, 320 to 8000 elements: 4-point rules 1.09 to
+// 1.65 times as fast (complex k 1.03 to 1.5, 0.92 to 1.3 on 320 elements); 9- and
+// 16-point rules 0.85 to 1.15 (complex k 0.57 to 1.14); targets off the surface,
+// where C takes a pass of its own, 0.6 to 1.2 (complex k 0.35 to 1.2).
+bool fix64_takes(const Ctx &c, const AssembleArgs &a, bool df64) {
+    if (df64 && !(on_nodes(c, a) && c.lay.Q[0] <= 4 && (a.k_im == 0.0 || c.n_elements >= 512))) return false;
+    return fix64_covers(c, a);
+}
+
 bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df64) {
-    if (!fix64_covers(c, args)) return false;
+    if (!fix64_takes(c, args, df64)) return false;
     AssembleArgs a = args;
     const bool cplx = a.k_im != 0.0;
     // C at points off the surface cancels to the quadrature error, where any other
-    // rounding would show: it keeps the FP64 (double-float) operations
-    const bool nodes = a.targets >= c.d_sources && a.targets + 3 * a.M <= c.d_sources + 3 * c.n_sources;
-    if ((a.flags & BIE_C) && !nodes) {
-        AssembleArgs f = a;
-        f.flags = BIE_C;
-        f.F = f.G = nullptr;
-        if (!(df64 && launch_assemble_k9(c, f))) launch_field_c_fp64(c, a.targets, a.M, a.C);
+    // rounding would show: it keeps the FP64 operations
+    struct Join {   // the call's stream waits for the side stream, whatever happens in between
+        Ctx &c;
+        bool on = false;
+        ~Join() {
+            if (on) cudaStreamWaitEvent(c.stream, c.side_ev[1], 0);
+        }
+    } join{c};
+    if ((a.flags & BIE_C) && !on_nodes(c, a)) {
+        // beside the fixed-point kernel (side streams are made outside captures)
+        const bool beside = (a.flags & (BIE_F | BIE_G)) && (c.side_stream || !c.capturing);
+        launch_field_c_fp64(c, a.targets, a.M, a.C, beside);
+        join.on = beside;
         a.flags &= ~BIE_C;
     }
     if (!(a.flags & (BIE_F | BIE_G | BIE_C))) return true;
@@ -919,8 +941,26 @@ bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df64) {
     auto reset = [&] { BIE_CUDA(cudaMemsetAsync(dbuf + dbytes, 0, 256 + (size_t)a.M * 8, c.stream)); };
     reset();
 
+    // The finest slicing with at least four elements per slice: blocks differ in
+    // cost (near pairs leave points out, midpoint rules add some), so many small
+    // ones even out.  Step at 128 / 64 / 32 slices: pulsating sphere 20.8 / 21.2 /
+    // 22.0 ms, rigid sphere P2 11.3 / 11.4 / 12.0, 5762 nodes P2 3.20 / 3.30 / 3.55,
+    // 362 nodes with 16-point rules 0.22 / 0.29 / 0.40.
+    int level = 0;
+    while (level + 1 < kMaxLevels && (c.n_elements >> (level + 1)) >= 4) ++level;
+    // Few rows do not fill the SMs with that (a pair takes microseconds, one after
+    // the other on its thread): four waves of blocks, on slices down to single
+    // elements, with every node shared (integer atomics).  8000 elements, 40 / 700 /
+    // 1333 / 2600 rows against the slices above: P2 with 16-point rules 2.00 -> 0.56,
+    // 6.0 -> 4.1, 8.4 -> 7.3, 14.4 -> 13.9 ms, P1 with 4-point rules 0.29 -> 0.13, 0.84
+    // -> 0.71, 1.33 -> 1.26, 2.29 -> 2.36; without shared nodes, whose entries need no
+    // atomics otherwise, 0.29 -> 0.15, 130 rows 0.37 -> 0.32, but 300 rows 0.45 -> 0.54.
+    const int64_t tiles = (a.M + kThreads - 1) / kThreads, resident = 4LL * c.num_sms;
+    // (BIE_PREC_DF64 keeps its tunable slices)
+    const bool few = !df64 && tiles << level <= (c.k2_nfix[level] > 0 ? 3 * resident : resident / 2);
+    const int spread = few ? (int)std::min<int64_t>(c.n_elements, 4 * resident / tiles) : 0;
     auto run = [&](const LaunchShape &sh) {
-        const int S = 1 << sh.level;
+        const int S = spread ? spread : 1 << sh.level;
         // phase table, point values of the block's threads, basis tables
         const size_t smem = ((size_t)fix64::kTrigEntries + 2 * kGroup * kThreads +
                              (size_t)L.R * phi_groups(L.qmax) * L.NP * 2) * 16 +
@@ -931,24 +971,17 @@ bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df64) {
         b.Cpart = reinterpret_cast<double *>(part);
         b.over = reinterpret_cast<int *>(part + cp);
         if (L.NP == 1) {
-            if (cplx) launch_np<1, true>(c, a, sh, smem, b);
-            else launch_np<1, false>(c, a, sh, smem, b);
+            if (cplx) launch_np<1, true>(c, a, sh, spread, smem, b);
+            else launch_np<1, false>(c, a, sh, spread, smem, b);
         } else if (L.NP == 3) {
-            if (cplx) launch_np<3, true>(c, a, sh, smem, b);
-            else launch_np<3, false>(c, a, sh, smem, b);
+            if (cplx) launch_np<3, true>(c, a, sh, spread, smem, b);
+            else launch_np<3, false>(c, a, sh, spread, smem, b);
         } else {
-            if (cplx) launch_np<6, true>(c, a, sh, smem, b);
-            else launch_np<6, false>(c, a, sh, smem, b);
+            if (cplx) launch_np<6, true>(c, a, sh, spread, smem, b);
+            else launch_np<6, false>(c, a, sh, spread, smem, b);
         }
-        if (a.flags & BIE_C) launch_reduce_c(c, b.Cpart, S, b.Cnear, a.M, a.C);
+        if (a.flags & BIE_C) launch_reduce_c(c, b.Cpart, S, b.Cnear, a.M, a.C, nullptr, true);
     };
-    // The finest slicing with at least four elements per slice: blocks differ in
-    // cost (near pairs leave points out, midpoint rules add some), so many small
-    // ones even out.  Step at 128 / 64 / 32 slices: pulsating sphere 20.8 / 21.2 /
-    // 22.0 ms, rigid sphere P2 11.3 / 11.4 / 12.0, 5762 nodes P2 3.20 / 3.30 / 3.55,
-    // 362 nodes with 16-point rules 0.22 / 0.29 / 0.40.
-    int level = 0;
-    while (level + 1 < kMaxLevels && (c.n_elements >> (level + 1)) >= 4) ++level;
     // (records are read through L1: the chunk is the double-float kernel's, which
     // shares the tuned shape)
     const int chunk0 = (int)std::max<size_t>(1, std::min<size_t>(32, (32u << 10) / ((size_t)c.dlay.stride * sizeof(float))));

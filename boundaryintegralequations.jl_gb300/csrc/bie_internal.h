@@ -109,7 +109,8 @@ enum ScratchSlot {
                                 // per level 1, 2 (solves inside another solve's product)
     kScratchFxWeight = 16, // fixed-point assembly: element factors as limbs
     kScratchK2Side = 17,   // mixed assembly: per-slice partial sums of nodes shared between slices
-    kScratchCount = 18
+    kScratchFieldC = 18,   // C at points off the surface, beside the fixed-point assembly: partial sums
+    kScratchCount = 19
 };
 
 // Mixed-precision element record (32-bit words, same element order as the FP64
@@ -176,6 +177,8 @@ struct Ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     bool owns_stream = true;             // false: the stream belongs to another context
+    cudaStream_t side_stream = nullptr;  // C at field points beside F and G
+    cudaEvent_t side_ev[2] = {};         // ... after the call's earlier work, ... done
     cudaStream_t copy_stream = nullptr;  // device-to-host copies overlapped with the assembly
                                          // (bie_assemble with host buffers), made on first use
     int num_sms = 0;
@@ -344,10 +347,12 @@ struct ShapeAxes {
 LaunchShape resolve_shape(Ctx &c, int kernel, int64_t M, const LaunchShape &base, const ShapeAxes &ax,
                           const std::function<void(const LaunchShape &)> &run, const std::function<void()> &reset);
 void launch_reduce_c(Ctx &c, const double *Cpart, int S, const double *Cextra, int64_t M,
-                     double *C);
+                     double *C, cudaStream_t st = nullptr, bool any_order = false);
 
 // C alone at targets off the surface, with K1's operations in K1's order
-void launch_field_c_fp64(Ctx &c, const double *targets, int64_t M, double *C);
+// beside: on c.side_stream, after the work on c.stream so far; the caller makes
+// c.stream wait for c.side_ev[1]
+void launch_field_c_fp64(Ctx &c, const double *targets, int64_t M, double *C, bool beside);
 
 // Matrix-free products yF = F x, yG = G v (bie_matvec.cu); all pointers device
 struct MatvecArgs {
@@ -597,7 +602,7 @@ bool launch_assemble_k9(Ctx &c, const AssembleArgs &a);   // the double-float ke
 // 2^+-300).  df64: BIE_PREC_DF64, which keeps its own slicing and off-surface C.
 void build_fix64_records(Ctx &c, const std::vector<double> &rec64);
 bool launch_assemble_fix64(Ctx &c, const AssembleArgs &a, bool df64);
-bool fix64_covers(const Ctx &c, const AssembleArgs &a);   // whether it launches
+bool fix64_takes(const Ctx &c, const AssembleArgs &a, bool df64);   // whether it launches
 
 // FMA throughput probe (bie_peaks.cu)
 void measure_peaks(int device, bie_peaks &out);

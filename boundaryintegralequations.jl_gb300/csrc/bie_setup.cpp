@@ -904,6 +904,15 @@ void destroy_context(Ctx &c) {
     c.ev_tensor.clear();
     c.ev_free.clear();
     c.d_qpe = nullptr;
+    if (c.side_stream) {
+        cudaStreamSynchronize(c.side_stream);
+        cudaStreamDestroy(c.side_stream);
+        c.side_stream = nullptr;
+    }
+    for (auto &e : c.side_ev) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
     if (c.copy_stream) {
         cudaStreamSynchronize(c.copy_stream);
         cudaStreamDestroy(c.copy_stream);

@@ -291,7 +291,8 @@ struct MeshRun {
     // before the recording, which sizes its scratch.
     void size_recorded(const double *ks, bool cplx) {
         const double ki = cplx ? 1.0 : 0.0;
-        if (!mixed && fix64_covers(c, assemble_args(ks[0], ks[1], nullptr)) != fix64_covers(c, assemble_args(0.0, ki, ks_d)))
+        if (!mixed && fix64_takes(c, assemble_args(ks[0], ks[1], nullptr), df64) !=
+                          fix64_takes(c, assemble_args(0.0, ki, ks_d), df64))
             assemble(0.0, ki, ks_d);
     }
     // amp[j] from y and A z

@@ -96,3 +96,23 @@ def test_graded_mesh():
     c = mesh.coordinates * s
     check(dataclasses.replace(mesh, coordinates=c, sources=c.copy()), 2.0, 2, 2)
 
+
+
+@pytest.mark.parametrize("geo,phys", [("linear", "geometry"), ("quadratic", "geometry"),
+                                      ("quadratic", "disctrilinear")])
+@pytest.mark.parametrize("k", [3.0, 2.0 + 0.4j])
+def test_few_rows_match_many(geo, phys, k):
+    """Few targets take slices down to single elements with every node shared, many
+    the flagged slices.  Every entry is a sum of the same integers, so rows agree
+    but for the FP64 additions of near pairs: some 30 at 2^-53 of the entries they
+    add to, below 1e-14 of the row."""
+    mesh = bm.icosphere(9, geometry=geo, physics=phys)
+    ctx = biegpu.get_context(mesh, n=2, m=2)
+    r = np.random.default_rng(4)
+    t = r.normal(size=(3, 2600))
+    t *= r.uniform(1.05, 4.0, 2600) / np.linalg.norm(t, axis=0)
+    F, G, _ = biegpu.assemble_parallel(mesh, k, t, n=2, m=2)
+    for M in (1, 40, 129, 300, 1792):
+        f, g, _ = biegpu.assemble_parallel(mesh, k, t[:, :M], n=2, m=2)
+        for a, b in ((f, F[:M]), (g, G[:M])):
+            assert np.max(np.abs(a - b) / np.max(np.abs(b), axis=1, keepdims=True)) <= 1e-14
