@@ -299,8 +299,11 @@ adjoint_grad_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
 // adjoint_grad_kernel is bound by the FP64 pipe (87 % busy, 79 ms for the
 // 4842-node ellipsoid, 46.9 M pairs).  Here the regular pairs run in double-float
 // (bie_df64.cuh) and only near pairs and nearest-node near-ties in FP64, in place:
-// 13.5 ms, bound by instruction issue (128 registers, 4 blocks per SM; two rows
-// per thread with one reduction for both took 19.7 ms at 255 registers).  Phases
+// 13.0 ms, bound by instruction issue and half by instruction fetch (128
+// registers, 16 warps per SM; two rows per thread with one reduction for both took
+// 19.7 ms at 255 registers): the loop over elements is longer than the
+// instruction caches, so the warps of a block stay together.  Whole gradient 28.2
+// ms without that, 26.9 in blocks of 128 threads, 25.8 of 256, 27.4 of 512.  Phases
 // are formed without cancellation, so gradients differ from the FP64 kernel's by
 // 3e-14 .. 8e-14, below the error of the solves (1e-13 .. 4e-13).  With
 // b = conj(w) p(x_q), z = b e^{ikr}, W = jw / 4 pi, n the unit normal, d = x_q - t,
@@ -418,7 +421,8 @@ __device__ __forceinline__ Acc warp_transpose_sum(Acc (&v)[32], int lane) {
     return v[0];
 }
 
-__global__ void __launch_bounds__(kT, 4)
+constexpr int kAT = 256;   // threads of the double-float reverse pass
+__global__ void __launch_bounds__(kAT, 512 / kAT)
 adjoint_df64_kernel(int64_t N, int64_t M, const double *__restrict__ src, const double *__restrict__ fpts,
                     const double2 *__restrict__ w, const double2 *__restrict__ p, const float *__restrict__ rec,
                     int stride, int nidx_off, const __grid_constant__ dev::RuleInfo ri,
@@ -433,14 +437,14 @@ adjoint_df64_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
     float *s_el = reinterpret_cast<float *>(s_ph + (size_t)chunk * 3 * qmax);    // chunk * 32: e_b, G0, centroid
     __shared__ dev::RuleInfo s_ri;
     if (threadIdx.x == 0) s_ri = ri;
-    for (int t = threadIdx.x; t < 3 * qmax * kAdjTab; t += kT) s_tab[t] = tab[t];
+    for (int t = threadIdx.x; t < 3 * qmax * kAdjTab; t += kAT) s_tab[t] = tab[t];
     const int lane = threadIdx.x & 31;
     const int s = blockIdx.y;
     const int64_t e0 = (int64_t)s * E / S, e1 = (int64_t)(s + 1) * E / S;
     const df K = dd::to_df(kre), K2 = dd::to_df(kre * kre);
     const float kf = K.hi, k3 = third(kre, K), k23 = third(kre * kre, K2);
 
-    const int64_t row = (int64_t)blockIdx.x * kT + threadIdx.x;
+    const int64_t row = (int64_t)blockIdx.x * kAT + threadIdx.x;
     const bool active = row < N + M, node = row < N;   // collocation row, else field row
     const float aF = node ? 1.0f : -1.0f;              // alpha_F, and the sign of alpha_G's factor
     double tx = 0, ty = 0, tz = 0;
@@ -463,10 +467,10 @@ adjoint_df64_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
         {
             const float4 *a = reinterpret_cast<const float4 *>(rec + cb * stride);
             float4 *b = reinterpret_cast<float4 *>(s_rec);
-            for (int t = threadIdx.x; t < n * stride / 4; t += kT) b[t] = a[t];
+            for (int t = threadIdx.x; t < n * stride / 4; t += kAT) b[t] = a[t];
         }
         __syncthreads();
-        for (int t = threadIdx.x; t < n * 3 * qmax; t += kT) {   // p at the points, in FP64
+        for (int t = threadIdx.x; t < n * 3 * qmax; t += kAT) {   // p at the points, in FP64
             const int el = t / (3 * qmax), c = (t - el * 3 * qmax) / qmax, q = t - el * 3 * qmax - c * qmax;
             const int32_t *nid = reinterpret_cast<const int32_t *>(s_rec + (size_t)el * stride + nidx_off);
             if (q >= s_ri.Q[c]) continue;
@@ -481,7 +485,7 @@ adjoint_df64_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
             const df x = dd::to_df(re), y = dd::to_df(im);
             s_ph[t] = make_float4(x.hi, x.lo, y.hi, y.lo);
         }
-        for (int t = threadIdx.x; t < n * 11; t += kT) {         // X_b - centroid, rhock (Im Y, -Re Y)
+        for (int t = threadIdx.x; t < n * 11; t += kAT) {         // X_b - centroid, rhock (Im Y, -Re Y)
             const int el = t / 11, j = t - el * 11;
             const float *r = s_rec + (size_t)el * stride;
             double x;
@@ -501,7 +505,11 @@ adjoint_df64_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
         }
         __syncthreads();
 
+#pragma unroll 1
         for (int el = 0; el < n; ++el) {
+            // (the warps stay together: the loop is longer than the instruction caches,
+            // and each would fetch it for itself)
+            __syncthreads();
             const float *r = s_rec + (size_t)el * stride;
             const float2 *se = reinterpret_cast<const float2 *>(s_el + 32 * el);
             const df G0r{se[9].x, se[9].y}, G0i{se[10].x, se[10].y};
@@ -518,7 +526,7 @@ adjoint_df64_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
                 for (int a = 0; a < 6; ++a) m[a] = Acc{0.f, 0.f};
 #pragma unroll
                 for (int a = 0; a < 3; ++a) sb[a] = Acc{0.f, 0.f};
-                                if (P.deferred || !(fabsf(kf * r0.hi) < df64::kDfMaxPhase)) {
+                if (P.deferred || !(fabsf(kf * r0.hi) < df64::kDfMaxPhase)) {
                     const cd g0 = {(double)G0r.hi + (double)G0r.lo, (double)G0i.hi + (double)G0i.lo};
                     const AdjPair o = adjoint_pair_fp64(
                         v64, cb + el, tx, ty, tz,
@@ -565,6 +573,7 @@ adjoint_df64_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
                     const float4 *g4 = reinterpret_cast<const float4 *>(r + s_ri.off[c]);
                     const float4 *ph = s_ph + ((size_t)el * 3 + c) * qmax;
                     const float4 *tb = reinterpret_cast<const float4 *>(s_tab + (size_t)c * qmax * kAdjTab);
+#pragma unroll 1
                     for (int q = 0; q < Q; ++q) {
                         const float4 A = g4[4 * q], B4 = g4[4 * q + 1], Cn = g4[4 * q + 2], Dn = g4[4 * q + 3];
                         const df ox{A.x, B4.x}, oy{A.y, B4.y}, oz{A.z, B4.z};
@@ -902,17 +911,17 @@ void run_adjoint(Ctx &c, const AdjointArgs &a, AdjointOut &out) {
             Buf dtab(tb.size() * 4), sums((size_t)E * kAdjSums * 8);
             BIE_CUDA(cudaMemcpyAsync(dtab.p, tb.data(), tb.size() * 4, cudaMemcpyHostToDevice, st));
             BIE_CUDA(cudaMemsetAsync(sums.p, 0, (size_t)E * kAdjSums * 8, st));
-            // chunks of ~24 KB: four blocks per SM with room for L1
+            // chunks of ~48 KB: two blocks per SM with room for L1
             const size_t el_bytes = (size_t)X.stride * 4 + (size_t)3 * L.qmax * 16 + 32 * 4;
-            const int chunk = (int)std::max<size_t>(1, std::min<size_t>(32, (24u << 10) / el_bytes));
+            const int chunk = (int)std::max<size_t>(1, std::min<size_t>(32, (48u << 10) / el_bytes));
             const size_t smem = tb.size() * 4 + chunk * el_bytes;
-            const int64_t tiles = (N + M + kT - 1) / kT;
+            const int64_t tiles = (N + M + kAT - 1) / kAT;
             int S = 1;
-            // many small blocks: their cost differs with the near pairs in them (13.5 ms
-            // at 64 blocks per SM, 14.0 at 32, 14.9 at 16, 16.4 at 8)
+            // many small blocks: their cost differs with the near pairs in them (blocks
+            // of 128 threads: 13.5 ms at 64 blocks per SM, 14.0 at 32, 14.9 at 16, 16.4 at 8)
             while (tiles * S < 64LL * c.num_sms && S * 2 * 8 <= E) S *= 2;
             BIE_CUDA(cudaFuncSetAttribute(adjoint_df64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            adjoint_df64_kernel<<<dim3((unsigned)tiles, (unsigned)S), kT, smem, st>>>(
+            adjoint_df64_kernel<<<dim3((unsigned)tiles, (unsigned)S), kAT, smem, st>>>(
                 N, M, c.d_sources, fp.d(), w.d2(), p.d2(), c.d_drecords, X.stride, X.nidx_off, ri, c.d_coords, Y.d2(),
                 E, S, static_cast<const float *>(dtab.p), L.qmax, v, a.k_re, rhock_re, deg, chunk, sums.d(), dX.d());
             BIE_CUDA(cudaGetLastError());

@@ -633,7 +633,7 @@ void launch_assemble_mixed(Ctx &c, const AssembleArgs &a) {
         else if (L.NP == 3) BIE_K2_LAUNCH(3);
         else BIE_K2_LAUNCH(6);
 #undef BIE_K2_LAUNCH
-        if (a.flags & BIE_C) launch_reduce_c(c, Cpart, S, Cnear, a.M, a.C);
+        if (a.flags & BIE_C) launch_reduce_c(c, Cpart, S, Cnear, a.M, a.C, nullptr, true);
     };
     auto reset = [&] {   // fresh deferred list (every entry of F, G is overwritten)
         BIE_CUDA(cudaMemsetAsync(dbuf + dbytes, 0, 256 + (size_t)a.M * 8, c.stream));
