@@ -754,8 +754,7 @@ __device__ __noinline__ double k9_pair_inplace(const Fp64View &v64, int64_t p, d
     return ce;
 }
 
-// FG = false: C alone (points off the surface, whose C keeps this arithmetic
-// while F and G come from the fixed-point kernel).
+// FG = false: C alone.
 template <int NP, bool CPLX_K, bool FG>
 __global__ void __launch_bounds__(kThreads, BIE_K9_MIN_BLOCKS)
 assemble_df64_kernel(const float *__restrict__ rec, int stride, int nidx_off, int64_t E, int S,
@@ -1012,10 +1011,7 @@ void build_df64_records(Ctx &c, const std::vector<double> &rec64, const std::vec
 }
 
 bool launch_assemble_df64(Ctx &c, const AssembleArgs &a) {
-    return launch_assemble_fix64(c, a, true) || launch_assemble_k9(c, a);
-}
-
-bool launch_assemble_k9(Ctx &c, const AssembleArgs &a) {
+    if (launch_assemble_fix64(c, a, true)) return true;
     const RecordLayout &L = c.lay;
     if (a.taylor_m >= 0 || (a.k_dev && !(a.k_abs_max > 0))) return false;
     df64::DfDegrees deg{};

@@ -588,18 +588,17 @@ void launch_nearfield(Ctx &c, const NearField &nf, double k_re, double k_im, int
 // host: builds d_mrecords / d_mphi from the FP64 records (E x lay.stride) and uploads them
 void build_mixed_records(Ctx &c, const std::vector<double> &rec64);
 void launch_assemble_mixed(Ctx &c, const AssembleArgs &a);
-// FP64-grade assembly (BIE_PREC_DF64): the fixed-point kernel (K10) or, where its
-// ranges end, the double-float kernel (K9); false when the arguments need the
-// FP64 kernel (k-derivatives, device-resident k, or phase rotations beyond the
-// Taylor tables)
+// FP64-grade assembly (BIE_PREC_DF64): the fixed-point kernel (K10) where
+// fix64_takes says so, else the double-float kernel (K9); false when the
+// arguments need BIE_PREC_FP64's kernels (k-derivatives, device-resident k without
+// a bound, or phase rotations beyond the Taylor tables)
 bool launch_assemble_df64(Ctx &c, const AssembleArgs &a);
-bool launch_assemble_k9(Ctx &c, const AssembleArgs &a);   // the double-float kernel itself
 
 // Fixed-point assembly at FP64 accuracy (K10, bie_assemble_fix64.cu): records
 // from the FP64 ones; the launch returns false, enqueuing nothing, where the
 // arguments need another kernel (k-derivatives, element factors, phases or
 // damping beyond the fixed-point ranges, coordinates outside
-// 2^+-300).  df64: BIE_PREC_DF64, which keeps its own slicing and off-surface C.
+// 2^+-300).  df64: BIE_PREC_DF64, of which it takes the calls where it is the faster.
 void build_fix64_records(Ctx &c, const std::vector<double> &rec64);
 bool launch_assemble_fix64(Ctx &c, const AssembleArgs &a, bool df64);
 bool fix64_takes(const Ctx &c, const AssembleArgs &a, bool df64);   // whether it launches

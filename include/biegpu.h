@@ -71,9 +71,9 @@ extern "C" {
 /* FP64 accuracy (the reference's results to FP64 rounding).  Assembly evaluates
  * the regular pairs in 64-bit fixed point with errors at or below FP64 rounding
  * (this GPU's FP64 pipe runs at 1/64 of its FP32 rate) and the near pairs in
- * FP64; C at points off the surface, k-derivatives, element factors and
- * wavenumbers beyond the fixed-point ranges use FP64 throughout, as do all
- * other operations. */
+ * FP64; dense complex128 products sum in fixed point as well, at the error of an
+ * FP64 sum.  C at points off the surface, k-derivatives and wavenumbers beyond the
+ * fixed-point ranges use FP64 throughout, as do all other operations. */
 #define BIE_PREC_FP64  0
 #define BIE_PREC_MIXED 1  /* FP32 regular pairs, FP64 near-singular pairs and C  */
 /* Multi-right-hand-side products only (bie_matvec_multi_device): matrix tiles
@@ -87,12 +87,11 @@ extern "C" {
 #define BIE_PREC_BF16_SPLIT 5   /* ~2e-5                        */
 /* Assembly, matrix-free products and GMRES operator arithmetic (bie_assemble*,
  * bie_matvec*, bie_gmres*; with `refine`, the residuals of refinement):
- * FP64-grade results, near pairs in FP64 with double-float sine and cosine.
- * Assembly takes the fixed-point kernel of BIE_PREC_FP64; products (and
- * assemblies with element factors or beyond the fixed-point ranges) evaluate
- * the regular pairs in double-float arithmetic (pairs of floats, ~48-bit
- * significand) on the FP32 pipes with every sum compensated, ~1e-14 from
- * BIE_PREC_FP64.  Falls
+ * FP64-grade results, near pairs in FP64.  The node rows of assemblies with rules
+ * of at most four points take the fixed-point kernel of BIE_PREC_FP64; other
+ * assemblies and products evaluate the regular pairs in double-float arithmetic
+ * (pairs of floats, ~48-bit significand) on the FP32 pipes with every sum
+ * compensated, ~1e-14 from BIE_PREC_FP64.  Falls
  * back to the FP64 kernels where the phase rotation k (r - r0) over one
  * element exceeds the Taylor tables (|k| x element radius > ~2.5).          */
 #define BIE_PREC_DF64       6
