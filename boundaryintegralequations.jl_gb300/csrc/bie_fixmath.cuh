@@ -129,6 +129,91 @@ FX_FN bool exp_minus(double x, const Table &table, double &v) {
     return true;
 }
 
+// ---- IEEE division and square root, rounded to nearest even ----------------
+// From an approximation of the quotient (root) to 2^-60 and the exact remainder
+// in 64-bit arithmetic, so the double is the one of the FP64 pipe's sequence.
+
+// 1 / B in Q62 of (1, 2], B: Q64 in [1/2, 1), to a few units: a float estimate and
+// two Newton steps
+FX_FN u64 reciprocal(u64 B) {
+    const float b = u32_to_float((unsigned)(B >> 32)) * 0x1p-32f;
+    const u64 y0 = (u64)(unsigned)round_to_int((1.0f / b) * 0x1p29f) << 33;      // Q62, 2^-23
+    const i64 e1 = (i64)(((u64)1 << 62) - mul_high(B, y0));                      // 1 - b y0, Q62
+    const u64 y1 = y0 + (u64)(wide((int)(e1 >> 10), (int)(y0 >> 33)) >> 19);     // Q62, 2^-45
+    const i64 e2 = (i64)(((u64)1 << 62) - mul_high(B, y1));
+    return y1 + (u64)(wide((int)e2, (int)(y1 >> 33)) >> 29);
+}
+FX_FN u64 mantissa(double x) { return (double_bits(x) & 0xfffffffffffffull) | 0x10000000000000ull; }
+FX_FN int exponent(double x) { return (int)(double_bits(x) >> 52) & 0x7ff; }
+
+// Division by one positive normal b
+struct Divisor {
+    u64 mb, R;
+    int eb;
+};
+FX_FN Divisor divisor(double b) {
+    const u64 mb = mantissa(b);
+    return Divisor{mb, reciprocal(mb << 11), exponent(b)};
+}
+// a / b for a zero or normal a and a normal quotient
+FX_FN double divide(double a, const Divisor &d) {
+    const u64 ma = mantissa(a);
+    const int s = ma < d.mb ? 1 : 0;
+    // ma 2^(53 + s) / mb in [2^53, 2^54); the reciprocal is of mb 2^-53
+    u64 Q = mul_high(ma << (9 + s), d.R) >> 7;
+    i64 rem = (i64)((ma << (53 + s)) - Q * d.mb);          // (the true value is small)
+    if (rem < 0) { --Q; rem += (i64)d.mb; }
+    if (rem >= (i64)d.mb) { ++Q; rem -= (i64)d.mb; }
+    const u64 m = (Q >> 1) + (Q & 1 & ((rem != 0 ? 1 : 0) | (Q >> 1)));
+    const u64 bits = ((u64)(unsigned)(exponent(a) - d.eb + 1022 - s) << 52) + m;
+    const u64 sign = double_bits(a) & ((u64)1 << 63);
+    return bits_double(exponent(a) == 0 ? sign : (bits | sign));
+}
+// sqrt of x in [1, 4)
+FX_FN double square_root(double x) {
+    const u64 mx = mantissa(x) << (exponent(x) - 1023);    // x in Q52
+    const i64 q = (i64)(mx << 6);                          // Q58
+    const Limb l = split(q), ri = split(rcp_sqrt(q, l));
+    u64 T = (u64)fold_up<5>(wide(l.h, ri.h), cross<5>(l, ri) + hi32(wide(l.l, ri.l))) >> 7;   // Q53
+    i64 rem = (i64)((mx << 54) - T * T);
+    if (rem < 0) { --T; rem += (i64)(2 * T + 1); }
+    if (rem > (i64)(2 * T)) ++T;
+    return bits_double(((u64)1022 << 52) + (T >> 1) + (T & 1));
+}
+// Julia's 3-argument hypot (maximum-abs scaling, IEEE division and square root,
+// ((a^2 + b^2) + c^2) summation), bit for bit; false (nothing set) where a
+// component other than zero is below 2^-100 times the largest, or that one
+// outside [2^-900, 2^900]
+FX_FN double mul_rn(double a, double b) {
+#ifdef __CUDA_ARCH__
+    return __dmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+FX_FN double add_rn(double a, double b) {
+#ifdef __CUDA_ARCH__
+    return __dadd_rn(a, b);
+#else
+    return a + b;
+#endif
+}
+FX_FN double magnitude(double x) { return bits_double(double_bits(x) & 0x7fffffffffffffffull); }
+FX_FN bool hypot3(double x, double y, double z, double &h) {
+    const u64 ux = double_bits(magnitude(x)), uy = double_bits(magnitude(y)), uz = double_bits(magnitude(z));
+    u64 um = ux > uy ? ux : uy;
+    um = uz > um ? uz : um;
+    const double m = bits_double(um);
+    const int em = exponent(m);
+    if ((unsigned)(em - 123) > 1800u) return false;
+    const u64 low = um - ((u64)100 << 52);                 // 2^-100 m
+    if ((ux != 0 && ux < low) || (uy != 0 && uy < low) || (uz != 0 && uz < low)) return false;
+    const Divisor d = divisor(m);
+    const double a = divide(x, d), b = divide(y, d), c = divide(z, d);
+    h = mul_rn(m, square_root(add_rn(add_rn(mul_rn(a, a), mul_rn(b, b)), mul_rn(c, c))));
+    return true;
+}
+
 }  // namespace fix64
 
 #ifdef __CUDACC__

@@ -13,8 +13,8 @@
 // (src/3d/jacobian.jl:78-87), and the F and G integrands of kernels.jl:13-37
 // accumulated per physics node.  A warp-shuffle reduction gives the element's
 // contributions, which the lanes add (FP64 atomics) to the pair's CSR slots.
-// FP64 throughout (roots, sine, cosine and exponential at FP64 accuracy on the
-// integer pipes): these are the singular and near-singular integrals.
+// FP64 throughout (roots, divisions, sine, cosine and exponential at FP64 accuracy
+// on the integer pipes): these are the singular and near-singular integrals.
 #include "bie_internal.h"
 #include "bie_device.cuh"
 #include "bie_fixmath.cuh"
@@ -57,6 +57,16 @@ __device__ __noinline__ double2 distance_library(double dx, double dy, double dz
     return make_double2(r, __ddiv_rn(1.0, r));
 }
 
+// negated unit normal and jacobian where the components leave the range of
+// fix64::hypot3
+struct Normal {
+    double x, y, z, jac;
+};
+__device__ __noinline__ Normal normal_library(double n0, double n1, double n2) {
+    const double jac = dev::julia_hypot3(n0, n1, n2);
+    return Normal{__ddiv_rn(-n0, jac), __ddiv_rn(-n1, jac), __ddiv_rn(-n2, jac), jac};
+}
+
 // FLAT: three-node elements with linear shape functions, whose derivatives and
 // so normal and jacobian are the same at every point.
 //
@@ -64,8 +74,10 @@ __device__ __noinline__ double2 distance_library(double dx, double dy, double dz
 // operations per point when roots, divisions, sine, cosine and exponential came
 // from the library and flat elements formed their normal at every point, some
 // 50 now, with about 280 integer instructions beside them.  Flat elements, 1962
-// nodes: 19.9 -> 4.3 ms (with a complex wavenumber 21.6 -> 4.8); 6-node elements,
-// whose geometry stays in FP64 at every point, 36.0 -> 27.4 ms at 2562 nodes.
+// nodes: 19.9 -> 4.2 ms (with a complex wavenumber 21.6 -> 4.8); 6-node elements,
+// 2562 nodes: 36.0 -> 19.0 ms (interpolation and cross product stay in FP64 at every
+// point; the hypot and divisions of the normal on the integer pipes with the same
+// roundings were worth 27.4 -> 21.4, the zero derivatives left out 2.4 more).
 template <int NS, int NP, bool CPLX_K, bool FLAT>
 __global__ void __launch_bounds__(256)
 nearfield_kernel(const int32_t *__restrict__ pairs, int pstride, int64_t npairs,
@@ -108,19 +120,30 @@ nearfield_kernel(const int32_t *__restrict__ pairs, int pstride, int64_t npairs,
 #pragma unroll
             for (int a = 0; a < NS; ++a) {
                 const double Ua = P[NS + a], Va = P[2 * NS + a];
+                // (dN/du of the third corner and dN/dv of the second are zero)
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
-                    tu[k] = __dadd_rn(tu[k], __dmul_rn(X[3 * a + k], Ua));
-                    tv[k] = __dadd_rn(tv[k], __dmul_rn(X[3 * a + k], Va));
+                    if (a != 2) tu[k] = a == 0 ? __dmul_rn(X[k], Ua) : __dadd_rn(tu[k], __dmul_rn(X[3 * a + k], Ua));
+                    if (a != 1) tv[k] = a == 0 ? __dmul_rn(X[k], Va) : __dadd_rn(tv[k], __dmul_rn(X[3 * a + k], Va));
                 }
             }
             const double n0 = __dsub_rn(__dmul_rn(tu[1], tv[2]), __dmul_rn(tu[2], tv[1]));
             const double n1 = __dsub_rn(__dmul_rn(tu[2], tv[0]), __dmul_rn(tu[0], tv[2]));
             const double n2 = __dsub_rn(__dmul_rn(tu[0], tv[1]), __dmul_rn(tu[1], tv[0]));
-            const double jac = dev::julia_hypot3(n0, n1, n2);
-            nx = __ddiv_rn(-n0, jac);
-            ny = __ddiv_rn(-n1, jac);
-            nz = __ddiv_rn(-n2, jac);
+            // hypot and divisions with the roundings of the FP64 pipe
+            double jac;
+            if (fix64::hypot3(n0, n1, n2, jac)) {
+                const fix64::Divisor d = fix64::divisor(jac);
+                nx = fix64::divide(-n0, d);
+                ny = fix64::divide(-n1, d);
+                nz = fix64::divide(-n2, d);
+            } else {
+                const Normal l = normal_library(n0, n1, n2);
+                jac = l.jac;
+                nx = l.x;
+                ny = l.y;
+                nz = l.z;
+            }
             jac4 = jac * kInv4Pi;
         };
         if (FLAT) normal(table + base * tstride);

@@ -46,3 +46,14 @@ def test_functions_against_long_double(tmp_path, seed):
     assert float(out[2]) <= 0.9
     assert float(out[3]) <= 1.0
     assert out[4] == "1"
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_division_and_roots_are_ieee(tmp_path, seed):
+    if GXX is None:
+        pytest.skip("g++ not available")
+    exe = tmp_path / "fix64_divide"
+    subprocess.run([GXX, "-O2", "-std=gnu++17", "-ffp-contract=off", "-I", str(PKG / "csrc"),
+                    str(ROOT / "tests" / "fix64_divide.cpp"), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe), str(seed)], check=True, capture_output=True, text=True).stdout.split()
+    assert out == ["0", "0", "0", "0", "1"]

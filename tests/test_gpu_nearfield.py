@@ -3,6 +3,8 @@ sparse_assemble_parallel! and partial_assemble_parallel!; FP64, relative
 2-norm error of the CSR values <= 1e-12."""
 from __future__ import annotations
 
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -52,3 +54,20 @@ def test_sparse_assemble_parallel_api():
     assert rel(F.data, Fo) <= 1e-12
     # the diagonal (self) entries of G are the largest single-layer values
     assert np.all(np.abs(G.diagonal()) > 0)
+
+
+def test_nearfield_flat_six_node_elements():
+    """Flat 6-node elements: F of connected pairs is the rounding of n . (x - t), so
+    it agrees with the oracle only if interpolation, cross product, hypot and
+    divisions round as there."""
+    mesh = bm.icosphere(3, geometry="quadratic")
+    X = np.array(mesh.coordinates)
+    T = np.asarray(mesh.topology) - np.min(mesh.topology)
+    T = T if T.shape[0] == 6 else T.T
+    for m, (a, b) in zip((3, 4, 5), ((0, 1), (1, 2), (2, 0))):
+        X[:, T[m]] = 0.5 * (X[:, T[a]] + X[:, T[b]])
+    mesh = dataclasses.replace(mesh, coordinates=X, sources=X.copy())
+    ctx = biegpu.get_context(mesh)
+    _, _, F, G = nearfield_values(ctx, 2.0, depth=1)
+    _, _, Fo, Go = oracle.nearfield(mesh, 2.0, depth=1)
+    assert rel(F, Fo) <= 1e-12 and rel(G, Go) <= 1e-12
