@@ -46,11 +46,12 @@ constexpr int kT = 256;
 // near the subnormals (where a zero's hidden bit would count) is summed in FP64
 // instead.
 //
-// Measured: 2562 nodes 92 -> 38 us, 4842 264 -> 103 us (3.65 TB/s), 10242
-// 1193 -> 430 us (3.9 TB/s); the integer issue slots (about 110 per entry and
+// Measured: 2562 nodes 92 -> 36 us, 4842 264 -> 94 us (4.0 TB/s), 10242
+// 1193 -> 397 us (4.2 TB/s); the integer issue slots (about 110 per entry and
 // warp) bound it now.  Error against extended precision, 5 to 2200 columns,
 // entries and vectors spread over up to 300 decades: 0.7 to 1.01 times the FP64
-// sum's.  Four columns per run or two blocks per SM are 2 to 8 % slower.
+// sum's.  Four columns are loaded ahead of the four in work (eight together
+// without that: 38 / 103 / 430 us); two or four blocks per SM take 2 to 17 % longer.
 constexpr int kGemvRadix = 29;
 constexpr int kGemvMask = (1 << kGemvRadix) - 1;
 __device__ __forceinline__ int biased_exponent(double a) { return (__double2hiint(a) >> 20) & 0x7ff; }
@@ -86,7 +87,7 @@ dense_gemv_kernel(const double2 *__restrict__ A, int64_t n, const double2 *__res
     __shared__ int4 xf[kT];        // Re, Im limbs
     __shared__ __align__(16) int xe[kT];   // exponents
     __shared__ int s_max[kT / 32];
-    constexpr int kRun = 8;              // columns loaded together
+    constexpr int kRun = 4;              // columns loaded together, one run ahead
     constexpr int kBlock = 64;           // columns between additions to the FP64 sum
     double re = 0, im = 0;
     int E = 0;                           // exponent of the row's products (doubly biased)
@@ -113,9 +114,13 @@ dense_gemv_kernel(const double2 *__restrict__ A, int64_t n, const double2 *__res
         int xmax = s_max[0];
 #pragma unroll
         for (int k = 1; k < kT / 32; ++k) xmax = max(xmax, s_max[k]);
+        const double2 *col = A + jb * n + i;
+        // (past the chunk: its last column again, against x = 0)
+        double2 next[kRun];
+#pragma unroll
+        for (int j = 0; j < kRun; ++j) next[j] = __ldcs(col + (int64_t)min(j, nb - 1) * n);
         for (int jc = 0; jc < nb; jc += kBlock) {
             const int ne = min(nb, jc + kBlock);
-            const double2 *col = A + jb * n + i;
             long long hr = 0, lr = 0, hm = 0, lm = 0;   // sums in units 2^58 and 2^29
             int amax = 0;
             for (int j8 = jc; j8 < ne; j8 += kRun) {
@@ -130,8 +135,10 @@ dense_gemv_kernel(const double2 *__restrict__ A, int64_t n, const double2 *__res
                     ex[j + 3] = e.w;
                 }
 #pragma unroll
-                for (int j = 0; j < kRun; ++j)   // (past the slice: its last column again, against x = 0)
-                    a[j] = __ldcs(col + (int64_t)min(j8 + j, nb - 1) * n);
+                for (int j = 0; j < kRun; ++j) {
+                    a[j] = next[j];
+                    next[j] = __ldcs(col + (int64_t)min(j8 + kRun + j, nb - 1) * n);
+                }
 #pragma unroll
                 for (int j = 0; j < kRun; ++j) {
                     er[j] = biased_exponent(a[j].x);
