@@ -245,7 +245,7 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
                       const int4 *__restrict__ trig, const int2 *__restrict__ damp, const double *__restrict__ tgt, int64_t M,
                       double kre, double kim, int flags, longlong2 *__restrict__ F, longlong2 *__restrict__ G,
                       const uint32_t *__restrict__ kflags, double *__restrict__ Cpart,
-                      int2 *__restrict__ defer, unsigned int *__restrict__ defer_count, unsigned int defer_cap,
+                      int2 *__restrict__ defer, u64 *__restrict__ defer_count, unsigned int defer_cap,
                       int *__restrict__ over, const int4 *__restrict__ gweight, const __grid_constant__ FxScale sc,
                       unsigned long long *__restrict__ qpe_count, const double *__restrict__ kdev) {
     if (kdev) {   // wavenumber read from device memory (recorded sweeps)
@@ -293,7 +293,7 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
     };
 
     double cacc = 0.0;
-    int over_at = 0x7fffffff;
+    int over_at = fix64::kNoOverflow;
     unsigned long long nqpe = 0;
     __syncthreads();
     const FxWave wv = s_wave;
@@ -314,9 +314,9 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
             const int e = I.e;
             int Q = 0;
             if (I.deferred) {   // no points here, but the pair may open or close entries
-                const unsigned int slot = atomicAdd(defer_count, 1u);
-                if (slot < defer_cap) defer[slot] = make_int2((int)i, (int)pe);
-                else over_at = min(over_at, (int)pe);   // rescanned by the correction kernel
+                u64 slot;
+                if (fix64::defer_slot([=] { return atomicAdd(defer_count, 1ull); }, defer_cap, (int)pe, over_at, slot))
+                    defer[slot] = make_int2((int)i, (int)pe);   // (else rescanned by the correction kernel)
             } else {
                 const int qs = T.st + 2 - e;   // 2^(59 - st) units -> Q61 of 2^e
                 P.Dx = (i64)((u64)P.Dx << qs);
@@ -556,7 +556,7 @@ __device__ __forceinline__ int fx_correct_pair(const Fp64View &v, int64_t i, int
 // gone through again from its first pair that found no place.
 template <int NP, bool CPLX_K>
 __global__ void __launch_bounds__(128)
-fx_correct_kernel(const int2 *__restrict__ defer, const unsigned int *__restrict__ defer_count,
+fx_correct_kernel(const int2 *__restrict__ defer, const u64 *__restrict__ defer_count,
                   unsigned int defer_cap, const __grid_constant__ Fp64View v, const double *__restrict__ tgt,
                   int64_t M, double kre, double kim, int flags, double2 *__restrict__ F, double2 *__restrict__ G,
                   double *__restrict__ Cnear, const int *__restrict__ over, const float *__restrict__ rec, int stride,
@@ -566,7 +566,8 @@ fx_correct_kernel(const int2 *__restrict__ defer, const unsigned int *__restrict
         kre = kdev[0];
         kim = kdev[1];
     }
-    const unsigned int total = *defer_count, n = min(total, defer_cap);
+    const u64 total = *defer_count;
+    const unsigned int n = (unsigned int)min(total, (u64)defer_cap);
     const bool doF = flags & BIE_F, doG = flags & BIE_G, doC = flags & BIE_C;
     unsigned long long nqpe = 0;
     for (unsigned int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
@@ -576,7 +577,7 @@ fx_correct_kernel(const int2 *__restrict__ defer, const unsigned int *__restrict
         const FxWave wv = fx_wave<CPLX_K>(kre, kim, sc);
         for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < M * S;
              j += (int64_t)gridDim.x * blockDim.x) {
-            if (over[j] == 0x7fffffff) continue;
+            if (over[j] == fix64::kNoOverflow) continue;
             const int64_t s = j / M, i = j - s * M;
             const FxTarget T = fx_target(tgt[3 * i], tgt[3 * i + 1], tgt[3 * i + 2], sc);
             for (int64_t p = over[j]; p < (s + 1) * E / S; ++p) {
@@ -598,7 +599,8 @@ inline unsigned stream_grid(const Ctx &c, int64_t total) {
 struct FxBuffers {
     double *Cpart, *Cnear;
     int2 *defer;
-    unsigned int *dcount, dcap;
+    u64 *dcount;
+    unsigned int dcap;
     int *over;
 };
 
@@ -936,7 +938,7 @@ bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df64) {
     const size_t dbytes = (size_t)b.dcap * sizeof(int2);
     char *dbuf = static_cast<char *>(c.scratch(kScratchDefer, dbytes + 256 + (size_t)a.M * 8));
     b.defer = reinterpret_cast<int2 *>(dbuf);
-    b.dcount = reinterpret_cast<unsigned int *>(dbuf + dbytes);
+    b.dcount = reinterpret_cast<u64 *>(dbuf + dbytes);
     b.Cnear = reinterpret_cast<double *>(dbuf + dbytes + 256);
     auto reset = [&] { BIE_CUDA(cudaMemsetAsync(dbuf + dbytes, 0, 256 + (size_t)a.M * 8, c.stream)); };
     reset();

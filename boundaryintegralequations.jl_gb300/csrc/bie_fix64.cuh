@@ -365,5 +365,20 @@ FX_FN int amplitude_exp(int kb, int e) { return kb + e > 1 ? kb + e - 1 : 0; }
 FX_FN int entry_exp_g(int ej, int fl) { return ej - (fl - 1) - 55; }
 FX_FN int entry_exp_f(int ej, int fl, int kb) { return ej - 2 * (fl - 1) + amplitude_exp(kb, fl - 1) - 55; }
 
+// Place in the list of deferred pairs of pair pe of a (row, slice), whose pairs come
+// in order: true and its slot, or false where the list is full.  Such a row's
+// slice is gone through again from over_at, its first pair without a place, so
+// later pairs need none and do not count: the counter ends at most one above the
+// list's length for each (row, slice), whatever the number of deferred pairs.
+constexpr int kNoOverflow = 0x7fffffff;
+template <class Count>
+FX_FN bool defer_slot(Count count, u64 capacity, int pe, int &over_at, u64 &slot) {
+    if (over_at < pe) return false;
+    slot = count();
+    if (slot < capacity) return true;
+    over_at = pe;
+    return false;
+}
+
 }  // namespace fix64
 }  // namespace bie

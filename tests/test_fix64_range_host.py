@@ -1,0 +1,37 @@
+"""Index arithmetic and scales of the fixed-point assembly on the host: the
+functions of csrc/bie_fix64.cuh at sizes and values no quick GPU test reaches."""
+from __future__ import annotations
+
+import shutil
+import subprocess
+
+import pytest
+
+from conftest import PKG, ROOT
+
+GXX = shutil.which("g++")
+
+
+@pytest.fixture(scope="module")
+def build(tmp_path_factory):
+    if GXX is None:
+        pytest.skip("g++ not available")
+    out = tmp_path_factory.mktemp("fix64_range")
+
+    def make(name):
+        exe = out / name
+        subprocess.run([GXX, "-O2", "-std=gnu++17", "-I", str(PKG / "csrc"), str(ROOT / "tests" / f"{name}.cpp"),
+                        "-o", str(exe)], check=True)
+
+        def run(*args):
+            return subprocess.run([str(exe), *map(str, args)], check=True, capture_output=True, text=True).stdout.split()
+        return run
+    return make
+
+
+@pytest.mark.parametrize("capacity,percent", [(0, 100), (7, 100), (500, 100), (500, 30), (100000, 100), (100000, 5)])
+def test_deferred_pairs_are_counted_once_per_row_and_slice(build, capacity, percent):
+    """Every deferred pair is integrated once, and the counter of list places stays
+    within the list's length and one per (row, slice) however many there are."""
+    out = build("fix64_defer")(1, 40, 5, 60, capacity, percent)
+    assert out[0] == "1" and out[1] == "1"
