@@ -41,6 +41,7 @@
 #include "bie_fixmath.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 
@@ -297,7 +298,6 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
     unsigned long long nqpe = 0;
     __syncthreads();
     const FxWave wv = s_wave;
-    const unsigned row_bytes = (unsigned)(M * 16);   // of a column
     char *Fi = reinterpret_cast<char *>(F + i), *Gi = reinterpret_cast<char *>(G + i);
     if (active) {
         for (int64_t pe = e0; pe < e1; ++pe) {
@@ -387,7 +387,7 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
                     const bool open = q0 == 0, close = q0 + kGroup >= Q;
 #pragma unroll 1
                     for (int a = 0; a < NP; ++a) {
-                        const u64 off = (u64)(unsigned)nid[a] * (u64)row_bytes;
+                        const u64 off = fix64::column_bytes(nid[a], M);
                         longlong2 *pF = reinterpret_cast<longlong2 *>(Fi + off);
                         longlong2 *pG = reinterpret_cast<longlong2 *>(Gi + off);
                         const bool shared = (fw >> (16 + a)) & 1u;
@@ -887,6 +887,7 @@ void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
 static bool fix64_covers(const Ctx &c, const AssembleArgs &a) {
     if (!c.fx_ok || a.taylor_m >= 0 || (a.g_weight && a.g_weight_exp == INT32_MIN)) return false;
     if (a.k_dev && !(a.k_abs_max > 0)) return false;   // no bound on |k|
+    if (a.M > INT32_MAX) return false;   // rows are 32-bit in the list of deferred pairs
     const bool cplx = a.k_im != 0.0;
     if (a.g_weight && (c.lay.NP != 3 || cplx)) return false;   // (the adjoint: 3-node physics, real k)
     // wavenumbers whose phase or damping over the mesh or an element leaves the

@@ -365,6 +365,9 @@ FX_FN int amplitude_exp(int kb, int e) { return kb + e > 1 ? kb + e - 1 : 0; }
 FX_FN int entry_exp_g(int ej, int fl) { return ej - (fl - 1) - 55; }
 FX_FN int entry_exp_f(int ej, int fl, int kb) { return ej - 2 * (fl - 1) + amplitude_exp(kb, fl - 1) - 55; }
 
+// Byte offset of a node's column of complex128 entries, rows in a column
+FX_FN u64 column_bytes(int node, i64 rows) { return (u64)(unsigned)node * (u64)rows << 4; }
+
 // Place in the list of deferred pairs of pair pe of a (row, slice), whose pairs come
 // in order: true and its slot, or false where the list is full.  Such a row's
 // slice is gone through again from over_at, its first pair without a place, so

@@ -35,3 +35,8 @@ def test_deferred_pairs_are_counted_once_per_row_and_slice(build, capacity, perc
     within the list's length and one per (row, slice) however many there are."""
     out = build("fix64_defer")(1, 40, 5, 60, capacity, percent)
     assert out[0] == "1" and out[1] == "1"
+
+
+def test_columns_of_many_rows(build):
+    # 2^28 rows and more: a column is 4 GB
+    assert build("fix64_columns")() == ["1"]
