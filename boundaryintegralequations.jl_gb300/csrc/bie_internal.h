@@ -107,11 +107,13 @@ enum ScratchSlot {
     kScratchLowp = 12,     // multi-RHS products: strips, 16-bit tiles, partial sums
     kScratchSolverNested = 13,  // GMRES workspace + partials of nested solves, two slots
                                 // per level 1, 2 (solves inside another solve's product)
-    kScratchFxWeight = 16, // fixed-point assembly: element factors as limbs
     kScratchK2Side = 17,   // mixed assembly: per-slice partial sums of nodes shared between slices
     kScratchFieldC = 18,   // C at points off the surface, beside the fixed-point assembly: partial sums
-    kScratchCount = 19
+    kScratchFxWeight = 19, // fixed-point assembly: element factors as limbs
+    kScratchCount = 20
 };
+constexpr int kMaxSolveLevel = 2;   // GMRES solves nested inside products
+static_assert(kScratchSolverNested + 2 * kMaxSolveLevel <= kScratchK2Side, "slots of nested solves overlap others");
 
 // Mixed-precision element record (32-bit words, same element order as the FP64
 // records):
@@ -478,8 +480,7 @@ struct DevOp {
     virtual bool honours_stop() const { return false; }
 };
 // run_gmres on a DevOp of size n; `level` 0, 1 or 2 selects the workspace, so a
-// solve may run inside the product of a solve one level up.
-constexpr int kMaxSolveLevel = 2;
+// solve may run inside the product of a solve one level up (kMaxSolveLevel).
 void run_gmres_devop(Ctx &c, DevOp &op, const double *b, double *x, const bie_gmres_opts &o,
                      bie_gmres_info &info, int level);
 void capture_gmres(Ctx &c, const bie_operator &op, const double *b, double *x, const bie_gmres_opts &o,
