@@ -27,7 +27,6 @@
 #include "bie_fixmath.cuh"
 
 #include <algorithm>
-#include <climits>
 #include <cmath>
 #include <complex>
 #include <vector>
@@ -771,26 +770,20 @@ void run_adjoint(Ctx &c, const AdjointArgs &a, AdjointOut &out) {
     const double2 aBc = make_double2(0.0, a.rho_c * a.k_re);
     // ---- forward: A, B ----------------------------------------------------------
     {
-        // |Re Y|, |Im Y| < 2^exp for the fixed-point assembly
-        double ymax = 0.0;
-        const std::complex<double> *Zh = reinterpret_cast<const std::complex<double> *>(a.Z);
-        for (int64_t e = 0; e < E; ++e) {
-            const double n = std::norm(Zh[e]);
-            const double y = std::max(std::fabs(Zh[e].real()), std::fabs(Zh[e].imag())) / n;
-            if (!(y <= ymax)) ymax = y;   // a NaN or infinity stays
-        }
-        int yexp = INT_MIN;
-        if (ymax > 0x1p-200 && ymax < 0x1p200) (void)std::frexp(ymax * 1.0001, &yexp);
+        // |Y| < 2^400 for the fixed-point assembly (an infinite Y, from |Z|^2 = 0, is not)
+        bool bounded = true;
+        for (int64_t e = 0; e < 2 * E; e += 2)
+            bounded = bounded && std::max(std::fabs(a.Z[e]), std::fabs(a.Z[e + 1])) > 0x1p-399;
         AssembleArgs s{a.k_re, a.k_im, c.d_sources, N, BIE_F | BIE_G | BIE_C, A.d(), G.d(), Cv.d()};
         s.g_weight = Y.d();
-        s.g_weight_exp = yexp;
+        s.g_weight_bounded = bounded;
         if (!(a.precision == BIE_PREC_DF64 && launch_assemble_df64(c, s))) launch_assemble_fp64(c, s);
         combine_system_kernel<<<std::min<unsigned>(nblocks(N * N), 65535u), 256, 0, st>>>(
             A.d2(), G.d2(), aAc, Cv.d2(), N, N);
         BIE_CUDA(cudaGetLastError());
         AssembleArgs f{a.k_re, a.k_im, fp.d(), M, BIE_F | BIE_G, B.d(), Gx.d(), nullptr};
         f.g_weight = Y.d();
-        f.g_weight_exp = yexp;
+        f.g_weight_bounded = bounded;
         if (!(a.precision == BIE_PREC_DF64 && launch_assemble_df64(c, f))) launch_assemble_fp64(c, f);
         // stored: F_x - i rho c k G_x  (= -B)
         combine_system_kernel<<<std::min<unsigned>(nblocks(M * N), 65535u), 256, 0, st>>>(

@@ -78,7 +78,7 @@ struct FxScale {
     int pe;              // basis values are stored times 2^-pe
     int extra;           // entry units times 2^extra (large node valences)
     float rho_max;       // largest rho of the mesh
-    int wexp;            // element factors on G are held times 2^-wexp
+    int extra_w;         // the same for G with element factors
 };
 
 // k as mantissas and exponents (see fix64::pair_wavenumber, pair_damping)
@@ -238,7 +238,14 @@ constexpr int kGroup = 4;
 constexpr int kInterleave = 2;   // points evaluated side by side
 inline int phi_groups(int qmax) { return (qmax + kGroup - 1) / kGroup; }
 
-// GW: per-element complex factors on G (the adjoint's element admittances)
+// GW: per-element complex factors on G (the adjoint's element admittances), each
+// against its own exponent; the unit of an entry of G then follows from the
+// largest weight exponent times factor exponent among the node's elements.
+struct FxFactors {
+    const int4 *limbs;   // E
+    const int *exps;     // E
+    const int *nodes;    // N
+};
 template <int NP, bool CPLX_K, bool GW>
 __global__ void __launch_bounds__(kThreads, 4)
 assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int S,
@@ -247,7 +254,7 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
                       double kre, double kim, int flags, longlong2 *__restrict__ F, longlong2 *__restrict__ G,
                       const uint32_t *__restrict__ kflags, double *__restrict__ Cpart,
                       int2 *__restrict__ defer, u64 *__restrict__ defer_count, unsigned int defer_cap,
-                      int *__restrict__ over, const int4 *__restrict__ gweight, const __grid_constant__ FxScale sc,
+                      int *__restrict__ over, const __grid_constant__ FxFactors gw, const __grid_constant__ FxScale sc,
                       unsigned long long *__restrict__ qpe_count, const double *__restrict__ kdev) {
     if (kdev) {   // wavenumber read from device memory (recorded sweeps)
         kre = kdev[0];
@@ -312,6 +319,7 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
             const int *node_ej = ir + kHdrNodes + 6 * NP;
             const int *nid = node_ej + NP;
             const int e = I.e;
+            const int ejw = GW ? ej + __ldg(gw.exps + pe) : ej;   // of G
             int Q = 0;
             if (I.deferred) {   // no points here, but the pair may open or close entries
                 u64 slot;
@@ -362,7 +370,7 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
                             const Limb a0 = fix64::split(v.Fr), a1 = fix64::split(v.Fi);
                             Limb a2 = fix64::split(v.Gr), a3 = fix64::split(v.Gi);
                             if (GW) {
-                                const int4 f = __ldg(gweight + pe);
+                                const int4 f = __ldg(gw.limbs + pe);
                                 const fix64::Values2 u = fix64::complex_mul(a2, a3, Limb{f.x, f.y}, Limb{f.z, f.w});
                                 a2 = fix64::split(u.re);
                                 a3 = fix64::split(u.im);
@@ -422,7 +430,8 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
                                                             abs_nodes[3 * a + 2], wv);
                         const int fl = en.fl, de = e - (fl - 1);
                         const int dj = node_ej[a] - ej + sc.extra + (CPLX_K ? P.base - en.base : 0);
-                        const int sg = max(0, dj + de);
+                        const int nw = GW ? __ldg(gw.nodes + nid[a]) : 0;
+                        const int sg = max(0, (GW ? nw - ejw + sc.extra_w : dj) + de);
                         const int sf = max(0, dj + 2 * de + fix64::amplitude_exp(wv.kb, fl - 1) - P.fe);
                         vF.x += fix64::shift_right(fix64::fold(fr, frl), sf);
                         vF.y += fix64::shift_right(fix64::fold(fi, fil), sf);
@@ -444,7 +453,8 @@ assemble_fix64_kernel(const float *__restrict__ rec, int stride, int64_t E, int 
                         if (last) {   // final complex128 entries
                             const int adj = sc.pe + sc.extra - en.base;
                             vF = fx_complex<CPLX_K>(vF, fix64::entry_exp_f(node_ej[a], fl, wv.kb) + adj);
-                            vG = fx_complex<CPLX_K>(vG, fix64::entry_exp_g(node_ej[a], fl) + adj + sc.S + sc.wexp);
+                            if (GW) vG = fx_complex<true>(vG, fix64::entry_exp_g(nw, fl) + sc.pe + sc.extra_w + sc.S);
+                            else vG = fx_complex<CPLX_K>(vG, fix64::entry_exp_g(node_ej[a], fl) + adj + sc.S);
                         }
                         if (doF) *pF = vF;
                         if (doG) *pG = vG;
@@ -482,7 +492,8 @@ template <bool CPLX_K>
 __global__ void fx_widen_kernel(const int32_t *__restrict__ fnode, int64_t nfix, const float4 *__restrict__ nodes,
                                 const double *__restrict__ tgt, int64_t M, double kre, double kim,
                                 const __grid_constant__ FxScale sc, longlong2 *__restrict__ F,
-                                longlong2 *__restrict__ G, const double *__restrict__ kdev) {
+                                longlong2 *__restrict__ G, const int *__restrict__ gnodes,
+                                const double *__restrict__ kdev) {
     if (kdev) {
         kre = kdev[0];
         kim = kdev[1];
@@ -502,16 +513,25 @@ __global__ void fx_widen_kernel(const int32_t *__restrict__ fnode, int64_t nfix,
         const FxEntry en = fx_entry<CPLX_K>(fx, fy, fz, x.x, x.y, x.z, wv);
         const int ej = __float_as_int(x.w), adj = sc.pe + sc.extra - en.base;
         if (F) F[off] = fx_complex<CPLX_K>(F[off], fix64::entry_exp_f(ej, en.fl, wv.kb) + adj);
-        if (G) G[off] = fx_complex<CPLX_K>(G[off], fix64::entry_exp_g(ej, en.fl) + adj + sc.S + sc.wexp);
+        if (G && gnodes)
+            G[off] = fx_complex<true>(G[off], fix64::entry_exp_g(gnodes[nd], en.fl) + sc.pe + sc.extra_w + sc.S);
+        else if (G)
+            G[off] = fx_complex<CPLX_K>(G[off], fix64::entry_exp_g(ej, en.fl) + adj + sc.S);
     }
 }
 
-// element factors as Q62 limbs times 2^-wexp
-__global__ void fx_weight_kernel(const double2 *__restrict__ w, int64_t E, int wexp, int4 *__restrict__ out) {
+// limbs and exponents of the element factors; nodes[j]: the largest exponent of
+// weight times factor among node j's elements (3-node physics)
+__global__ void fx_factor_kernel(const double2 *__restrict__ w, int64_t E, const float *__restrict__ rec, int stride,
+                                 int4 *__restrict__ limbs, int *__restrict__ exps, int *__restrict__ nodes) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= E) return;
-    const Limb a = fix64::split(fx_round(w[p].x, 0.0, 62 - wexp)), b = fix64::split(fx_round(w[p].y, 0.0, 62 - wexp));
-    out[p] = make_int4(a.h, a.l, b.h, b.l);
+    const fix64::Factor f = fix64::element_factor(w[p].x, w[p].y);
+    limbs[p] = make_int4(f.re.h, f.re.l, f.im.h, f.im.l);
+    exps[p] = f.e;
+    const int *r = reinterpret_cast<const int *>(rec + p * stride);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) atomicMax(nodes + r[kHdrNodes + 7 * 3 + a], r[kHdrEj] + f.e);
 }
 
 template <int NP, bool CPLX_K>
@@ -622,14 +642,18 @@ void launch_np(Ctx &c, const AssembleArgs &a, const LaunchShape &sh, int spread,
     sc.pe = c.fx_phi_exp;
     sc.extra = c.fx_extra;
     sc.rho_max = c.fx_rho_max;
-    int4 *gw = nullptr;
+    FxFactors gw{};
     if (a.g_weight && (a.flags & BIE_G)) {
-        sc.wexp = a.g_weight_exp;
-        gw = static_cast<int4 *>(c.scratch(kScratchFxWeight, (size_t)c.n_elements * sizeof(int4)));
-        fx_weight_kernel<<<(unsigned)((c.n_elements + 255) / 256), 256, 0, c.stream>>>(
-            reinterpret_cast<const double2 *>(a.g_weight), c.n_elements, sc.wexp, gw);
+        const size_t E = (size_t)c.n_elements, N = (size_t)c.n_sources;
+        int4 *limbs = static_cast<int4 *>(c.scratch(kScratchFxWeight, E * 20 + N * 4));
+        int *exps = reinterpret_cast<int *>(limbs + E), *nodes = exps + E;
+        BIE_CUDA(cudaMemsetAsync(nodes, 0xc0, N * 4, c.stream));   // far below every exponent
+        fx_factor_kernel<<<(unsigned)((E + 255) / 256), 256, 0, c.stream>>>(
+            reinterpret_cast<const double2 *>(a.g_weight), c.n_elements, c.d_xrecords, X.stride, limbs, exps, nodes);
         BIE_CUDA(cudaGetLastError());
         ++c.kernel_launches;
+        gw = FxFactors{limbs, exps, nodes};
+        sc.extra_w = c.fx_extra_w;
     }
     const Fp64View v{c.d_records, L.stride, L.nidx_off, c.d_phi, L.qmax, ri64, c.d_xtrig};
     const int level = sh.level, S = spread ? spread : 1 << level;
@@ -644,7 +668,7 @@ void launch_np(Ctx &c, const AssembleArgs &a, const LaunchShape &sh, int spread,
     }
     auto kern = assemble_fix64_kernel<NP, CPLX, false>;
     if constexpr (NP == 3 && !CPLX)
-        if (gw) kern = assemble_fix64_kernel<NP, CPLX, true>;
+        if (gw.limbs) kern = assemble_fix64_kernel<NP, CPLX, true>;
     BIE_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const dim3 grid((unsigned)((a.M + kThreads - 1) / kThreads), (unsigned)S);
     cudaEvent_t t0 = c.timer_begin();
@@ -660,7 +684,7 @@ void launch_np(Ctx &c, const AssembleArgs &a, const LaunchShape &sh, int spread,
     if (nfix > 0 && (F || G)) {
         fx_widen_kernel<CPLX><<<stream_grid(c, nfix * a.M), 256, 0, c.stream>>>(
             fnode, nfix, reinterpret_cast<const float4 *>(c.d_xnodes), a.targets, a.M, a.k_re, a.k_im, sc, F, G,
-            a.k_dev);
+            gw.nodes, a.k_dev);
         BIE_CUDA(cudaGetLastError());
         ++c.kernel_launches;
     }
@@ -857,17 +881,25 @@ void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
         }
     }
     // entries hold |sum| <= 4 sqrt(2) 2^55 sum of the reaches: below 2^62
-    std::vector<double> node_reach(N, 0.0);
+    // (with element factors each contribution may be the node's largest, and a
+    // factor's modulus is up to sqrt(2) of its unit: G is below half of F's bound)
+    std::vector<double> node_reach(N, 0.0), node_all(N, 0.0);
     for (int64_t p = 0; p < E; ++p)
         for (int a = 0; a < NP; ++a) {
             const int32_t nd = c.ptopo[NP * c.order[p] + a];
             rec[(size_t)p * X.stride + kHdrNodes + 6 * NP + a] = node_ej[nd];
             node_reach[nd] += std::ldexp(reach[(size_t)p * NP + a], ej[p] - node_ej[nd]);
+            node_all[nd] += reach[(size_t)p * NP + a];
         }
-    double worst = 0.0;
-    for (double v : node_reach) worst = std::max(worst, v);
-    c.fx_extra = 0;
-    while (std::ldexp(worst * 5.7, -c.fx_extra) > 127.0) ++c.fx_extra;
+    auto extra_of = [](const std::vector<double> &reach) {
+        double worst = 0.0;
+        for (double v : reach) worst = std::max(worst, v);
+        int x = 0;
+        while (std::ldexp(worst * 5.7, -x) > 127.0) ++x;
+        return x;
+    };
+    c.fx_extra = extra_of(node_reach);
+    c.fx_extra_w = extra_of(node_all);
 
     std::vector<float> nodes((size_t)4 * N);
     for (int64_t j = 0; j < N; ++j) {
@@ -885,7 +917,7 @@ void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
 }
 
 static bool fix64_covers(const Ctx &c, const AssembleArgs &a) {
-    if (!c.fx_ok || a.taylor_m >= 0 || (a.g_weight && a.g_weight_exp == INT32_MIN)) return false;
+    if (!c.fx_ok || a.taylor_m >= 0 || (a.g_weight && !a.g_weight_bounded)) return false;
     if (a.k_dev && !(a.k_abs_max > 0)) return false;   // no bound on |k|
     if (a.M > INT32_MAX) return false;   // rows are 32-bit in the list of deferred pairs
     const bool cplx = a.k_im != 0.0;

@@ -108,6 +108,29 @@ FX_FN Values2 complex_mul(Limb ar, Limb ai, Limb br, Limb bi) {
                    fold_up<2>(high(wide(ar.h, bi.h), ai, br), cross(cross<2>(ar, bi), ai, br))};
 }
 
+// An element's complex factor on G as Q62 limbs times 2^-e and that e, its own
+// exponent (largest component in [1/2, 1)): factors of a mesh may spread over any
+// range without losing bits.  Zero has the exponent kZeroFactor, below every
+// other one's.
+constexpr int kZeroFactor = -4096;
+struct Factor {
+    Limb re, im;
+    int e;
+};
+FX_FN Factor element_factor(double re, double im) {
+    const double m = re < 0 ? -re : re, n = im < 0 ? -im : im, top = m > n ? m : n;
+    if (top == 0.0) return Factor{Limb{0, 0}, Limb{0, 0}, kZeroFactor};
+#ifdef __CUDA_ARCH__
+    int e;
+    (void)frexp(top, &e);
+    return Factor{split(__double2ll_rn(ldexp(re, 62 - e))), split(__double2ll_rn(ldexp(im, 62 - e))), e};
+#else
+    int e;
+    (void)std::frexp(top, &e);
+    return Factor{split((i64)std::llrint(std::ldexp(re, 62 - e))), split((i64)std::llrint(std::ldexp(im, 62 - e))), e};
+#endif
+}
+
 constexpr int kTrigBits = 10;                      // e^{2 pi i j / 1024}
 constexpr int kTrigEntries = 1 << kTrigBits;
 constexpr int kCoordBits = 59;                     // fixed coordinates: largest |x| -> 2^59

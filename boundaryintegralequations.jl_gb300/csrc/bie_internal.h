@@ -252,6 +252,7 @@ struct Ctx {
     float fx_rho_max = 0.f;              // largest point or node offset from a centroid (scaled)
     int fx_phi_exp = 0;                  // basis values are stored times 2^-fx_phi_exp
     int fx_extra = 0;                    // entry units times 2^fx_extra (nodes with many elements)
+    int fx_extra_w = 0;                  // ... of G with element factors
     float *d_xrecords = nullptr;         // E x xlay.stride words, element order
     int32_t *d_xphi = nullptr;           // R x qmax x (4, 8, 12) limb words
     float *d_xnodes = nullptr;           // N x (x, y, z, entry weight exponent)
@@ -324,8 +325,8 @@ struct AssembleArgs {
     bool c64_out = false;    // mixed only: F, G are complex64 (float2) buffers, not widened
     const double *g_weight = nullptr;   // not mixed: per-element complex factor on G
                                         // (record order), e.g. an element admittance
-    int g_weight_exp = INT32_MIN;       // |Re|, |Im| of the factors < 2^g_weight_exp; INT32_MIN:
-                                        // not known (no fixed-point assembly)
+    bool g_weight_bounded = false;      // the factors are finite, below 2^400 (else no
+                                        // fixed-point assembly)
     int taylor_m = -1;                  // FP64 only: >= 0 assembles the taylor_m-th
                                         // k-derivative (corner rules only)
     const double *k_dev = nullptr;      // device (re, im): the kernels read k here instead

@@ -40,3 +40,14 @@ def test_deferred_pairs_are_counted_once_per_row_and_slice(build, capacity, perc
 def test_columns_of_many_rows(build):
     # 2^28 rows and more: a column is 4 GB
     assert build("fix64_columns")() == ["1"]
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_element_factors_of_any_magnitude(build, seed):
+    """Value times factor, in the value's unit (2^-59 of its range): the final
+    shift rounds to half a unit, the two products of low limbs that are left out
+    are below 2^62 2^-62 = 1 each, and the factor's own rounding 2^-62 of a
+    component counts an eighth: 2.7 units.  The factor's exponent is its own, so
+    this holds whatever other elements carry."""
+    out = build("fix64_factor")(seed)
+    assert float(out[0]) <= 2.7 and out[1] == "1"
