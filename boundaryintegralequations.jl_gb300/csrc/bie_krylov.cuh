@@ -83,6 +83,7 @@ __device__ __forceinline__ double row_product(const int64_t *__restrict__ rp, co
 __device__ __forceinline__ void rotate_column(double2 *col, const double2 *sn, const double *cs, int j, int lane) {
     const bool im = lane & 1, fin = lane & 2;
     double2 a = col[0];
+    __syncwarp(0xfu);   // lanes 2, 3 store col[0] in the first pass (the shuffles order the later entries)
     for (int k = 0; k < j; ++k) {
         const double2 b = col[k + 1], s = sn[k];
         const double2 p = fin ? a : b, q = fin ? b : a;
