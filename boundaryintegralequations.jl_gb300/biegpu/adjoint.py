@@ -22,8 +22,9 @@ def farfield_objective(mesh: Mesh3d, k: float, Z, field_points, rho_c: float = 1
                        direction=(0.0, 0.0, 1.0), gradient: bool = True, reltol: float = 1e-13,
                        n: int = 2, m: int = 2, device: int = 0, precision: str = "fp64"):
     """(J, p_field, dJ/dX (3 x N_c) or None, dJ/dZ (E complex) or None, info).
-    ``precision="df64"`` assembles the forward model in double-float
-    arithmetic (FP64-grade, faster on GB300); the reverse pass is FP64."""
+    ``precision="df64"`` takes the double-float kernels of the library for the
+    forward model and the reverse pass (gradients to about 1e-13, faster on
+    GB300); with "fp64" the reverse pass is FP64."""
     ctx = get_context(mesh, n=n, m=m, device=device)
     Zc = np.ascontiguousarray(Z, dtype=np.complex128)
     if Zc.shape != (mesh.n_elements,):

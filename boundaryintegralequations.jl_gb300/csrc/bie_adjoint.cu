@@ -19,8 +19,9 @@
 // The reverse pass recomputes the quadrature of every (row, element) pair
 // with the forward rule choice (the nearest-node rule is piecewise constant
 // in the geometry) and accumulates analytic derivatives of the integrands
-// with respect to the element vertices, the collocation point and Y_e.
-// FP64 throughout.
+// with respect to the element vertices, the collocation point and Y_e: in FP64
+// for BIE_PREC_FP64 (adjoint_grad_kernel), in double-float with the near pairs in
+// FP64 for BIE_PREC_DF64 (adjoint_df64_kernel).
 #include "bie_internal.h"
 #include "bie_device.cuh"
 #include "bie_df64.cuh"
@@ -293,9 +294,9 @@ adjoint_grad_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
 }
 
 // ---------------------------------------------------------------------------
-// The reverse pass on the FP32 pipes.
+// The reverse pass on the FP32 pipes (BIE_PREC_DF64).
 //
-// adjoint_grad_kernel is bound by the FP64 pipe (87 % busy, 79 ms for the
+// adjoint_grad_kernel is bound by the FP64 pipe (87 % busy, 67 ms for the
 // 4842-node ellipsoid, 46.9 M pairs).  Here the regular pairs run in double-float
 // (bie_df64.cuh) and only near pairs and nearest-node near-ties in FP64, in place:
 // 13.0 ms, bound by instruction issue and half by instruction fetch (128
@@ -303,8 +304,11 @@ adjoint_grad_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
 // 19.7 ms at 255 registers): the loop over elements is longer than the
 // instruction caches, so the warps of a block stay together.  Whole gradient 28.2
 // ms without that, 26.9 in blocks of 128 threads, 25.8 of 256, 27.4 of 512.  Phases
-// are formed without cancellation, so gradients differ from the FP64 kernel's by
-// 3e-14 .. 8e-14, below the error of the solves (1e-13 .. 4e-13).  With
+// are formed without cancellation.  Error of a gradient with the solves carried on
+// to 3e-16 (a tolerance of 1e-13 leaves 1e-13 .. 9e-13), ellipsoids of 252 to 2562
+// nodes at k = 3, field points at 10: 2e-14 .. 4e-14, with the FP64 kernel 3e-15 ..
+// 1e-14; at k = 0.3 or with field points at 1.5 it is 5e-15 .. 5e-14 against 1e-15 ..
+// 6e-15, so FP64 callers keep the FP64 kernel.  With
 // b = conj(w) p(x_q), z = b e^{ikr}, W = jw / 4 pi, n the unit normal, d = x_q - t,
 // g = z alpha_G Y_e, sc = Re conj(w) p_i (collocation rows):
 //   t3 = alpha_F (z_r + k r z_i) - sc,     gp = Re g (i k r - 1),
@@ -877,7 +881,8 @@ void run_adjoint(Ctx &c, const AdjointArgs &a, AdjointOut &out) {
         BIE_CUDA(cudaMemsetAsync(sY.p, 0, E * 16, st));
         const double rhock_re = a.rho_c * a.k_re;
         df64::DfDegrees deg{};
-        if (df64::df_degrees(std::fabs(a.k_re) * c.df_rho_max, 0.0, deg)) {
+        // (a caller of BIE_PREC_FP64 gets FP64 here too)
+        if (a.precision == BIE_PREC_DF64 && df64::df_degrees(std::fabs(a.k_re) * c.df_rho_max, 0.0, deg)) {
             deg.tab = reinterpret_cast<const float4 *>(c.d_phase_tab);
             const RecordLayout &L = c.lay;
             const Df64Layout &X = c.dlay;
@@ -922,7 +927,7 @@ void run_adjoint(Ctx &c, const AdjointArgs &a, AdjointOut &out) {
                                                               dX.d(), sY.d2());
             BIE_CUDA(cudaGetLastError());
             BIE_CUDA(cudaStreamSynchronize(st));   // the call's buffers go out of scope
-        } else {   // phase rotations beyond the double-float tables
+        } else {   // FP64, or phase rotations beyond the double-float tables
             int S = 1;
             const int64_t tiles = (N + M + kT - 1) / kT;
             while (tiles * S < 8LL * c.num_sms && S < 256 && S * 2 <= E) S *= 2;

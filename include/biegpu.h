@@ -648,7 +648,8 @@ typedef struct bie_adjoint_opts {
     double rho_c;        /* characteristic impedance rho0 c of the fluid (e.g. 1.21 * 343) */
     double dir[3];       /* incident plane-wave direction (unit vector)                  */
     double reltol;       /* GMRES tolerance of the forward and adjoint solves (<= 0: 1e-13) */
-    int32_t precision;   /* forward-model assembly: BIE_PREC_FP64 (0) or BIE_PREC_DF64       */
+    int32_t precision;   /* BIE_PREC_FP64 (0), or BIE_PREC_DF64: double-float assembly of the
+                            forward model and regular pairs of the reverse pass          */
 } bie_adjoint_opts;
 
 typedef struct bie_adjoint_info {
@@ -666,7 +667,8 @@ typedef struct bie_adjoint_info {
  * The reference has no gradient code (its only prior art is finite differences
  * in 2D, examples/2d_optimization.jl:187-219; nodal impedance form
  * examples/3d_cube_wave_anechoic.jl:62-68).  Gradients by the adjoint method
- * with a reverse pass that recomputes the quadrature (FP64):
+ * with a reverse pass that recomputes the quadrature (in FP64; for
+ * opts->precision = BIE_PREC_DF64 the regular pairs in double-float):
  *   dX: 3 x N_c, dJ/d(vertex coordinates);  dZ: E complex, dJ/dRe Z_e + i dJ/dIm Z_e.
  * Z: E complex impedances in the element order of the mesh.  Outputs may be
  * NULL (J alone costs one forward solve).  Host buffers; blocking.

@@ -1,5 +1,5 @@
 """Adjoint gradients where the arithmetic's ranges matter: admittances of very
-different size in one mesh."""
+different size in one mesh, meshes away from the origin."""
 from __future__ import annotations
 
 import numpy as np
@@ -7,6 +7,7 @@ import pytest
 
 import biegpu
 import oracle
+from biegpu import mesh as bm
 
 from test_gpu_adjoint import RHO_C, setup
 
@@ -26,3 +27,37 @@ def test_soft_patch_beside_hard_elements(ratio, precision):
     _, want = oracle.farfield_objective(mesh, 3.0, Z, X, rho_c=RHO_C)
     assert info["forward_converged"]
     assert np.linalg.norm(pf - want) <= 1e-12 * np.linalg.norm(want)
+
+
+def moved(mesh, shift, scale=1.0):
+    P = mesh.coordinates * scale + np.asarray(shift, dtype=np.float64)[:, None]
+    return bm._finish(P, mesh.topology, "linear", "geometry")
+
+
+def against_forward_mode(mesh, k, Z, X, precision, tol):
+    from oracle import forward_mode as fm
+    _, _, dX, dZ, info = biegpu.farfield_objective(mesh, k, Z, X, rho_c=RHO_C, precision=precision)
+    assert info["forward_converged"] and info["adjoint_converged"]
+    rng = np.random.default_rng(11)
+    for _ in range(3):
+        V = rng.normal(size=mesh.coordinates.shape)
+        _, dJ = fm.farfield_directional_derivative(mesh, k, Z, X, Vdir=V, rho_c=RHO_C)
+        assert abs(float(np.sum(dX * V)) - dJ) <= tol * np.linalg.norm(dX) * np.linalg.norm(V)
+        dz = rng.normal(size=mesh.n_elements) + 1j * rng.normal(size=mesh.n_elements)
+        _, dJz = fm.farfield_directional_derivative(mesh, k, Z, X, dZ=dz, rho_c=RHO_C)
+        gz = float(np.sum(dZ.real * dz.real + dZ.imag * dz.imag))
+        assert abs(gz - dJz) <= tol * np.linalg.norm(dZ) * np.linalg.norm(dz)
+
+
+@pytest.mark.parametrize("shift", [(0.0, 0.0, 0.0), (300.0, -200.0, 150.0)])
+@pytest.mark.parametrize("precision", ["fp64"])
+def test_gradient_to_the_precision_asked_for(precision, shift):
+    """Gradients against the exact derivative of the CPU restatement.  A point's
+    coordinate carries 2^-53 |x| (|x| about 400 on the moved mesh: 4.4e-14), the
+    nearest pairs are some 0.03 away and the derivative goes with the third power
+    of the distance: 4.4e-12 at most, and 1e-12 from the solves (1e-13 each, a
+    decade for the system's condition).  Double-float coordinates (2^-48) would
+    be 32 times as far off."""
+    mesh, Z, X = setup(3, nfield=8)
+    tol = 5.4e-12 if shift[0] else 1e-12
+    against_forward_mode(moved(mesh, shift), 3.0, Z, X + np.asarray(shift)[:, None], precision, tol)
