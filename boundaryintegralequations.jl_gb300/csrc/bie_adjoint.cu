@@ -460,7 +460,6 @@ adjoint_df64_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
         wv = w[row];
         if (node) pv = p[row];
     }
-    const mixed::Target T{dd::to_df(tx), dd::to_df(ty), dd::to_df(tz)};
     const df cwr = dd::to_df(wv.x), cwi = dd::to_df(-wv.y);
     const df sc = dd::to_df(node ? wv.x * pv.x + wv.y * pv.y : 0.0);   // Re conj(w) p_i
     Acc gt[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
@@ -520,7 +519,11 @@ adjoint_df64_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = Acc{0.f, 0.f};
             if (active) {
-                const mixed::PairSetup P = mixed::pair_setup<3>(r, T);
+                // D = centroid - t in FP64 before it is split: of absolute coordinates
+                // rounded to float pairs it would lose 2^-48 |x|
+                const double *cen = reinterpret_cast<const double *>(s_el + 32 * el + 24);
+                const double ax = cen[0] - tx, ay = cen[1] - ty, az = cen[2] - tz;
+                const mixed::PairSetup P = mixed::pair_setup<3>(r, r[6], dd::to_df(ax), dd::to_df(ay), dd::to_df(az));
                 df r0, ri0;
                 dd::sqrt_rcp_df(dev::df_add(dev::df_add(dev::df_sqr(P.Dxd), dev::df_sqr(P.Dyd)), dev::df_sqr(P.Dzd)),
                                 r0, ri0);
@@ -551,8 +554,6 @@ adjoint_df64_kernel(int64_t N, int64_t M, const double *__restrict__ src, const 
                     // otherwise idle pipe), series in double-float
                     df E0r, E0i;
                     {
-                        const double *cen = reinterpret_cast<const double *>(s_el + 32 * el + 24);
-                        const double ax = cen[0] - tx, ay = cen[1] - ty, az = cen[2] - tz;
                         const double q2 = ax * ax + ay * ay + az * az;
                         const double x = kre * (q2 * rsqrt(q2));
                         const double nq = rint(x * 0.63661977236758134308);   // 2 / pi
@@ -699,7 +700,9 @@ __global__ void adjoint_finish_kernel(const double *__restrict__ sums, const dou
     for (int k = 0; k < 3; ++k) {
         cen[k] = X[0][k] / 3.0;
         cen[k] += X[1][k] / 3.0;
-        cen[k] += X[2][k] / 3.0;   // as the records form it
+        cen[k] += X[2][k] / 3.0;
+        const float hi = (float)cen[k];   // as the records hold it
+        cen[k] = (double)hi + (double)(float)(cen[k] - (double)hi);
         u[k] = X[1][k] - X[0][k];
         v[k] = X[2][k] - X[0][k];
         for (int b = 0; b < 3; ++b) eb[b][k] = X[b][k] - cen[k];

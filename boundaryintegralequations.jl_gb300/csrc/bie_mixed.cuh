@@ -50,13 +50,11 @@ struct PairSetup {
 
 // Nearest physics node in FP32 with near / near-tie detection.
 template <int NP>
-__device__ __forceinline__ PairSetup pair_setup(const float *r, const Target &T) {
+__device__ __forceinline__ PairSetup pair_setup(const float *r, float near2, df Dx, df Dy, df Dz) {
     PairSetup P;
-    const float4 h0 = *reinterpret_cast<const float4 *>(r);       // c_hi xyz, c_lo x
-    const float4 h1 = *reinterpret_cast<const float4 *>(r + 4);   // c_lo yz, near2, -
-    P.Dxd = dev::df_sub({h0.x, h0.w}, T.x);
-    P.Dyd = dev::df_sub({h0.y, h1.x}, T.y);
-    P.Dzd = dev::df_sub({h0.z, h1.y}, T.z);
+    P.Dxd = Dx;
+    P.Dyd = Dy;
+    P.Dzd = Dz;
     P.Dx = P.Dxd.hi;
     P.Dy = P.Dyd.hi;
     P.Dz = P.Dzd.hi;
@@ -79,10 +77,16 @@ __device__ __forceinline__ PairSetup pair_setup(const float *r, const Target &T)
 #pragma unroll
     for (int a = 0; a < NP; ++a) tie |= (a != c) && (d2[a] <= lim);
     const float r0f2 = P.Dx * P.Dx + P.Dy * P.Dy + P.Dz * P.Dz;
-    const float near2 = h1.z;
     P.c = c;
     P.deferred = tie || r0f2 < near2 || 4.0f * b < near2;
     return P;
+}
+template <int NP>
+__device__ __forceinline__ PairSetup pair_setup(const float *r, const Target &T) {
+    const float4 h0 = *reinterpret_cast<const float4 *>(r);       // c_hi xyz, c_lo x
+    const float4 h1 = *reinterpret_cast<const float4 *>(r + 4);   // c_lo yz, near2, -
+    return pair_setup<NP>(r, h1.z, dev::df_sub({h0.x, h0.w}, T.x), dev::df_sub({h0.y, h1.x}, T.y),
+                          dev::df_sub({h0.z, h1.y}, T.z));
 }
 
 struct Phase {

@@ -61,3 +61,19 @@ def test_gradient_to_the_precision_asked_for(precision, shift):
     mesh, Z, X = setup(3, nfield=8)
     tol = 5.4e-12 if shift[0] else 1e-12
     against_forward_mode(moved(mesh, shift), 3.0, Z, X + np.asarray(shift)[:, None], precision, tol)
+
+
+@pytest.mark.parametrize("shift,scale", [((0.0, 0.0, 0.0), 1.0), ((0.0, 0.0, 0.0), 1e-3), ((0.0, 0.0, 0.0), 3e4),
+                                         ((300.0, -200.0, 160.0), 1.0)])
+def test_double_float_gradient_beside_fp64(shift, scale):
+    """Regular pairs in 48 bits stay within 1e-13 of FP64 where the mesh is near the
+    origin (1e-12 with the solves).  Moved by 400 both precisions carry the
+    coordinates' 2^-53 |x| = 4.4e-14, over the nearest distance of 0.03 1.5e-12; a
+    distance taken between coordinates that were rounded to float pairs (2^-48)
+    would put 32 times that into the nearer pairs."""
+    mesh, Z, X = setup(6, nfield=8)
+    mesh = moved(mesh, shift, scale)
+    X = X * scale + np.asarray(shift)[:, None]
+    a, b = (biegpu.farfield_objective(mesh, 3.0 / scale, Z, X, rho_c=RHO_C, precision=p) for p in ("fp64", "df64"))
+    for i in (2, 3):
+        assert np.linalg.norm(b[i] - a[i]) <= (1.5e-12 if shift[0] else 1e-12) * np.linalg.norm(a[i])
