@@ -738,6 +738,26 @@ __global__ void adjoint_finish_kernel(const double *__restrict__ sums, const dou
 
 inline unsigned nblocks(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 
+// Whether the double-float kernel's values stay clear of the ends of FP32's range.
+// They go with the adjoint pressure over the mesh size L (a gradient's terms, and
+// about 2^-14 of it per point); the error term of a product of pairs is 2^-72 of
+// it.  Largest adjoint pressure over L and error against the FP64 kernel: 2^-37
+// 3e-14, 2^-47 5e-14, 2^-53 3e-10, 2^-57 6e-11 .. 1e-4.
+bool double_float_range(const Ctx &c, const std::vector<std::complex<double>> &lam,
+                        const std::vector<std::complex<double>> &pf, const AdjointArgs &a) {
+    auto largest = [](const std::vector<std::complex<double>> &v) {
+        double m = 0.0;
+        for (const auto &x : v) m = std::max(m, std::max(std::fabs(x.real()), std::fabs(x.imag())));
+        return m;
+    };
+    const double l = largest(lam), p = largest(pf);
+    double z = INFINITY;
+    for (int64_t e = 0; e < 2 * c.n_elements; e += 2)
+        z = std::min(z, std::max(std::fabs(a.Z[e]), std::fabs(a.Z[e + 1])));
+    return l >= std::ldexp(1.0, c.fx_exp - 40) && l <= 0x1p40 && p <= 0x1p40 &&
+           std::fabs(a.rho_c * a.k_re) <= 0x1p60 * z;
+}
+
 }  // namespace
 
 void run_adjoint(Ctx &c, const AdjointArgs &a, AdjointOut &out) {
@@ -772,6 +792,9 @@ void run_adjoint(Ctx &c, const AdjointArgs &a, AdjointOut &out) {
         BIE_CUDA(cudaMalloc(&c.d_topo, c.topo.size() * sizeof(int32_t)));
         BIE_CUDA(cudaMemcpy(c.d_topo, c.topo.data(), c.topo.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     }
+    // double-float holds squares and cubes of lengths: mesh sizes within 2^+-30
+    // (gradient error 4e-14 at 2^-43, 3e-12 to 8e-12 at 2^-50)
+    const bool use_df = a.precision == BIE_PREC_DF64 && c.fx_ok && std::abs(c.fx_exp) <= 30;
     // -i rho c k and +i rho c k (k real)
     const double2 aAc = make_double2(0.0, -a.rho_c * a.k_re);
     const double2 aBc = make_double2(0.0, a.rho_c * a.k_re);
@@ -784,14 +807,14 @@ void run_adjoint(Ctx &c, const AdjointArgs &a, AdjointOut &out) {
         AssembleArgs s{a.k_re, a.k_im, c.d_sources, N, BIE_F | BIE_G | BIE_C, A.d(), G.d(), Cv.d()};
         s.g_weight = Y.d();
         s.g_weight_bounded = bounded;
-        if (!(a.precision == BIE_PREC_DF64 && launch_assemble_df64(c, s))) launch_assemble_fp64(c, s);
+        if (!(use_df && launch_assemble_df64(c, s))) launch_assemble_fp64(c, s);
         combine_system_kernel<<<std::min<unsigned>(nblocks(N * N), 65535u), 256, 0, st>>>(
             A.d2(), G.d2(), aAc, Cv.d2(), N, N);
         BIE_CUDA(cudaGetLastError());
         AssembleArgs f{a.k_re, a.k_im, fp.d(), M, BIE_F | BIE_G, B.d(), Gx.d(), nullptr};
         f.g_weight = Y.d();
         f.g_weight_bounded = bounded;
-        if (!(a.precision == BIE_PREC_DF64 && launch_assemble_df64(c, f))) launch_assemble_fp64(c, f);
+        if (!(use_df && launch_assemble_df64(c, f))) launch_assemble_fp64(c, f);
         // stored: F_x - i rho c k G_x  (= -B)
         combine_system_kernel<<<std::min<unsigned>(nblocks(M * N), 65535u), 256, 0, st>>>(
             B.d2(), Gx.d2(), make_double2(-aBc.x, -aBc.y), nullptr, M, N);
@@ -885,7 +908,8 @@ void run_adjoint(Ctx &c, const AdjointArgs &a, AdjointOut &out) {
         const double rhock_re = a.rho_c * a.k_re;
         df64::DfDegrees deg{};
         // (a caller of BIE_PREC_FP64 gets FP64 here too)
-        if (a.precision == BIE_PREC_DF64 && df64::df_degrees(std::fabs(a.k_re) * c.df_rho_max, 0.0, deg)) {
+        if (use_df && double_float_range(c, hl, hp, a) &&
+            df64::df_degrees(std::fabs(a.k_re) * c.df_rho_max, 0.0, deg)) {
             deg.tab = reinterpret_cast<const float4 *>(c.d_phase_tab);
             const RecordLayout &L = c.lay;
             const Df64Layout &X = c.dlay;
@@ -930,7 +954,7 @@ void run_adjoint(Ctx &c, const AdjointArgs &a, AdjointOut &out) {
                                                               dX.d(), sY.d2());
             BIE_CUDA(cudaGetLastError());
             BIE_CUDA(cudaStreamSynchronize(st));   // the call's buffers go out of scope
-        } else {   // FP64, or phase rotations beyond the double-float tables
+        } else {   // FP64, or values or phase rotations beyond the double-float kernel's
             int S = 1;
             const int64_t tiles = (N + M + kT - 1) / kT;
             while (tiles * S < 8LL * c.num_sms && S < 256 && S * 2 <= E) S *= 2;

@@ -77,3 +77,17 @@ def test_double_float_gradient_beside_fp64(shift, scale):
     a, b = (biegpu.farfield_objective(mesh, 3.0 / scale, Z, X, rho_c=RHO_C, precision=p) for p in ("fp64", "df64"))
     for i in (2, 3):
         assert np.linalg.norm(b[i] - a[i]) <= (1.5e-12 if shift[0] else 1e-12) * np.linalg.norm(a[i])
+
+
+@pytest.mark.parametrize("scale,radius", [(1.0, 1e10), (1e9, 1e6), (1e15, 10.0), (1e-15, 10.0)])
+def test_double_float_gradient_at_the_ends_of_its_range(scale, radius):
+    """Lengths and distances whose products leave FP32's range (the adjoint pressure
+    falls with the field points' distance): such calls take the FP64 reverse pass."""
+    mesh, Z, X = setup(5, nfield=8)
+    mesh = moved(mesh, (0.0, 0.0, 0.0), scale)
+    k = (3.0 if radius == 10.0 else 1e-3) / scale
+    X = X * (radius / 10.0 * scale)
+    a, b = (biegpu.farfield_objective(mesh, k, Z, X, rho_c=RHO_C, precision=p) for p in ("fp64", "df64"))
+    for i in (2, 3):
+        size = np.max(np.abs(a[i]))
+        assert np.linalg.norm((b[i] - a[i]) / size) <= 1e-12 * np.linalg.norm(a[i] / size)
