@@ -8,7 +8,7 @@
 // argument's bits are taken apart, the function is evaluated on 64-bit integers
 // (about 150 and 80 instructions) and the double is put together from bits.
 // Errors against extended precision: roots 0.51 ulp, exponential 0.7 ulp, sine
-// and cosine 2^-60 of 1 besides the final rounding (an error of the modulus of
+// and cosine 2^-59 of 1 besides the final rounding (an error of the modulus of
 // e^{ikr}).  Arguments beyond the ranges below take the library's
 // functions.  Measured: corrections of the near pairs of the mixed assembly at 11562
 // nodes 232 -> 202 us and of the mixed product at 40962 nodes 1.56 -> 1.36 ms
@@ -86,9 +86,10 @@ FX_FN bool root(double r2, double &rinv, double &r) {
     return true;
 }
 
-// (m j) >> sh of a 53-bit and a 64-bit number, 0 < sh: the low 64 bits, the rest in top
-FX_FN u64 scaled_product(u64 m, u64 j, int sh, u64 &top) {
-    const u64 hi = mul_high(m, j), lo = m * j;
+// (m j + more) >> sh of a 53-bit and a 64-bit number, 0 < sh: the low 64 bits, the rest
+// in top
+FX_FN u64 scaled_product(u64 m, u64 j, int sh, u64 &top, u64 more = 0) {
+    const u64 lo = m * j + more, hi = mul_high(m, j) + (lo < more ? 1 : 0);
     const int a = sh < 64 ? sh : 63, b = sh < 64 ? 0 : (sh < 127 ? sh - 64 : 63);
     top = sh < 64 ? hi >> a : 0;
     return sh < 64 ? (hi << (64 - a)) | (lo >> a) : hi >> b;
@@ -100,9 +101,14 @@ FX_FN bool sine_cosine(double x, const Table &table, double &s, double &c) {
     const u64 u = double_bits(x);
     const int ex = (int)(u >> 52) & 0x7ff;
     if (ex >= 1043) return false;
-    // x / 2 pi as a 64-bit fraction of a turn (2^66 / 2 pi; a subnormal is below 2^-64)
+    // x / 2 pi as a 64-bit fraction of a turn (a subnormal is below 2^-64): 2^66 / 2 pi
+    // in two words, the second for |x| >= 2^9 (rounded to one word it is good to
+    // 2^-69 |x|)
+    const u64 m = (u & 0xfffffffffffffull) | 0x10000000000000ull;
     u64 top;
-    const u64 frac = scaled_product((u & 0xfffffffffffffull) | 0x10000000000000ull, 0xa2f9836e4e44152aull, 1077 - ex, top);
+    const u64 frac = ex < 1032 ? scaled_product(m, 0xa2f9836e4e44152aull, 1077 - ex, top)
+                               : scaled_product(m, 0xa2f9836e4e441529ull, 1077 - ex, top,
+                                                mul_high(m, 0xfc2757d1f534ddc0ull));
     i64 Er, Ei;
     unit_circle<true>(frac, table, Er, Ei);
     c = fixed_double(Er, -62);
