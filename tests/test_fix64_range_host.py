@@ -59,3 +59,12 @@ def test_sine_and_cosine_over_their_range(build, exponent):
     2^-60, the truncated turn 2 pi 2^-64, and below 2^9 1 / 2 pi in one word
     (2^-69.4 |x|)."""
     assert float(build("fix64_sine")(1, exponent)[0]) <= 1.0
+
+
+@pytest.mark.parametrize("exponent", [-1022, -300, -60, -31, -30, -29, -20, -15, -12, -10, -9])
+def test_sine_of_small_arguments(build, exponent):
+    """Below 2^-8 the sine is relative to its argument: half a unit of rounding, and
+    2^-58 of the value from x^2 (Q72), the two series terms (the next one is
+    x^6 / 5040 < 2^-60) and the product: 0.52 units."""
+    out = build("fix64_sine")(1, exponent)
+    assert float(out[0]) <= 1.0 and float(out[1]) <= 0.52

@@ -1,0 +1,45 @@
+"""Imaginary parts at small wavenumbers.  With k r small e^{ikr} is nearly real: the
+imaginary part of G is about k times its real part, that of F about k^3, and each is
+a result of its own (it carries the radiated power).  FP64 calls keep each part to
+FP64, not only the modulus."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+import biegpu
+import oracle
+from biegpu import mesh as bm
+
+from conftest import rel_fro
+
+pytestmark = pytest.mark.gpu
+
+
+def check_parts(F, G, wantF, wantG, k):
+    """G: sin(k r) to a few units, summed over some ten points: 1e-14.  F: the
+    difference k r cos(k r) - sin(k r) of terms that round at 2^-53 k r (r at most 2
+    here), a few dozen points of either sign: 2^-48 k of the modulus."""
+    assert rel_fro(G.imag, wantG.imag) <= 1e-14
+    assert np.linalg.norm(F.imag - wantF.imag) <= 2.0**-48 * k * np.linalg.norm(wantF.real)
+    assert rel_fro(F, wantF) <= 1e-12 and rel_fro(G, wantG) <= 1e-12
+
+
+@pytest.mark.parametrize("k", [1e-8, 1e-5, 1e-2, 0.3])
+def test_near_field(k):
+    mesh = bm.icosphere(3, geometry="quadratic")
+    F, G = biegpu.assemble_parallel(mesh, k, sparse=True, depth=1, offset=0.2)
+    o = oracle.nearfield(mesh, k, depth=1, offset=0.2)
+    check_parts(F.data, G.data, *o[2:4], k)
+
+
+@pytest.mark.parametrize("geometry", ["linear", "quadratic"])
+@pytest.mark.parametrize("k", [1e-8, 1e-5, 1e-2, 0.3])
+def test_matrix_free_product(geometry, k):
+    mesh = bm.icosphere(4, geometry=geometry)
+    want = oracle.assemble(mesh, k, n=2, m=2)
+    x = np.random.default_rng(2).uniform(0.5, 1.5, mesh.n_sources).astype(np.complex128)
+    F, G = ((op(mesh, k, n=2, m=2, precision="fp64") @ torch.from_numpy(x).cuda()).cpu().numpy()
+            for op in (biegpu.GPUFOperator, biegpu.GPUGOperator))
+    check_parts(F, G, want[0] @ x, want[1] @ x, k)
