@@ -166,6 +166,7 @@ struct MeshRun {
     bool mixed;
     bool df64;        // FP64-grade assembly in double-float arithmetic
     double kmax = 0;  // largest |k| of the sweep (the double-float phase tables' bound)
+    double kmin = 0;  // smallest |Re k| other than 0
     DevBuf F, G, vec, P, dinfo, kb, ctl, tsb;
     double2 *Cv, *dg, *b, *wd, *X;
     double2 *pz = nullptr, *py = nullptr, *pw = nullptr;   // sensitivity probe: z, y ~ A^-1 z, A z
@@ -251,6 +252,7 @@ struct MeshRun {
         a.c64_out = mixed;
         a.k_dev = kd;
         a.k_abs_max = kmax;
+        a.k_re_min = kmin;
         return a;
     }
     void assemble(double kr, double ki, const double *kd) {
@@ -497,7 +499,12 @@ void run_sweep(Ctx *const *ctxs, int nmesh, const double *ks, int nk, const doub
         Ctx &c = *ctxs[m];
         c.autotune = true;
         runs.push_back(std::make_unique<MeshRun>(c, nk, ks, w[m], o));
-        for (int j = 0; j < nk; ++j) runs.back()->kmax = std::max(runs.back()->kmax, std::hypot(ks[2 * j], ks[2 * j + 1]));
+        MeshRun &run = *runs.back();
+        for (int j = 0; j < nk; ++j) {
+            const double re = std::fabs(ks[2 * j]);
+            run.kmax = std::max(run.kmax, std::hypot(ks[2 * j], ks[2 * j + 1]));
+            if (re > 0 && (run.kmin == 0 || re < run.kmin)) run.kmin = re;
+        }
         runs.back()->eager(0, ks, ev.e);   // sizes the scratch, tunes the slicing
         runs.back()->size_recorded(ks, cplx);
     }

@@ -43,3 +43,35 @@ def test_matrix_free_product(geometry, k):
     F, G = ((op(mesh, k, n=2, m=2, precision="fp64") @ torch.from_numpy(x).cuda()).cpu().numpy()
             for op in (biegpu.GPUFOperator, biegpu.GPUGOperator))
     check_parts(F, G, want[0] @ x, want[1] @ x, k)
+
+
+@pytest.mark.parametrize("geometry", ["linear", "quadratic"])
+@pytest.mark.parametrize("targets", [0, 40])
+@pytest.mark.parametrize("k", [0.0, 1e-8, 1e-5, 1e-2, 0.3])
+def test_assembly(geometry, targets, k):
+    mesh = bm.icosphere(4, geometry=geometry)
+    t = None
+    if targets:
+        t = np.random.default_rng(3).normal(size=(3, targets))
+        t *= 1.8 / np.linalg.norm(t, axis=0)
+    ctx = biegpu.get_context(mesh, n=2, m=2)
+    F, G, _ = ctx.assemble(k, targets=t)
+    want = oracle.assemble(mesh, k, targets=t, n=2, m=2)
+    if k == 0.0:
+        assert not np.any(F.imag) and not np.any(G.imag)
+        assert rel_fro(F, want[0]) <= 1e-12 and rel_fro(G, want[1]) <= 1e-12
+    else:
+        check_parts(F, G, want[0], want[1], k)
+
+
+def test_sweep_over_both_kernels():
+    """A sweep whose wavenumbers lie on both sides of the line records the FP64 kernel;
+    solutions as with one wavenumber at a time."""
+    mesh = bm.icosphere(5)
+    ks = np.array([1e-3, 0.2, 0.8, 2.0, 3.0])
+    w = np.random.default_rng(4).normal(size=mesh.n_sources) + 0j
+    p, _ = biegpu.sweep([mesh], ks, [w], precision="fp64", n=2, m=2)
+    for j, k in enumerate(ks):
+        q, _ = biegpu.sweep([mesh], ks[j:j + 1], [w], precision="fp64", n=2, m=2)
+        a, b = np.asarray(p[0])[:, j], np.asarray(q[0])[:, 0]
+        assert np.linalg.norm(a - b) <= 1e-7 * np.linalg.norm(b)
