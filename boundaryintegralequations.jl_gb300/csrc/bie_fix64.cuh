@@ -136,7 +136,7 @@ constexpr int kTrigEntries = 1 << kTrigBits;
 constexpr int kCoordBits = 59;                     // fixed coordinates: largest |x| -> 2^59
 constexpr int kMinExp = -7;                        // pairs with rmin < 2^(kMinExp - 1) go to FP64
 constexpr float kRhoFactor = 2.01f;                // regular: |D| >= kRhoFactor rho
-constexpr int kMaxTurnExp = 9;                     // k 2^e / 2 pi < 2^9
+constexpr int kMaxTurnExp = 25;                    // k 2^e / 2 pi < 2^25 (Pair::fsh below 32)
 constexpr int kDampBits = 8;                       // 2^(-j / 256)
 constexpr int kDampEntries = 1 << kDampBits;
 constexpr int kMaxDampExp = 9;                     // |Im k| 2^e log2(e) < 2^9

@@ -68,3 +68,13 @@ def test_sine_of_small_arguments(build, exponent):
     x^6 / 5040 < 2^-60) and the product: 0.52 units."""
     out = build("fix64_sine")(1, exponent)
     assert float(out[0]) <= 1.0 and float(out[1]) <= 0.52
+
+
+@pytest.mark.parametrize("cplx", [0, 1])
+@pytest.mark.parametrize("turns", [-8, 0, 9, 15, 25])
+def test_points_of_many_turns_and_complex_wavenumbers(build, turns, cplx):
+    """As the real points of few turns: 2^-50 for the roundings and 2^-53 of the phase
+    (r to 2^-55, the turn's fraction with 58 + 32 bits), and for complex k 2^-53 of
+    the damping's exponent, relative to the element's near end."""
+    out = build("fix64_complex")(1, turns, cplx)
+    assert out[0] == "1" and float(out[1]) <= 1.0
