@@ -31,7 +31,7 @@ int main(int argc, char **argv) {
     for (int n = 0; n < 200000; ++n) {
         const double x = (U() < 0.5 ? -1 : 1) * std::ldexp(1.0 + U(), e);
         double s, c;
-        if (!sine_cosine(x, trig, s, c)) return 3;
+        if (!sine_cosine<1076>(x, trig, s, c)) return 3;
         // reduced with 2 pi in two parts
         const Q hi = ldexpl((Q)0xc90fdaa22168c235ULL, -61), lo = -1.0033115225336664e-19L;
         const Q turns = rintl((Q)x / hi);

@@ -53,7 +53,7 @@ def test_element_factors_of_any_magnitude(build, seed):
     assert float(out[0]) <= 2.7 and out[1] == "1"
 
 
-@pytest.mark.parametrize("exponent", [-6, -3, 0, 3, 6, 8, 9, 12, 15, 17, 19])
+@pytest.mark.parametrize("exponent", [-6, -3, 0, 3, 6, 8, 9, 12, 15, 17, 19, 24, 31, 40, 48])
 def test_sine_and_cosine_over_their_range(build, exponent):
     """Besides the final rounding 2^-59 for every argument that is taken: the series
     2^-60, the truncated turn 2 pi 2^-64, and below 2^9 1 / 2 pi in one word
