@@ -616,6 +616,10 @@ inline unsigned stream_grid(const Ctx &c, int64_t total) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, 16LL * c.num_sms));
 }
 
+bool on_nodes(const Ctx &c, const AssembleArgs &a) {
+    return a.targets >= c.d_sources && a.targets + 3 * a.M <= c.d_sources + 3 * c.n_sources;
+}
+
 struct FxBuffers {
     double *Cpart, *Cnear;
     int2 *defer;
@@ -689,7 +693,11 @@ void launch_np(Ctx &c, const AssembleArgs &a, const LaunchShape &sh, int spread,
         ++c.kernel_launches;
     }
     auto corr = fx_correct_kernel<NP, CPLX>;
-    corr<<<(unsigned)(4 * c.num_sms), 128, 0, c.stream>>>(
+    // (far from the surface every pair can be here: 30000 points at 10^5 sizes 96 ms
+    // with 4 blocks per SM, 84 with 16, the FP64 kernel alone 95; on the surface a few
+    // per cent of the pairs)
+    const int64_t most = (a.M * E + 127) / 128;
+    corr<<<(unsigned)std::min<int64_t>(most, (on_nodes(c, a) ? 4LL : 16LL) * c.num_sms), 128, 0, c.stream>>>(
         b.defer, b.dcount, b.dcap, v, a.targets, a.M, a.k_re, a.k_im, a.flags, reinterpret_cast<double2 *>(F),
         reinterpret_cast<double2 *>(G), b.Cnear, b.over, c.d_xrecords, X.stride, E, S, sc, c.d_qpe, a.k_dev,
         reinterpret_cast<const double2 *>(a.g_weight));
@@ -934,10 +942,6 @@ static bool fix64_covers(const Ctx &c, const AssembleArgs &a) {
     // (3e-16), 2e-16 (1e-16); k = 0.01 6e-10 (1e-14), 5e-15 (1e-16).
     const double kmin = (a.k_dev ? a.k_re_min : std::fabs(a.k_re)) * len;
     return kmin == 0.0 || kmin >= 1.0;
-}
-
-static bool on_nodes(const Ctx &c, const AssembleArgs &a) {
-    return a.targets >= c.d_sources && a.targets + 3 * a.M <= c.d_sources + 3 * c.n_sources;
 }
 
 // Where the double-float kernel is available (BIE_PREC_DF64), the fixed-point one
