@@ -959,6 +959,37 @@ bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df64) {
     if (!fix64_takes(c, args, df64)) return false;
     AssembleArgs a = args;
     const bool cplx = a.k_im != 0.0;
+    // The finest slicing with at least four elements per slice: blocks differ in
+    // cost (near pairs leave points out, midpoint rules add some), so many small
+    // ones even out.  Step at 128 / 64 / 32 slices: pulsating sphere 20.8 / 21.2 /
+    // 22.0 ms, rigid sphere P2 11.3 / 11.4 / 12.0, 5762 nodes P2 3.20 / 3.30 / 3.55,
+    // 362 nodes with 16-point rules 0.22 / 0.29 / 0.40.
+    int level = 0;
+    while (level + 1 < kMaxLevels && (c.n_elements >> (level + 1)) >= 4) ++level;
+    // Few rows do not fill the SMs with that (a pair takes microseconds, one after
+    // the other on its thread): four waves of blocks, on slices down to single
+    // elements, with every node shared (integer atomics).  8000 elements, 40 / 700 /
+    // 1333 / 2600 rows against the slices above: P2 with 16-point rules 2.00 -> 0.56,
+    // 6.0 -> 4.1, 8.4 -> 7.3, 14.4 -> 13.9 ms, P1 with 4-point rules 0.29 -> 0.13, 0.84
+    // -> 0.71, 1.33 -> 1.26, 2.29 -> 2.36; without shared nodes, whose entries need no
+    // atomics otherwise, 0.29 -> 0.15, 130 rows 0.37 -> 0.32, but 300 rows 0.45 -> 0.54.
+    const int64_t tiles = (a.M + kThreads - 1) / kThreads, resident = 4LL * c.num_sms;
+    // (BIE_PREC_DF64 keeps its tunable slices)
+    const bool few = !df64 && tiles << level <= (c.k2_nfix[level] > 0 ? 3 * resident : resident / 2);
+    const int spread = few ? (int)std::min<int64_t>(c.n_elements, 4 * resident / tiles) : 0;
+    // list of deferred pairs, counter, C of these; and per (slice, row) the C partial
+    // sums and the overflow marks: up to 2 KB a row, where the FP64 kernel needs 8 bytes
+    // a slice.  It takes over where the device has no room for that beside the outputs.
+    const unsigned int dcap = (unsigned int)std::min<int64_t>(a.M * 64 + 4096, (int64_t)1 << 30);
+    const size_t dbytes = (size_t)dcap * sizeof(int2);
+    const size_t part_row = (size_t)(spread ? spread : 1 << level) * (sizeof(double) + sizeof(int));
+    if ((a.flags & (BIE_F | BIE_G)) || on_nodes(c, a)) {
+        if (!c.scratch_fits(kScratchDefer, dbytes + 256 + (size_t)a.M * 8)) return false;
+        if (!c.scratch_fits(kScratchCpart, part_row * a.M)) {
+            c.drop_scratch(kScratchDefer);
+            return false;
+        }
+    }
     // C at points off the surface cancels to the quadrature error, where any other
     // rounding would show: it keeps the FP64 operations
     struct Join {   // the call's stream waits for the side stream, whatever happens in between
@@ -978,8 +1009,7 @@ bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df64) {
     if (!(a.flags & (BIE_F | BIE_G | BIE_C))) return true;
     const RecordLayout &L = c.lay;
     FxBuffers b{};
-    b.dcap = (unsigned int)std::min<int64_t>(a.M * 64 + 4096, (int64_t)1 << 30);
-    const size_t dbytes = (size_t)b.dcap * sizeof(int2);
+    b.dcap = dcap;
     char *dbuf = static_cast<char *>(c.scratch(kScratchDefer, dbytes + 256 + (size_t)a.M * 8));
     b.defer = reinterpret_cast<int2 *>(dbuf);
     b.dcount = reinterpret_cast<u64 *>(dbuf + dbytes);
@@ -987,24 +1017,6 @@ bool launch_assemble_fix64(Ctx &c, const AssembleArgs &args, bool df64) {
     auto reset = [&] { BIE_CUDA(cudaMemsetAsync(dbuf + dbytes, 0, 256 + (size_t)a.M * 8, c.stream)); };
     reset();
 
-    // The finest slicing with at least four elements per slice: blocks differ in
-    // cost (near pairs leave points out, midpoint rules add some), so many small
-    // ones even out.  Step at 128 / 64 / 32 slices: pulsating sphere 20.8 / 21.2 /
-    // 22.0 ms, rigid sphere P2 11.3 / 11.4 / 12.0, 5762 nodes P2 3.20 / 3.30 / 3.55,
-    // 362 nodes with 16-point rules 0.22 / 0.29 / 0.40.
-    int level = 0;
-    while (level + 1 < kMaxLevels && (c.n_elements >> (level + 1)) >= 4) ++level;
-    // Few rows do not fill the SMs with that (a pair takes microseconds, one after
-    // the other on its thread): four waves of blocks, on slices down to single
-    // elements, with every node shared (integer atomics).  8000 elements, 40 / 700 /
-    // 1333 / 2600 rows against the slices above: P2 with 16-point rules 2.00 -> 0.56,
-    // 6.0 -> 4.1, 8.4 -> 7.3, 14.4 -> 13.9 ms, P1 with 4-point rules 0.29 -> 0.13, 0.84
-    // -> 0.71, 1.33 -> 1.26, 2.29 -> 2.36; without shared nodes, whose entries need no
-    // atomics otherwise, 0.29 -> 0.15, 130 rows 0.37 -> 0.32, but 300 rows 0.45 -> 0.54.
-    const int64_t tiles = (a.M + kThreads - 1) / kThreads, resident = 4LL * c.num_sms;
-    // (BIE_PREC_DF64 keeps its tunable slices)
-    const bool few = !df64 && tiles << level <= (c.k2_nfix[level] > 0 ? 3 * resident : resident / 2);
-    const int spread = few ? (int)std::min<int64_t>(c.n_elements, 4 * resident / tiles) : 0;
     auto run = [&](const LaunchShape &sh) {
         const int S = spread ? spread : 1 << sh.level;
         // phase table, point values of the block's threads, basis tables

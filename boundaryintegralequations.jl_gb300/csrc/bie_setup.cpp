@@ -339,13 +339,28 @@ void *Ctx::scratch(int slot, size_t bytes) {
     if (bytes == 0) bytes = 16;
     if (scratch_bytes[slot] < bytes) {
         if (capturing) fail(BIE_ERR_INVALID, "device scratch would grow while a CUDA graph is recorded");
-        if (d_scratch[slot]) BIE_CUDA(cudaFree(d_scratch[slot]));
-        d_scratch[slot] = nullptr;
-        scratch_bytes[slot] = 0;
+        drop_scratch(slot);
         BIE_CUDA(cudaMalloc(&d_scratch[slot], bytes));
         scratch_bytes[slot] = bytes;
     }
     return d_scratch[slot];
+}
+
+void Ctx::drop_scratch(int slot) {
+    if (d_scratch[slot]) BIE_CUDA(cudaFree(d_scratch[slot]));
+    d_scratch[slot] = nullptr;
+    scratch_bytes[slot] = 0;
+}
+
+bool Ctx::scratch_fits(int slot, size_t bytes) {
+    try {
+        scratch(slot, bytes);
+    } catch (const Error &e) {
+        if (e.code != BIE_ERR_NOMEM) throw;
+        cudaGetLastError();   // (a failed allocation stays the last error otherwise)
+        return false;
+    }
+    return true;
 }
 
 cudaEvent_t Ctx::take_event() {
