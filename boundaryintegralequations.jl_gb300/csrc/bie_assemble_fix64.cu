@@ -705,6 +705,170 @@ void launch_np(Ctx &c, const AssembleArgs &a, const LaunchShape &sh, int spread,
     ++c.kernel_launches;
 }
 
+// ---- records ------------------------------------------------------------------
+// Built on the device from the FP64 records: one thread per element (thousands of
+// elements, a few hundred FP64 operations each).  On the host, one thread, this
+// made a context 18 to 44 % more expensive (rigid sphere P2, 5780 elements: 5.9 ms).
+struct FxBuild {
+    double x0[3], inv, area;      // origin, 2^-S, 2^-2S / 4 pi
+    int NP, R, qmax, pe;          // pe: basis values are stored times 2^-pe
+    int stride64, stride;
+    int Q[kMaxRules], off64[kMaxRules], off[kMaxRules];
+};
+struct FxSummary {                // (non-negative doubles and floats compare as integers)
+    unsigned long long reach, reach_all;
+    unsigned int rho, bad;
+};
+
+__device__ __forceinline__ i64 fx_fixed(double h, double l, double scale) {
+    return __double2ll_rn(h * scale) + __double2ll_rn(l * scale);
+}
+__device__ __forceinline__ void fx_put64(int *w, i64 v) {
+    w[0] = fix64::lo32(v);
+    w[1] = fix64::hi32(v);
+}
+__device__ __forceinline__ void fx_put_limbs(int *w, i64 v) {
+    const Limb l = fix64::split(v);
+    w[0] = l.h;
+    w[1] = l.l;
+}
+// a - b = s + err exactly
+__device__ __forceinline__ double fx_diff(double a, double b, double &err) {
+    const double s = __dsub_rn(a, b), bb = __dsub_rn(s, a);
+    err = __dadd_rn(__dsub_rn(a, __dsub_rn(s, bb)), __dsub_rn(-b, bb));
+    return s;
+}
+
+// corners: the three corner vertices of every element.  nodes: largest weight
+// exponent per node; reach: max over rules of sum |jw| |phi| in 2^(ej + pe).
+__global__ void __launch_bounds__(64)
+fx_build_kernel(const double *__restrict__ rec64, const double *__restrict__ corners, const double *__restrict__ phi,
+                int64_t E, const __grid_constant__ FxBuild b, int *__restrict__ rec, int *__restrict__ nodes,
+                double *__restrict__ reach, FxSummary *__restrict__ sum, const int32_t *__restrict__ nidx, int nidx_off) {
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= E) return;
+    const int NP = b.NP;
+    const double *R0 = rec64 + p * b.stride64, *V = corners + 9 * p;
+    int *w = rec + p * b.stride;
+    float *wf = reinterpret_cast<float *>(w);
+    double cen[3], hmax = 0.0;
+    for (int k = 0; k < 3; ++k) {
+        cen[k] = __dadd_rn(__dadd_rn(__ddiv_rn(V[k], 3.0), __ddiv_rn(V[3 + k], 3.0)), __ddiv_rn(V[6 + k], 3.0));
+        double err;
+        const double s = fx_diff(cen[k], b.x0[k], err);
+        fx_put64(w + kHdrCen + 2 * k, fx_fixed(s * b.inv, err * b.inv, 0x1p59));
+    }
+    for (int a = 0; a < 3; ++a) {
+        const double *A = V + 3 * a, *B = V + 3 * ((a + 1) % 3);
+        double d2 = 0.0;
+        for (int k = 0; k < 3; ++k) {
+            const double d = (A[k] - B[k]) * b.inv;
+            d2 += d * d;
+        }
+        hmax = fmax(hmax, d2);
+    }
+    wf[kHdrNear2] = (float)hmax;
+    double rho2 = 0.0, omax = 0.0, jmax = 0.0, jsum = 0.0;
+    for (int a = 0; a < NP; ++a) {
+        double d2 = 0.0;
+        for (int k = 0; k < 3; ++k) {
+            const double x = R0[3 * a + k], d = (x - cen[k]) * b.inv;
+            d2 += d * d;
+            wf[kHdrNodes + 3 * a + k] = (float)d;
+            wf[kHdrNodes + 3 * NP + 3 * a + k] = (float)((x - b.x0[k]) * b.inv);
+        }
+        rho2 = fmax(rho2, d2);
+    }
+    for (int r = 0; r < b.R; ++r) {
+        const int Q = b.Q[r];
+        const double *g = R0 + b.off64[r];
+        double js = 0.0;
+        for (int q = 0; q < Q; ++q) {
+            double d2 = 0.0;
+            for (int k = 0; k < 3; ++k) {
+                const double d = (g[k * Q + q] - cen[k]) * b.inv;
+                d2 += d * d;
+                omax = fmax(omax, fabs(d));
+            }
+            rho2 = fmax(rho2, d2);
+            const double j = fabs(g[6 * Q + q]) * b.area;
+            jmax = fmax(jmax, j);
+            js += j;
+        }
+        jsum = fmax(jsum, js);
+    }
+    const float rho = (float)(sqrt(rho2) * (1.0 + 1e-6));
+    wf[kHdrRho] = rho;
+    atomicMax(&sum->rho, __float_as_uint(rho));
+    int eo = 0, je = 0;
+    (void)frexp(omax > 0 ? omax * (1.0 + 1e-9) : 0x1p-60, &eo);
+    (void)frexp(jmax > 0 ? jmax * 1.01 : 0x1p-200, &je);
+    while (ldexp(jsum, -je) > 8.0) ++je;   // sums over a rule: |sum t| < 8 * 4 2^57
+    if (je < -900) {
+        sum->bad = 1;
+        return;
+    }
+    w[kHdrEj] = je;
+    w[kHdrEo] = eo;
+    const double so = ldexp(1.0, 62 - eo), sj = ldexp(b.area, 63 - je);
+    for (int r = 0; r < b.R; ++r) {
+        const int Q = b.Q[r];
+        const double *g = R0 + b.off64[r];
+        for (int q = 0; q < Q; ++q) {
+            int *P = w + b.off[r] + kPointWords * q;
+            for (int k = 0; k < 3; ++k) {
+                double err;
+                const double s = fx_diff(g[k * Q + q], cen[k], err);
+                fx_put64(P + 2 * k, fx_fixed(s * b.inv, err * b.inv, so));
+                fx_put_limbs(P + 6 + 2 * k, __double2ll_rn(g[(3 + k) * Q + q] * 0x1p61));
+            }
+            fx_put_limbs(P + 12, __double2ll_rn(g[6 * Q + q] * sj));
+        }
+    }
+    const int32_t *nid = nidx + 2 * (p * b.stride64 + nidx_off);
+    for (int a = 0; a < NP; ++a) {
+        double best = 0.0;
+        for (int r = 0; r < b.R; ++r) {
+            double s = 0.0;
+            for (int q = 0; q < b.Q[r]; ++q)
+                s += fabs(R0[b.off64[r] + 6 * b.Q[r] + q] * phi[((int64_t)r * b.qmax + q) * NP + a]);
+            best = fmax(best, s);
+        }
+        reach[p * NP + a] = ldexp(best * b.area, -je - b.pe);
+        w[kHdrNodes + 7 * NP + a] = nid[a];
+        atomicMax(nodes + nid[a], je);
+    }
+}
+
+// The node's weight exponent into every record, and the sums of the reaches per
+// node: in units of that exponent, and each in its own (element factors may make
+// any contribution the node's largest).
+__global__ void fx_build_nodes_kernel(int64_t E, const __grid_constant__ FxBuild b, int *__restrict__ rec,
+                                      const int *__restrict__ nodes, const double *__restrict__ reach,
+                                      double *__restrict__ sums, int64_t N) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= E * b.NP) return;
+    const int64_t p = t / b.NP;
+    const int a = (int)(t - p * b.NP);
+    int *w = rec + p * b.stride;
+    const int nd = w[kHdrNodes + 7 * b.NP + a], je = nodes[nd];
+    w[kHdrNodes + 6 * b.NP + a] = je;
+    atomicAdd(sums + nd, ldexp(reach[t], w[kHdrEj] - je));
+    atomicAdd(sums + N + nd, reach[t]);
+}
+
+__global__ void fx_build_finish_kernel(int64_t N, const __grid_constant__ FxBuild b, const double *__restrict__ src,
+                                       const int *__restrict__ nodes, const double *__restrict__ sums,
+                                       float4 *__restrict__ xnodes, FxSummary *__restrict__ sum) {
+    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= N) return;
+    const int je = nodes[j];
+    xnodes[j] = make_float4((float)((src[3 * j] - b.x0[0]) * b.inv), (float)((src[3 * j + 1] - b.x0[1]) * b.inv),
+                            (float)((src[3 * j + 2] - b.x0[2]) * b.inv), __int_as_float(je == INT_MIN ? 0 : je));
+    atomicMax(&sum->reach, (unsigned long long)__double_as_longlong(sums[j]));
+    atomicMax(&sum->reach_all, (unsigned long long)__double_as_longlong(sums[N + j]));
+}
+
 }  // namespace
 
 // e^{2 pi i j / 1024} and 2^(-j / 256) as Q62 limbs (constants: built once; the
@@ -730,8 +894,8 @@ static const std::vector<int32_t> &unit_tables() {
     return table;
 }
 
-// Records of the fixed-point kernels from the FP64 ones (E x lay.stride).
-void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
+// Records of the fixed-point kernels from the FP64 ones (c.d_records).
+void build_fix64_records(Ctx &c) {
     const RecordLayout &L = c.lay;
     Fix64Layout &X = c.xlay;
     X = Fix64Layout{};
@@ -764,8 +928,6 @@ void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
     if (!(top > 0x1p-300 && top < 0x1p300)) return;   // such meshes stay with the FP64 kernel
     (void)std::frexp(top, &c.fx_exp);
     const double inv = std::ldexp(1.0, -c.fx_exp);
-    // integer nearest to (hi + lo) 2^n
-    auto fixed = [](double h, double l, double scale) { return (long long)std::llrint(h * scale) + (long long)std::llrint(l * scale); };
     auto put_limbs = [](int32_t *w, long long v) {
         const fix64::Limb s = fix64::split(v);
         w[0] = s.h;
@@ -793,134 +955,81 @@ void build_fix64_records(Ctx &c, const std::vector<double> &rec64) {
                 put_limbs(&phi[((((size_t)r * ng + q / kGroup) * NP + a) * kGroup + q % kGroup) * 2],
                           (long long)std::llrint(std::ldexp(c.phi[((size_t)r * L.qmax + q) * NP + a], 61 - c.fx_phi_exp)));
 
-    std::vector<int32_t> rec((size_t)E * X.stride, 0);
-    std::vector<int> ej(E);
-    std::vector<int> node_ej(N, INT32_MIN);
-    std::vector<double> reach((size_t)E * NP);   // max over rules of sum |jw| |phi| in 2^(ej + pe)
-    for (int64_t p = 0; p < E; ++p) {
-        const int64_t e = c.order[p];
-        const double *R0 = &rec64[(size_t)p * L.stride];
-        int32_t *w = &rec[(size_t)p * X.stride];
-        float *wf = reinterpret_cast<float *>(w);
-        double cen[3] = {0, 0, 0}, hmax = 0;
-        for (int a = 0; a < 3; ++a)
-            for (int k = 0; k < 3; ++k) cen[k] += c.coords[3 * (int64_t)c.topo[c.NS * e + a] + k] / 3.0;
-        for (int a = 0; a < 3; ++a) {
-            const double *A = &c.coords[3 * (int64_t)c.topo[c.NS * e + a]];
-            const double *B = &c.coords[3 * (int64_t)c.topo[c.NS * e + (a + 1) % 3]];
-            const double d[3] = {(A[0] - B[0]) * inv, (A[1] - B[1]) * inv, (A[2] - B[2]) * inv};
-            hmax = std::max(hmax, std::sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]));
-        }
-        long long fc[3];
-        for (int k = 0; k < 3; ++k) {
-            const double s = cen[k] - c.fx_origin[k], bb = s - cen[k];
-            const double err = (cen[k] - (s - bb)) + (-c.fx_origin[k] - bb);   // two-sum
-            fc[k] = fixed(s * inv, err * inv, 0x1p59);
-            std::memcpy(w + kHdrCen + 2 * k, &fc[k], 8);
-        }
-        wf[kHdrNear2] = (float)(hmax * hmax);
-        double rho2 = 0.0, jmax = 0.0, omax = 0.0, jsum = 0.0;
-        for (int a = 0; a < NP; ++a) {
-            double d2 = 0.0;
-            for (int k = 0; k < 3; ++k) {
-                const double x = R0[3 * a + k], d = (x - cen[k]) * inv;
-                d2 += d * d;
-                wf[kHdrNodes + 3 * a + k] = (float)d;
-                wf[kHdrNodes + 3 * NP + 3 * a + k] = (float)((x - c.fx_origin[k]) * inv);
-            }
-            rho2 = std::max(rho2, d2);
-        }
-        for (int r = 0; r < L.R; ++r) {
-            const int Q = L.Q[r];
-            const double *g = R0 + L.rule_off[r];
-            double js = 0.0;
-            for (int q = 0; q < Q; ++q) {
-                double d2 = 0.0;
-                for (int k = 0; k < 3; ++k) {
-                    const double d = (g[k * Q + q] - cen[k]) * inv;
-                    d2 += d * d;
-                    omax = std::max(omax, std::fabs(d));
-                }
-                rho2 = std::max(rho2, d2);
-                const double j = std::fabs(g[6 * Q + q]) * (inv * inv) * dev::kInv4Pi;
-                jmax = std::max(jmax, j);
-                js += j;
-            }
-            jsum = std::max(jsum, js);
-        }
-        wf[kHdrRho] = (float)(std::sqrt(rho2) * (1.0 + 1e-6));
-        c.fx_rho_max = std::max(c.fx_rho_max, wf[kHdrRho]);
-        int eo = 0, je = 0;
-        (void)std::frexp(omax > 0 ? omax * (1.0 + 1e-9) : 0x1p-60, &eo);
-        (void)std::frexp(jmax > 0 ? jmax * 1.01 : 0x1p-200, &je);
-        while (std::ldexp(jsum, -je) > 8.0) ++je;   // sums over a rule: |sum t| < 8 * 4 2^57
-        if (je < -900) return;
-        ej[p] = je;
-        w[kHdrEj] = je;
-        w[kHdrEo] = eo;
-        const double so = std::ldexp(1.0, 62 - eo), sj = std::ldexp(inv * inv * dev::kInv4Pi, 63 - je);
-        for (int r = 0; r < L.R; ++r) {
-            const int Q = L.Q[r];
-            const double *g = R0 + L.rule_off[r];
-            for (int q = 0; q < Q; ++q) {
-                int32_t *P = w + X.rule_off[r] + kPointWords * q;
-                for (int k = 0; k < 3; ++k) {
-                    const double x = g[k * Q + q], s = x - cen[k], bb = s - x;
-                    const double err = (x - (s - bb)) + (-cen[k] - bb);
-                    const long long o = fixed(s * inv, err * inv, so);
-                    std::memcpy(P + 2 * k, &o, 8);
-                    put_limbs(P + 6 + 2 * k, (long long)std::llrint(g[(3 + k) * Q + q] * 0x1p61));
-                }
-                put_limbs(P + 12, (long long)std::llrint(g[6 * Q + q] * sj));
-            }
-        }
-        for (int a = 0; a < NP; ++a) {
-            const int32_t nd = c.ptopo[NP * e + a];
-            w[kHdrNodes + 7 * NP + a] = nd;
-            node_ej[nd] = std::max(node_ej[nd], je);
-            double best = 0.0;
-            for (int r = 0; r < L.R; ++r) {
-                double s = 0.0;
-                for (int q = 0; q < L.Q[r]; ++q)
-                    s += std::fabs(R0[L.rule_off[r] + 6 * L.Q[r] + q] * c.phi[((size_t)r * L.qmax + q) * NP + a]);
-                best = std::max(best, s);
-            }
-            reach[(size_t)p * NP + a] = std::ldexp(best * inv * inv * dev::kInv4Pi, -je - c.fx_phi_exp);
-        }
+    FxBuild b{};
+    for (int k = 0; k < 3; ++k) b.x0[k] = c.fx_origin[k];
+    b.inv = inv;
+    b.area = inv * inv * dev::kInv4Pi;
+    b.NP = NP;
+    b.R = L.R;
+    b.qmax = L.qmax;
+    b.pe = c.fx_phi_exp;
+    b.stride64 = L.stride;
+    b.stride = X.stride;
+    for (int r = 0; r < L.R; ++r) {
+        b.Q[r] = L.Q[r];
+        b.off64[r] = L.rule_off[r];
+        b.off[r] = X.rule_off[r];
     }
-    // entries hold |sum| <= 4 sqrt(2) 2^55 sum of the reaches: below 2^62
-    // (with element factors each contribution may be the node's largest, and a
-    // factor's modulus is up to sqrt(2) of its unit: G is below half of F's bound)
-    std::vector<double> node_reach(N, 0.0), node_all(N, 0.0);
+    std::vector<double> corners((size_t)9 * E);
     for (int64_t p = 0; p < E; ++p)
-        for (int a = 0; a < NP; ++a) {
-            const int32_t nd = c.ptopo[NP * c.order[p] + a];
-            rec[(size_t)p * X.stride + kHdrNodes + 6 * NP + a] = node_ej[nd];
-            node_reach[nd] += std::ldexp(reach[(size_t)p * NP + a], ej[p] - node_ej[nd]);
-            node_all[nd] += reach[(size_t)p * NP + a];
-        }
-    auto extra_of = [](const std::vector<double> &reach) {
-        double worst = 0.0;
-        for (double v : reach) worst = std::max(worst, v);
+        for (int a = 0; a < 3; ++a)
+            for (int k = 0; k < 3; ++k)
+                corners[9 * p + 3 * a + k] = c.coords[3 * (int64_t)c.topo[c.NS * c.order[p] + a] + k];
+    // temporary: corners, reaches, sums per node, summary, exponents per node
+    struct Temp {
+        char *p = nullptr;
+        ~Temp() { cudaFree(p); }
+    } tmp;
+    const size_t nc = corners.size() * 8, nr = (size_t)E * NP * 8, ns = (size_t)2 * N * 8;
+    FxSummary sum{};
+    try {
+        BIE_CUDA(cudaMalloc(&tmp.p, nc + nr + ns + sizeof(FxSummary) + (size_t)N * 4));
+        BIE_CUDA(cudaMalloc(&c.d_xrecords, (size_t)E * X.stride * 4));
+        BIE_CUDA(cudaMalloc(&c.d_xphi, phi.size() * 4));
+        BIE_CUDA(cudaMalloc(&c.d_xnodes, (size_t)N * 16));
+    } catch (const Error &e) {   // no room: the other kernels do without
+        if (e.code != BIE_ERR_NOMEM) throw;
+        cudaGetLastError();
+        cudaFree(c.d_xrecords);
+        cudaFree(c.d_xphi);
+        c.d_xrecords = nullptr;
+        c.d_xphi = nullptr;
+        return;
+    }
+    double *d_corners = reinterpret_cast<double *>(tmp.p), *d_reach = d_corners + 9 * E, *d_sums = d_reach + E * NP;
+    FxSummary *d_sum = reinterpret_cast<FxSummary *>(d_sums + 2 * N);
+    int *d_nodes = reinterpret_cast<int *>(d_sum + 1);
+    // (all on the default stream: in order with the uploads of the FP64 records)
+    BIE_CUDA(cudaMemcpy(d_corners, corners.data(), nc, cudaMemcpyHostToDevice));
+    BIE_CUDA(cudaMemcpy(c.d_xphi, phi.data(), phi.size() * 4, cudaMemcpyHostToDevice));
+    BIE_CUDA(cudaMemsetAsync(d_sums, 0, ns + sizeof(FxSummary), 0));
+    BIE_CUDA(cudaMemsetAsync(c.d_xrecords, 0, (size_t)E * X.stride * 4, 0));
+    const std::vector<int> none((size_t)N, INT_MIN);
+    BIE_CUDA(cudaMemcpy(d_nodes, none.data(), (size_t)N * 4, cudaMemcpyHostToDevice));
+    int *rec = reinterpret_cast<int *>(c.d_xrecords);
+    fx_build_kernel<<<(unsigned)((E + 63) / 64), 64>>>(c.d_records, d_corners, c.d_phi, E, b, rec, d_nodes, d_reach,
+                                                       d_sum, reinterpret_cast<const int32_t *>(c.d_records),
+                                                       L.nidx_off);
+    BIE_CUDA(cudaGetLastError());
+    fx_build_nodes_kernel<<<(unsigned)((E * NP + 255) / 256), 256>>>(E, b, rec, d_nodes, d_reach, d_sums, N);
+    BIE_CUDA(cudaGetLastError());
+    fx_build_finish_kernel<<<(unsigned)((N + 255) / 256), 256>>>(N, b, c.d_sources, d_nodes, d_sums,
+                                                                 reinterpret_cast<float4 *>(c.d_xnodes), d_sum);
+    BIE_CUDA(cudaGetLastError());
+    BIE_CUDA(cudaMemcpy(&sum, d_sum, sizeof(sum), cudaMemcpyDeviceToHost));
+    if (sum.bad) return;
+    std::memcpy(&c.fx_rho_max, &sum.rho, 4);
+    // entries hold |sum| <= 4 sqrt(2) 2^55 sum of the reaches: below 2^62 (a factor's
+    // modulus is up to sqrt(2) of its unit: G with factors is below half of F's bound)
+    auto extra_of = [](unsigned long long bits) {
+        double worst;
+        std::memcpy(&worst, &bits, 8);
         int x = 0;
         while (std::ldexp(worst * 5.7, -x) > 127.0) ++x;
         return x;
     };
-    c.fx_extra = extra_of(node_reach);
-    c.fx_extra_w = extra_of(node_all);
-
-    std::vector<float> nodes((size_t)4 * N);
-    for (int64_t j = 0; j < N; ++j) {
-        for (int k = 0; k < 3; ++k) nodes[4 * j + k] = (float)((c.sources[3 * j + k] - c.fx_origin[k]) * inv);
-        const int32_t v = node_ej[j] == INT32_MIN ? 0 : node_ej[j];
-        std::memcpy(&nodes[4 * j + 3], &v, 4);
-    }
-    BIE_CUDA(cudaMalloc(&c.d_xrecords, rec.size() * 4));
-    BIE_CUDA(cudaMalloc(&c.d_xphi, phi.size() * 4));
-    BIE_CUDA(cudaMalloc(&c.d_xnodes, nodes.size() * 4));
-    BIE_CUDA(cudaMemcpy(c.d_xrecords, rec.data(), rec.size() * 4, cudaMemcpyHostToDevice));
-    BIE_CUDA(cudaMemcpy(c.d_xphi, phi.data(), phi.size() * 4, cudaMemcpyHostToDevice));
-    BIE_CUDA(cudaMemcpy(c.d_xnodes, nodes.data(), nodes.size() * 4, cudaMemcpyHostToDevice));
+    c.fx_extra = extra_of(sum.reach);
+    c.fx_extra_w = extra_of(sum.reach_all);
     c.fx_ok = true;
 }
 

@@ -604,7 +604,7 @@ bool launch_assemble_df64(Ctx &c, const AssembleArgs &a);
 // arguments need another kernel (k-derivatives, element factors, phases or
 // damping beyond the fixed-point ranges, coordinates outside
 // 2^+-300).  df64: BIE_PREC_DF64, of which it takes the calls where it is the faster.
-void build_fix64_records(Ctx &c, const std::vector<double> &rec64);
+void build_fix64_records(Ctx &c);
 bool launch_assemble_fix64(Ctx &c, const AssembleArgs &a, bool df64);
 bool fix64_takes(const Ctx &c, const AssembleArgs &a, bool df64);   // whether it launches
 

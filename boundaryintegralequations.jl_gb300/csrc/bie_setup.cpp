@@ -861,7 +861,7 @@ void build_context(Ctx &c, const bie_mesh_desc &d, int device, int gauss_rule,
     if (!k2_fix.empty())
         BIE_CUDA(cudaMemcpy(c.d_k2_fix, k2_fix.data(), k2_fix.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     build_mixed_records(c, rec);
-    build_fix64_records(c, rec);
+    build_fix64_records(c);
     prepare_noalloc(c);
 }
 
