@@ -294,8 +294,11 @@ struct MeshRun {
     void size_recorded(const double *ks, bool cplx) {
         const double ki = cplx ? 1.0 : 0.0;
         if (!mixed && fix64_takes(c, assemble_args(ks[0], ks[1], nullptr), df64) !=
-                          fix64_takes(c, assemble_args(0.0, ki, ks_d), df64))
+                          fix64_takes(c, assemble_args(0.0, ki, ks_d), df64)) {
             assemble(0.0, ki, ks_d);
+            // (the recorded sweep starts on a stream of its own and writes the same matrices)
+            BIE_CUDA(cudaStreamSynchronize(c.stream));
+        }
     }
     // amp[j] from y and A z
     void finish_probe(const int *jdev, int jhost) {

@@ -120,3 +120,20 @@ def test_sweep_graph_small_restart_and_maxiter():
     assert ig["converged"] == ie["converged"] == 3
     for j in range(len(ks)):
         assert rel(pg[0][:, j], pe[0][:, j]) <= 1e-6
+
+
+@pytest.mark.parametrize("f", [5, 16])
+def test_recorded_route_other_than_the_first(f):
+    """The recording's bounds (largest |k| for Re k and Im k) send it to another kernel
+    than the first wavenumber's, which runs once beforehand to size its scratch; the
+    recorded sweep waits for that run, whose matrices it writes again."""
+    mesh = bm.icosphere(f)
+    # |k| 2^S beyond 100 bounds Im k out of the fixed-point range; the wavenumbers
+    # themselves are inside it
+    ks = np.array([3.0 + 0.01j, 55.0 + 0.01j, 2.0 + 0.01j])
+    w = np.random.default_rng(1).normal(size=mesh.n_sources) + 0j
+    p, _ = biegpu.sweep([mesh], ks, [w], precision="fp64", n=2, m=2)
+    for j, k in enumerate(ks):
+        q, _ = biegpu.sweep([mesh], [k], [w], precision="fp64", n=2, m=2)
+        a, b = np.asarray(p[0])[:, j], np.asarray(q[0])[:, 0]
+        assert np.linalg.norm(a - b) <= 1e-6 * np.linalg.norm(b)
