@@ -1033,6 +1033,15 @@ void build_fix64_records(Ctx &c) {
     c.fx_ok = true;
 }
 
+// Small phases stay in floating point: values here are good to 2^-55 of the modulus,
+// but with k r small the imaginary parts, k and k^3 times the real ones, are
+// results of their own.  Error of Im F and Im G on the unit sphere (2^S = 2), with
+// the FP64 kernel in brackets: k = 1 8e-16 (2e-16), 1e-16 (1e-16); k = 0.3 2e-14
+// (3e-16), 2e-16 (1e-16); k = 0.01 6e-10 (1e-14), 5e-15 (1e-16).
+bool fix64_small_phase(const Ctx &c, double k_re) {
+    return k_re != 0.0 && std::fabs(k_re) * std::ldexp(1.0, c.fx_exp) < 1.0;
+}
+
 static bool fix64_covers(const Ctx &c, const AssembleArgs &a) {
     if (!c.fx_ok || a.taylor_m >= 0 || (a.g_weight && !a.g_weight_bounded)) return false;
     if (a.k_dev && !(a.k_abs_max > 0)) return false;   // no bound on |k|
@@ -1044,13 +1053,7 @@ static bool fix64_covers(const Ctx &c, const AssembleArgs &a) {
     const double bound = a.k_dev ? a.k_abs_max : 0.0, len = std::ldexp(1.0, c.fx_exp);
     const double kr = std::max(std::fabs(a.k_re), bound) * len, ki = cplx ? std::max(std::fabs(a.k_im), bound) * len : 0.0;
     if (!(kr < 500.0 && ki < 100.0 && ki * c.fx_rho_max * 1.45 < fix64::kMaxDampSpread)) return false;
-    // Small phases stay in floating point: values here are good to 2^-55 of the modulus,
-    // but with k r small the imaginary parts, k and k^3 times the real ones, are
-    // results of their own.  Error of Im F and Im G on the unit sphere (2^S = 2), with
-    // the FP64 kernel in brackets: k = 1 8e-16 (2e-16), 1e-16 (1e-16); k = 0.3 2e-14
-    // (3e-16), 2e-16 (1e-16); k = 0.01 6e-10 (1e-14), 5e-15 (1e-16).
-    const double kmin = (a.k_dev ? a.k_re_min : std::fabs(a.k_re)) * len;
-    return kmin == 0.0 || kmin >= 1.0;
+    return !fix64_small_phase(c, a.k_dev ? a.k_re_min : a.k_re);
 }
 
 // Where the double-float kernel is available (BIE_PREC_DF64), the fixed-point one

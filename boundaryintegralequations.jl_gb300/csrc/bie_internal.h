@@ -607,6 +607,7 @@ bool launch_assemble_df64(Ctx &c, const AssembleArgs &a);
 void build_fix64_records(Ctx &c);
 bool launch_assemble_fix64(Ctx &c, const AssembleArgs &a, bool df64);
 bool fix64_takes(const Ctx &c, const AssembleArgs &a, bool df64);   // whether it launches
+bool fix64_small_phase(const Ctx &c, double k_re);   // too small a wavenumber for it
 
 // FMA throughput probe (bie_peaks.cu)
 void measure_peaks(int device, bie_peaks &out);

@@ -166,7 +166,8 @@ struct MeshRun {
     bool mixed;
     bool df64;        // FP64-grade assembly in double-float arithmetic
     double kmax = 0;  // largest |k| of the sweep (the double-float phase tables' bound)
-    double kmin = 0;  // smallest |Re k| other than 0
+    double kmin = 0;  // smallest |Re k| other than 0 of the recorded wavenumbers
+    int first = 1;    // the recorded wavenumbers are first .. nk-1
     DevBuf F, G, vec, P, dinfo, kb, ctl, tsb;
     double2 *Cv, *dg, *b, *wd, *X;
     double2 *pz = nullptr, *py = nullptr, *pw = nullptr;   // sensitivity probe: z, y ~ A^-1 z, A z
@@ -307,11 +308,37 @@ struct MeshRun {
         BIE_CUDA(cudaGetLastError());
         ++c.kernel_launches;
     }
-    // record wavenumbers 1 .. nk-1 as a WHILE node appended on `top`; the loop
+    // The recording takes one assembly kernel for its wavenumbers.  Where some of them
+    // are too small for the fixed-point one, everything up to the last of these goes
+    // launch by launch, so that the others keep it (FP64, 2562 nodes, one of six
+    // wavenumbers too small: 54 ms with the FP64 kernel throughout, 21 ms so).
+    void choose_first(const double *ks, bool cplx) {
+        int last = 0, small = 0;
+        for (int j = 0; j < nk; ++j) {
+            kmax = std::max(kmax, std::hypot(ks[2 * j], ks[2 * j + 1]));
+            if (j > 0 && fix64_small_phase(c, ks[2 * j])) {
+                last = j;
+                ++small;
+            }
+        }
+        auto begin_at = [&](int j0) {
+            first = j0;
+            kmin = 0;
+            for (int j = j0; j < nk; ++j) {
+                const double re = std::fabs(ks[2 * j]);
+                if (re > 0 && (kmin == 0 || re < kmin)) kmin = re;
+            }
+        };
+        begin_at(1);
+        if (mixed || small == 0 || small == nk - 1) return;
+        begin_at(last + 1);
+        if (!fix64_takes(c, assemble_args(0.0, cplx ? 1.0 : 0.0, ks_d), df64)) begin_at(1);
+    }
+    // record wavenumbers first .. nk-1 as a WHILE node appended on `top`; the loop
     // body is captured on the context stream, the GMRES bodies on body[0..3]
     void record(cudaStream_t top, const cudaStream_t *body, bool cplx) {
         const cudaGraphConditionalHandle h = graph_new_handle(top);
-        sweep_begin_kernel<<<1, 1, 0, top>>>(jd, 1, nk, h);
+        sweep_begin_kernel<<<1, 1, 0, top>>>(jd, first, nk, h);
         BIE_CUDA(cudaGetLastError());
         cudaGraph_t loop_body;
         graph_add_conditional(top, h, cudaGraphCondTypeWhile, 1, &loop_body);
@@ -341,11 +368,12 @@ struct MeshRun {
     // statistics and timestamps of the recorded wavenumbers (after the launch)
     void collect() {
         std::vector<unsigned long long> hts((size_t)3 * nk);
-        BIE_CUDA(cudaMemcpyAsync(hinfo.data() + 1, dgi + 1, (size_t)(nk - 1) * sizeof(bie_gmres_info),
+        if (first >= nk) return;
+        BIE_CUDA(cudaMemcpyAsync(hinfo.data() + first, dgi + first, (size_t)(nk - first) * sizeof(bie_gmres_info),
                                  cudaMemcpyDeviceToHost, c.stream));
         BIE_CUDA(cudaMemcpyAsync(hts.data(), ts, hts.size() * 8, cudaMemcpyDeviceToHost, c.stream));
         BIE_CUDA(cudaStreamSynchronize(c.stream));
-        for (int j = 1; j < nk; ++j) {
+        for (int j = first; j < nk; ++j) {
             asm_ms += 1e-6 * (double)(hts[3 * j + 1] - hts[3 * j]);
             sol_ms += 1e-6 * (double)(hts[3 * j + 2] - hts[3 * j + 1]);
         }
@@ -503,18 +531,15 @@ void run_sweep(Ctx *const *ctxs, int nmesh, const double *ks, int nk, const doub
         c.autotune = true;
         runs.push_back(std::make_unique<MeshRun>(c, nk, ks, w[m], o));
         MeshRun &run = *runs.back();
-        for (int j = 0; j < nk; ++j) {
-            const double re = std::fabs(ks[2 * j]);
-            run.kmax = std::max(run.kmax, std::hypot(ks[2 * j], ks[2 * j + 1]));
-            if (re > 0 && (run.kmin == 0 || re < run.kmin)) run.kmin = re;
-        }
-        runs.back()->eager(0, ks, ev.e);   // sizes the scratch, tunes the slicing
-        runs.back()->size_recorded(ks, cplx);
+        run.choose_first(ks, cplx);
+        for (int j = 0; j < run.first; ++j) run.eager(j, ks, ev.e);   // sizes the scratch, tunes the slicing
+        run.size_recorded(ks, cplx);
     }
     GraphScope gs(uniq);
     const auto t0 = std::chrono::steady_clock::now();
     gs.begin();
-    for (auto &r : runs) r->record(gs.top, gs.body, cplx);
+    for (auto &r : runs)
+        if (r->first < nk) r->record(gs.top, gs.body, cplx);
     gs.end();
     BIE_CUDA(cudaGraphInstantiate(&gs.exec, gs.graph, 0));
     info.record_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();

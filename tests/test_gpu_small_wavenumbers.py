@@ -4,6 +4,8 @@ a result of its own (it carries the radiated power).  FP64 calls keep each part 
 FP64, not only the modulus."""
 from __future__ import annotations
 
+import dataclasses
+
 import numpy as np
 import pytest
 import torch
@@ -75,3 +77,21 @@ def test_sweep_over_both_kernels():
         q, _ = biegpu.sweep([mesh], ks[j:j + 1], [w], precision="fp64", n=2, m=2)
         a, b = np.asarray(p[0])[:, j], np.asarray(q[0])[:, 0]
         assert np.linalg.norm(a - b) <= 1e-7 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("order", [[0, 1, 2, 3, 4, 5], [5, 4, 3, 2, 1, 0], [3, 0, 4, 1, 5, 2]])
+@pytest.mark.parametrize("precision", ["fp64", "df64"])
+def test_sweep_in_any_order(order, precision):
+    """Wavenumbers on both sides of the line, in three orders, on two meshes of which
+    the smaller one puts the line elsewhere."""
+    small = bm.icosphere(4)
+    meshes = [bm.icosphere(5), dataclasses.replace(small, sources=0.2 * small.sources, coordinates=0.2 * small.coordinates)]
+    ks = np.array([0.1, 0.3, 0.6, 1.5, 2.5, 3.5])
+    rng = np.random.default_rng(4)
+    w = [rng.normal(size=m.n_sources) + 0j for m in meshes]
+    p, _ = biegpu.sweep(meshes, ks[order], w, precision=precision, n=2, m=2)
+    for i, mesh in enumerate(meshes):
+        for j, k in enumerate(ks[order]):
+            q, _ = biegpu.sweep([mesh], [k], [w[i]], precision=precision, n=2, m=2)
+            a, b = np.asarray(p[i])[:, j], np.asarray(q[0])[:, 0]
+            assert np.linalg.norm(a - b) <= 1e-7 * np.linalg.norm(b)
