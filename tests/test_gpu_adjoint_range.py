@@ -91,3 +91,16 @@ def test_double_float_gradient_at_the_ends_of_its_range(scale, radius):
     for i in (2, 3):
         size = np.max(np.abs(a[i]))
         assert np.linalg.norm((b[i] - a[i]) / size) <= 1e-12 * np.linalg.norm(a[i] / size)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "df64"])
+def test_few_and_many_field_points(precision):
+    """Few field points take slices down to single elements with every node shared,
+    many the flagged slices; with admittances over six decades both sum the same
+    integers, so the pressures agree to the FP64 additions (1e-13 of the largest)."""
+    mesh, Z, X = setup(9, nfield=2000)
+    Z = Z * 10.0 ** np.random.default_rng(8).uniform(-3, 3, mesh.n_elements)
+    many = biegpu.farfield_objective(mesh, 3.0, Z, X, rho_c=RHO_C, precision=precision, gradient=False)[1]
+    for M in (1, 8, 200):
+        few = biegpu.farfield_objective(mesh, 3.0, Z, X[:, :M], rho_c=RHO_C, precision=precision, gradient=False)[1]
+        assert np.max(np.abs(few - many[:M])) <= 1e-13 * np.max(np.abs(many))
