@@ -717,7 +717,7 @@ struct FxBuild {
 };
 struct FxSummary {                // (non-negative doubles and floats compare as integers)
     unsigned long long reach, reach_all;
-    unsigned int rho, bad;
+    unsigned int rho, bad, small, unused;
 };
 
 __device__ __forceinline__ i64 fx_fixed(double h, double l, double scale) {
@@ -800,6 +800,8 @@ fx_build_kernel(const double *__restrict__ rec64, const double *__restrict__ cor
     const float rho = (float)(sqrt(rho2) * (1.0 + 1e-6));
     wf[kHdrRho] = rho;
     atomicMax(&sum->rho, __float_as_uint(rho));
+    // (regular pairs of such elements lie closer than the fixed range: FP64)
+    if (ldexpf(fix64::kRhoFactor * rho, 1 - fix64::kMinExp) < 1.0f) atomicAdd(&sum->small, 1u);
     int eo = 0, je = 0;
     (void)frexp(omax > 0 ? omax * (1.0 + 1e-9) : 0x1p-60, &eo);
     (void)frexp(jmax > 0 ? jmax * 1.01 : 0x1p-200, &je);
@@ -1019,6 +1021,7 @@ void build_fix64_records(Ctx &c) {
     BIE_CUDA(cudaMemcpy(&sum, d_sum, sizeof(sum), cudaMemcpyDeviceToHost));
     if (sum.bad) return;
     std::memcpy(&c.fx_rho_max, &sum.rho, 4);
+    c.fx_small = sum.small;
     // entries hold |sum| <= 4 sqrt(2) 2^55 sum of the reaches: below 2^62 (a factor's
     // modulus is up to sqrt(2) of its unit: G with factors is below half of F's bound)
     auto extra_of = [](unsigned long long bits) {
@@ -1061,8 +1064,12 @@ static bool fix64_covers(const Ctx &c, const AssembleArgs &a) {
 // Against the double-float kernel, 320 to 8000 elements: 4-point rules 1.09 to
 // 1.65 times as fast (complex k 1.03 to 1.5, 0.92 to 1.3 on 320 elements); 9- and
 // 16-point rules 0.85 to 1.15 (complex k 0.57 to 1.14); targets off the surface,
-// where C takes a pass of its own, 0.6 to 1.2 (complex k 0.35 to 1.2).
+// where C takes a pass of its own, 0.6 to 1.2 (complex k 0.35 to 1.2).  On graded
+// meshes the pairs among elements below 2^-9 of the mesh go to FP64: 2562 nodes with
+// element sizes over a factor of 1000 3.2 and 4.8 ms (36 and 69 % of the elements
+// small), the double-float kernel 1.9.
 bool fix64_takes(const Ctx &c, const AssembleArgs &a, bool df64) {
+    if (df64 && 8 * (int64_t)c.fx_small > c.n_elements) return false;
     if (df64 && !(on_nodes(c, a) && c.lay.Q[0] <= 4 && (a.k_im == 0.0 || c.n_elements >= 512))) return false;
     return fix64_covers(c, a);
 }

@@ -253,6 +253,7 @@ struct Ctx {
     int fx_phi_exp = 0;                  // basis values are stored times 2^-fx_phi_exp
     int fx_extra = 0;                    // entry units times 2^fx_extra (nodes with many elements)
     int fx_extra_w = 0;                  // ... of G with element factors
+    unsigned int fx_small = 0;           // elements whose regular pairs may be too close for them
     float *d_xrecords = nullptr;         // E x xlay.stride words, element order
     int32_t *d_xphi = nullptr;           // R x qmax x (4, 8, 12) limb words
     float *d_xnodes = nullptr;           // N x (x, y, z, entry weight exponent)

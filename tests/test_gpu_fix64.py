@@ -116,3 +116,13 @@ def test_few_rows_match_many(geo, phys, k):
         f, g, _ = biegpu.assemble_parallel(mesh, k, t[:, :M], n=2, m=2)
         for a, b in ((f, F[:M]), (g, G[:M])):
             assert np.max(np.abs(a - b) / np.max(np.abs(b), axis=1, keepdims=True)) <= 1e-14
+
+
+@pytest.mark.parametrize("power", [1, 4, 12])
+@pytest.mark.parametrize("precision", ["fp64", "df64"])
+def test_graded_meshes_in_both_precisions(power, precision):
+    # few, half and most of the elements small against the mesh
+    mesh = bm.icosphere(6)
+    s = 1e-3 + (1 - 1e-3) * ((1 + mesh.coordinates[2]) / 2) ** power
+    c = mesh.coordinates * s
+    check(dataclasses.replace(mesh, coordinates=c, sources=c.copy()), 2.0, 2, 2, precision=precision)
