@@ -1038,11 +1038,12 @@ void build_fix64_records(Ctx &c) {
 
 // Small phases stay in floating point: values here are good to 2^-55 of the modulus,
 // but with k r small the imaginary parts, k and k^3 times the real ones, are
-// results of their own.  Error of Im F and Im G on the unit sphere (2^S = 2), with
-// the FP64 kernel in brackets: k = 1 8e-16 (2e-16), 1e-16 (1e-16); k = 0.3 2e-14
-// (3e-16), 2e-16 (1e-16); k = 0.01 6e-10 (1e-14), 5e-15 (1e-16).
+// results of their own.  FP64 rounds k r cos(k r) - sin(k r) to 2^-53 k r, so at
+// k r = 1/4 both are alike; below that the fixed-point parts lose: on the unit
+// sphere (2^S = 2) Im F and Im G differ from plain FP64 by 2e-14 and 2e-16 at k = 0.3,
+// 6e-13 and 5e-16 at 0.1, 6e-10 and 5e-15 at 0.01.
 bool fix64_small_phase(const Ctx &c, double k_re) {
-    return k_re != 0.0 && std::fabs(k_re) * std::ldexp(1.0, c.fx_exp) < 1.0;
+    return k_re != 0.0 && std::fabs(k_re) * std::ldexp(1.0, c.fx_exp) < 0.25;
 }
 
 static bool fix64_covers(const Ctx &c, const AssembleArgs &a) {
