@@ -610,6 +610,7 @@ def adjoint_bench(args, max_over_ranks):
             "workload": f"ellipsoid 3:2:1 f=22 ({mesh.n_sources} nodes, {mesh.n_elements} elements), ka=3, "
                         "32 field points at radius 10",
             "ms_per_gradient": 1e3 * t_grad, "ms_per_forward": 1e3 * t_fwd, "parameters": n_params,
+            # (double-float forward assembly and reverse pass)
             "df64_forward": {"ms_per_gradient": 1e3 * t_grad_df,
                              "J_rel_diff": abs(Jd - J) / abs(J),
                              "dX_rel_diff": float(np.linalg.norm(dXd - dX) / np.linalg.norm(dX))},

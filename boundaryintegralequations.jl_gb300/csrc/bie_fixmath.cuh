@@ -9,8 +9,8 @@
 // (about 150 and 80 instructions) and the double is put together from bits.
 // Errors against extended precision: roots 0.51 ulp, exponential 0.7 ulp, sine
 // and cosine 2^-59 of 1 besides the final rounding (an error of the modulus of
-// e^{ikr}), the sine below 2^-8 0.51 ulp.  Arguments beyond the ranges below take the library's
-// functions.  Measured: corrections of the near pairs of the mixed assembly at 11562
+// e^{ikr}), the sine below 2^-8 0.51 ulp.  Arguments beyond the ranges below take
+// the library's functions.  Measured: corrections of the near pairs of the mixed assembly at 11562
 // nodes 232 -> 202 us and of the mixed product at 40962 nodes 1.56 -> 1.36 ms
 // (which had sine and cosine in double-float), FP64 matrix-free product at 5762
 // nodes 16.7 -> 11.7 ms.

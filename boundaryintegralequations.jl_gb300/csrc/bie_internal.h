@@ -255,7 +255,7 @@ struct Ctx {
     int fx_extra_w = 0;                  // ... of G with element factors
     unsigned int fx_small = 0;           // elements whose regular pairs may be too close for them
     float *d_xrecords = nullptr;         // E x xlay.stride words, element order
-    int32_t *d_xphi = nullptr;           // R x qmax x (4, 8, 12) limb words
+    int32_t *d_xphi = nullptr;           // R x groups of four points x NP x 8 limb words
     float *d_xnodes = nullptr;           // N x (x, y, z, entry weight exponent)
     int32_t *d_xtrig = nullptr;          // 1024 x (cos, sin) limbs, 256 x 2^(-j/256) limbs
     double *d_coords = nullptr;          // 3 x Nc geometry nodes (near-field kernels)
@@ -602,9 +602,10 @@ bool launch_assemble_df64(Ctx &c, const AssembleArgs &a);
 
 // Fixed-point assembly at FP64 accuracy (K10, bie_assemble_fix64.cu): records
 // from the FP64 ones; the launch returns false, enqueuing nothing, where the
-// arguments need another kernel (k-derivatives, element factors, phases or
-// damping beyond the fixed-point ranges, coordinates outside
-// 2^+-300).  df64: BIE_PREC_DF64, of which it takes the calls where it is the faster.
+// arguments need another kernel (k-derivatives, element factors but for 3-node
+// physics and real k, phases or damping beyond the fixed-point ranges, wavenumbers
+// with small phases, coordinates outside 2^+-300, no room for its scratch).  df64:
+// BIE_PREC_DF64, of which it takes the calls where it is the faster.
 void build_fix64_records(Ctx &c);
 bool launch_assemble_fix64(Ctx &c, const AssembleArgs &a, bool df64);
 bool fix64_takes(const Ctx &c, const AssembleArgs &a, bool df64);   // whether it launches

@@ -17,7 +17,7 @@
 // Every gmres is this library's device GMRES (run_gmres_devop) with the
 // reference's defaults; the solves nest two deep (a Gv solve inside the inner
 // operator inside the outer product), each level on its own workspace.
-// The sparse and derivative kernels are HBM/latency bound, one row per thread.
+// The sparse and derivative kernels are latency bound, eight lanes per row.
 #include "bie_internal.h"
 #include "bie_krylov.cuh"
 

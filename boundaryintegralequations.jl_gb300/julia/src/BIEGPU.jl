@@ -425,7 +425,7 @@ struct AdjointOpts
     rho_c::Float64
     dir::NTuple{3,Float64}
     reltol::Float64
-    precision::Int32   # 0: FP64 forward assembly, 6: double-float (BIE_PREC_DF64)
+    precision::Int32   # 0: FP64, 6: double-float forward assembly and reverse pass (BIE_PREC_DF64)
 end
 struct AdjointInfo
     forward_iterations::Int32; forward_converged::Int32
@@ -451,7 +451,7 @@ function farfield_objective(coordinates, Z, mesh, k, field; rho_c=1.21 * 343.0, 
     dX = gradient ? zeros(Float64, size(coordinates)) : Matrix{Float64}(undef, 0, 0)
     dZ = gradient ? zeros(ComplexF64, length(Zv)) : Vector{ComplexF64}(undef, 0)
     d = collect(Float64, dir); d ./= norm(d)
-    # precision: forward-model assembly, :fp64 or :df64 (double-float)
+    # precision: forward assembly and regular pairs of the reverse pass, :fp64 or :df64
     opts = Ref(AdjointOpts(rho_c, (d[1], d[2], d[3]), reltol, precision_code(precision)))
     info = Ref{AdjointInfo}()
     GC.@preserve Zv X pf dX dZ begin

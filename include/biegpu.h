@@ -73,7 +73,10 @@ extern "C" {
  * (this GPU's FP64 pipe runs at 1/64 of its FP32 rate) and the near pairs in
  * FP64; dense complex128 products sum in fixed point as well, at the error of an
  * FP64 sum.  C at points off the surface, k-derivatives and wavenumbers beyond the
- * fixed-point ranges use FP64 throughout, as do all other operations. */
+ * fixed-point ranges or of small phase (0 < |k| times the mesh's size below about
+ * 1/4, where the imaginary parts are results of their own) use FP64 throughout, as
+ * do all other operations; sine, cosine, exponential and roots of FP64 pairs are
+ * evaluated on the integer pipes at FP64 accuracy. */
 #define BIE_PREC_FP64  0
 #define BIE_PREC_MIXED 1  /* FP32 regular pairs, FP64 near-singular pairs and C  */
 /* Multi-right-hand-side products only (bie_matvec_multi_device): matrix tiles
@@ -88,8 +91,8 @@ extern "C" {
 /* Assembly, matrix-free products and GMRES operator arithmetic (bie_assemble*,
  * bie_matvec*, bie_gmres*; with `refine`, the residuals of refinement):
  * FP64-grade results, near pairs in FP64.  The node rows of assemblies with rules
- * of at most four points take the fixed-point kernel of BIE_PREC_FP64; other
- * assemblies and products evaluate the regular pairs in double-float arithmetic
+ * of at most four points take the fixed-point kernel of BIE_PREC_FP64 (not on
+ * meshes with many elements below 1/500 of the mesh); other assemblies and products evaluate the regular pairs in double-float arithmetic
  * (pairs of floats, ~48-bit significand) on the FP32 pipes with every sum
  * compensated, ~1e-14 from BIE_PREC_FP64.  Falls
  * back to the FP64 kernels where the phase rotation k (r - r0) over one
