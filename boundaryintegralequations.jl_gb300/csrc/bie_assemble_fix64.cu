@@ -1057,7 +1057,8 @@ static bool fix64_covers(const Ctx &c, const AssembleArgs &a) {
     const double bound = a.k_dev ? a.k_abs_max : 0.0, len = std::ldexp(1.0, c.fx_exp);
     const double kr = std::max(std::fabs(a.k_re), bound) * len, ki = cplx ? std::max(std::fabs(a.k_im), bound) * len : 0.0;
     if (!(kr < 500.0 && ki < 100.0 && ki * c.fx_rho_max * 1.45 < fix64::kMaxDampSpread)) return false;
-    return !fix64_small_phase(c, a.k_dev ? a.k_re_min : a.k_re);
+    // (C does not depend on k)
+    return !(a.flags & (BIE_F | BIE_G)) || !fix64_small_phase(c, a.k_dev ? a.k_re_min : a.k_re);
 }
 
 // Where the double-float kernel is available (BIE_PREC_DF64), the fixed-point one

@@ -266,7 +266,8 @@ struct Ctx {
     void *d_scratch[kScratchCount] = {};
     size_t scratch_bytes[kScratchCount] = {};
     void *scratch(int slot, size_t bytes);
-    bool scratch_fits(int slot, size_t bytes);   // the same, false where the device has no room
+    bool scratch_fits(int slot, size_t bytes);   // the same, false where there is no room for it
+                                                 // (on the device; or a recording would grow it)
     void drop_scratch(int slot);                 // gives a slot's memory back
     // set while the context stream records a CUDA graph: scratch must not grow
     // then (a reallocation would leave the graph pointing at freed memory)

@@ -353,6 +353,8 @@ void Ctx::drop_scratch(int slot) {
 }
 
 bool Ctx::scratch_fits(int slot, size_t bytes) {
+    // (a recording keeps the route of the run that sized its scratch)
+    if (capturing && scratch_bytes[slot] < bytes) return false;
     try {
         scratch(slot, bytes);
     } catch (const Error &e) {
